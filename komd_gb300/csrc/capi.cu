@@ -156,7 +156,7 @@ int check_launch(const char *what) {
 
 int ensure_partials(komd_gpu *h) {
     Engine &e = h->e;
-    int need = e.g.ncell;                      // pair kernels write at most one partial row per cell
+    int need = std::max(e.g.ncell, pair_cell_grid(e));   // one partial row per block of the pair kernels
     need = std::max(need, atm_grid(e));
     need = std::max(need, kinetic_grid(e));
     if (need > h->partial_cap) {
@@ -719,6 +719,7 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
         CK(cudaMemcpy(e.exact_com, exact.data(), e.n_mol, cudaMemcpyHostToDevice));
         e.fused_drift = e.verlet && e.n_mol == n;
         for (int64_t k = 0; k < e.n_mol && e.fused_drift; k++) e.fused_drift = exact[k] != 0;
+        e.multi_key = (int64_t)dense.size() < n;
         e.uniform = true;
         for (int64_t s = 1; s < n && e.uniform; s++) e.uniform = eps[s] == eps[0] && sig[s] == sig[0];
         e.eps0 = (float)eps[0];

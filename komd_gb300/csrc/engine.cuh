@@ -80,6 +80,30 @@ __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
 
+// a > b for a >= 0 and b >= 0 (false when a is NaN), on the bits: GB300
+// compares doubles on its narrow FP64 pipe
+__device__ __forceinline__ bool dabove(double a, double b) {
+    const long long ka = __double_as_longlong(a);
+    return ka > __double_as_longlong(b) && ka <= 0x7ff0000000000000LL;
+}
+
+// the warp sums of (x, y, z): a butterfly over offsets 16, 8, 4, 2, 1 whose
+// lanes split the components on the way (lanes 0-7 end with x, 8-15 with y,
+// 16-31 with z): 6 additions a lane instead of 15, the same pairing of partial
+// sums as a butterfly per component
+template <typename Real>
+__device__ __forceinline__ Real warp_sum3(Real x, Real y, Real z, int lane) {
+    const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+    const Real r1 = __shfl_xor_sync(0xffffffffu, up16 ? x : z, 16);
+    const Real r2 = __shfl_xor_sync(0xffffffffu, y, 16);
+    Real c0 = (up16 ? z : x) + r1;
+    const Real c1 = y + r2;
+    const Real r3 = __shfl_xor_sync(0xffffffffu, (up16 || up8) ? c0 : c1, 8);
+    c0 = ((up16 || !up8) ? c0 : c1) + r3;
+    for (int o = 4; o > 0; o >>= 1) c0 += __shfl_xor_sync(0xffffffffu, c0, o);
+    return c0;
+}
+
 // Reference point of a cell for the FP32 cell-local coordinates.  Any fixed
 // choice works as long as the sort and the force kernels agree; the centre
 // keeps |local| <= half a cell so FP32 keeps ~1e-7 absolute precision.
@@ -127,6 +151,21 @@ __host__ __device__ inline int atm_code(int nb, bool crosses, int slot) {
     return nb | (crosses ? 32 : 0) | (slot << 6);
 }
 constexpr int kMaxAtmSlot = (1 << 25) - 1;
+struct alignas(16) AtmEntryD { double x, y, z; long long code; };   // the list entry of the FP64 kernels
+
+// The squared range of an FP32 pre-test in home-cell coordinates that must not
+// drop a pair inside scan2: coordinates of up to two cell edges carry about
+// 5e-7 edges of rounding per component, so r^2 up to 3.5 r times that; the
+// margin is that bound, rounded up, on top of 1e-4 of the range.
+inline float pair_pre2(const Grid &g, double scan2) {
+    double edge = 0.0;
+    for (int d = 0; d < 3; d++) {
+        const double last = g.L[d] - (g.nd[d] - 1) * g.cs;   // the stretched last cell
+        edge = edge > last ? edge : last;
+        edge = edge > g.cs ? edge : g.cs;
+    }
+    return (float)(scan2 * (1.0 + 1e-4) + 4e-6 * edge * sqrt(scan2));
+}
 
 // The order in which the Verlet rows put a site's neighbours "above" it (the
 // front region that the half-list pass reads): j is above i when j's z at the
@@ -167,6 +206,10 @@ struct PairParams {
     int lj_bins;
     double max_sigma;
     double rc2, rc3sq, scan2;  // LJ cutoff^2, ATM cutoff^2, max of both
+    float pre2;                // scan2 with the margin of the FP32 pre-test
+    int uniform;               // one eps and one sigma for every site
+    int multi_key;             // some sites share a molecule key
+    int lj_scaled;             // lj_fscale is not 1
     double stiffness;
     int use_lj;
     int virial_compat;
@@ -189,6 +232,14 @@ struct PairParams {
     float sw_rc2, sw_iw;       // cutoff^2 and 1 / (cutoff^2 - (cutoff - width)^2)
     float4 *fown;              // per slot, optional: the half-list pass writes each site's own FP32 force here
                                // (the flush widens it) instead of FP64 into f
+};
+
+// the tabulated force F(r): ascending nodes xs, values ys, segment slopes,
+// lo below and hi above the nodes
+struct PairTable {
+    int n;
+    const double *xs, *ys, *slope;
+    double lo, hi;
 };
 
 struct AtmParams {
@@ -403,6 +454,7 @@ struct Engine {
     unsigned char *exact_com = nullptr;
     // all sites share eps and sigma: the list kernel uses constants
     bool uniform = false;
+    bool multi_key = false;         // some sites share a molecule key (a molecule of several sites)
     float eps0 = 1.f, sig0 = 1.f;
     double lj_fscale = 1.0;         // ATM2B factor (KOMD_TERM_ATM2B), else 1
     bool fused_drift = false;       // Verlet path, single-site molecules with exact COM: k_step0_fused

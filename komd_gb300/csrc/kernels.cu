@@ -235,242 +235,13 @@ __global__ void __launch_bounds__(kBlock) k_cell_sort(SortArgs a) {
     cell_sort_body(a, blockIdx.x, gridDim.x);
 }
 
-// ===========================================================================
-// pair kernel: LJ 12-6 (LJ12_6.cpp:15-43), FENE (FENE.cpp:15-43), the ATM
-// neighbour list inside cutoff_3b, energy / virial / histograms / counts.
-//
-// One warp per home cell, full shell (27 neighbour cells, periodic images by
-// cell wrap), no atomics on forces: lane = (home site il, group grp); the G
-// groups split each neighbour cell's sites and their partial forces are
-// reduced through shared memory.  Real = float: cell-local FP32 coordinates;
-// Real = double: absolute FP64 positions with the reference's exact
-// dr = r_i - (r_j + shift) arithmetic.
-// ===========================================================================
+// the ATM neighbour list's entry: r_i - r_j and the packed code
 template <typename Real>
 struct AtmEntry;
 template <>
 struct AtmEntry<float> { using T = float4; };
-struct alignas(16) AtmEntryD { double x, y, z; long long code; };
 template <>
 struct AtmEntry<double> { using T = AtmEntryD; };
-
-__device__ __forceinline__ float4 make_entry(float x, float y, float z, int code) {
-    return make_float4(x, y, z, __int_as_float(code));
-}
-__device__ __forceinline__ AtmEntryD make_entry(double x, double y, double z, int code) {
-    AtmEntryD e; e.x = x; e.y = y; e.z = z; e.code = code; return e;
-}
-
-template <typename Real, bool MEASURE, bool EMIT, bool FENE, bool COUNT>
-__global__ void __launch_bounds__(kBlock) k_pair(PairParams p) {
-    using Entry = typename AtmEntry<Real>::T;
-    constexpr bool FP64 = sizeof(Real) == 8;
-    __shared__ int s_cnt[kWarpsPerBlock][32];
-    __shared__ Real s_red[kWarpsPerBlock][32][3];
-    __shared__ double s_part[kWarpsPerBlock][R_NSLOTS];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cell = blockIdx.x * kWarpsPerBlock + wib;
-    double a_u = 0.0, a_w[6] = {0, 0, 0, 0, 0, 0}, a_pairs = 0.0;
-    const Real rc2 = (Real)p.rc2, rc3sq = (Real)p.rc3sq, scan2 = (Real)p.scan2;
-    Entry *nl = reinterpret_cast<Entry *>(p.nl);
-
-    if (cell < p.g.ncell) {
-        int cx, cy, cz;
-        cell_coords(p.g, cell, cx, cy, cz);
-        const double cen[3] = {cell_centre(p.g, 0, cx), cell_centre(p.g, 1, cy), cell_centre(p.g, 2, cz)};
-        const int hs = p.cell_start[cell], hn = p.cell_start[cell + 1] - hs;
-        for (int base = 0; base < hn; base += 32) {
-            const int hc = min(32, hn - base);
-            const int G = 32 / hc;
-            const int il = lane % hc, grp = lane / hc;
-            const bool act = grp < G;
-            const int is = hs + base + il;
-            Real pix, piy, piz, sgi, epi;
-            if (FP64) {
-                pix = (Real)p.posd[3 * is]; piy = (Real)p.posd[3 * is + 1]; piz = (Real)p.posd[3 * is + 2];
-                sgi = (Real)p.sig_d[is]; epi = (Real)p.seps_d[is];
-            } else {
-                const float4 q = p.pos4[is];
-                pix = q.x; piy = q.y; piz = q.z; sgi = q.w; epi = p.seps[is];
-            }
-            const int ki = p.skey[is];
-            const int site_i = p.slot_site[is];
-            Real fx = 0, fy = 0, fz = 0;
-            int cnt = 0;
-            if (EMIT && lane < hc) s_cnt[wib][lane] = 0;
-            __syncwarp();
-            for (int nb = 0; nb < 27; nb++) {
-                const NbCell q = neighbour_cell(p.g, cx, cy, cz, nb);
-                const int js = p.cell_start[q.cell], jn = p.cell_start[q.cell + 1] - js;
-                int qx, qy, qz;
-                cell_coords(p.g, q.cell, qx, qy, qz);
-                Real ox, oy, oz;
-                if (FP64) {
-                    ox = (Real)q.shift[0]; oy = (Real)q.shift[1]; oz = (Real)q.shift[2];
-                } else {
-                    ox = (Real)((cell_centre(p.g, 0, qx) + q.shift[0]) - cen[0]);
-                    oy = (Real)((cell_centre(p.g, 1, qy) + q.shift[1]) - cen[1]);
-                    oz = (Real)((cell_centre(p.g, 2, qz) + q.shift[2]) - cen[2]);
-                }
-                const bool vir_full = p.virial_compat && q.crosses;  // COMPAT: images counted per list entry
-                if (!act) continue;
-                for (int jj = grp; jj < jn; jj += G) {
-                    const int j = js + jj;
-                    if (j == is) continue;
-                    Real dx, dy, dz, r2;
-                    if (FP64) {
-                        const double *pj = p.posd + 3 * j;
-                        dx = (Real)dsub((double)pix, dadd(pj[0], (double)ox));
-                        dy = (Real)dsub((double)piy, dadd(pj[1], (double)oy));
-                        dz = (Real)dsub((double)piz, dadd(pj[2], (double)oz));
-                        r2 = (Real)dadd(dadd(dmul((double)dx, (double)dx), dmul((double)dy, (double)dy)),
-                                        dmul((double)dz, (double)dz));
-                    } else {
-                        const float4 pj = p.pos4[j];
-                        dx = pix - (pj.x + ox);
-                        dy = piy - (pj.y + oy);
-                        dz = piz - (pj.z + oz);
-                        r2 = dx * dx + dy * dy + dz * dz;
-                    }
-                    int kj = 0;
-                    if (FENE) {
-                        kj = p.skey[j];
-                        if (kj == ki && !q.crosses) {
-                            // FENE on same-molecule pairs, no cutoff: force on i
-                            // along (r_j - r_i), overstretch -> 1e30 / (r_j - r_i)
-                            const Real sgj = FP64 ? (Real)p.sig_d[j] : (Real)(2.0f * p.pos4[j].w);
-                            const Real sgm = FP64 ? (sgi + sgj) / (Real)2.0 : (sgi + (Real)0.5 * sgj);
-                            const Real R0 = (Real)1.5 * sgm;
-                            const Real R02 = R0 * R0;
-                            if (R02 <= r2) {
-                                // invdr * 1e+30 with invdr = 1 / (r_j - r_i), as FENE.cpp:28-33
-                                fx += ((Real)1 / (-dx)) * (Real)1e30;
-                                fy += ((Real)1 / (-dy)) * (Real)1e30;
-                                fz += ((Real)1 / (-dz)) * (Real)1e30;
-                            } else {
-                                Real e;
-                                if (FP64) e = (Real)sqrt((double)epi * (double)p.seps_d[j]);
-                                else e = epi * p.seps[j];
-                                const Real k = (Real)p.stiffness * e / (sgm * sgm);
-                                const Real fac = k / ((Real)1 - (r2 / R02));
-                                fx -= dx * fac; fy -= dy * fac; fz -= dz * fac;
-                            }
-                        }
-                    }
-                    if (r2 > scan2) continue;
-                    if (!FENE) kj = p.skey[j];
-                    if (EMIT && r2 <= rc3sq) {
-                        const int c = atomicAdd(&s_cnt[wib][il], 1);
-                        if (c < p.nl_cap) nl[(size_t)is * p.nl_cap + c] = make_entry(dx, dy, dz, atm_code(nb, q.crosses, j));
-                    }
-                    if (!p.use_lj || r2 > rc2 || kj == ki) continue;
-                    if (COUNT) { cnt++; continue; }
-                    Real fac, u, ljd;
-                    if (FP64) {
-                        // LJ12_6_Force arithmetic in FP64 (pow(x, 3.0), pow(lj6, 2.0) as products)
-                        const double inv = ddiv(1.0, (double)r2);
-                        const double sgm = (p.sig_d[is] + p.sig_d[j]) / 2.0;
-                        const double e = sqrt(p.seps_d[is] * p.seps_d[j]);
-                        const double x = sgm * sgm * inv;
-                        const double lj6 = x * x * x, lj12 = lj6 * lj6;
-                        fac = (Real)(24.0 * e * (2.0 * lj12 - lj6) * inv);
-                        u = (Real)(4.0 * e * (lj12 - lj6));
-                        ljd = (Real)(24.0 * e * (2.0 * lj12 - lj6));
-                    } else {
-                        const float inv = __frcp_rn((float)r2);
-                        const float sgm = (float)sgi + p.pos4[j].w;
-                        const float x = sgm * sgm * inv;
-                        const float lj6 = x * x * x, lj12 = lj6 * lj6;
-                        const float e = (float)epi * p.seps[j];
-                        ljd = 24.0f * e * (2.0f * lj12 - lj6);
-                        fac = ljd * inv;
-                        u = 4.0f * e * (lj12 - lj6);
-                    }
-                    if (!MEASURE) fac *= (Real)p.lj_fscale;   // ATM2B (1 otherwise); sensors stay unscaled
-                    fx += dx * fac; fy += dy * fac; fz += dz * fac;
-                    if (MEASURE) {
-                        const double wt = vir_full ? 1.0 : 0.5;
-                        const double gx = (double)dx * (double)fac, gy = (double)dy * (double)fac,
-                                     gz = (double)dz * (double)fac;
-                        a_u += 0.5 * (double)u;
-                        a_pairs += 0.5;
-                        a_w[0] += wt * ((double)dx * gx);
-                        a_w[1] += wt * 0.5 * ((double)dx * gy + (double)dy * gx);
-                        a_w[2] += wt * ((double)dy * gy);
-                        a_w[3] += wt * 0.5 * ((double)dx * gz + (double)dz * gx);
-                        a_w[4] += wt * 0.5 * ((double)dy * gz + (double)dz * gy);
-                        a_w[5] += wt * ((double)dz * gz);
-                        if (p.lj_hist) {
-                            const int site_j = p.slot_site[j];
-                            if (site_i < site_j) {
-                                const double rp = sqrt((double)r2);
-                                const double bw = 3.0 * p.max_sigma / (double)p.lj_bins;
-                                unsigned long long bin = (unsigned long long)(rp / bw);
-                                if (bin > (unsigned long long)(p.lj_bins - 1)) bin = p.lj_bins - 1;
-                                atomicAdd(&p.lj_hist[bin], (double)u);
-                                atomicAdd(&p.lj_hist[p.lj_bins + bin], (double)ljd / rp);
-                                atomicAdd(&p.lj_hist[2 * p.lj_bins + bin], 1.0);
-                                atomicAdd(&p.lj_hist[3 * p.lj_bins + bin], 1.0);
-                            }
-                        }
-                    }
-                }
-            }
-            // reduce the G partial sums of every home site
-            if (COUNT) {
-                s_cnt[wib][lane] = cnt;
-                __syncwarp();
-                if (act && grp == 0) {
-                    long long c = 0;
-                    for (int k = 0; k < G; k++) c += s_cnt[wib][il + k * hc];
-                    p.counts[site_i] = c;
-                }
-                __syncwarp();
-                continue;
-            }
-            s_red[wib][lane][0] = fx; s_red[wib][lane][1] = fy; s_red[wib][lane][2] = fz;
-            __syncwarp();
-            if (act && grp == 0) {
-                Real sx = 0, sy = 0, sz = 0;
-                for (int k = 0; k < G; k++) {
-                    sx += s_red[wib][il + k * hc][0];
-                    sy += s_red[wib][il + k * hc][1];
-                    sz += s_red[wib][il + k * hc][2];
-                }
-                p.f[3 * site_i] = (double)sx;
-                p.f[3 * site_i + 1] = (double)sy;
-                p.f[3 * site_i + 2] = (double)sz;
-            }
-            if (EMIT && lane < hc) {
-                const int c = s_cnt[wib][lane];
-                p.nl_count[hs + base + lane] = min(c, p.nl_cap);
-                if (c > p.nl_cap) atomicOr(&p.err[E_ATM_OVERFLOW], 1);
-            }
-            __syncwarp();
-        }
-    }
-    if (MEASURE) {
-        double vals[9] = {a_u, a_w[0], a_w[1], a_w[2], a_w[3], a_w[4], a_w[5], a_pairs, 0.0};
-        for (int k = 0; k < 8; k++) {
-            double x = vals[k];
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            vals[k] = x;
-        }
-        if (lane == 0) {
-            s_part[wib][R_ULJ] = vals[0];
-            for (int k = 0; k < 6; k++) s_part[wib][R_W0 + k] = vals[1 + k];
-            s_part[wib][R_PAIRS] = vals[7];
-        }
-        __syncthreads();
-        if (threadIdx.x < R_NSLOTS) {
-            const int t = threadIdx.x;
-            double s = 0.0;
-            if (t == R_ULJ || t == R_PAIRS || (t >= R_W0 && t <= R_W5))
-                for (int w = 0; w < kWarpsPerBlock; w++) s += s_part[w][t];
-            p.partials[(size_t)blockIdx.x * R_NSLOTS + t] = s;
-        }
-    }
-}
 
 // ===========================================================================
 // ATM triplet kernel (ATM.cpp:22-62 / ATM_NOLIST.cpp:124-159): one warp per
@@ -1349,165 +1120,6 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_partials(int nblocks, const
     }
 }
 
-// Tabulated pair force (IBI_ForceFunctor<IBI_Default>::IBI_Force,
-// plugins/IBI/IBI_ForceFunctor.cpp:18-37, FunctionPL::evaluateAt,
-// plugins/IBI/IBI_Math.h:30-44): for every pair inside the cutoff (no
-// same-molecule exclusion) F = table(r), force = (dr / r) * F on the site.
-// FP64: the exact separation and cutoff test, r = sqrt(r^2) and the table
-// value as the reference forms them (the upper node is the first node >= r,
-// by binary search, the node the reference's linear scan finds, and slope[k] =
-// (y[k+1] - y[k]) / (x[k+1] - x[k]) is the reference's quotient, computed once
-// with the same IEEE operations); dr / r as dr * (1 / r), one division per
-// pair instead of three (within an ulp of the reference's quotients; the FP64
-// pipe bounds this kernel).  At r == x[0] the reference reads x[-1]; here the
-// first segment is used.
-__device__ __forceinline__ double table_eval(double x, int n, const double *__restrict__ xs,
-                                             const double *__restrict__ ys, const double *__restrict__ slope,
-                                             double lo, double hi) {
-    if (x > xs[n - 1]) return hi;
-    if (x < xs[0]) return lo;
-    int a = 0, b = n - 1;           // lower_bound: first index with xs[i] >= x
-    while (a < b) {
-        const int m = (a + b) >> 1;
-        if (x > xs[m]) a = m + 1;
-        else b = m;
-    }
-    const int lb = (a < 1 ? 1 : a) - 1;
-    return dadd(ys[lb], dmul(slope[lb], dsub(x, xs[lb])));
-}
-
-// One warp per home cell.  The 27-cell neighbourhood is staged in shared
-// memory in FP32 home-cell coordinates (cell-local position plus the
-// neighbour cell's centre offset); for each home site the lanes test 32
-// staged sites at a time against the cutoff with a 1e-4 relative margin (the
-// FP32 separation is good to ~1e-7, so the test only drops pairs that are
-// clearly outside), queue the hits by ballot, and evaluate the queue 32 pairs
-// at a time in FP64 from the FP64 positions and the neighbour cell's periodic
-// shift, with the exact cutoff test.  Per home site the lanes' sums are
-// reduced in a fixed tree and added to f.
-constexpr int kTabWarps = 4;
-constexpr int kTabStage = 416;   // staged sites per round (more rounds for a larger neighbourhood)
-
-__global__ void __launch_bounds__(32 * kTabWarps) k_pair_table(
-    Grid g, const int *__restrict__ cell_start, const int *__restrict__ slot_site, const double *__restrict__ posd,
-    const float4 *__restrict__ pos4, const float *__restrict__ offtab, double rc2, int n,
-    const double *__restrict__ xs, const double *__restrict__ ys, const double *__restrict__ slope, double lo,
-    double hi, double *__restrict__ f) {
-    __shared__ float4 s_p[kTabWarps][kTabStage];
-    __shared__ int2 s_j[kTabWarps][kTabStage];   // slot, neighbour-cell index
-    __shared__ double s_sh[kTabWarps][27][3];
-    __shared__ float s_o[kTabWarps][27][3];
-    __shared__ int s_st[kTabWarps][27], s_pre[kTabWarps][28];
-    __shared__ int s_q[kTabWarps][64];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cell = blockIdx.x * kTabWarps + w;
-    if (cell >= g.ncell) return;   // warp-uniform; the kernel uses no block barrier
-    unsigned lt;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-    int cx, cy, cz;
-    cell_coords(g, cell, cx, cy, cz);
-    int cnt = 0;
-    if (lane < 27) {
-        const NbCell q = neighbour_cell(g, cx, cy, cz, lane);
-        const int s0 = cell_start[q.cell];
-        cnt = cell_start[q.cell + 1] - s0;
-        s_st[w][lane] = s0;
-        for (int d = 0; d < 3; d++) s_sh[w][lane][d] = q.shift[d];
-        s_o[w][lane][0] = offtab[cx * 3 + lane % 3];
-        s_o[w][lane][1] = offtab[g.nd[0] * 3 + cy * 3 + (lane / 3) % 3];
-        s_o[w][lane][2] = offtab[(g.nd[0] + g.nd[1]) * 3 + cz * 3 + lane / 9];
-    }
-    int inc = cnt;   // inclusive prefix of the 27 counts
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane < 27) s_pre[w][lane] = inc - cnt;
-    const int total = __shfl_sync(0xffffffffu, inc, 26);
-    if (lane == 0) s_pre[w][27] = total;
-    __syncwarp();
-    const int hs = s_st[w][13], hn = s_pre[w][14] - s_pre[w][13];   // neighbour 13 is the home cell
-    const float pre2 = (float)(rc2 * (1.0 + 1e-4));
-    for (int sb = 0; sb < total; sb += kTabStage) {
-        const int ns = min(kTabStage, total - sb);
-        __syncwarp();
-        for (int t = lane; t < ns; t += 32) {
-            const int gi = sb + t;
-            int a = 0, b = 27;   // the neighbour cell holding staged site gi
-            while (b - a > 1) {
-                const int mid = (a + b) >> 1;
-                if (s_pre[w][mid] <= gi) a = mid;
-                else b = mid;
-            }
-            const int j = s_st[w][a] + (gi - s_pre[w][a]);
-            float4 q = pos4[j];
-            q.x += s_o[w][a][0];
-            q.y += s_o[w][a][1];
-            q.z += s_o[w][a][2];
-            s_p[w][t] = q;
-            s_j[w][t] = make_int2(j, a);
-        }
-        __syncwarp();
-        for (int h = 0; h < hn; h++) {
-            const int is = hs + h;
-            const float4 hp = pos4[is];
-            const double xi = posd[3 * is], yi = posd[3 * is + 1], zi = posd[3 * is + 2];
-            double fx = 0.0, fy = 0.0, fz = 0.0;
-            auto eval = [&](int c) {
-                if (c < 0) return;
-                const int2 jn = s_j[w][c];
-                const double *pj = posd + 3 * (size_t)jn.x;
-                const double dx = dsub(xi, dadd(pj[0], s_sh[w][jn.y][0]));
-                const double dy = dsub(yi, dadd(pj[1], s_sh[w][jn.y][1]));
-                const double dz = dsub(zi, dadd(pj[2], s_sh[w][jn.y][2]));
-                const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-                if (r2 > rc2) return;
-                const double r = __dsqrt_rn(r2);
-                const double F = table_eval(r, n, xs, ys, slope, lo, hi);
-                const double ir = ddiv(1.0, r);
-                fx = dadd(fx, dmul(dmul(dx, ir), F));
-                fy = dadd(fy, dmul(dmul(dy, ir), F));
-                fz = dadd(fz, dmul(dmul(dz, ir), F));
-            };
-            int qn = 0;
-            for (int c0 = 0; c0 < ns; c0 += 32) {
-                const int c = c0 + lane;
-                bool hit = false;
-                if (c < ns && s_j[w][c].x != is) {
-                    const float4 pj = s_p[w][c];
-                    const float dx = hp.x - pj.x, dy = hp.y - pj.y, dz = hp.z - pj.z;
-                    hit = dx * dx + dy * dy + dz * dz <= pre2;
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, hit);
-                if (hit) s_q[w][qn + __popc(m & lt)] = c;
-                qn += __popc(m);
-                if (qn >= 32) {   // a full batch: one queued pair per lane
-                    __syncwarp();
-                    eval(s_q[w][lane]);
-                    __syncwarp();
-                    qn -= 32;
-                    if (lane < qn) s_q[w][lane] = s_q[w][32 + lane];
-                    __syncwarp();
-                }
-            }
-            __syncwarp();
-            eval(lane < qn ? s_q[w][lane] : -1);
-            for (int o = 16; o > 0; o >>= 1) {
-                fx = dadd(fx, __shfl_xor_sync(0xffffffffu, fx, o));
-                fy = dadd(fy, __shfl_xor_sync(0xffffffffu, fy, o));
-                fz = dadd(fz, __shfl_xor_sync(0xffffffffu, fz, o));
-            }
-            if (lane == 0) {
-                const int site = slot_site[is];
-                f[3 * site] = dadd(f[3 * site], fx);
-                f[3 * site + 1] = dadd(f[3 * site + 1], fy);
-                f[3 * site + 2] = dadd(f[3 * site + 2], fz);
-            }
-            __syncwarp();
-        }
-    }
-}
-
 // VelocityScaling (VelocityScaling.cpp:12-25): v *= beta; beta from the
 // caller, or (acc != nullptr) sqrt(T_target / T) with T from the summed
 // kinetic slots as TemperatureSensor computes it.  A non-finite T (an
@@ -1614,9 +1226,14 @@ PairParams pair_params(Engine &e) {
     p.scan2 = 0.0;
     if (lj) p.scan2 = p.rc2;
     if (atm && p.rc3sq > p.scan2) p.scan2 = p.rc3sq;
+    p.pre2 = pair_pre2(e.g, p.scan2);
     p.stiffness = e.cfg.stiffness;
     p.use_lj = lj ? 1 : 0;
     p.lj_fscale = e.lj_fscale;
+    p.lj_scaled = e.lj_fscale != 1.0;
+    // constants for one species: sqrt(eps eps) is eps while the square stays normal
+    p.uniform = e.uniform && e.eps0 > 1e-30f && e.eps0 < 1e30f;
+    p.multi_key = e.multi_key;
     p.lj_fscalef = (float)e.lj_fscale;
     p.virial_compat = e.cfg.virial_mode == KOMD_VIRIAL_COMPAT;
     p.offtab = e.offtab;
@@ -1638,52 +1255,23 @@ PairParams pair_params(Engine &e) {
     return p;
 }
 
-template <typename Real, bool M, bool E, bool F>
-static void pair_dispatch_c(PairParams &p, int grid, cudaStream_t st) {
-    k_pair<Real, M, E, F, false><<<grid, kBlock, 0, st>>>(p);
-}
-
-template <typename Real>
-static void pair_dispatch(PairParams &p, bool measure, bool emit, bool fene, int grid, cudaStream_t st) {
-    const int code = (measure ? 4 : 0) | (emit ? 2 : 0) | (fene ? 1 : 0);
-    switch (code) {
-        case 0: pair_dispatch_c<Real, false, false, false>(p, grid, st); break;
-        case 1: pair_dispatch_c<Real, false, false, true>(p, grid, st); break;
-        case 2: pair_dispatch_c<Real, false, true, false>(p, grid, st); break;
-        case 3: pair_dispatch_c<Real, false, true, true>(p, grid, st); break;
-        case 4: pair_dispatch_c<Real, true, false, false>(p, grid, st); break;
-        case 5: pair_dispatch_c<Real, true, false, true>(p, grid, st); break;
-        case 6: pair_dispatch_c<Real, true, true, false>(p, grid, st); break;
-        default: pair_dispatch_c<Real, true, true, true>(p, grid, st); break;
-    }
-}
-
 int atm_grid(const Engine &e) { return nblk(e.n, kWarpsPerBlock); }
 
 // The FP32 force path runs the tiled kernel (pair_tile.cu, one CTA per cell);
-// FP64 mode, FENE and the LJ sensor histograms use the warp-per-cell kernel
-// above.  Returns the number of blocks whose partial sums were written.
+// FP64 mode, FENE and the LJ sensor histograms use pair_cell.cu.  FENE acts
+// between sites of one molecule ID only: without such a pair the term is
+// empty.  Returns the number of blocks whose partial sums were written.
 int launch_pair(Engine &e, cudaStream_t st, bool measure, double *lj_hist) {
     PairParams p = pair_params(e);
     p.lj_hist = lj_hist;
     const bool emit = (e.cfg.terms & KOMD_TERM_ATM) != 0;
-    const bool fene = (e.cfg.terms & KOMD_TERM_FENE) != 0;
+    const bool fene = (e.cfg.terms & KOMD_TERM_FENE) != 0 && e.multi_key;
     if (e.verlet && !lj_hist) return launch_lj_vlist(e, p, measure, emit, st);
     if (e.cfg.precision == KOMD_FP32 && !fene && !lj_hist) {
         launch_pair_tile(p, e.g.ncell, measure, emit, st);
         return e.g.ncell;
     }
-    const int grid = nblk(e.g.ncell, kWarpsPerBlock);
-    if (e.cfg.precision == KOMD_FP64) pair_dispatch<double>(p, measure, emit, fene, grid, st);
-    else pair_dispatch<float>(p, measure, emit, fene, grid, st);
-    return grid;
-}
-
-void launch_counts(Engine &e, cudaStream_t st) {
-    PairParams p = pair_params(e);
-    p.use_lj = 1;
-    p.scan2 = p.rc2;
-    k_pair<double, false, false, false, true><<<nblk(e.g.ncell, kWarpsPerBlock), kBlock, 0, st>>>(p);
+    return launch_pair_cell(e, p, measure, emit, fene, st);
 }
 
 void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc) {
@@ -1912,13 +1500,6 @@ void launch_step1(Engine &e, cudaStream_t st) {
 }
 
 int kinetic_grid(const Engine &e) { return std::min(nblk(e.n, kBlock), e.num_sms * 2); }
-
-void launch_pair_table(Engine &e, cudaStream_t st) {
-    if (!e.tab_x || !e.tab_s || e.tab_n < 2) return;
-    k_pair_table<<<nblk(e.g.ncell, kTabWarps), 32 * kTabWarps, 0, st>>>(
-        e.g, e.cell_start, e.slot_site, e.posd, e.pos4, e.offtab, e.cfg.cutoff * e.cfg.cutoff, e.tab_n, e.tab_x,
-        e.tab_y, e.tab_s, e.tab_lo, e.tab_hi, e.f);
-}
 
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta) {
     const int blocks = std::min(nblk(3 * e.n, 256), e.num_sms * 8);

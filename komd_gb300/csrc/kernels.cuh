@@ -7,6 +7,9 @@ void launch_container(Engine &e, cudaStream_t st);
 int launch_pair(Engine &e, cudaStream_t st, bool measure, double *lj_hist);
 void launch_pair_tile(PairParams &p, int ncell, bool measure, bool emit, cudaStream_t st);
 PairParams pair_params(Engine &e);
+// pair_cell.cu: FP64 forces, FENE, histograms (blocks launched: rows of partial sums when measuring)
+int launch_pair_cell(Engine &e, const PairParams &p, bool measure, bool emit, bool fene, cudaStream_t st);
+int pair_cell_grid(const Engine &e);
 void launch_vlist_build(Engine &e, cudaStream_t st);
 int launch_lj_vlist(Engine &e, PairParams &p, bool measure, bool emit, cudaStream_t st);
 int vlist_grid(const Engine &e);

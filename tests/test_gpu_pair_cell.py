@@ -1,0 +1,62 @@
+"""The per-step pair kernel (FP64 forces, FENE, the tabulated force) and the FP64
+triplets against the FP64 oracle, where their shapes change: cells emptier
+than a block's warps, neighbourhoods of several staging rounds, rows around a
+warp's 32 entries, two species, molecules.  Bars as in test_gpu_parity: FP64
+forces to 1e-12, FP32 forces to a relative RMSE of 1e-5."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_rmse(a, b):
+    return float(np.sqrt(((a - b) ** 2).sum(1).mean()) / np.sqrt((b ** 2).sum(1).mean()))
+
+
+def _system(form):
+    """(system, cell edge): sparse -- about one site per cell; liquid -- 18;
+    crowded -- 76 (four staging rounds); molecules -- three-site, two species."""
+    from komd_gb300 import lattice
+    if form == "molecules":
+        s = lattice.triatomic_sc(5, rho_site=0.3, t_star=0.5, seed=71, r0=0.97, theta0_deg=90.0)
+        return s, 2.5
+    if form == "sparse":
+        s = lattice.argon_fcc(4, rho=0.07, t_star=0.7, seed=72, jitter=0.35)
+        return s, 2.5
+    s = lattice.argon_fcc(6 if form == "liquid" else 8, rho=0.8442, t_star=0.722, seed=73, jitter=0.05)
+    return s, float(s.high[0]) / (4.0 if form == "liquid" else 3.0)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("form", ["sparse", "liquid", "crowded", "molecules"])
+def test_cell_list_forces_match_oracle(oracle_lib, form, mixed):
+    """LJ + FENE in both precisions, and the tabulated force."""
+    from komd_gb300 import gpu
+    s, cell = _system(form)
+    if mixed:
+        s.eps[::2], s.sig[::2] = 0.7, 0.95
+    sim = oracle_lib.OracleSim(s, cell, 2.4, fene=True)
+    sim.update_container()
+    sim.forces()
+    assert np.isfinite(sim.f).all()
+    for precision, bar in ((gpu.FP64, 1e-12), (gpu.FP32, 1e-5)):
+        g = gpu.GpuSystem(s, gpu.make_config(s.low, s.high, cell, cutoff=2.4, terms=gpu.TERM_LJ | gpu.TERM_FENE,
+                                             precision=precision))
+        g.update_container()
+        g.forces()
+        f = g.download()[2]
+        u = g.measure(gpu.MEASURE_ENERGY)["u_lj"]
+        g.close()
+        assert rel_rmse(f, sim.f) < bar
+        assert u == pytest.approx(sim.lj_out.u_total, rel=1e-11 if precision == gpu.FP64 else 2e-5)
+    x = np.concatenate([[0.3], np.sort(np.random.default_rng(5).uniform(0.31, 2.2, 41))])   # uneven nodes, r beyond the last
+    table = (x, 2.0 / x ** 2, 50.0, 0.25)
+    sim = oracle_lib.OracleSim(s, cell, 2.4, lj=False, table=table)
+    sim.update_container()
+    sim.forces()
+    g = gpu.GpuSystem(s, gpu.make_config(s.low, s.high, cell, cutoff=2.4, terms=gpu.TERM_TABULATED, precision=gpu.FP64))
+    g.set_pair_table(*table)
+    g.update_container()
+    g.forces()
+    assert rel_rmse(g.download()[2], sim.f) < 1e-12
+    g.close()
