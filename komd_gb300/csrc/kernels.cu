@@ -235,141 +235,153 @@ __global__ void __launch_bounds__(kBlock) k_cell_sort(SortArgs a) {
     cell_sort_body(a, blockIdx.x, gridDim.x);
 }
 
-// the ATM neighbour list's entry: r_i - r_j and the packed code
-template <typename Real>
-struct AtmEntry;
-template <>
-struct AtmEntry<float> { using T = float4; };
-template <>
-struct AtmEntry<double> { using T = AtmEntryD; };
-
 // ===========================================================================
-// ATM triplet kernel (ATM.cpp:22-62 / ATM_NOLIST.cpp:124-159): one warp per
+// ATM triplets in FP64 (ATM.cpp:22-62 / ATM_NOLIST.cpp:124-159): one warp per
 // site i, every pair (a, b) of i's neighbours inside cutoff_3b with
 // |r_a - r_b| inside too.  Force on i only (each triplet is visited from all
-// three vertices, no atomics).  With A=|r_ia|^2, B=|r_ib|^2, C=|r_ab|^2:
+// three vertices, no atomics: the sums are reproducible).  With A=|r_ia|^2,
+// B=|r_ib|^2, C=|r_ab|^2:
 //   V = nu [ (ABC)^-3/2 + 3/8 P (ABC)^-5/2 ],  P = (A+B-C)(A-B+C)(-A+B+C)
 //   dV/dA = nu (ABC)^-5/2 [ -3/2 BC + 3/8 dP/dA - 15/16 P/A ]
 //   F_i(physical) = -2 (dV/dA e_a + dV/dB e_b),  e_a = r_i - r_a
 // which equals the reference's comp_force terms (comp_force = 2 dV/dA).
+//
+// GB300's FP64 pipe (about 1/64 of the FP32 rate) bounds this kernel, so only
+// the triplets reach it: the lanes test the candidate pairs in FP32 with a
+// 1e-4 margin over the cutoff (the vectors' rounding is below 1e-6 of it),
+// queue the hits by ballot and evaluate 32 queued pairs at a time, with the
+// exact FP64 test of C.  A, 1/A and 1/sqrt(A) are staged once per neighbour.
+// 32,000 sites of liquid argon: 1688 -> 418 us a launch (every candidate tested
+// and both roots taken in FP64 before), sensors' form 3051 -> 928 us.
 // ===========================================================================
-__device__ __forceinline__ int entry_code(const float4 &e) { return __float_as_int(e.w); }
-__device__ __forceinline__ int entry_code(const AtmEntryD &e) { return (int)e.code; }
-__device__ __forceinline__ float rsqrt_r(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double rsqrt_r(double x) { return 1.0 / sqrt(x); }
+struct AtmStageD { double x, y, z, A, iA, wA; };   // r_i - r_a, |.|^2, its reciprocal and reciprocal root
 
-template <typename Real, bool MEASURE, bool COMPAT>
-__global__ void __launch_bounds__(kBlock) k_atm(AtmParams p) {
-    using Entry = typename AtmEntry<Real>::T;
-    struct Q2 { Real A, invA; };
+template <bool MEASURE, bool COMPAT>
+__global__ void __launch_bounds__(kBlock) k_atm_d(AtmParams p) {
     extern __shared__ float4 s_dyn[];
-    __shared__ double s_part[kWarpsPerBlock][4 + 6];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int s_q[kWarpsPerBlock][64];
+    __shared__ double s_part[kWarpsPerBlock][8];
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int cap = p.nl_cap;
-    Entry *se = reinterpret_cast<Entry *>(s_dyn) + wib * cap;
-    Q2 *sq = reinterpret_cast<Q2 *>(reinterpret_cast<Entry *>(s_dyn) + kWarpsPerBlock * cap) + wib * cap;
-    const Entry *nl = reinterpret_cast<const Entry *>(p.nl);
-    const int i = blockIdx.x * kWarpsPerBlock + wib;
-    Real gx = 0, gy = 0, gz = 0;
-    double a_e = 0.0, a_t = 0.0, a_w[6] = {0, 0, 0, 0, 0, 0};
-    const Real rc2 = (Real)p.rc2;
-    if (i < p.n) {
+    float4 *sf = s_dyn + wib * cap;   // FP32 vector and code (the candidate test)
+    AtmStageD *sd = reinterpret_cast<AtmStageD *>(s_dyn + warps * cap) + wib * cap;
+    const AtmEntryD *nl = reinterpret_cast<const AtmEntryD *>(p.nl);
+    const double rc2 = p.rc2;
+    const float pre2 = (float)(p.rc2 * (1.0 + 1e-4));
+    double a_e = 0.0, a_w[6] = {0, 0, 0, 0, 0, 0};
+    int a_t = 0;
+    unsigned lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    for (int i = blockIdx.x * warps + wib; i < p.n; i += gridDim.x * warps) {
         const int ni = p.nl_count[i];
         for (int k = lane; k < ni; k += 32) {
-            const Entry e = nl[(size_t)i * cap + k];
-            const Real A = (Real)e.x * (Real)e.x + (Real)e.y * (Real)e.y + (Real)e.z * (Real)e.z;
-            se[k] = e;
-            sq[k] = Q2{A, (Real)1 / A};
+            const AtmEntryD e = nl[(size_t)i * cap + k];
+            const double A = e.x * e.x + e.y * e.y + e.z * e.z;
+            sf[k] = make_float4((float)e.x, (float)e.y, (float)e.z, __int_as_float((int)e.code));
+            sd[k] = AtmStageD{e.x, e.y, e.z, A, __drcp_rn(A), rsqrt(A)};
         }
         __syncwarp();
-        for (int a0 = 0; a0 < ni; a0 += 32) {
+        double gx = 0.0, gy = 0.0, gz = 0.0;
+        auto triplet = [&](int q, bool valid) {
+            if (!valid) return;
+            const AtmStageD ea = sd[q & 0xffff], eb = sd[q >> 16];
+            const double cx = eb.x - ea.x, cy = eb.y - ea.y, cz = eb.z - ea.z;
+            const double C = cx * cx + cy * cy + cz * cz;
+            if (dabove(C, rc2)) return;
+            const double A = ea.A, B = eb.A;
+            const double wc = rsqrt(C);
+            const double sv = ea.wA * eb.wA * wc;       // 1/(abc)
+            const double s2 = sv * sv;
+            const double s5 = s2 * s2 * sv;
+            const double S = A + B + C;
+            const double t1 = fma(-2.0, C, S), t2 = fma(-2.0, B, S), t3 = fma(-2.0, A, S);
+            const double u = t2 * t3, v = t1 * t3, w = t1 * t2;
+            const double P = t1 * u;
+            const double K = u + v + w, nP = -2.5 * P;
+            // 8/3 dV/dA: u + v - w - 4 B C - 5/2 P / A  (B: v and A C; C: u and A B)
+            const double vA = s5 * fma(nP, ea.iA, fma(-2.0, w, fma(-4.0 * B, C, K)));
+            const double vB = s5 * fma(nP, eb.iA, fma(-2.0, v, fma(-4.0 * A, C, K)));
+            gx = fma(vA, ea.x, fma(vB, eb.x, gx));
+            gy = fma(vA, ea.y, fma(vB, eb.y, gy));
+            gz = fma(vA, ea.z, fma(vB, eb.z, gz));
+            if (MEASURE) {
+                const double vC = s5 * fma(nP, wc * wc, fma(-2.0, u, fma(-4.0 * A, B, K)));
+                a_e += s2 * sv * fma(0.375 * P, s2, 1.0);   // a third of it per visit, applied at the end
+                a_t++;
+                double wt = 1.0 / 3.0;
+                if (p.virial_compat) {
+                    const int ca = __float_as_int(sf[q & 0xffff].w), cb = __float_as_int(sf[q >> 16].w);
+                    const int k = 1 + ((ca & 32) ? 0 : 1) + ((cb & 32) ? 0 : 1);
+                    wt = p.atm_direct ? 0.0 : 1.0 / (double)k;
+                }
+                // pair-decomposed virial sum_pairs P_ab d (x) d with P_ab = -2 dV/d(r_ab^2)
+                const double sc = -0.75 * wt;
+                const double pa = sc * vA, pb = sc * vB, pc = sc * vC;
+                a_w[0] += pa * ea.x * ea.x + pb * eb.x * eb.x + pc * cx * cx;
+                a_w[1] += pa * ea.x * ea.y + pb * eb.x * eb.y + pc * cx * cy;
+                a_w[2] += pa * ea.y * ea.y + pb * eb.y * eb.y + pc * cy * cy;
+                a_w[3] += pa * ea.x * ea.z + pb * eb.x * eb.z + pc * cx * cz;
+                a_w[4] += pa * ea.y * ea.z + pb * eb.y * eb.z + pc * cy * cz;
+                if (!p.virial_compat) a_w[5] += pa * ea.z * ea.z + pb * eb.z * eb.z + pc * cz * cz;
+            }
+        };
+        int qn = 0;
+        const int half = ni / 2;
+        for (int a0 = 0; a0 < ni; a0 += 32) {   // round robin (a, a + d mod n): every pair once
             const int a = a0 + lane;
             const bool av = a < ni;
-            Real ax = 0, ay = 0, az = 0;
-            Q2 qa{1, 1};
-            int ca = 0;
-            if (av) {
-                const Entry ea = se[a];
-                ax = (Real)ea.x; ay = (Real)ea.y; az = (Real)ea.z;
-                ca = entry_code(ea);
-                qa = sq[a];
-            }
-            const Real wa = rsqrt_r(qa.A);
-            for (int d = 1; d <= ni / 2; d++) {
-                if (!av || (2 * d == ni && a >= d)) continue;
-                int b = a + d;
-                if (b >= ni) b -= ni;
-                const Entry eb = se[b];
-                const Q2 qb = sq[b];
-                const int cb = entry_code(eb);
-                if (COMPAT) {
-                    const int nba = ca & 31, nbb = cb & 31;
-                    const bool ok = (nba == 13 && nbb == 13) || (nba != 13 && nbb != 13 && nba != nbb);
-                    if (!ok) continue;
-                }
-                const Real bx = (Real)eb.x, by = (Real)eb.y, bz = (Real)eb.z;
-                const Real cx = bx - ax, cy = by - ay, cz = bz - az;
-                const Real C = cx * cx + cy * cy + cz * cz;
-                if (C > rc2) continue;
-                const Real A = qa.A, B = qb.A;
-                const Real wc = rsqrt_r(C);
-                const Real sv = wa * rsqrt_r(B) * wc;       // 1/(abc)
-                const Real s2 = sv * sv;
-                const Real s5 = s2 * s2 * sv;
-                const Real t1 = A + B - C, t2 = A - B + C, t3 = B + C - A;
-                const Real u = t2 * t3, v = t1 * t3, w = t1 * t2;
-                const Real P = t1 * u;
-                const Real vA = s5 * ((Real)-1.5 * B * C + (Real)0.375 * (u + v - w) - (Real)0.9375 * P * qa.invA);
-                const Real vB = s5 * ((Real)-1.5 * A * C + (Real)0.375 * (u - v + w) - (Real)0.9375 * P * qb.invA);
-                gx += vA * ax + vB * bx;
-                gy += vA * ay + vB * by;
-                gz += vA * az + vB * bz;
-                if (MEASURE) {
-                    const Real vC = s5 * ((Real)-1.5 * A * B + (Real)0.375 * (-u + v + w) - (Real)0.9375 * P * (wc * wc));
-                    a_e += (double)(s2 * sv * ((Real)1 + (Real)0.375 * P * s2)) * (1.0 / 3.0);
-                    a_t += 1.0 / 3.0;
-                    double wt;
-                    if (p.virial_compat) {
-                        const int k = 1 + ((ca & 32) ? 0 : 1) + ((cb & 32) ? 0 : 1);
-                        wt = p.atm_direct ? 0.0 : 1.0 / (double)k;
-                    } else {
-                        wt = 1.0 / 3.0;
+            float4 ea = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (av) ea = sf[a];
+            for (int d = 1; d <= half; d++) {
+                bool hit = false;
+                int b = 0;
+                if (av && !(2 * d == ni && a >= d)) {
+                    b = a + d;
+                    if (b >= ni) b -= ni;
+                    const float4 eb = sf[b];
+                    const float cx = eb.x - ea.x, cy = eb.y - ea.y, cz = eb.z - ea.z;
+                    hit = !(cx * cx + cy * cy + cz * cz > pre2);
+                    if (COMPAT) {
+                        const int nba = __float_as_int(ea.w) & 31, nbb = __float_as_int(eb.w) & 31;
+                        hit = hit && ((nba == 13 && nbb == 13) || (nba != 13 && nbb != 13 && nba != nbb));
                     }
-                    // pair-decomposed virial sum_pairs P_ab d (x) d with P_ab = -2 dV/d(r_ab^2)
-                    const double pa = -2.0 * (double)vA, pb = -2.0 * (double)vB, pc = -2.0 * (double)vC;
-                    const double dax = ax, day = ay, daz = az, dbx = bx, dby = by, dbz = bz;
-                    const double dcx = cx, dcy = cy, dcz = cz;
-                    a_w[0] += wt * (pa * dax * dax + pb * dbx * dbx + pc * dcx * dcx);
-                    a_w[1] += wt * (pa * dax * day + pb * dbx * dby + pc * dcx * dcy);
-                    a_w[2] += wt * (pa * day * day + pb * dby * dby + pc * dcy * dcy);
-                    a_w[3] += wt * (pa * dax * daz + pb * dbx * dbz + pc * dcx * dcz);
-                    a_w[4] += wt * (pa * day * daz + pb * dby * dbz + pc * dcy * dcz);
-                    if (!p.virial_compat) a_w[5] += wt * (pa * daz * daz + pb * dbz * dbz + pc * dcz * dcz);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                if (hit) s_q[wib][qn + __popc(m & lt)] = a | (b << 16);
+                qn += __popc(m);
+                if (qn >= 32) {
+                    __syncwarp();
+                    const int q = s_q[wib][lane], tail = s_q[wib][32 + lane];
+                    __syncwarp();
+                    qn -= 32;
+                    if (lane < qn) s_q[wib][lane] = tail;
+                    __syncwarp();
+                    triplet(q, true);
                 }
             }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            gx += __shfl_xor_sync(0xffffffffu, gx, o);
-            gy += __shfl_xor_sync(0xffffffffu, gy, o);
-            gz += __shfl_xor_sync(0xffffffffu, gz, o);
-        }
-        if (lane == 0) {
-            const int site = p.slot_site[i];
+        __syncwarp();
+        if (qn > 0) triplet(lane < qn ? s_q[wib][lane] : 0, lane < qn);
+        const double gs = warp_sum3(gx, gy, gz, lane);
+        if ((lane & 7) == 0 && lane < 24) {
             // reference sign: +2 nu (vA e_a + vB e_b); physical: the negative
-            const double sc = 2.0 * (double)p.sign * p.nu;
-            p.f[3 * site] += sc * (double)gx;
-            p.f[3 * site + 1] += sc * (double)gy;
-            p.f[3 * site + 2] += sc * (double)gz;
+            const double sc = 0.75 * p.sign * p.nu;
+            p.f[3 * (size_t)p.slot_site[i] + (lane >> 3)] += sc * gs;
         }
+        __syncwarp();   // the staging is refilled by the next vertex
     }
     if (MEASURE) {
-        double vals[8] = {a_e, a_t, a_w[0], a_w[1], a_w[2], a_w[3], a_w[4], a_w[5]};
+        double vals[8] = {a_e * (1.0 / 3.0), 0.0, a_w[0], a_w[1], a_w[2], a_w[3], a_w[4], a_w[5]};
         for (int k = 0; k < 8; k++) {
             double x = vals[k];
             for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
             vals[k] = x;
         }
-        if (lane == 0) for (int k = 0; k < 8; k++) s_part[wib][k] = vals[k];
+        const int visits = __reduce_add_sync(0xffffffffu, a_t);
+        if (lane == 0) {
+            for (int k = 0; k < 8; k++) s_part[wib][k] = vals[k];
+            s_part[wib][1] = (double)visits / 3.0;
+        }
         __syncthreads();
         if (threadIdx.x < R_NSLOTS) {
             const int t = threadIdx.x;
@@ -379,7 +391,7 @@ __global__ void __launch_bounds__(kBlock) k_atm(AtmParams p) {
             else if (t == R_TRIPS) src = 1;
             else if (t >= R_W0 && t <= R_W5) src = 2 + (t - R_W0);
             if (src >= 0)
-                for (int w = 0; w < kWarpsPerBlock; w++) sum += s_part[w][src];
+                for (int w = 0; w < warps; w++) sum += s_part[w][src];
             // nu scaling of energy and virial
             if (t == R_UATM || (t >= R_W0 && t <= R_W5)) sum *= p.nu;
             p.partials[(size_t)blockIdx.x * R_NSLOTS + t] = sum;
@@ -1255,7 +1267,19 @@ PairParams pair_params(Engine &e) {
     return p;
 }
 
-int atm_grid(const Engine &e) { return nblk(e.n, kWarpsPerBlock); }
+// FP64: a resident grid whose warps stride over the vertices (at most one row
+// of partial sums per block, whatever the list capacity)
+int atm_grid(const Engine &e) {
+    const int g = nblk(e.n, kWarpsPerBlock);
+    return e.cfg.precision == KOMD_FP64 ? std::min(g, e.num_sms * 16) : g;
+}
+// warps per block of the FP64 kernel: eight, fewer where their staging (64
+// bytes a neighbour) would pass 96 KB
+static int atm_warps(const Engine &e) {
+    int w = kWarpsPerBlock;
+    while (w > 1 && (size_t)w * e.nl_cap * (sizeof(AtmStageD) + sizeof(float4)) > 96 * 1024) w >>= 1;
+    return w;
+}
 
 // The FP32 force path runs the tiled kernel (pair_tile.cu, one CTA per cell);
 // FP64 mode, FENE and the LJ sensor histograms use pair_cell.cu.  FENE acts
@@ -1288,9 +1312,8 @@ void launch_limit(Engine &e, cudaStream_t st) {
 }
 
 size_t atm_smem(const Engine &e) {
-    const size_t per = e.cfg.precision == KOMD_FP64 ? (sizeof(AtmEntryD) + 2 * sizeof(double))
-                                                    : (2 * sizeof(float4));
-    return (size_t)kWarpsPerBlock * e.nl_cap * per;
+    if (e.cfg.precision == KOMD_FP64) return (size_t)atm_warps(e) * e.nl_cap * (sizeof(AtmStageD) + sizeof(float4));
+    return (size_t)kWarpsPerBlock * e.nl_cap * 2 * sizeof(float4);
 }
 
 // stage vertex i's neighbours above i (ballot compaction); returns their count
@@ -1414,25 +1437,23 @@ __global__ void k_atm_flush(int n, const int *__restrict__ slot_site, unsigned l
     }
 }
 
-template <typename Real>
-static void atm_dispatch(AtmParams &p, bool measure, bool compat, int grid, size_t sm, cudaStream_t st) {
-    if (measure) {
-        if (compat) k_atm<Real, true, true><<<grid, kBlock, sm, st>>>(p);
-        else k_atm<Real, true, false><<<grid, kBlock, sm, st>>>(p);
-    } else {
-        if (compat) k_atm<Real, false, true><<<grid, kBlock, sm, st>>>(p);
-        else k_atm<Real, false, false><<<grid, kBlock, sm, st>>>(p);
-    }
-}
-
-template <>
-void atm_dispatch<float>(AtmParams &p, bool measure, bool compat, int grid, size_t sm, cudaStream_t st) {
+static void atm_dispatch_f(AtmParams &p, bool measure, bool compat, int grid, size_t sm, cudaStream_t st) {
     if (measure) {
         if (compat) k_atm_q<true, true><<<grid, kBlock, sm, st>>>(p);
         else k_atm_q<true, false><<<grid, kBlock, sm, st>>>(p);
     } else {
         if (compat) k_atm_q<false, true><<<grid, kBlock, sm, st>>>(p);
         else k_atm_q<false, false><<<grid, kBlock, sm, st>>>(p);
+    }
+}
+
+static void atm_dispatch_d(AtmParams &p, bool measure, bool compat, int grid, int warps, size_t sm, cudaStream_t st) {
+    if (measure) {
+        if (compat) k_atm_d<true, true><<<grid, 32 * warps, sm, st>>>(p);
+        else k_atm_d<true, false><<<grid, 32 * warps, sm, st>>>(p);
+    } else {
+        if (compat) k_atm_d<false, true><<<grid, 32 * warps, sm, st>>>(p);
+        else k_atm_d<false, false><<<grid, 32 * warps, sm, st>>>(p);
     }
 }
 
@@ -1478,8 +1499,9 @@ bool launch_atm(Engine &e, cudaStream_t st, bool measure, bool with_step1) {
         k_atm_s<<<atm_grid(e), kBlock, atm_smem(e), st>>>(p);
         return launch_atm_flush(e, st, with_step1, false);
     }
-    if (e.cfg.precision == KOMD_FP64) atm_dispatch<double>(p, measure, compat, atm_grid(e), atm_smem(e), st);
-    else atm_dispatch<float>(p, measure, compat, atm_grid(e), atm_smem(e), st);
+    if (e.cfg.precision == KOMD_FP64)
+        atm_dispatch_d(p, measure, compat, atm_grid(e), atm_warps(e), atm_smem(e), st);
+    else atm_dispatch_f(p, measure, compat, atm_grid(e), atm_smem(e), st);
     return false;
 }
 
@@ -1529,18 +1551,23 @@ void launch_rdf_bins(Engine &e, cudaStream_t st, double *bins, bool cells, doubl
         k_rdf_all<<<nblk(e.n_mol, 128), 128, 0, st>>>(e.g, (int)e.n_mol, e.com, max_r, dr, nbins, bins);
 }
 
+// the ATM kernels' staging; with their static arrays (up to 5 KB) it passes
+// the default 48 KB above 40
 void set_kernel_attributes(Engine &e) {
     const int sm = (int)atm_smem(e);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_atm_s, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (sm > 48 * 1024) {
-        cudaFuncSetAttribute(k_atm_q<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm_q<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm_q<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm_q<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm<double, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm<double, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm<double, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_atm<double, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (sm <= 40 * 1024) return;
+    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (e.cfg.precision == KOMD_FP64) {
+        cudaFuncSetAttribute(k_atm_d<true, true>, attr, sm);
+        cudaFuncSetAttribute(k_atm_d<true, false>, attr, sm);
+        cudaFuncSetAttribute(k_atm_d<false, true>, attr, sm);
+        cudaFuncSetAttribute(k_atm_d<false, false>, attr, sm);
+    } else {
+        cudaFuncSetAttribute(k_atm_s, attr, sm);
+        cudaFuncSetAttribute(k_atm_q<true, true>, attr, sm);
+        cudaFuncSetAttribute(k_atm_q<true, false>, attr, sm);
+        cudaFuncSetAttribute(k_atm_q<false, true>, attr, sm);
+        cudaFuncSetAttribute(k_atm_q<false, false>, attr, sm);
     }
 }
 

@@ -60,3 +60,30 @@ def test_cell_list_forces_match_oracle(oracle_lib, form, mixed):
     g.forces()
     assert rel_rmse(g.download()[2], sim.f) < 1e-12
     g.close()
+
+
+@pytest.mark.parametrize("full", [False, True])
+@pytest.mark.parametrize("form", ["sparse", "liquid", "crowded"])
+def test_fp64_triplets_match_oracle(oracle_lib, form, full):
+    """FP64 ATM forces in both triplet sets, energy and count in the full one
+    (the oracle's compat sweep counts list entries, images among them); the
+    cutoffs give vertices with no neighbour, with partly filled batches, and
+    (crowded) with more than 32 neighbours and several batches each."""
+    from komd_gb300 import gpu
+    s, cell = _system(form)
+    rc3 = 2.4 if form == "crowded" else 1.9
+    sim = oracle_lib.OracleSim(s, cell, 2.4, nu=0.073, cutoff_atm=rc3, atm=True, atm_mode="full" if full else "compat")
+    sim.update_container()
+    sim.forces()
+    g = gpu.GpuSystem(s, gpu.make_config(s.low, s.high, cell, cutoff=2.4, cutoff_3b=rc3, nu=0.073,
+                                         terms=gpu.TERM_LJ | gpu.TERM_ATM, precision=gpu.FP64,
+                                         atm_enum=gpu.ATM_ENUM_FULL if full else gpu.ATM_ENUM_COMPAT))
+    g.update_container()
+    g.forces()
+    f = g.download()[2]
+    o = g.measure(gpu.MEASURE_ENERGY)
+    g.close()
+    assert rel_rmse(f, sim.f) < 1e-12
+    if full:
+        assert o["triplets"] == sim.atm_out.triplets
+        assert o["u_atm"] == pytest.approx(sim.atm_out.energy, rel=1e-11)
