@@ -1843,10 +1843,12 @@ int packed_group(komd_batch *b, PackedStep &pk, int r0, int r1, int pr) {
     std::vector<ScatterArgs> sm;
     std::vector<SortArgs> so;
     std::vector<FlushArgs> fl;
+    double sites = 0.0;    // the fullest replica's mean sites per cell
+    int64_t cells = 0;
     std::vector<PairParams> pp;
     std::vector<AtmParams> ap;
     std::vector<float> sa;
-    std::vector<int> n, per, two, b_io, b_cont, b_sort, b_vb, b_force;
+    std::vector<int> n, per, b_io, b_cont, b_sort, b_vb, b_force;
     for (komd_gpu *h : reps) {
         Engine &e = h->e;
         s0.push_back(step0_args(e));
@@ -1864,7 +1866,8 @@ int packed_group(komd_batch *b, PackedStep &pk, int r0, int r1, int pr) {
         sa.push_back((float)(2.0 * a.sign * a.nu));
         n.push_back((int)e.n);
         per.push_back(pr);
-        two.push_back(vbuild_two(e) ? 1 : 0);
+        cells += e.g.ncell;
+        sites = std::max(sites, (double)e.n / e.g.ncell);
         b_io.push_back((int)((e.n + 255) / 256));
         b_cont.push_back(packed_blocks_container(e));
         b_sort.push_back(std::max(1, std::min((e.g.ncell + kWarpsPerBlock - 1) / kWarpsPerBlock, 16)));
@@ -1886,7 +1889,8 @@ int packed_group(komd_batch *b, PackedStep &pk, int r0, int r1, int pr) {
     if (!rc) rc = packed_upload(b, sa, pk.sa);
     if (!rc) rc = packed_upload(b, n, pk.n);
     if (!rc) rc = packed_upload(b, per, pk.per);
-    if (!rc) rc = packed_upload(b, two, pk.two);
+    // about one replica in eight rebuilds its list in a step
+    pk.vb = vb_shape(sites, cells / 8, b->reps[0]->e.num_sms);
     return rc;
 }
 

@@ -234,6 +234,12 @@ struct PairParams {
                                // (the flush widens it) instead of FP64 into f
 };
 
+// the Verlet list build's launch shape: warps per block, staged sites per
+// round, parts of a home cell's sites
+struct VbShape {
+    int warps = 4, stage = 640, split = 1;
+};
+
 // the tabulated force F(r): ascending nodes xs, values ys, segment slopes,
 // lo below and hi above the nodes
 struct PairTable {

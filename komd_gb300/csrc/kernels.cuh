@@ -57,7 +57,7 @@ struct PackedStage {
 struct PackedStep {
     int nrep = 0;
     PackedStage step0, bin, scan, scatter, sort, vbuild, force, flush;
-    int *two = nullptr;       // per replica: the two-home form of the list build
+    VbShape vb;               // the list build's shape for every replica of the group
     PairParams *pp = nullptr; // per replica (list build and force pass)
     AtmParams *ap = nullptr;
     float *sa = nullptr;      // per replica: 2 sign nu
@@ -77,7 +77,8 @@ size_t lj_atm_half_smem(const Engine &e);
 // the blocks a stage gives one replica (the same shapes as the single-system launches)
 int packed_blocks_container(const Engine &e);
 int packed_blocks_vbuild(const Engine &e);
-bool vbuild_two(const Engine &e);
+VbShape vb_shape(double sites, int64_t cells, int num_sms);
+size_t vb_smem(const VbShape &v);
 void launch_packed_step(const PackedStep &pk, cudaStream_t st);          // kernels.cu: all eight stages
 void launch_packed_pair_stages(const PackedStep &pk, cudaStream_t st, bool vbuild);   // pair_tile.cu
 int kinetic_grid(const Engine &e);

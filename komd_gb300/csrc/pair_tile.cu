@@ -267,30 +267,30 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Verlet list build (rebuild steps only): one warp per home cell, one lane per
-// home site (groups of 32 when a cell holds more, or two homes per lane in
-// the form for crowded cells).  The warp walks the 27
-// neighbour cells in order and stages each one's sites (position with the
-// cell's periodic offset, list word, molecule key) in warp-private shared
-// memory; every lane tests them all against its site and appends the hits to
-// its row.  Rows hold the pairs inside cutoff + skin by neighbour cell, then
-// by slot (deterministic); bit 31 marks a same-molecule pair (no LJ).
+// Verlet list build (rebuild steps only).  Blocks of a resident grid take units
+// -- part of a home cell's sites -- from a counter the scan resets (cells
+// differ in cost, and steps without a rebuild launch few blocks).  A block
+// stages the cell's 27-cell neighbourhood in shared memory, by neighbour cell
+// then slot (1024 sites a round); each warp then tests the staged sites, 32 at
+// a time, against up to four home sites at once (one shared read serves the
+// four).  Lane t keeps the ballot of batch t, so the test loop is 9
+// instructions a home and batch; the hits are then expanded from the lanes'
+// words in order and appended 32 at a time, so that the append (order key,
+// molecule key, row write) runs on full warps and row writes are contiguous.
+// Rows hold the pairs inside cutoff + skin in
+// staging order (deterministic); bit 31 marks a same-molecule pair (no LJ).
 // A row has two regions: the neighbours above the site (vl_above: larger z
 // at the rebuild, ties by slot) from the front, the others from the back
 // (row[cap-1] downwards); the count word holds both (above | below << 16).
 // The half-list force pass reads the front region alone, full-row readers
 // both (vl_entry).
+// Issue-bound (79 % issue activity, 232M instructions at 256k sites).  Against a
+// warp per home cell with a lane per home site, a launch takes 247 us (320) at
+// 256,000 sites and skin 0.6, 16 us (118; 216 cells left most SMs idle) at
+// 4,000, and 565 us (1157) on 300,000 sites of molecules in cells of 4.8.
+// Per-lane shares of the staged sites without ballots, and classifying the hits
+// in the test loop, took 254 and 375 us at 256,000.
 // ---------------------------------------------------------------------------
-constexpr int kVbWarps = 4;   // home cells per block
-
-// appends one hit to a two-region row: the front for a neighbour above the
-// site (vl_above), the back otherwise (a full row drops the hit and the count
-// still grows: the caller flags the overflow)
-__device__ __forceinline__ void vl_put(unsigned *row, int cap, int &chi, int &clo, unsigned word, bool up) {
-    if (chi + clo < cap) row[up ? chi : cap - 1 - clo] = word;
-    if (up) chi++; else clo++;
-}
-
 // the count word of a row (both regions clamped so that they never overlap)
 __device__ __forceinline__ int vl_count_word(int chi, int clo, int cap) {
     const int a = min(chi, cap), b = min(clo, cap - a);
@@ -300,167 +300,180 @@ __device__ __forceinline__ int vl_count_word(int chi, int clo, int cap) {
 // logical entry k of a full row (the front region, then the back region)
 __device__ __forceinline__ int vl_entry(int k, int chi, int cap) { return k < chi ? k : cap - 1 - (k - chi); }
 
-// one lane's home site in the build: position, key, row and hit count
-struct VbHome {
-    float4 p;
-    int key, slot, c, clo, zk;
-    unsigned self;
-    bool active;
-};
+constexpr int kVbMaxWarps = 8;
+constexpr int kVbRound = 1024;   // staged sites a round: a ballot word per lane and 32 sites
+constexpr int kVbQueue = 256;    // hits expanded at a time per warp
 
-__device__ __forceinline__ void vb_home(const PairParams &p, int hs, int hn, int h, VbHome &o) {
-    o.active = h < hn;
-    o.slot = hs + min(h, hn - 1);
-    o.p = p.pos4[o.slot];
-    o.key = p.skey[o.slot];
-    o.self = (13u << 26) | (unsigned)o.slot;   // the site itself, in the home cell
-    o.c = 0;
-    o.clo = 0;
-    o.zk = p.zkey[o.slot];
-}
-
-__device__ __forceinline__ bool vb_hit(const VbHome &o, const float4 &pj, float rl2) {
-    const float ax = o.p.x - pj.x, ay = o.p.y - pj.y, az = o.p.z - pj.z;
-    return ax * ax + ay * ay + az * az <= rl2;
-}
-
-__device__ __forceinline__ void vb_emit(const PairParams &p, VbHome &o, const uint2 &ww, int zk) {
-    if (ww.x != o.self)
-        vl_put(p.vl + (size_t)o.slot * p.vl_cap, p.vl_cap, o.c, o.clo, ((int)ww.y == o.key ? 0x80000000u : 0u) | ww.x,
-               vl_above(o.zk, zk, (unsigned)o.slot, ww.x & 0x3ffffffu));
-}
-
-__device__ __forceinline__ void vb_done(const PairParams &p, const VbHome &o) {
-    if (o.active) {
-        p.vl_count[o.slot] = vl_count_word(o.c, o.clo, p.vl_cap);
-        if (o.c + o.clo > p.vl_cap) atomicOr(&p.err[E_VL_OVERFLOW], 1);
+// H home sites h0, h0 + 1, ... (those below h1) of one warp against the ns
+// staged sites, and their rows
+template <int H>
+__device__ __forceinline__ void vb_homes(const PairParams &p, const float4 *s_p, const unsigned *s_w, short *s_q, int hs,
+                                         int h0, int h1, int ns, int self0, bool first, bool last, float rl2, int lane,
+                                         unsigned lt) {
+    float hx[H], hy[H], hz[H];
+    unsigned word[H];
+#pragma unroll
+    for (int k = 0; k < H; k++) {
+        const float4 q = p.pos4[hs + min(h0 + k, h1 - 1)];
+        hx[k] = q.x; hy[k] = q.y; hz[k] = q.z;
+        word[k] = 0u;
     }
-}
-
-// the 27 cells around a home cell, staged 32 sites at a time in the warp's
-// shared arrays (position in the home cell's frame; list word without the
-// same-molecule bit and molecule key; order key); visit(jc) tests the jc
-// staged sites
-template <typename Visit>
-__device__ __forceinline__ void vb_walk(const PairParams &p, int cx, int cy, int cz, const float4 *nbo, float4 *sq,
-                                        uint2 *sw, int *sz, int lane, Visit &&visit) {
-    for (int nb = 0; nb < 27; nb++) {
-        int kx, ky, kz;
-        bool cr;
-        const int q = nb_cell(p.g, cx, cy, cz, nb, kx, ky, kz, cr);
-        const int qs = p.cell_start[q], qn = p.cell_start[q + 1] - qs;
-        const float4 o = nbo[nb];
-        for (int jb = 0; jb < qn; jb += 32) {
-            const int jc = min(32, qn - jb);
-            __syncwarp();
-            if (lane < jc) {
-                const int j = qs + jb + lane;
-                float4 pj = p.pos4[j];
-                pj.x += o.x;
-                pj.y += o.y;
-                pj.z += o.z;
-                sq[lane] = pj;
-                sw[lane] = make_uint2(((unsigned)nb << 26) | (unsigned)j, (unsigned)p.skey[j]);
-                sz[lane] = p.zkey[j];
-            }
-            __syncwarp();
-            visit(jc);
+    const int nb = (ns + 31) >> 5;   // the staging is padded to whole batches with sites out of range
+    for (int t = 0; t < nb; t++) {
+        const float4 pj = s_p[32 * t + lane];
+#pragma unroll
+        for (int k = 0; k < H; k++) {
+            const float ax = hx[k] - pj.x, ay = hy[k] - pj.y, az = hz[k] - pj.z;
+            const unsigned m = __ballot_sync(0xffffffffu, ax * ax + ay * ay + az * az <= rl2);
+            if (lane == t) word[k] = m;
         }
     }
+#pragma unroll
+    for (int k = 0; k < H; k++) {
+        if (h0 + k >= h1) break;
+        const int hslot = hs + h0 + k;
+        const int self = self0 + h0 + k;   // the site itself, if it is staged in this round
+        unsigned m = word[k];
+        if ((self >> 5) == lane && self >= 0) m &= ~(1u << (self & 31));
+        const int zi = p.zkey[hslot], hkey = p.skey[hslot];
+        unsigned *row = p.vl + (size_t)hslot * p.vl_cap;
+        int chi = 0, clo = 0;   // run on over the rounds
+        if (!first) {
+            const int cw = p.vl_count[hslot];
+            chi = cw & 0xffff;
+            clo = cw >> 16;
+        }
+        const int mine = __popc(m);
+        int off = mine;   // exclusive prefix of the lanes' hits
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, off, o);
+            if (lane >= o) off += y;
+        }
+        const int hits = __shfl_sync(0xffffffffu, off, 31);
+        off -= mine;
+        for (int q0 = 0; q0 < hits; q0 += kVbQueue) {   // one trip unless a round holds more hits
+            const int qe = min(hits, q0 + kVbQueue);
+            __syncwarp();
+            while (m && off < qe) {
+                s_q[off - q0] = (short)(32 * lane + __ffs(m) - 1);
+                m &= m - 1;
+                off++;
+            }
+            __syncwarp();
+            for (int c0 = q0; c0 < qe; c0 += 32) {
+                const bool valid = c0 + lane < qe;
+                unsigned wd = 0;
+                bool up = false;
+                if (valid) {
+                    const int c = s_q[c0 - q0 + lane];
+                    wd = s_w[c];
+                    const unsigned j = wd & 0x3ffffffu;
+                    up = vl_above(zi, __float_as_int(s_p[c].w), (unsigned)hslot, j);
+                    if (p.multi_key && p.skey[j] == hkey) wd |= 0x80000000u;
+                }
+                const unsigned mu = __ballot_sync(0xffffffffu, valid && up);
+                const unsigned md = __ballot_sync(0xffffffffu, valid && !up);
+                // a full row drops hits and the counts still grow: flagged below
+                const int at = up ? chi + __popc(mu & lt) : clo + __popc(md & lt);
+                if (valid && at < p.vl_cap) row[up ? at : p.vl_cap - 1 - at] = wd;
+                chi += __popc(mu);
+                clo += __popc(md);
+            }
+        }
+        if (lane == 0) {
+            if (last) {
+                p.vl_count[hslot] = vl_count_word(chi, clo, p.vl_cap);
+                if (chi + clo > p.vl_cap) atomicOr(&p.err[E_VL_OVERFLOW], 1);
+            } else {   // past 0x7fff the row has overflowed already
+                p.vl_count[hslot] = min(chi, 0x7fff) | (min(clo, 0x7fff) << 16);
+            }
+        }
+    }
+    __syncwarp();
 }
 
-// TWO = false: a home site per lane, one walk per 32 homes (cells of up to
-// about 26 sites on average); TWO = true: cells of more than 32 sites walk
-// their neighbourhood once per 64 homes.  Both write the same rows.
-template <bool TWO>
-__device__ __forceinline__ void vlist_build_body(const PairParams &p, int bid) {
-    __shared__ float4 s_q[kVbWarps][32];
-    __shared__ uint2 s_w[kVbWarps][32];
-    __shared__ int s_z[kVbWarps][32];
+__device__ __forceinline__ void vlist_build_body(const PairParams &p, const VbShape &shape, int bid) {
+    extern __shared__ float4 s_dyn[];
+    __shared__ int s_st[27], s_pre[28];
+    __shared__ short s_q[kVbMaxWarps][kVbQueue];
+    __shared__ int s_unit;
     if (!*p.rebuild) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const unsigned lt = lanemask_lt();
     if (bid == 0 && threadIdx.x == 0 && p.rebuild_count) atomicAdd(p.rebuild_count, 1);
     const float rl2 = (float)p.rl2;
-    float4 *sq = s_q[w];
-    uint2 *sw = s_w[w];
-    int *sz = s_z[w];
-    // warps take home cells from a counter (reset by the scan of this rebuild):
-    // cells differ in cost, and a resident grid keeps every SM busy to the end
+    const int stage = shape.stage, split = shape.split;
+    float4 *s_p = s_dyn;                                            // position in the home cell's frame, order key
+    unsigned *s_w = reinterpret_cast<unsigned *>(s_dyn + stage);    // list word without the same-molecule bit
     for (;;) {
-        int cell = 0;
-        if (lane == 0) cell = atomicAdd(p.vb_next, 1);
-        cell = __shfl_sync(0xffffffffu, cell, 0);
-        if (cell < 0 || cell >= p.g.ncell) break;
-        int cx, cy, cz;
-        cell_coords(p.g, cell, cx, cy, cz);
-        const int hs = p.cell_start[cell], hn = p.cell_start[cell + 1] - hs;
-        const float4 *nbo = p.nboff + (size_t)cell * 27;
-        if (!TWO || hn <= 32) {
-          for (int hb = 0; hb < hn; hb += 32) {   // one trip unless TWO is false and hn > 32
-            // a home site per lane
-            const int h = hb + lane;
-            const bool active = h < hn;
-            const int hslot = hs + min(h, hn - 1);
-            const float4 hp = p.pos4[hslot];
-            const int hkey = p.skey[hslot];
-            const int hz = p.zkey[hslot];
-            const unsigned self = (13u << 26) | (unsigned)hslot;   // the site itself, in the home cell
-            unsigned *row = p.vl + (size_t)hslot * p.vl_cap;
-            int c = 0, clo = 0;
-            vb_walk(p, cx, cy, cz, nbo, sq, sw, sz, lane, [&](int jc) {
-                if (active) {
-#pragma unroll 4
-                    for (int t = 0; t < jc; t++) {
-                        const float4 pj = sq[t];
-                        const float ax = hp.x - pj.x, ay = hp.y - pj.y, az = hp.z - pj.z;
-                        if (ax * ax + ay * ay + az * az <= rl2) {   // the word is read only for hits
-                            const uint2 ww = sw[t];
-                            if (ww.x != self)
-                                vl_put(row, p.vl_cap, c, clo, ((int)ww.y == hkey ? 0x80000000u : 0u) | ww.x,
-                                       vl_above(hz, sz[t], (unsigned)hslot, ww.x & 0x3ffffffu));
-                        }
-                    }
-                }
-            });
-            if (active) {
-                p.vl_count[hslot] = vl_count_word(c, clo, p.vl_cap);
-                if (c + clo > p.vl_cap) atomicOr(&p.err[E_VL_OVERFLOW], 1);
+        __syncthreads();   // the previous unit's shared data is read to the end
+        if (threadIdx.x == 0) s_unit = atomicAdd(p.vb_next, 1);
+        __syncthreads();
+        const int unit = s_unit;
+        if (unit < 0 || unit >= p.g.ncell * split) break;
+        const int cell = unit / split, part = unit - cell * split;
+        if (w == 0) {
+            int cx, cy, cz, cnt = 0;
+            cell_coords(p.g, cell, cx, cy, cz);
+            if (lane < 27) {
+                int kx, ky, kz;
+                bool cr;
+                const int q = nb_cell(p.g, cx, cy, cz, lane, kx, ky, kz, cr);
+                const int s0 = p.cell_start[q];
+                cnt = p.cell_start[q + 1] - s0;
+                s_st[lane] = s0;
             }
-          }
-        } else {
-            // up to 64 home sites per walk of the neighbourhood: lane l serves
-            // homes hb + l and, while more than 32 remain, hb + 32 + l
-            for (int hb = 0; hb < hn; hb += 64) {
-                const bool two = hn - hb > 32;   // warp-uniform
-                VbHome h0, h1;
-                vb_home(p, hs, hn, hb + lane, h0);
-                if (two) vb_home(p, hs, hn, hb + 32 + lane, h1);
-                vb_walk(p, cx, cy, cz, nbo, sq, sw, sz, lane, [&](int jc) {
-                    if (two) {   // h0 is active: hn - hb > 32
-#pragma unroll 2
-                        for (int t = 0; t < jc; t++) {
-                            const float4 pj = sq[t];
-                            const uint2 ww = sw[t];   // one read for both homes
-                            if (vb_hit(h0, pj, rl2)) vb_emit(p, h0, ww, sz[t]);
-                            if (h1.active && vb_hit(h1, pj, rl2)) vb_emit(p, h1, ww, sz[t]);
-                        }
-                    } else if (h0.active) {
-#pragma unroll 4
-                        for (int t = 0; t < jc; t++)
-                            if (vb_hit(h0, sq[t], rl2)) vb_emit(p, h0, sw[t], sz[t]);
-                    }
-                });
-                vb_done(p, h0);
-                if (two) vb_done(p, h1);
+            int inc = cnt;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane < 27) s_pre[lane] = inc - cnt;
+            if (lane == 26) s_pre[27] = inc;
+        }
+        __syncthreads();
+        const int hs = s_st[13], hn = s_pre[14] - s_pre[13];   // neighbour 13 is the home cell
+        // this unit's homes, in contiguous shares of the warps
+        const int u0 = (int)((long long)hn * part / split), u1 = (int)((long long)hn * (part + 1) / split);
+        const int w0 = u0 + (u1 - u0) * w / warps, w1 = u0 + (u1 - u0) * (w + 1) / warps;
+        const int total = u1 > u0 ? s_pre[27] : 0;
+        for (int sb = 0; sb < total; sb += stage) {
+            const int ns = min(stage, total - sb);
+            if (sb > 0) __syncthreads();
+            for (int nb = w; nb < 27; nb += warps) {   // a neighbour cell per warp
+                const int s0 = s_st[nb], t0 = s_pre[nb] - sb;
+                const int k0 = max(0, -t0), k1 = min(s_pre[nb + 1] - s_pre[nb], ns - t0);
+                if (k0 >= k1) continue;
+                const float4 o = p.nboff[(size_t)cell * 27 + nb];
+                for (int k = k0 + lane; k < k1; k += 32) {
+                    const int j = s0 + k;
+                    const float4 q = p.pos4[j];
+                    s_p[t0 + k] = make_float4(q.x + o.x, q.y + o.y, q.z + o.z, __int_as_float(p.zkey[j]));
+                    s_w[t0 + k] = ((unsigned)nb << 26) | (unsigned)j;
+                }
+            }
+            for (int t = ns + threadIdx.x; t < ((ns + 31) & ~31); t += blockDim.x)   // out of range of every home
+                s_p[t] = make_float4(1e30f, 1e30f, 1e30f, 0.f);
+            __syncthreads();
+            const bool first = sb == 0, last = sb + stage >= total;
+            const int self0 = s_pre[13] - sb;
+            for (int h = w0; h < w1;) {
+                const int rem = w1 - h;
+                if (rem >= 3) {
+                    vb_homes<4>(p, s_p, s_w, s_q[w], hs, h, w1, ns, self0, first, last, rl2, lane, lt);
+                    h += 4;
+                } else {
+                    vb_homes<2>(p, s_p, s_w, s_q[w], hs, h, w1, ns, self0, first, last, rl2, lane, lt);
+                    h += 2;
+                }
             }
         }
     }
 }
-template <bool TWO>
-__global__ void __launch_bounds__(32 * kVbWarps) k_vlist_build(PairParams p) {
+__global__ void __launch_bounds__(32 * kVbMaxWarps) k_vlist_build(PairParams p, VbShape shape) {
     pdl_trigger();
     pdl_wait();
-    vlist_build_body<TWO>(p, blockIdx.x);
+    vlist_build_body(p, shape, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -919,12 +932,10 @@ __device__ __forceinline__ int packed_replica(const int *__restrict__ start, int
     return lo;
 }
 
-__global__ void __launch_bounds__(32 * kVbWarps) k_vlist_build_p(const PairParams *__restrict__ p,
-                                                                const int *__restrict__ two,
-                                                                const int *__restrict__ start, int nrep) {
+__global__ void __launch_bounds__(32 * kVbMaxWarps) k_vlist_build_p(const PairParams *__restrict__ p, VbShape shape,
+                                                                   const int *__restrict__ start, int nrep) {
     const int r = packed_replica(start, nrep, blockIdx.x);
-    if (two[r]) vlist_build_body<true>(p[r], blockIdx.x - start[r]);
-    else vlist_build_body<false>(p[r], blockIdx.x - start[r]);
+    vlist_build_body(p[r], shape, blockIdx.x - start[r]);
 }
 
 template <bool UNIFORM, bool SW, bool PLAIN>
@@ -948,7 +959,12 @@ static void launch_half_p(const PackedStep &pk, cudaStream_t st) {
 
 void launch_packed_pair_stages(const PackedStep &pk, cudaStream_t st, bool vbuild) {
     if (vbuild) {
-        k_vlist_build_p<<<pk.vbuild.blocks, 32 * kVbWarps, 0, st>>>(pk.pp, pk.two, pk.vbuild.start, pk.nrep);
+        // the force pass's shared-memory carve-out: an SM that runs one group's
+        // list build beside another group's force pass would otherwise have to
+        // drain to change it (48 replicas: 21.1 against 20.1 ms a pass)
+        cudaFuncSetAttribute(k_vlist_build_p, cudaFuncAttributePreferredSharedMemoryCarveout, 72);
+        k_vlist_build_p<<<pk.vbuild.blocks, 32 * pk.vb.warps, vb_smem(pk.vb), st>>>(pk.pp, pk.vb, pk.vbuild.start,
+                                                                                    pk.nrep);
         return;
     }
     if (pk.sw) {
@@ -961,23 +977,32 @@ void launch_packed_pair_stages(const PackedStep &pk, cudaStream_t st, bool vbuil
     }
 }
 
-int packed_blocks_vbuild(const Engine &e) {
-    // up to 1024 warps for a rebuilding replica (a warp per home cell here);
-    // the blocks of replicas without a rebuild exit at once
-    return std::max(1, std::min((e.g.ncell + kVbWarps - 1) / kVbWarps, 256));
+// The list build's shape for systems of up to `sites` sites per cell on average
+// and `cells` cells in all: the staging holds a mean neighbourhood and a
+// quarter, up to a round's 1024; eight warps where a cell keeps them busy, and
+// parts of a cell's homes where the cells alone give fewer than six blocks per SM.
+VbShape vb_shape(double sites, int64_t cells, int num_sms) {
+    VbShape v;
+    v.warps = sites >= 48.0 ? 8 : 4;
+    v.stage = std::min(kVbRound, std::max(256, ((int)(27.0 * sites * 1.25) + 127) / 128 * 128));
+    const int most = std::max(1, (int)(sites / v.warps + 0.999));
+    const int64_t want = ((int64_t)num_sms * 6 + cells - 1) / std::max<int64_t>(cells, 1);
+    v.split = (int)std::max<int64_t>(1, std::min<int64_t>(most, want));
+    return v;
 }
+size_t vb_smem(const VbShape &v) { return (size_t)v.stage * (sizeof(float4) + sizeof(unsigned)); }
 
-bool vbuild_two(const Engine &e) {
-    return (double)e.n / ((double)e.g.nd[0] * e.g.nd[1] * e.g.nd[2]) > 26.0;
+int packed_blocks_vbuild(const Engine &e) {
+    // up to 256 blocks for a rebuilding replica; those of replicas without a
+    // rebuild exit at once
+    return std::max(1, std::min(e.g.ncell, 256));
 }
 
 void launch_vlist_build(Engine &e, cudaStream_t st) {
     PairParams p = pair_params(e);
-    // a resident grid (12 blocks of 4 warps per SM at this kernel's register count)
-    const int blocks = std::min((e.g.ncell + kVbWarps - 1) / kVbWarps, e.num_sms * 12);
-    // the two-home form pays off once many cells hold more than 32 sites
-    if (vbuild_two(e)) launch_pdl(k_vlist_build<true>, blocks, 32 * kVbWarps, 0, st, p);
-    else launch_pdl(k_vlist_build<false>, blocks, 32 * kVbWarps, 0, st, p);
+    const VbShape v = vb_shape((double)e.n / e.g.ncell, e.g.ncell, e.num_sms);
+    const int blocks = std::min(e.g.ncell * v.split, e.num_sms * 48 / v.warps);   // resident
+    launch_pdl(k_vlist_build, blocks, 32 * v.warps, vb_smem(v), st, p, v);
 }
 
 template <bool UNIFORM>

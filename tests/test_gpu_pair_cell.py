@@ -87,3 +87,28 @@ def test_fp64_triplets_match_oracle(oracle_lib, form, full):
     if full:
         assert o["triplets"] == sim.atm_out.triplets
         assert o["u_atm"] == pytest.approx(sim.atm_out.energy, rel=1e-11)
+
+
+@pytest.mark.parametrize("form", ["sparse", "liquid", "crowded", "molecules"])
+def test_verlet_list_forces_match_oracle(oracle_lib, form):
+    """The Verlet list build where its units change: parts of few cells, cells
+    with no or one site, neighbourhoods of several staging rounds, molecules
+    (the same-molecule bit).  After 30 steps from the list, the forces are the
+    oracle's at the engine's positions."""
+    from komd_gb300 import gpu, lattice
+    s, cell = _system(form)
+    rc = 1.5 if form == "molecules" else 2.1   # every site pair in range lies in adjacent cells
+    if form == "molecules":
+        cell = float(s.high[0]) / 3.0
+    g = gpu.GpuSystem(s, gpu.make_config(s.low, s.high, cell, cutoff=rc, terms=gpu.TERM_LJ, skin=0.3, dt=0.002,
+                                         virial_mode=gpu.VIRIAL_CORRECT))
+    g.update_container()
+    g.forces()
+    g.step(30)
+    r, v, f = g.download()
+    g.close()
+    at = lattice.System(r=r, v=v, m=s.m, eps=s.eps, sig=s.sig, mol_id=s.mol_id, low=s.low, high=s.high)
+    sim = oracle_lib.OracleSim(at, cell, rc)
+    sim.update_container()
+    sim.forces()
+    assert rel_rmse(f, sim.f) < 1e-5
