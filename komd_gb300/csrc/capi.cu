@@ -409,6 +409,7 @@ int validate(const komd_config *c, Grid &g) {
             return fail(KOMD_ERR_ARG, "with a Verlet skin the cell size must be >= cutoff + skin");
     }
     g.cs = c->cell_size;
+    g.ics = 1.0 / c->cell_size;
     g.ncell = 1;
     for (int d = 0; d < 3; d++) {
         g.low[d] = c->domain_low[d];
@@ -617,7 +618,7 @@ int komd_gpu_destroy(komd_gpu *h) {
     dfree(e.tab_x); dfree(e.tab_y); dfree(e.tab_s); dfree(e.atm_acc); dfree(e.fown);
     dfree(e.rdf); dfree(e.lj_hist); dfree(e.counts); dfree(h->f_scratch); dfree(h->prof); dfree(h->acc); dfree(h->thermo_acc); dfree(e.offtab);
     dfree(e.nboff); dfree(e.vb_next); dfree(e.rebuild); dfree(e.bias); dfree(e.ref4); dfree(e.slot_cell); dfree(e.zkey); dfree(e.vl); dfree(e.vl_count);
-    dfree(e.rebuild_count); dfree(e.hdtm); dfree(e.exact_com);
+    dfree(e.rebuild_count); dfree(e.hdtm); dfree(e.site_lj); dfree(e.exact_com);
     {
         Surrogate &u = h->sur;
         dfree(u.x); dfree(u.mom); dfree(u.dedx); dfree(u.esite); dfree(u.fsur); dfree(u.w1); dfree(u.w1t);
@@ -713,6 +714,10 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
             const double mk = m[off[k]];
             exact[k] = (off[k + 1] - off[k] == 1 && std::frexp(mk, &ex) == 0.5) ? 1 : 0;
         }
+        std::vector<float2> lj(n);
+        for (int64_t s = 0; s < n; s++) lj[s] = make_float2((float)std::sqrt(eps[s]), (float)(0.5 * sig[s]));
+        CK(dalloc(e.site_lj, n));
+        CK(cudaMemcpy(e.site_lj, lj.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
         CK(dalloc(e.hdtm, n));
         CK(dalloc(e.exact_com, e.n_mol));
         CK(cudaMemcpy(e.hdtm, hdtm.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
@@ -1870,7 +1875,7 @@ int packed_group(komd_batch *b, PackedStep &pk, int r0, int r1, int pr) {
         sites = std::max(sites, (double)e.n / e.g.ncell);
         b_io.push_back((int)((e.n + 255) / 256));
         b_cont.push_back(packed_blocks_container(e));
-        b_sort.push_back(std::max(1, std::min((e.g.ncell + kWarpsPerBlock - 1) / kWarpsPerBlock, 16)));
+        b_sort.push_back(std::max(1, std::min((e.g.ncell + kWarpsPerBlock - 1) / kWarpsPerBlock, 128)));
         b_vb.push_back(packed_blocks_vbuild(e));
         b_force.push_back((vlist_grid(e) + pr - 1) / pr);
         pk.force_smem = std::max(pk.force_smem, lj_atm_half_smem(e));

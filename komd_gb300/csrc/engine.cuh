@@ -56,7 +56,7 @@ constexpr int kBlock = 32 * kWarpsPerBlock;
 // dimension of edge cs, the last one stretched to the domain's high bound.
 struct Grid {
     double low[3], high[3], L[3];
-    double cs;
+    double cs, ics;   // cell edge and its reciprocal
     int nd[3];
     int ncell;
 };
@@ -298,6 +298,7 @@ struct BinArgs {              // k_com_wrap_bin: COM, periodic wrap, binning
     const int *rebuild;
     const unsigned char *exact_com;
     int wrapped;
+    int single;               // every molecule has one site (the counts of both kinds are equal)
 };
 struct ScanArgs {             // k_scan2: exclusive scans of the cell counts
     int nc;
@@ -315,6 +316,7 @@ struct SortArgs {             // k_cell_sort: slots and the cell-ordered arrays
     Grid g;
     const int *mol_off, *cell_mstart, *cell_start, *cell_mols;
     const double *r, *eps, *sig;
+    const float2 *site_lj;
     const int *key;
     int *slot_site, *site_slot;
     float4 *pos4;
@@ -324,6 +326,7 @@ struct SortArgs {             // k_cell_sort: slots and the cell-ordered arrays
     float4 *ref4;
     int *slot_cell, *zkey;
     const int *rebuild;
+    int single;
 };
 struct Step0Args {            // k_step0_fused: half-kick, drift, wrap, skin test
     int n;
@@ -457,6 +460,7 @@ struct Engine {
     int *rebuild_count = nullptr;    // list builds since the last profile reset
     // per-site (dt/2)/m and per-molecule exact-COM flags (single site, power-of-two mass)
     double *hdtm = nullptr;
+    float2 *site_lj = nullptr;   // per site: FP32 sqrt(eps) and sigma/2
     unsigned char *exact_com = nullptr;
     // all sites share eps and sigma: the list kernel uses constants
     bool uniform = false;

@@ -23,6 +23,22 @@ namespace komd {
 // container: COM, periodic wrap, binning (LinkedCells.cpp:65-121,390-400;
 // MoleculeContainer.cpp:55-75).  One thread per molecule.
 // ===========================================================================
+// (int64)(x / cs) clamped to [0, nd - 1] (writeIndices).  The truncated quotient
+// is read off x * (1 / cs) where that is not within 1e-9 of an integer (its
+// error is below 4e-10 for quotients up to 1e6); the IEEE division, a dozen
+// instructions on the narrow FP64 pipe, runs for the rest.
+__device__ __forceinline__ int cell_index(double x, double cs, double ics, int nd) {
+    const double t = dmul(x, ics);
+    const int q0 = __double2int_rz(t);
+    const long long fr = __double_as_longlong(dsub(t, (double)q0));   // ordered as the value where positive
+    long long q;
+    if (q0 >= 0 && q0 < 1000000 && fr > __double_as_longlong(1e-9) && fr < __double_as_longlong(1.0 - 1e-9)) q = q0;
+    else q = __double2ll_rz(ddiv(x, cs));
+    if (q < 0) q = 0;
+    if (q > nd - 1) q = nd - 1;
+    return (int)q;
+}
+
 __device__ __forceinline__ void com_wrap_bin_body(const BinArgs &a, int bid, int nblk) {
     const Grid &g = a.g;
     const int n_mol = a.n_mol;
@@ -38,7 +54,7 @@ __device__ __forceinline__ void com_wrap_bin_body(const BinArgs &a, int bid, int
     if (a.wrapped && rebuild && !*rebuild) return;   // k_step0_fused wrapped this step; no rebuild
     const bool bin = !(rebuild && !*rebuild);        // no rebuild in this step: cells stay as built
     for (int k = bid * blockDim.x + threadIdx.x; k < n_mol; k += nblk * blockDim.x) {
-    const int s0 = mol_off[k], s1 = mol_off[k + 1];
+    const int s0 = a.single ? k : mol_off[k], s1 = a.single ? k + 1 : mol_off[k + 1];
     // com += r * m ; M += m ; com /= M   (updateCOM, no FMA).  For a single
     // site of power-of-two mass the scaling is exact and the result is r
     // itself (up to the sign of a zero), so the FP64 division is skipped.
@@ -86,17 +102,11 @@ __device__ __forceinline__ void com_wrap_bin_body(const BinArgs &a, int bid, int
     if (!bin) continue;
     // writeIndices: (int64)((com - low) / cs) clamped to [0, nd-1]
     int b[3];
-    for (int d = 0; d < 3; d++) {
-        const double fbin = ddiv(dsub(c[d], g.low[d]), g.cs);
-        long long q = __double2ll_rz(fbin);
-        if (q < 0) q = 0;
-        if (q > g.nd[d] - 1) q = g.nd[d] - 1;
-        b[d] = (int)q;
-    }
+    for (int d = 0; d < 3; d++) b[d] = cell_index(dsub(c[d], g.low[d]), g.cs, g.ics, g.nd[d]);
     const int cell = b[0] + g.nd[0] * (b[1] + g.nd[1] * b[2]);
     mol_cell[k] = cell;
     mol_rank[k] = atomicAdd(&cell_mcount[cell], 1);
-    atomicAdd(&cell_count[cell], s1 - s0);
+    if (!a.single) atomicAdd(&cell_count[cell], s1 - s0);   // else the scan takes the molecules' counts
     }
 }
 __global__ void k_com_wrap_bin(BinArgs a) {
@@ -105,48 +115,78 @@ __global__ void k_com_wrap_bin(BinArgs a) {
     com_wrap_bin_body(a, blockIdx.x, gridDim.x);
 }
 
-// exclusive scan of two count arrays of length nc (one block of 1024 threads,
-// each owning a contiguous chunk); the counts are zeroed once read, ready for
-// the next binning (work: the Verlet list build's cell counter, reset here for
-// this rebuild)
+// exclusive scans of the cells' site and molecule counts (length nc; one block
+// of 1024 threads over tiles of 4096 cells, four consecutive cells a thread);
+// the counts are zeroed once read, ready for the next binning.  Without site
+// counts (q.a null: one site per molecule) both scans are the molecules'.
+// work: the Verlet list build's unit counter, reset here for this rebuild.
 __device__ __forceinline__ void scan2_body(const ScanArgs &q) {
-    __shared__ int wa[32], wb[32];
+    __shared__ int2 s_w[2][32];
     const int nc = q.nc;
     int *__restrict__ a = q.a, *__restrict__ sa = q.sa, *__restrict__ b = q.b, *__restrict__ sb = q.sb;
-    int *__restrict__ work = q.work;
     if (q.rebuild && !*q.rebuild) return;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if (work && t == 0) *work = 0;
-    const int per = (nc + 1023) / 1024;
-    const int lo = min(t * per, nc), hi = min(lo + per, nc);
-    int ta = 0, tb = 0;
-    for (int i = lo; i < hi; i++) { ta += a[i]; tb += b[i]; }
-    // inclusive warp scan
-    int xa = ta, xb = tb;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int ya = __shfl_up_sync(0xffffffffu, xa, o), yb = __shfl_up_sync(0xffffffffu, xb, o);
-        if (lane >= o) { xa += ya; xb += yb; }
-    }
-    if (lane == 31) { wa[w] = xa; wb[w] = xb; }
-    __syncthreads();
-    if (w == 0) {
-        int va = wa[lane], vb = wb[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            const int ya = __shfl_up_sync(0xffffffffu, va, o), yb = __shfl_up_sync(0xffffffffu, vb, o);
-            if (lane >= o) { va += ya; vb += yb; }
+    if (q.work && t == 0) *q.work = 0;
+    int ca = 0, cb = 0;   // sums of the tiles before
+    for (int base = 0, turn = 0; base < nc; base += 4096, turn ^= 1) {
+        const int i = base + 4 * t;
+        int va[4] = {0, 0, 0, 0}, vb[4] = {0, 0, 0, 0};
+        const bool whole = i + 4 <= nc;
+        if (whole) {
+            const int4 y = *reinterpret_cast<const int4 *>(b + i);
+            vb[0] = y.x; vb[1] = y.y; vb[2] = y.z; vb[3] = y.w;
+            *reinterpret_cast<int4 *>(b + i) = make_int4(0, 0, 0, 0);
+            if (a) {
+                const int4 x = *reinterpret_cast<const int4 *>(a + i);
+                va[0] = x.x; va[1] = x.y; va[2] = x.z; va[3] = x.w;
+                *reinterpret_cast<int4 *>(a + i) = make_int4(0, 0, 0, 0);
+            }
+        } else {
+            for (int k = 0; k < 4 && i + k < nc; k++) {
+                vb[k] = b[i + k];
+                b[i + k] = 0;
+                if (a) {
+                    va[k] = a[i + k];
+                    a[i + k] = 0;
+                }
+            }
         }
-        wa[lane] = va;
-        wb[lane] = vb;
+        const int ta = va[0] + va[1] + va[2] + va[3], tb = vb[0] + vb[1] + vb[2] + vb[3];
+        int xa = ta, xb = tb;   // inclusive warp scan
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ya = __shfl_up_sync(0xffffffffu, xa, o), yb = __shfl_up_sync(0xffffffffu, xb, o);
+            if (lane >= o) { xa += ya; xb += yb; }
+        }
+        if (lane == 31) s_w[turn][w] = make_int2(xa, xb);
+        __syncthreads();
+        const int2 mine = s_w[turn][lane];   // every warp scans the 32 warp sums itself
+        int wa = mine.x, wb = mine.y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ya = __shfl_up_sync(0xffffffffu, wa, o), yb = __shfl_up_sync(0xffffffffu, wb, o);
+            if (lane >= o) { wa += ya; wb += yb; }
+        }
+        const int suma = __shfl_sync(0xffffffffu, wa, 31), sumb = __shfl_sync(0xffffffffu, wb, 31);
+        int pa = ca + __shfl_sync(0xffffffffu, wa - mine.x, w) + xa - ta;
+        int pb = cb + __shfl_sync(0xffffffffu, wb - mine.y, w) + xb - tb;
+        int ea[4], eb[4];
+        for (int k = 0; k < 4; k++) {
+            ea[k] = pa; pa += va[k];
+            eb[k] = pb; pb += vb[k];
+        }
+        if (whole) {
+            const int4 y = make_int4(eb[0], eb[1], eb[2], eb[3]);
+            *reinterpret_cast<int4 *>(sb + i) = y;
+            *reinterpret_cast<int4 *>(sa + i) = a ? make_int4(ea[0], ea[1], ea[2], ea[3]) : y;
+        } else {
+            for (int k = 0; k < 4 && i + k < nc; k++) {
+                sb[i + k] = eb[k];
+                sa[i + k] = a ? ea[k] : eb[k];
+            }
+        }
+        ca += suma;
+        cb += sumb;
     }
-    __syncthreads();
-    int pa = xa - ta + (w > 0 ? wa[w - 1] : 0), pb = xb - tb + (w > 0 ? wb[w - 1] : 0);
-    for (int i = lo; i < hi; i++) {
-        sa[i] = pa; pa += a[i];
-        sb[i] = pb; pb += b[i];
-        a[i] = 0;
-        b[i] = 0;
-    }
-    if (t == 1023) { sa[nc] = wa[31]; sb[nc] = wb[31]; }
+    if (t == 0) { sa[nc] = a ? ca : cb; sb[nc] = cb; }
 }
 __global__ void __launch_bounds__(1024) k_scan2(ScanArgs q) {
     pdl_trigger();
@@ -167,12 +207,14 @@ __global__ void k_scatter_mol(ScatterArgs a) {
 
 // One warp per domain cell: order the cell's molecules by index (ascending
 // site index, the reference's cell-list order), assign slots and gather the
-// cell-ordered arrays.
+// cell-ordered arrays.  A lane holds a molecule, and its place is the summed
+// size of the cell's molecules with a lower index, counted over warp shuffles.
 __device__ __forceinline__ void cell_sort_body(const SortArgs &a, int bid, int nblk) {
     const Grid &g = a.g;
     const int *__restrict__ mol_off = a.mol_off, *__restrict__ cell_mstart = a.cell_mstart;
     const int *__restrict__ cell_start = a.cell_start, *__restrict__ cell_mols = a.cell_mols;
-    const double *__restrict__ r = a.r, *__restrict__ eps = a.eps, *__restrict__ sig = a.sig;
+    const double *__restrict__ r = a.r;
+    const float2 *__restrict__ site_lj = a.site_lj;
     const int *__restrict__ key = a.key;
     int *__restrict__ slot_site = a.slot_site, *__restrict__ site_slot = a.site_slot;
     float4 *__restrict__ pos4 = a.pos4;
@@ -182,51 +224,68 @@ __device__ __forceinline__ void cell_sort_body(const SortArgs &a, int bid, int n
     double *__restrict__ bias = a.bias;
     float4 *__restrict__ ref4 = a.ref4;
     int *__restrict__ slot_cell = a.slot_cell, *__restrict__ zkey = a.zkey;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     if (a.rebuild && !*a.rebuild) return;
-    for (int cell = bid * kWarpsPerBlock + (threadIdx.x >> 5); cell < g.ncell;
-         cell += nblk * kWarpsPerBlock) {
-    int cx, cy, cz;
-    cell_coords(g, cell, cx, cy, cz);
-    const double cen[3] = {cell_centre(g, 0, cx), cell_centre(g, 1, cy), cell_centre(g, 2, cz)};
-    const int ms = cell_mstart[cell], mc = cell_mstart[cell + 1] - ms;
-    const int ss = cell_start[cell];
-    for (int base = 0; base < mc; base += 32) {
-        const int t = base + lane;
-        const int mine = (t < mc) ? cell_mols[ms + t] : INT_MAX;
-        int off = 0;
-        for (int u = 0; u < mc; u++) {
-            const int other = cell_mols[ms + u];
-            if (other < mine) off += mol_off[other + 1] - mol_off[other];
-        }
-        if (t < mc) {
-            const int s0 = mol_off[mine], s1 = mol_off[mine + 1];
-            for (int s = s0; s < s1; s++) {
-                const int slot = ss + off + (s - s0);
-                slot_site[slot] = s;
-                site_slot[s] = slot;
-                const double x = r[3 * s], y = r[3 * s + 1], z = r[3 * s + 2];
-                const float4 p4 = make_float4(__double2float_rn(x - cen[0]), __double2float_rn(y - cen[1]),
-                                              __double2float_rn(z - cen[2]), __double2float_rn(0.5 * sig[s]));
-                pos4[slot] = p4;
-                skey[slot] = key[s];
-                seps[slot] = __double2float_rn(sqrt(eps[s]));
-                if (bias) {
-                    bias[3 * s] = cen[0]; bias[3 * s + 1] = cen[1]; bias[3 * s + 2] = cen[2];
-                    ref4[s] = p4;
-                    slot_cell[slot] = cell;
-                    // the half-list order key: z quantized over the box (see vl_above)
-                    long long q = (long long)floor((z - g.low[2]) / g.L[2] * (double)kZq);
-                    zkey[slot] = (int)(q < 0 ? 0 : (q >= kZq ? kZq - 1 : q));
+    for (int cell = bid * warps + (threadIdx.x >> 5); cell < g.ncell; cell += nblk * warps) {
+        const int ms = cell_mstart[cell], mc = cell_mstart[cell + 1] - ms;
+        const int ss = cell_start[cell];
+        int cx, cy, cz;
+        cell_coords(g, cell, cx, cy, cz);
+        const double cen[3] = {cell_centre(g, 0, cx), cell_centre(g, 1, cy), cell_centre(g, 2, cz)};
+        for (int base = 0; base < mc; base += 32) {
+            const int t = base + lane;
+            const int mine = (t < mc) ? cell_mols[ms + t] : INT_MAX;
+            int s0 = mine, size = 1;
+            if (!a.single && t < mc) {
+                s0 = mol_off[mine];
+                size = mol_off[mine + 1] - s0;
+            }
+            int off = 0;
+            for (int cb = 0; cb < mc; cb += 32) {
+                int other = mine, osize = size;
+                if (cb != base) {
+                    const int u = cb + lane;
+                    other = u < mc ? cell_mols[ms + u] : INT_MAX;
+                    osize = !a.single && u < mc ? mol_off[other + 1] - mol_off[other] : 1;
                 }
-                if (posd) {
-                    posd[3 * slot] = x; posd[3 * slot + 1] = y; posd[3 * slot + 2] = z;
-                    seps_d[slot] = eps[s];
-                    sig_d[slot] = sig[s];
+                const int nu = min(32, mc - cb);
+                if (a.single) {
+                    for (int u = 0; u < nu; u++) off += __shfl_sync(0xffffffffu, other, u) < mine ? 1 : 0;
+                } else {
+                    for (int u = 0; u < nu; u++) {
+                        const int o = __shfl_sync(0xffffffffu, other, u), z = __shfl_sync(0xffffffffu, osize, u);
+                        off += o < mine ? z : 0;
+                    }
+                }
+            }
+            if (t < mc) {
+                for (int s = s0; s < s0 + size; s++) {
+                    const int slot = ss + off + (s - s0);
+                    slot_site[slot] = s;
+                    site_slot[s] = slot;
+                    const double x = r[3 * s], y = r[3 * s + 1], z = r[3 * s + 2];
+                    const float2 lj = site_lj[s];   // sqrt(eps), sigma/2
+                    const float4 p4 = make_float4(__double2float_rn(x - cen[0]), __double2float_rn(y - cen[1]),
+                                                  __double2float_rn(z - cen[2]), lj.y);
+                    pos4[slot] = p4;
+                    skey[slot] = key[s];
+                    seps[slot] = lj.x;
+                    if (bias) {
+                        bias[3 * s] = cen[0]; bias[3 * s + 1] = cen[1]; bias[3 * s + 2] = cen[2];
+                        ref4[s] = p4;
+                        slot_cell[slot] = cell;
+                        // the half-list order key: z quantized over the box (see vl_above)
+                        long long q = (long long)floor((z - g.low[2]) / g.L[2] * (double)kZq);
+                        zkey[slot] = (int)(q < 0 ? 0 : (q >= kZq ? kZq - 1 : q));
+                    }
+                    if (posd) {
+                        posd[3 * slot] = x; posd[3 * slot + 1] = y; posd[3 * slot + 2] = z;
+                        seps_d[slot] = a.eps[s];
+                        sig_d[slot] = a.sig[s];
+                    }
                 }
             }
         }
-    }
     }
 }
 __global__ void __launch_bounds__(kBlock) k_cell_sort(SortArgs a) {
@@ -1166,10 +1225,11 @@ static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
 BinArgs bin_args(const Engine &e) {
     return BinArgs{e.g, (int)e.n_mol, e.mol_off, e.r, e.m, e.com, e.mol_cell, e.mol_rank, e.cell_count, e.cell_mcount,
-                   e.verlet ? e.bias : nullptr, e.verlet ? e.rebuild : nullptr, e.exact_com, e.fused_drift ? 1 : 0};
+                   e.verlet ? e.bias : nullptr, e.verlet ? e.rebuild : nullptr, e.exact_com, e.fused_drift ? 1 : 0,
+                   e.n_mol == e.n ? 1 : 0};
 }
 ScanArgs scan_args(const Engine &e) {
-    return ScanArgs{e.g.ncell, e.cell_count, e.cell_start, e.cell_mcount, e.cell_mstart,
+    return ScanArgs{e.g.ncell, e.n_mol == e.n ? nullptr : e.cell_count, e.cell_start, e.cell_mcount, e.cell_mstart,
                     e.verlet ? e.rebuild : nullptr, e.vb_next};
 }
 ScatterArgs scatter_args(const Engine &e) {
@@ -1177,10 +1237,10 @@ ScatterArgs scatter_args(const Engine &e) {
                        e.verlet ? e.rebuild : nullptr};
 }
 SortArgs sort_args(const Engine &e) {
-    return SortArgs{e.g, e.mol_off, e.cell_mstart, e.cell_start, e.cell_mols, e.r, e.eps, e.sig, e.key,
+    return SortArgs{e.g, e.mol_off, e.cell_mstart, e.cell_start, e.cell_mols, e.r, e.eps, e.sig, e.site_lj, e.key,
                     e.slot_site, e.site_slot, e.pos4, e.skey, e.seps, e.posd, e.seps_d, e.sig_d,
                     e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.verlet ? e.slot_cell : nullptr,
-                    e.verlet ? e.zkey : nullptr, e.verlet ? e.rebuild : nullptr};
+                    e.verlet ? e.zkey : nullptr, e.verlet ? e.rebuild : nullptr, e.n_mol == e.n ? 1 : 0};
 }
 Step0Args step0_args(const Engine &e) {
     const float hs = (float)(0.5 * e.cfg.skin);
@@ -1202,7 +1262,8 @@ void launch_container(Engine &e, cudaStream_t st) {
     launch_pdl(k_com_wrap_bin, std::min(nblk(e.n_mol, 256), res), 256, 0, st, bin_args(e));
     launch_pdl(k_scan2, 1, 1024, 0, st, scan_args(e));
     launch_pdl(k_scatter_mol, std::min(nblk(e.n_mol, 256), res), 256, 0, st, scatter_args(e));
-    launch_pdl(k_cell_sort, std::min(nblk(g.ncell, kWarpsPerBlock), res), kBlock, 0, st, sort_args(e));
+    // four warps a block: with few cells the chain of loads bounds the sort, not its throughput
+    launch_pdl(k_cell_sort, std::min(nblk(g.ncell, 4), 2 * res), 128, 0, st, sort_args(e));
     if (e.verlet) {
         if (!e.fused_drift)
             k_refresh<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.slot_site, e.r, e.bias, e.pos4, e.rebuild);
@@ -1598,7 +1659,7 @@ __global__ void k_scatter_mol_p(const ScatterArgs *a, const int *start, int nrep
     const int r = packed_rep(start, nrep, blockIdx.x);
     scatter_mol_body(a[r], blockIdx.x - start[r], start[r + 1] - start[r]);
 }
-__global__ void __launch_bounds__(kBlock) k_cell_sort_p(const SortArgs *a, const int *start, int nrep) {
+__global__ void __launch_bounds__(kBlock, 4) k_cell_sort_p(const SortArgs *a, const int *start, int nrep) {
     const int r = packed_rep(start, nrep, blockIdx.x);
     cell_sort_body(a[r], blockIdx.x - start[r], start[r + 1] - start[r]);
 }
@@ -1610,7 +1671,7 @@ __global__ void __launch_bounds__(kIoBlock, 8) k_atm_flush_step1_p(const FlushAr
 // blocks per replica of the container stages: on a step without a rebuild
 // they exit at once; on a rebuild step a replica's blocks do its whole
 // binning, so too few of them make a long tail for the launch
-int packed_blocks_container(const Engine &e) { return std::max(1, std::min(nblk(e.n_mol, 256), 16)); }
+int packed_blocks_container(const Engine &e) { return std::max(1, std::min(nblk(e.n_mol, 256), 64)); }
 
 // one step of every replica: the stages of enqueue_step on the Verlet path
 // with the fused drift and the half-list pass, each stage one launch
