@@ -87,6 +87,38 @@ __device__ __forceinline__ bool dabove(double a, double b) {
     return ka > __double_as_longlong(b) && ka <= 0x7ff0000000000000LL;
 }
 
+// Reciprocal square root and square root in FP64 for kernels that GB300's FP64
+// pipe bounds: an FP32 seed y0 (24 bits, from the hardware's approximation; both
+// conversions are integer shifts of the bits) and one Householder step of third
+// order in the residual e (Householder 1970):
+//   e = 1 - x y0^2,  y = y0 + y0 e (1/2 + 3/8 e)     (y0^2 is exact)
+// |e| < 2^-21, so the truncation is below 2^-62 and the last fused operation
+// rounds once: 5 FP64 instructions, an error below 0.51 ulp.  sqrt(x) = x y
+// with one Newton correction from the exact residual x - r^2 (4 more; both
+// restated in tests/test_fp64_roots.py).  Arguments outside the FP32 normal
+// range (zero, inf, NaN among them) take CUDA's functions.
+__device__ __forceinline__ bool fp32_range(double x) {   // 2^-125 <= x < 2^125
+    return (unsigned)(__double2hiint(x) - 0x38200000) < 0x0fa00000u;
+}
+__device__ __forceinline__ double rsqrt_d(double x) {
+    if (!fp32_range(x)) return rsqrt(x);
+    // x truncated to 24 bits
+    const float xf = __int_as_float((int)__funnelshift_l((unsigned)__double2loint(x),
+                                                         (unsigned)(__double2hiint(x) - 0x38000000), 3));
+    float s;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(xf));
+    const int b = __float_as_int(s);
+    const double y0 = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+    const double e = __fma_rn(-x, __dmul_rn(y0, y0), 1.0);
+    return __fma_rn(__dmul_rn(y0, e), __fma_rn(e, 0.375, 0.5), y0);
+}
+// sqrt(x) from y = rsqrt_d(x)
+__device__ __forceinline__ double sqrt_d(double x, double y) {
+    if (!fp32_range(x)) return __dsqrt_rn(x);
+    const double r = __dmul_rn(x, y);
+    return __fma_rn(__fma_rn(-r, r, x), __dmul_rn(0.5, y), r);
+}
+
 // the warp sums of (x, y, z): a butterfly over offsets 16, 8, 4, 2, 1 whose
 // lanes split the components on the way (lanes 0-7 end with x, 8-15 with y,
 // 16-31 with z): 6 additions a lane instead of 15, the same pairing of partial

@@ -16,8 +16,10 @@
 // range test.  GB300 issues FP64 at about 1/64 of its FP32 rate, so the FP64
 // pipe bounds this form, and only pairs near or inside the range may reach
 // it; comparisons are made on the doubles' bits (integer pipe), a division
-// 1 / x is one correctly rounded reciprocal, and the warp's sums split their
-// components over the lanes (6 additions instead of 15).
+// 1 / x is one correctly rounded reciprocal, r and 1 / r of the table's force
+// come from one reciprocal root (rsqrt_d: 181 -> 145 us a launch at 32,000
+// sites against a square root and a reciprocal), and the warp's sums split
+// their components over the lanes (6 additions instead of 15).
 // Real = float: the staged coordinates are the operands; issue-bound.
 //
 // Against one warp per home cell with every candidate in the result type (10
@@ -184,14 +186,13 @@ __global__ void __launch_bounds__(32 * kPcWarps) k_pair_cell(PairParams p, PairT
                     }
                 }
                 if constexpr (KIND == PC_TABLE) {
-                    // (dr / r) * F as dr * (1 / r) * F: one division per pair
+                    // (dr / r) * F as dr * (F / r), 1 / r and r from one reciprocal root
                     if (valid && !above(r2, rc2)) {
-                        const double r = __dsqrt_rn((double)r2);
-                        const double F = table_eval(r, tab);
-                        const double ir = __drcp_rn(r);
-                        fx += (Real)dmul(dmul((double)dx, ir), F);
-                        fy += (Real)dmul(dmul((double)dy, ir), F);
-                        fz += (Real)dmul(dmul((double)dz, ir), F);
+                        const double ir = rsqrt_d((double)r2);
+                        const double Fr = dmul(ir, table_eval(sqrt_d((double)r2, ir), tab));
+                        fx = (Real)__fma_rn((double)dx, Fr, (double)fx);
+                        fy = (Real)__fma_rn((double)dy, Fr, (double)fy);
+                        fz = (Real)__fma_rn((double)dz, Fr, (double)fz);
                     }
                     return;
                 }
