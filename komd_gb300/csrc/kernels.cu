@@ -12,6 +12,7 @@
 #include <cfloat>
 #include <climits>
 #include <cstdint>
+#include <cstring>
 
 #include "engine.cuh"
 #include "kernels.cuh"
@@ -1025,135 +1026,169 @@ __device__ __forceinline__ void rdf_pair(const double *ca, const double *cb, Gri
     atomicAdd(&bins[b], 1.0);
 }
 
-// Cell path (max_r <= cell edge): one warp per home cell.  The molecules of the
-// 27 neighbour cells are staged in shared memory as FP32 COMs relative to the
-// home cell's centre (formed in FP64, then rounded); for each home molecule
-// the lanes test 32 staged molecules at a time against max_r with a 1e-4
-// relative margin and queue the hits, and the queued pairs take rdf_pair's
-// FP64 arithmetic, so the bin of every pair is the reference's.  The counts go
-// to a per-block shared histogram of integers (hist_smem) or straight to bins,
-// and the block adds its integer counts to bins at the end: the sums are
-// exact, whatever the order.
+// Cell path (max_r <= cell edge).  A block takes part of a home cell's
+// molecules: it stages the 27 neighbour cells' COMs in shared memory in FP32
+// relative to the home cell's centre (formed in FP64, then rounded); for each
+// home molecule a warp's lanes test 32 staged molecules at a time against
+// max_r with a margin and queue the hits of higher index -- the reference
+// counts ordered pairs, and (k, o) and (o, k) give the same bin exactly (the
+// differences are negatives, and rounding is symmetric), so each pair is
+// evaluated once and counted twice.  The queued pairs take rdf_pair_bin's FP64
+// arithmetic, whose bins are the reference's.  The counts go to a per-block
+// shared histogram of integers (hist_smem) or straight to bins, and the block
+// adds its integer counts to bins at the end: the sums are exact, whatever the
+// order.  The FP64 pipe bounds it: 32,000 molecules, max_r 2.5 and 100 bins,
+// 326 -> 135 us a sample (a warp per cell, ordered pairs, two divisions a pair).
 constexpr int kRdfWarps = 4;
-constexpr int kRdfStage = 320;
+constexpr int kRdfStage = 640;
 constexpr int kRdfSmemBins = 2048;   // with the staging arrays, under the 48 KB default
 
-__device__ __forceinline__ long long rdf_pair_bin(const double *ca, const double *cb, Grid g, double max_r, double dr,
-                                                  long long nbins) {
+// what a bin needs of the RDF's parameters; lo, up, top: the high words of
+// 0.4 L, 0.6 L and 1.4 L
+struct RdfArgs {
+    double max_r, dr, idr;
+    float pre2;
+    long long nbins;
+    int lo[3], up[3], top[3];
+};
+
+// the bin of a pair, or -1 beyond max_r: RDF_Kernel's arithmetic.  The minimum
+// image round(delta / L) is 0 below 0.4 L and +-1 between 0.6 L and 1.4 L,
+// whatever the quotient's rounding.  Away from the bin edges and max_r the bin
+// is read off sqrt(r2) / dr by a product with 1 / dr (both within 2e-15 of the
+// reference's values, the distance to the edges at least 1e-9 of a bin).  The
+// divisions and the square root of the reference run for the rest.
+__device__ __forceinline__ long long rdf_pair_bin(const double *ca, const double *cb, const Grid &g,
+                                                  const RdfArgs &a) {
     double q[3];
+#pragma unroll
     for (int d = 0; d < 3; d++) {
-        const double delta = dsub(ca[d], cb[d]);
-        // round(delta / L) is 0 for |delta| < 0.4 L whatever the quotient's rounding; the
-        // division runs only where the minimum image can move the pair
-        const double img = fabs(delta) < 0.4 * g.L[d] ? 0.0 : (double)(long long)round(ddiv(delta, g.L[d]));
-        q[d] = dsub(delta, dmul(g.L[d], img));
+        q[d] = dsub(ca[d], cb[d]);
+        const int hi = __double2hiint(q[d]) & 0x7fffffff;
+        if (hi >= a.lo[d]) {
+            if (hi > a.up[d] && hi < a.top[d]) {
+                q[d] = dsub(q[d], copysign(g.L[d], q[d]));
+            } else {
+                const double img = (double)(long long)round(ddiv(q[d], g.L[d]));
+                q[d] = dsub(q[d], dmul(g.L[d], img));
+            }
+        }
     }
-    const double rr = sqrt(dadd(dadd(dmul(q[0], q[0]), dmul(q[1], q[1])), dmul(q[2], q[2])));
-    if (rr > max_r) return -1;
-    unsigned long long b = (unsigned long long)ddiv(rr, dr);
-    if (b > (unsigned long long)(nbins - 1)) b = nbins - 1;
+    const double r2 = dadd(dadd(dmul(q[0], q[0]), dmul(q[1], q[1])), dmul(q[2], q[2]));
+    const double t = dmul(sqrt_d(r2, rsqrt_d(r2)), a.idr);
+    const int q0 = __double2int_rz(t);
+    const long long fr = __double_as_longlong(dsub(t, (double)q0));   // ordered as the value where positive
+    if (q0 >= 0 && q0 + 2 < a.nbins && q0 < 1000000 && fr > __double_as_longlong(1e-9) &&
+        fr < __double_as_longlong(1.0 - 1e-9))
+        return q0;   // below the last bin, so below max_r too
+    const double rr = sqrt(r2);
+    if (rr > a.max_r) return -1;
+    unsigned long long b = (unsigned long long)ddiv(rr, a.dr);
+    if (b > (unsigned long long)(a.nbins - 1)) b = a.nbins - 1;
     return (long long)b;
 }
 
 __global__ void __launch_bounds__(32 * kRdfWarps) k_rdf_cells(Grid g, const double *__restrict__ com,
                                                               const int *__restrict__ cell_mstart,
-                                                              const int *__restrict__ cell_mols, double max_r,
-                                                              double dr, long long nbins, bool hist_smem,
-                                                              double *bins) {
+                                                              const int *__restrict__ cell_mols, RdfArgs a,
+                                                              bool hist_smem, int split, double *bins) {
     extern __shared__ unsigned s_hist[];   // nbins counts when hist_smem
-    __shared__ float4 s_p[kRdfWarps][kRdfStage];
-    __shared__ int2 s_j[kRdfWarps][kRdfStage];   // molecule, neighbour-cell index
-    __shared__ double s_sh[kRdfWarps][27][3];
-    __shared__ int s_st[kRdfWarps][27], s_pre[kRdfWarps][28];
+    const long long nbins = a.nbins;
+    __shared__ float4 s_p[kRdfStage];      // home-cell coordinates, molecule
+    __shared__ double s_sh[27][3], s_ctr[3];
+    __shared__ int s_st[27], s_pre[28], s_im[27];
     __shared__ int s_q[kRdfWarps][64];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (hist_smem)
         for (int b = threadIdx.x; b < nbins; b += blockDim.x) s_hist[b] = 0u;
-    __syncthreads();
-    const int cell = blockIdx.x * kRdfWarps + w;
-    if (cell < g.ncell) {
-        unsigned lt;
-        asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-        int cx, cy, cz;
+    const int cell = blockIdx.x / split, part = blockIdx.x - cell * split;
+    unsigned lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    if (w == 0) {
+        int cx, cy, cz, cnt = 0;
         cell_coords(g, cell, cx, cy, cz);
-        const double ctr[3] = {cell_centre(g, 0, cx), cell_centre(g, 1, cy), cell_centre(g, 2, cz)};
-        int cnt = 0;
         if (lane < 27) {
             const NbCell q = neighbour_cell(g, cx, cy, cz, lane);
             const int s0 = cell_mstart[q.cell];
             cnt = cell_mstart[q.cell + 1] - s0;
-            s_st[w][lane] = s0;
-            for (int d = 0; d < 3; d++) s_sh[w][lane][d] = q.shift[d];
+            s_st[lane] = s0;
+            s_im[lane] = q.crosses;
+            for (int d = 0; d < 3; d++) s_sh[lane][d] = q.shift[d];
         }
         int inc = cnt;
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += y;
         }
-        if (lane < 27) s_pre[w][lane] = inc - cnt;
-        const int total = __shfl_sync(0xffffffffu, inc, 26);
-        if (lane == 0) s_pre[w][27] = total;
-        __syncwarp();
-        const int hs = s_st[w][13], hn = s_pre[w][14] - s_pre[w][13];
-        const float pre2 = (float)(max_r * max_r * (1.0 + 1e-4));
-        auto rel = [&](int o, int nb) {   // FP32 COM relative to the home centre, through the periodic shift
-            const double *c = com + 3 * (size_t)o;
-            return make_float4((float)dsub(dadd(c[0], s_sh[w][nb][0]), ctr[0]),
-                               (float)dsub(dadd(c[1], s_sh[w][nb][1]), ctr[1]),
-                               (float)dsub(dadd(c[2], s_sh[w][nb][2]), ctr[2]), 0.f);
-        };
-        for (int sb = 0; sb < total; sb += kRdfStage) {
-            const int ns = min(kRdfStage, total - sb);
-            __syncwarp();
-            for (int t = lane; t < ns; t += 32) {
-                const int gi = sb + t;
-                int a = 0, b = 27;
-                while (b - a > 1) {
-                    const int mid = (a + b) >> 1;
-                    if (s_pre[w][mid] <= gi) a = mid;
-                    else b = mid;
+        if (lane < 27) s_pre[lane] = inc - cnt;
+        if (lane == 26) s_pre[27] = inc;
+        if (lane < 3) s_ctr[lane] = cell_centre(g, lane, lane == 0 ? cx : (lane == 1 ? cy : cz));
+    }
+    __syncthreads();
+    const int hs = s_st[13], hn = s_pre[14] - s_pre[13];
+    const int total = part * kRdfWarps < hn ? s_pre[27] : 0;
+    const double ctr[3] = {s_ctr[0], s_ctr[1], s_ctr[2]};
+    auto rel = [&](int o, int nb) {   // FP32 COM relative to the home centre, through the periodic shift
+        const double *c = com + 3 * (size_t)o;
+        double x = c[0], y = c[1], z = c[2];
+        if (s_im[nb]) {
+            x = dadd(x, s_sh[nb][0]);
+            y = dadd(y, s_sh[nb][1]);
+            z = dadd(z, s_sh[nb][2]);
+        }
+        return make_float4(d2f_rn(dsub(x, ctr[0])), d2f_rn(dsub(y, ctr[1])), d2f_rn(dsub(z, ctr[2])),
+                           __int_as_float(o));
+    };
+    for (int sb = 0; sb < total; sb += kRdfStage) {
+        const int ns = min(kRdfStage, total - sb);
+        if (sb > 0) __syncthreads();
+        for (int t = threadIdx.x; t < ns; t += blockDim.x) {
+            const int gi = sb + t;
+            int nb = 0, e = 27;
+            while (e - nb > 1) {
+                const int mid = (nb + e) >> 1;
+                if (s_pre[mid] <= gi) nb = mid;
+                else e = mid;
+            }
+            s_p[t] = rel(cell_mols[s_st[nb] + (gi - s_pre[nb])], nb);
+        }
+        __syncthreads();
+        for (int h = part * kRdfWarps + w; h < hn; h += split * kRdfWarps) {
+            const int k = cell_mols[hs + h];
+            const float4 hp = rel(k, 13);
+            auto count = [&](int c) {
+                if (c < 0) return;
+                const long long b = rdf_pair_bin(com + 3 * (size_t)k, com + 3 * (size_t)__float_as_int(s_p[c].w), g,
+                                                 a);
+                if (b < 0) return;
+                if (hist_smem) atomicAdd(&s_hist[b], 2u);
+                else atomicAdd(&bins[b], 2.0);
+            };
+            int qn = 0;
+            for (int c0 = 0; c0 < ns; c0 += 32) {
+                const int c = c0 + lane;
+                bool hit = false;
+                if (c < ns) {
+                    const float4 pj = s_p[c];
+                    const float dx = hp.x - pj.x, dy = hp.y - pj.y, dz = hp.z - pj.z;
+                    hit = __float_as_int(pj.w) > k && dx * dx + dy * dy + dz * dz <= a.pre2;
                 }
-                const int o = cell_mols[s_st[w][a] + (gi - s_pre[w][a])];
-                s_p[w][t] = rel(o, a);
-                s_j[w][t] = make_int2(o, a);
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                if (hit) s_q[w][qn + __popc(m & lt)] = c;
+                qn += __popc(m);
+                if (qn >= 32) {
+                    __syncwarp();
+                    const int c1 = s_q[w][lane], c2 = s_q[w][32 + lane];
+                    __syncwarp();
+                    qn -= 32;
+                    if (lane < qn) s_q[w][lane] = c2;
+                    __syncwarp();
+                    count(c1);
+                }
             }
             __syncwarp();
-            for (int h = 0; h < hn; h++) {
-                const int k = cell_mols[hs + h];
-                const float4 hp = rel(k, 13);
-                auto count = [&](int c) {
-                    if (c < 0) return;
-                    const long long b = rdf_pair_bin(com + 3 * (size_t)k, com + 3 * (size_t)s_j[w][c].x, g, max_r, dr,
-                                                     nbins);
-                    if (b < 0) return;
-                    if (hist_smem) atomicAdd(&s_hist[b], 1u);
-                    else atomicAdd(&bins[b], 1.0);
-                };
-                int qn = 0;
-                for (int c0 = 0; c0 < ns; c0 += 32) {
-                    const int c = c0 + lane;
-                    bool hit = false;
-                    if (c < ns && s_j[w][c].x != k) {
-                        const float4 pj = s_p[w][c];
-                        const float dx = hp.x - pj.x, dy = hp.y - pj.y, dz = hp.z - pj.z;
-                        hit = dx * dx + dy * dy + dz * dz <= pre2;
-                    }
-                    const unsigned m = __ballot_sync(0xffffffffu, hit);
-                    if (hit) s_q[w][qn + __popc(m & lt)] = c;
-                    qn += __popc(m);
-                    if (qn >= 32) {
-                        __syncwarp();
-                        count(s_q[w][lane]);
-                        __syncwarp();
-                        qn -= 32;
-                        if (lane < qn) s_q[w][lane] = s_q[w][32 + lane];
-                        __syncwarp();
-                    }
-                }
-                __syncwarp();
-                count(lane < qn ? s_q[w][lane] : -1);
-                __syncwarp();
-            }
+            count(lane < qn ? s_q[w][lane] : -1);
+            __syncwarp();
         }
     }
     if (hist_smem) {
@@ -1605,8 +1640,22 @@ void launch_rdf(Engine &e, cudaStream_t st, double *bins, bool cells) {
 void launch_rdf_bins(Engine &e, cudaStream_t st, double *bins, bool cells, double max_r, double dr, int64_t nbins) {
     if (cells) {
         const bool hist_smem = nbins <= kRdfSmemBins;
-        k_rdf_cells<<<nblk(e.g.ncell, kRdfWarps), 32 * kRdfWarps, hist_smem ? sizeof(unsigned) * nbins : 0, st>>>(
-            e.g, e.com, e.cell_mstart, e.cell_mols, max_r, dr, nbins, hist_smem, bins);
+        // parts of a cell's molecules where there are few cells, as in pair_cell.cu
+        const int most = std::max(1, (int)((double)e.n_mol / e.g.ncell / kRdfWarps + 0.999));
+        const int split = std::max(1, std::min(most, (e.num_sms * 8 + e.g.ncell - 1) / e.g.ncell));
+        RdfArgs a{max_r, dr, 1.0 / dr, pair_pre2(e.g, max_r * max_r), nbins, {0}, {0}, {0}};
+        auto high = [](double x) {
+            uint64_t b;
+            std::memcpy(&b, &x, sizeof(b));
+            return (int)(b >> 32);
+        };
+        for (int d = 0; d < 3; d++) {
+            a.lo[d] = high(0.4 * e.g.L[d]);
+            a.up[d] = high(0.6 * e.g.L[d]);
+            a.top[d] = high(1.4 * e.g.L[d]);
+        }
+        k_rdf_cells<<<e.g.ncell * split, 32 * kRdfWarps, hist_smem ? sizeof(unsigned) * nbins : 0, st>>>(
+            e.g, e.com, e.cell_mstart, e.cell_mols, a, hist_smem, split, bins);
     }
     else
         k_rdf_all<<<nblk(e.n_mol, 128), 128, 0, st>>>(e.g, (int)e.n_mol, e.com, max_r, dr, nbins, bins);

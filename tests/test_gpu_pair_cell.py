@@ -112,3 +112,29 @@ def test_verlet_list_forces_match_oracle(oracle_lib, form):
     sim.update_container()
     sim.forces()
     assert rel_rmse(f, sim.f) < 1e-5
+
+
+@pytest.mark.parametrize("nbins", [7, 250, 3001])
+@pytest.mark.parametrize("form", ["sparse", "liquid", "crowded", "molecules"])
+def test_rdf_counts_are_exact(form, nbins):
+    """The cell path of the RDF against the reference's arithmetic on every
+    ordered pair of centres: few and many bins (shared and global counts; 7
+    does not divide max_r evenly), some staging rounds, parts of cells."""
+    from komd_gb300 import gpu
+    s, cell = _system(form)
+    max_r, mol = 2.4, np.searchsorted(np.unique(s.mol_id), s.mol_id)
+    L = s.high - s.low
+    g = gpu.GpuSystem(s, gpu.make_config(s.low, s.high, cell, cutoff=2.4, terms=gpu.TERM_LJ))
+    g.update_container()
+    got = g.rdf_profile(max_r, nbins)
+    r = g.download()[0]
+    g.close()
+    com = np.stack([np.bincount(mol, r[:, d]) for d in range(3)], 1) / np.bincount(mol)[:, None]
+    dr, expect = max_r / nbins, np.zeros(nbins)
+    for k in range(com.shape[0]):
+        q = com[k] - com
+        q -= L * np.round(q / L)
+        rr = np.sqrt((q[:, 0] * q[:, 0] + q[:, 1] * q[:, 1]) + q[:, 2] * q[:, 2])
+        rr = np.delete(rr, k)
+        np.add.at(expect, np.minimum((rr[rr <= max_r] / dr).astype(np.int64), nbins - 1), 1.0)
+    assert np.array_equal(got, expect)
