@@ -193,14 +193,16 @@ bool surrogate_on(komd_gpu *h) {
     return (h->e.cfg.terms & KOMD_TERM_ATM_SURROGATE) && h->sur.loaded && !h->sur.fallback;
 }
 
-// surrogate three-body forces: into f (fout == nullptr) or written to fout
-void enqueue_surrogate(komd_gpu *h, double *fout) {
+// surrogate three-body forces: into f (fout == nullptr), with integrate1 of the
+// step (with_step1), or written to fout
+void enqueue_surrogate(komd_gpu *h, double *fout, bool with_step1 = false) {
     Engine &e = h->e;
     SurParams p = sur_params(h);
     launch_sur_desc(p, e.stream);
     launch_sur_mlp(p, e.stream);
     launch_sur_force(p, e.stream);
-    launch_sur_apply(p, e.slot_site, e.f, fout, e.stream);
+    if (with_step1) launch_sur_apply_step1(p, e, e.stream);
+    else launch_sur_apply(p, e.slot_site, e.f, fout, e.stream);
 }
 
 bool fused_lj_atm(komd_gpu *h, bool measure) {
@@ -248,7 +250,8 @@ bool enqueue_forces(komd_gpu *h, bool measure, double *lj_hist, bool with_step1 
     if (surrogate_on(h)) {
         {
             ProfScope ps(h, F_SURROGATE);
-            enqueue_surrogate(h, nullptr);
+            enqueue_surrogate(h, nullptr, with_step1);
+            fused = with_step1;
         }
         if (measure) launch_sum_sites((int)e.n, h->sur.esite, h->acc + R_UATM, st);
     } else if (e.cfg.terms & KOMD_TERM_ATM) {

@@ -78,6 +78,8 @@ void launch_sur_desc(SurParams &p, cudaStream_t st);
 void launch_sur_mlp(SurParams &p, cudaStream_t st);
 void launch_sur_force(SurParams &p, cudaStream_t st);
 void launch_sur_apply(SurParams &p, const int *slot_site, double *f, double *fout, cudaStream_t st);
+struct Engine;
+void launch_sur_apply_step1(SurParams &p, const Engine &e, cudaStream_t st);
 void launch_sur_probe(int n, const double *fa, const double *fb, double *out2, cudaStream_t st);
 void launch_sum_sites(int n, const float *e, double *out, cudaStream_t st);
 void launch_train_step(TrainParams &t, int step, cudaStream_t st);
