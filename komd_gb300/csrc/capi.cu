@@ -1684,7 +1684,7 @@ int komd_sur_fit_grad(komd_sur_data *d, const float *params, const float *fmean,
     CK(cudaMemcpy(b.snaps, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice));
     CK(cudaMemset(b.fs, 0, sizeof(float) * 3 * (size_t)p.nb));
     CK(cudaMemset(b.grad, 0, sizeof(float) * kSurNParam));
-    launch_fit_step(p, b.grad, nullptr);
+    launch_fit_step(p, b.grad, true, nullptr);
     rc = check_launch("sur_fit_grad");
     if (rc) return rc;
     CK(cudaMemcpy(grad, b.grad, sizeof(float) * kSurNParam, cudaMemcpyDeviceToHost));
@@ -1716,10 +1716,11 @@ int komd_sur_fit(komd_sur_data *d, float *params, const float *fmean, const floa
         for (int64_t k = 0; k < per_epoch; k++, step++) {
             p.snaps = b.snaps + k * bs;
             const float lr = o->lr * std::pow(o->lr_end / o->lr, total > 1 ? (float)step / (float)(total - 1) : 0.f);
-            CK(cudaMemsetAsync(b.fs, 0, sizeof(float) * 3 * (size_t)p.nb, nullptr));
-            CK(cudaMemsetAsync(b.grad, 0, sizeof(float) * kSurNParam, nullptr));
-            launch_fit_step(p, b.grad, nullptr);
-            launch_fit_adam(b.params, b.grad, b.m, b.v, lr, (int)step, nullptr);
+            // Adam leaves the gradient zero and the fragments packed, the tensor-core form fs zero
+            if (step == 0) CK(cudaMemsetAsync(b.grad, 0, sizeof(float) * kSurNParam, nullptr));
+            if (step == 0 || !p.tc) CK(cudaMemsetAsync(b.fs, 0, sizeof(float) * 3 * (size_t)p.nb, nullptr));
+            launch_fit_step(p, b.grad, step == 0, nullptr);
+            launch_fit_adam(p, b.params, b.grad, b.m, b.v, lr, (int)step, nullptr);
         }
         rc = check_launch("sur_fit");
         if (rc) return rc;

@@ -171,17 +171,32 @@ __device__ __forceinline__ float sym_dot(const float *A, const float *B) {
 // residual, force loss and the adjoint w (warp per batch site)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_fit_adjoint(FitParams p) {
+    __shared__ double s_loss[8];
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.x * 8 + (threadIdx.x >> 5);
+    // the block's force loss in one atomic (one a site queued up on the one address)
+    if (lane == 0) {
+        double le = 0.0;
+        if (b < p.nb) {
+            const size_t gs = fit_site(p, b);
+            float dF[3];
+            for (int d = 0; d < 3; d++) dF[d] = p.fs[3 * b + d] - p.f3[3 * gs + d];
+            le = (double)(p.lam_f * p.inv_f2 * (dF[0] * dF[0] + dF[1] * dF[1] + dF[2] * dF[2]) / (float)p.nb);
+        }
+        s_loss[threadIdx.x >> 5] = le;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double le = 0.0;
+        for (int w = 0; w < 8; w++) le += s_loss[w];
+        atomicAdd(&p.loss[1], le);
+    }
     if (b >= p.nb) return;
     const size_t gs = fit_site(p, b);
     const size_t gbase = gs - (size_t)(b % p.n_site);
     const int base = (b / p.n_site) * p.n_site;
     float dFi[3];
     for (int d = 0; d < 3; d++) dFi[d] = p.fs[3 * b + d] - p.f3[3 * gs + d];
-    if (lane == 0)
-        atomicAdd(&p.loss[1], (double)(p.lam_f * p.inv_f2 * (dFi[0] * dFi[0] + dFi[1] * dFi[1] + dFi[2] * dFi[2]) /
-                                       (float)p.nb));
     float acc[kSurNR + kSurNC * 9];      // directional derivatives: radial (16), per channel dM1 (3) + dM2 (6)
 #pragma unroll
     for (int k = 0; k < kSurNR + kSurNC * 9; k++) acc[k] = 0.f;
@@ -363,15 +378,46 @@ __global__ void __launch_bounds__(128) k_fit_grad(const float *__restrict__ rec,
     atomicAdd(&grad[q], s);
 }
 
-__global__ void k_fit_adam(float *params, const float *__restrict__ grad, float *m, float *v, float lr, int step) {
+namespace {
+// FitParams::wf: W1, W1^T, W2, W2^T as the N x K matrices of load_frag
+constexpr int kWfW1 = 0, kWfW1T = kSurH * kSurNF, kWfW2 = 2 * kSurH * kSurNF, kWfW2T = kWfW2 + kSurH * kSurH;
+static_assert(kWfW2T + kSurH * kSurH == kFitWf, "fragment buffer");
+// place of element (n, k) of an N x K matrix in the B-fragment order of load_frag:
+// ((t S + s) 32 + lane) 4 + j with n = 8t + lane/4, k = 16s + 2(lane%4) + (j%2) + 8(j/2)
+__device__ __forceinline__ int wf_at(int n, int k, int K) {
+    const int kk = k & 15, lane = ((n & 7) << 2) | ((kk & 7) >> 1), j = (kk & 1) | ((kk >> 3) << 1);
+    return ((((n >> 3) * (K / 16) + (k >> 4)) * 32 + lane) << 2) + j;
+}
+// parameter q in BF16 in the fragment buffers that hold it (a weight and its transpose)
+__device__ __forceinline__ void wf_put(__nv_bfloat16 *wf, int q, float v) {
+    const __nv_bfloat16 h = __float2bfloat16(v);
+    if (q >= kOW1 && q < kOW1 + kSurH * kSurNF) {
+        const int o = (q - kOW1) / kSurNF, k = (q - kOW1) % kSurNF;
+        wf[kWfW1 + wf_at(o, k, kSurNF)] = h;
+        wf[kWfW1T + wf_at(k, o, kSurH)] = h;
+    } else if (q >= kOW2 && q < kOW2 + kSurH * kSurH) {
+        const int o = (q - kOW2) / kSurH, k = (q - kOW2) % kSurH;
+        wf[kWfW2 + wf_at(o, k, kSurH)] = h;
+        wf[kWfW2T + wf_at(k, o, kSurH)] = h;
+    }
+}
+}  // namespace
+
+// one Adam step; the gradient is zeroed for the next, and (wf) the new weights
+// go to the BF16 fragment buffers of the next step's network kernels
+__global__ void k_fit_adam(float *params, float *__restrict__ grad, float *m, float *v, float lr, int step,
+                           __nv_bfloat16 *__restrict__ wf) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= kSurNParam) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float g = grad[q];
+    grad[q] = 0.f;
     const float mq = m[q] = b1 * m[q] + (1.f - b1) * g;
     const float vq = v[q] = b2 * v[q] + (1.f - b2) * g * g;
     const float mh = mq / (1.f - powf(b1, (float)(step + 1))), vh = vq / (1.f - powf(b2, (float)(step + 1)));
-    params[q] -= lr * mh / (sqrtf(vh) + eps);
+    const float pq = params[q] - lr * mh / (sqrtf(vh) + eps);
+    params[q] = pq;
+    if (wf) wf_put(wf, q, pq);
 }
 
 
@@ -379,9 +425,6 @@ __global__ void k_fit_adam(float *params, const float *__restrict__ grad, float 
 // tensor-core form
 // ===========================================================================
 namespace {
-// FitParams::wf: W1, W1^T, W2, W2^T as the N x K matrices of load_frag
-constexpr int kWfW1 = 0, kWfW1T = kSurH * kSurNF, kWfW2 = 2 * kSurH * kSurNF, kWfW2T = kWfW2 + kSurH * kSurH;
-static_assert(kWfW2T + kSurH * kSurH == kFitWf, "fragment buffer");
 // BF16 record of one batch site (tensor-core form), element offsets:
 //   left factors  Z1B | ZD1B (dW1), Z2B | ZD2B (dW2)
 //   right factors X | W (dW1),  H1 | HD1 (dW2)
@@ -391,25 +434,10 @@ constexpr int kGradChunk = 32;            // batch sites per shared-memory stage
 constexpr int kRecPad = kRecTc + 8;       // 912-byte rows: the 8 rows of an ldmatrix hit distinct banks
 }  // namespace
 
-// the weight matrices of the parameters, rounded to BF16, in the B-fragment
-// order of load_frag (element (n, k) of an N x K matrix at
-// ((t S + s) 32 + lane) 4 + j with n = 8t + lane/4, k = 16s + 2(lane%4) + (j%2) + 8(j/2))
+// the weight matrices of the parameters, rounded to BF16, in fragment order
 __global__ void k_fit_pack(const float *__restrict__ params, __nv_bfloat16 *__restrict__ wf) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= kFitWf) return;
-    const int which = e < kWfW1T ? 0 : e < kWfW2 ? 1 : e < kWfW2T ? 2 : 3;
-    const int base = which == 0 ? kWfW1 : which == 1 ? kWfW1T : which == 2 ? kWfW2 : kWfW2T;
-    const int K = which == 0 ? kSurNF : kSurH;
-    const int q = e - base, j = q & 3, chunk = q >> 2, lane = chunk & 31, ts = chunk >> 5;
-    const int S = K / 16, s = ts % S, t = ts / S;
-    const int n = 8 * t + (lane >> 2), k = 16 * s + 2 * (lane & 3) + (j & 1) + 8 * (j >> 1);
-    const float *W1 = params + kOW1, *W2 = params + kOW2;
-    float v;
-    if (which == 0) v = W1[n * kSurNF + k];        // W1 (64 x 32)
-    else if (which == 1) v = W1[k * kSurNF + n];   // W1^T (32 x 64)
-    else if (which == 2) v = W2[n * kSurH + k];    // W2
-    else v = W2[k * kSurH + n];                    // W2^T
-    wf[e] = __float2bfloat16(v);
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < kSurNParam) wf_put(wf, q, params[q]);
 }
 
 // shared-memory copy of the BF16 weights and the FP32 biases (every block of
@@ -433,17 +461,24 @@ __device__ __forceinline__ float fit_target(const FitParams &p, int b) {
 // forward + input gradient of 16 batch sites per warp on the tensor cores:
 // the tile's standardised features go to their g rows, which sur_mlp_tile
 // overwrites with dE/dx
-__global__ void __launch_bounds__(128) k_fit_fwd_tc(FitParams p) {
+__global__ void __launch_bounds__(128) k_fit_fwd_tc(FitParams p, int tpb) {
     __shared__ __align__(16) FitSmemW sw;
+    const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3, w = threadIdx.x >> 5;
+    const int b0 = (blockIdx.x * tpb + w) * 16;
+    const bool mine = w < tpb && b0 < p.nb;
+    static_assert(kSurNF == 32, "a feature per lane");
+    float xr[16];   // the tile's features, all rows in flight beside the weights' staging
+    if (mine)
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            xr[u] = p.x[fit_site(p, min(b0 + u, p.nb - 1)) * kSurNF + lane];
     const SurW W = fit_stage(p, sw);
-    const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int b0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 16;
     float le = 0.f;
-    if (b0 < p.nb) {
-        for (int q = lane; q < 16 * kSurNF; q += 32) {
-            const int b = b0 + q / kSurNF, k = q % kSurNF;
-            if (b < p.nb) p.g[(size_t)b * kSurNF + k] = (p.x[fit_site(p, b) * kSurNF + k] - p.fmean[k]) / p.fstd[k];
-        }
+    if (mine) {
+        const float mean = p.fmean[lane], std = p.fstd[lane];
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            if (b0 + u < p.nb) p.g[(size_t)(b0 + u) * kSurNF + lane] = (xr[u] - mean) / std;
         __syncwarp();
         const int r0 = b0 + g, r1 = r0 + 8;
         const bool v0 = r0 < p.nb, v1 = r1 < p.nb;
@@ -486,12 +521,14 @@ __device__ __forceinline__ void st_bf16x2(__nv_bfloat16 *dst, uint32_t v) { *rei
 // tensor cores (the algebra of k_fit_bwd): the BF16 left and right factors of
 // the weight gradients go to the records, and the gradients of the biases,
 // the output weights and the output bias (column sums) straight into grad
-__global__ void __launch_bounds__(128) k_fit_bwd_tc(FitParams p, float *grad) {
+__global__ void __launch_bounds__(128) k_fit_bwd_tc(FitParams p, float *grad, int tpb) {
     __shared__ __align__(16) FitSmemW sw;
     const SurW W = fit_stage(p, sw);
     const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int b0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 16;
-    if (b0 >= p.nb) return;
+    const int b0 = (blockIdx.x * tpb + (threadIdx.x >> 5)) * 16;
+    if ((threadIdx.x >> 5) >= tpb || b0 >= p.nb) return;
+    for (int q = lane; q < 48; q += 32)   // the learned forces are read: zero for the next step
+        if (3 * b0 + q < 3 * p.nb) p.fs[3 * (size_t)b0 + q] = 0.f;
     const int r0 = b0 + g, r1 = r0 + 8;
     const bool v0 = r0 < p.nb, v1 = r1 < p.nb;
     const size_t s0 = v0 ? fit_site(p, r0) : 0, s1 = v1 ? fit_site(p, r1) : 0;
@@ -499,10 +536,9 @@ __global__ void __launch_bounds__(128) k_fit_bwd_tc(FitParams p, float *grad) {
     __nv_bfloat16 *q0 = rec + (size_t)(v0 ? r0 : 0) * kRecTc, *q1 = rec + (size_t)(v1 ? r1 : 0) * kRecTc;
     // A fragments of the standardised features and of the tangent w
     uint32_t ax[2][4], aw[2][4];
+    float xs[2][2][4], ws[2][2][4];   // [s][row][k, k + 1, k + 8, k + 9], every load before the first store
 #pragma unroll
-    for (int s = 0; s < 2; s++) {
-        const int k = 16 * s + tig * 2;
-        float x[2][4], w[2][4];   // [row][k, k + 1, k + 8, k + 9]
+    for (int s = 0; s < 2; s++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const bool v = h ? v1 : v0;
@@ -510,11 +546,15 @@ __global__ void __launch_bounds__(128) k_fit_bwd_tc(FitParams p, float *grad) {
             const int b = h ? r1 : r0;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int kk = k + (u & 1) + 8 * (u >> 1);
-                x[h][u] = v ? (p.x[gs * kSurNF + kk] - p.fmean[kk]) / p.fstd[kk] : 0.f;
-                w[h][u] = v ? p.w[(size_t)b * kSurNF + kk] : 0.f;
+                const int kk = 16 * s + tig * 2 + (u & 1) + 8 * (u >> 1);
+                xs[s][h][u] = v ? (p.x[gs * kSurNF + kk] - p.fmean[kk]) / p.fstd[kk] : 0.f;
+                ws[s][h][u] = v ? p.w[(size_t)b * kSurNF + kk] : 0.f;
             }
         }
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        const int k = 16 * s + tig * 2;
+        const float (*x)[4] = xs[s], (*w)[4] = ws[s];
         ax[s][0] = pack_bf16(x[0][0], x[0][1]);
         ax[s][1] = pack_bf16(x[1][0], x[1][1]);
         ax[s][2] = pack_bf16(x[0][2], x[0][3]);
@@ -776,16 +816,24 @@ void launch_fit_capture(int n, const float4 *nl, const int *nl_count, int nl_cap
                                                dcount, dcap, dx, dmom, de3, df3, dsite, err);
 }
 
-// fs (nb x 3) and grad (kSurNParam) must be zero on entry
-void launch_fit_step(FitParams &p, float *grad, cudaStream_t st) {
+// warps of a block with a 16-site tile of their own: all four where the tiles
+// fill the chip that way, else one tile per block, so that a small batch spreads
+// over the SMs (the other warps help to stage the weights).  At 2,000 batch
+// sites (125 tiles) k_fit_fwd_tc took 18.5 us on 32 blocks with a dependent
+// load per feature row, 9.5 us with a tile per block and the rows in flight.
+static int fit_tiles_per_block(int tiles) { return std::max(1, std::min(4, tiles / 304)); }
+
+// fs (nb x 3) and grad (kSurNParam) must be zero on entry; the tensor-core form
+// leaves fs zero.  pack: the weights' fragment buffer is not up to date
+void launch_fit_step(FitParams &p, float *grad, bool pack, cudaStream_t st) {
     if (p.tc) {
-        const int tiles = (p.nb + 15) / 16;
+        const int tiles = (p.nb + 15) / 16, tpb = fit_tiles_per_block(tiles);
         const int chunks = (p.nb + kGradChunk - 1) / kGradChunk;
-        k_fit_pack<<<(kFitWf + 255) / 256, 256, 0, st>>>(p.params, p.wf);
-        k_fit_fwd_tc<<<(tiles + 3) / 4, 128, 0, st>>>(p);
+        if (pack) k_fit_pack<<<(kSurNParam + 255) / 256, 256, 0, st>>>(p.params, p.wf);
+        k_fit_fwd_tc<<<(tiles + tpb - 1) / tpb, 128, 0, st>>>(p, tpb);
         k_fit_force<<<(p.nb + 7) / 8, 256, 0, st>>>(p);
         k_fit_adjoint<<<(p.nb + 7) / 8, 256, 0, st>>>(p);
-        k_fit_bwd_tc<<<(tiles + 3) / 4, 128, 0, st>>>(p, grad);
+        k_fit_bwd_tc<<<(tiles + tpb - 1) / tpb, 128, 0, st>>>(p, grad, tpb);
         k_fit_grad_tc<<<chunks < 256 ? chunks : 256, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16 *>(p.rec),
                                                                    p.nb, grad);
         return;
@@ -797,8 +845,9 @@ void launch_fit_step(FitParams &p, float *grad, cudaStream_t st) {
     k_fit_grad<<<dim3((kSurNParam + 127) / 128, (p.nb + 255) / 256), 128, 0, st>>>(p.rec, p.nb, grad);
 }
 
-void launch_fit_adam(float *params, const float *grad, float *m, float *v, float lr, int step, cudaStream_t st) {
-    k_fit_adam<<<(kSurNParam + 127) / 128, 128, 0, st>>>(params, grad, m, v, lr, step);
+void launch_fit_adam(const FitParams &p, float *params, float *grad, float *m, float *v, float lr, int step,
+                     cudaStream_t st) {
+    k_fit_adam<<<(kSurNParam + 127) / 128, 128, 0, st>>>(params, grad, m, v, lr, step, p.tc ? p.wf : nullptr);
 }
 
 }  // namespace komd

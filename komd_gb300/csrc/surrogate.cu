@@ -99,24 +99,86 @@ __global__ void __launch_bounds__(128) k_sur_desc(SurParams p) {
     // this lane's features: radials 4c .. 4c + 3 and the channel's four invariants
     float raw[8] = {tot[0], tot[1], tot[2], tot[3], v[0] * v[0] + v[1] * v[1] + v[2] * v[2], i2,
                     v[0] * Mv[0] + v[1] * Mv[1] + v[2] * Mv[2], i4};
-    if (p.fstd) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int f = k < 4 ? 4 * c4 + k : kSurNR + 4 * (k - 4) + c4;
-            raw[k] = (raw[k] - p.fmean[f]) / p.fstd[f];
-        }
+    for (int k = 0; k < 8; k++) {
+        const int f = k < 4 ? 4 * c4 + k : kSurNR + 4 * (k - 4) + c4;
+        raw[k] = (raw[k] - p.fmean[f]) / p.fstd[f];
     }
     float *xo = p.x + (size_t)i * kSurNF;
     reinterpret_cast<float4 *>(xo)[c4] = make_float4(raw[0], raw[1], raw[2], raw[3]);
 #pragma unroll
     for (int k = 0; k < 4; k++) xo[kSurNR + kSurNC * k + c4] = raw[4 + k];
-    if (p.mom) {
-        float *mo = p.mom + (size_t)i * kSurNC * 9 + 9 * c4;
+    float *mo = p.mom + (size_t)i * kSurNC * 9 + 9 * c4;
 #pragma unroll
-        for (int k = 0; k < 9; k++) mo[k] = tot[4 + k];
-    }
+    for (int k = 0; k < 9; k++) mo[k] = tot[4 + k];
 }
 
+// raw features and moments of a training sample: one thread per slot, the sums
+// in the row's order.  Samples are rare, and training rounds the features to
+// BF16, which turns a change in a sum's last bit into one of 2^-9: their order
+// stays as datasets and fits were made with it.
+__global__ void __launch_bounds__(128) k_sur_sample(SurParams p) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= p.n) return;
+    float *xo = p.x + (size_t)i * kSurNF, *mo = p.mom ? p.mom + (size_t)i * kSurNC * 9 : nullptr;
+    const int ni = min(p.nl_count[i], p.nl_cap);
+    float acc[kSurNR + kSurNC * 9];   // G (16), then per channel M1 (3) + M2 (6: xx xy xz yy yz zz)
+#pragma unroll
+    for (int k = 0; k < kSurNR + kSurNC * 9; k++) acc[k] = 0.f;
+    const float4 *row = p.nl + (size_t)i * p.nl_cap;
+    for (int k = 0; k < ni; k++) {
+        SurNb q;
+        if (!sur_nb(row[k], p.rc, q)) continue;
+        float G[kSurNR];
+        radial_basis(q.r, q.fc, 0.f, G, nullptr);
+#pragma unroll
+        for (int c = 0; c < kSurNR; c++) acc[c] += G[c];
+#pragma unroll
+        for (int c = 0; c < kSurNC; c++) {
+            const float t = q.r - sur_mu_a(c);
+            const float g = __expf(-kSurEtaA * t * t) * q.fc;
+            float *m = acc + kSurNR + 9 * c;
+            const float gx = g * q.u[0], gy = g * q.u[1], gz = g * q.u[2];
+            m[0] += gx; m[1] += gy; m[2] += gz;
+            m[3] += gx * q.u[0]; m[4] += gx * q.u[1]; m[5] += gx * q.u[2];
+            m[6] += gy * q.u[1]; m[7] += gy * q.u[2]; m[8] += gz * q.u[2];
+        }
+    }
+    float raw[kSurNF];
+#pragma unroll
+    for (int k = 0; k < kSurNR; k++) raw[k] = acc[k];
+#pragma unroll
+    for (int c = 0; c < kSurNC; c++) {
+        const float *v = acc + kSurNR + 9 * c, *m = v + 3;
+        float M[3][3], Mv[3], M2[3][3];
+        sym_full(m, M);
+#pragma unroll
+        for (int x = 0; x < 3; x++) Mv[x] = M[x][0] * v[0] + M[x][1] * v[1] + M[x][2] * v[2];
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+#pragma unroll
+            for (int y = 0; y < 3; y++) M2[x][y] = M[x][0] * M[0][y] + M[x][1] * M[1][y] + M[x][2] * M[2][y];
+        float i2 = 0.f, i4 = 0.f;
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+#pragma unroll
+            for (int y = 0; y < 3; y++) { i2 += M[x][y] * M[x][y]; i4 += M2[x][y] * M[y][x]; }
+        raw[kSurNR + c] = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+        raw[kSurNR + kSurNC + c] = i2;
+        raw[kSurNR + 2 * kSurNC + c] = v[0] * Mv[0] + v[1] * Mv[1] + v[2] * Mv[2];
+        raw[kSurNR + 3 * kSurNC + c] = i4;
+    }
+    float4 *x4 = reinterpret_cast<float4 *>(xo);
+#pragma unroll
+    for (int k = 0; k < kSurNF / 4; k++) x4[k] = make_float4(raw[4 * k], raw[4 * k + 1], raw[4 * k + 2], raw[4 * k + 3]);
+    if (mo) {
+        float4 *m4 = reinterpret_cast<float4 *>(mo);
+#pragma unroll
+        for (int k = 0; k < kSurNC * 9 / 4; k++)
+            m4[k] = make_float4(acc[kSurNR + 4 * k], acc[kSurNR + 4 * k + 1], acc[kSurNR + 4 * k + 2],
+                                acc[kSurNR + 4 * k + 3]);
+    }
+}
 
 __device__ __forceinline__ void sur_stage_weights(const SurParams &p, __nv_bfloat16 *sW1, __nv_bfloat16 *sW1T,
                                                   __nv_bfloat16 *sW2, __nv_bfloat16 *sW2T, float *sb1, float *sb2,
@@ -379,7 +441,11 @@ __global__ void k_train_adam(TrainParams t, int step) {
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-void launch_sur_desc(SurParams &p, cudaStream_t st) { k_sur_desc<<<(p.n + 31) / 32, 128, 0, st>>>(p); }
+// fstd == nullptr: raw features (training samples)
+void launch_sur_desc(SurParams &p, cudaStream_t st) {
+    if (p.fstd) k_sur_desc<<<(p.n + 31) / 32, 128, 0, st>>>(p);
+    else k_sur_sample<<<(p.n + 127) / 128, 128, 0, st>>>(p);
+}
 void launch_sur_mlp(SurParams &p, cudaStream_t st) {
     const int tiles = (p.n + 15) / 16;
     int blocks = (tiles + 3) / 4;

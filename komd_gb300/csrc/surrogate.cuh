@@ -71,8 +71,9 @@ void launch_fit_capture(int n, const float4 *nl, const int *nl_count, int nl_cap
                         const double *e3_site, const double *f3_site, const int *slot_site, float4 *dnl,
                         int *dcount, int dcap, float *dx, float *dmom, float *de3, float *df3, int *dsite, int *err,
                         cudaStream_t st);
-void launch_fit_step(FitParams &p, float *grad, cudaStream_t st);
-void launch_fit_adam(float *params, const float *grad, float *m, float *v, float lr, int step, cudaStream_t st);
+void launch_fit_step(FitParams &p, float *grad, bool pack, cudaStream_t st);
+void launch_fit_adam(const FitParams &p, float *params, float *grad, float *m, float *v, float lr, int step,
+                     cudaStream_t st);
 
 void launch_sur_desc(SurParams &p, cudaStream_t st);
 void launch_sur_mlp(SurParams &p, cudaStream_t st);
