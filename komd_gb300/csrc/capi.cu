@@ -45,7 +45,7 @@ cudaError_t dalloc(T *&p, size_t count) {
 }
 
 // TemperatureSensor's conversion (TemperatureSensor.cpp:44-47), restated in engine.cuh
-double temperature_from(double mv2, double n_in_box) { return sci_temperature(mv2, n_in_box); }
+double temperature_from(double mv2, double n_in_box) { return sci_temperature(sci_factor(), mv2, n_in_box); }
 
 // ---------------------------------------------------------------------------
 // profiling: event pairs per kernel family
@@ -79,7 +79,7 @@ struct komd_gpu {
     Engine e;
     Surrogate sur;
     double *f_scratch = nullptr;
-    double *acc = nullptr;            // R_NSLOTS
+    double *acc = nullptr;            // a measure's sums (R_NSLOTS), with the error flags (Engine::err) behind them
     double *thermo_acc = nullptr;     // R_NSLOTS, the device thermostat's kinetic sums
     int partial_cap = 0;
     bool want_posd = false;
@@ -96,7 +96,7 @@ struct komd_gpu {
     double ms[kNumFamilies] = {0};
     int64_t graph_steps = 0;
     uint64_t graph_epoch = 0;         // step graphs captured so far
-    int *flags_h = nullptr;           // pinned landing buffer of the error flags
+    double *land = nullptr;           // pinned landing buffer of acc and the flags, the copies' layout
     // komd_gpu_step_host's one-step graph (the step graph with the caller's
     // buffers bound), valid for one capture of the step graph and one set of buffers
     cudaGraphExec_t hgraph = nullptr;
@@ -296,9 +296,7 @@ void enqueue_step(komd_gpu *h) {
     }
     if (e.cfg.thermostat) {   // Simulation.cpp:72, after the step's sensors
         ProfScope ps(h, F_INTEGRATE);
-        cudaMemsetAsync(h->thermo_acc, 0, sizeof(double) * R_NSLOTS, e.stream);
-        launch_kinetic(e, e.stream, 0);
-        launch_sum_partials(e.stream, kinetic_grid(e), e.partials, h->thermo_acc);
+        launch_kinetic(e, e.stream, 0, h->thermo_acc);
         launch_velocity_scale(e, e.stream, h->thermo_acc, 1.0);
     }
     if (r_async) {
@@ -310,13 +308,23 @@ void enqueue_step(komd_gpu *h) {
     }
 }
 
+// the flags' place in a landing buffer of a measure's sums
+int *land_flags(double *land) { return reinterpret_cast<int *>(land + R_NSLOTS); }
+constexpr size_t kLandBytes = sizeof(double) * R_NSLOTS + sizeof(int) * E_NFLAGS;
+
+// the error flags, after everything on the stream; `clear` zeroes those that were raised
 int read_flags(komd_gpu *h, int flags[E_NFLAGS], bool clear) {
     Engine &e = h->e;
-    int *land = h->flags_h ? h->flags_h : flags;   // a pinned landing buffer copies without staging
+    int *land = h->land ? land_flags(h->land) : flags;   // a pinned landing buffer copies without staging
     CK(cudaMemcpyAsync(land, e.err, sizeof(int) * E_NFLAGS, cudaMemcpyDeviceToHost, e.stream));
-    if (clear) CK(cudaMemsetAsync(e.err, 0, sizeof(int) * E_NFLAGS, e.stream));
     CK(cudaStreamSynchronize(e.stream));
     if (land != flags) std::memcpy(flags, land, sizeof(int) * E_NFLAGS);
+    bool raised = false;
+    for (int k = 0; k < E_NFLAGS; k++) raised |= flags[k] != 0;
+    if (clear && raised) {
+        CK(cudaMemsetAsync(e.err, 0, sizeof(int) * E_NFLAGS, e.stream));
+        CK(cudaStreamSynchronize(e.stream));   // a batch runs the engine on another stream
+    }
     return KOMD_OK;
 }
 
@@ -429,13 +437,14 @@ int validate(const komd_config *c, Grid &g) {
 }
 
 // the launches of a measure on the engine's stream, and the copies of the
-// sums (acc_h, R_NSLOTS doubles), the RDF and the LJ histograms to the host
-// buffers given (asynchronous: valid once the stream has synchronised)
-int measure_enqueue(komd_gpu *h, uint32_t mask, double *acc_h, double *rdf, double *lj_hist) {
+// sums and the error flags (land, kLandBytes), the RDF and the LJ histograms to
+// the host buffers given (asynchronous: valid once the stream has synchronised)
+int measure_enqueue(komd_gpu *h, uint32_t mask, double *land, double *rdf, double *lj_hist) {
     Engine &e = h->e;
     cudaStream_t st = e.stream;
     ProfScope ps(h, F_MEASURE);
-    CK(cudaMemsetAsync(h->acc, 0, sizeof(double) * R_NSLOTS, st));
+    // first: it also clears the slots that the force terms add to
+    launch_kinetic(e, st, e.cfg.virial_mode == KOMD_VIRIAL_COMPAT ? (int)e.n_mol : (int)e.n, h->acc);
     const bool need_forces = (mask & (KOMD_MEASURE_ENERGY | KOMD_MEASURE_PRESSURE | KOMD_MEASURE_LJ_HIST)) != 0;
     if (need_forces) {
         // re-evaluate the force terms into a scratch force buffer (the sensors of
@@ -443,16 +452,12 @@ int measure_enqueue(komd_gpu *h, uint32_t mask, double *acc_h, double *rdf, doub
         if (mask & KOMD_MEASURE_LJ_HIST) CK(cudaMemsetAsync(e.lj_hist, 0, sizeof(double) * 4 * e.cfg.lj_bins, st));
         double *keep = e.f;
         const uint32_t force_terms = e.cfg.terms;
-        CK(cudaMemsetAsync(h->f_scratch, 0, sizeof(double) * 3 * e.n, st));
-        e.f = h->f_scratch;
+        e.f = h->f_scratch;   // the pair pass writes every site's force first
         e.cfg.terms = h->sensor_terms;
         enqueue_forces(h, true, (mask & KOMD_MEASURE_LJ_HIST) ? e.lj_hist : nullptr);
         e.cfg.terms = force_terms;
         e.f = keep;
     }
-    const int n_terms = e.cfg.virial_mode == KOMD_VIRIAL_COMPAT ? (int)e.n_mol : (int)e.n;
-    launch_kinetic(e, st, n_terms);
-    launch_sum_partials(st, kinetic_grid(e), e.partials, h->acc);
     if ((mask & KOMD_MEASURE_RDF) && e.rdf_bins > 0) {
         if (e.verlet) launch_rebuild(h);   // the cells of the last rebuild may be stale
         CK(cudaMemsetAsync(e.rdf, 0, sizeof(double) * e.rdf_bins, st));
@@ -462,7 +467,7 @@ int measure_enqueue(komd_gpu *h, uint32_t mask, double *acc_h, double *rdf, doub
     }
     int rc = check_launch("measure");
     if (rc) return rc;
-    CK(cudaMemcpyAsync(acc_h, h->acc, sizeof(double) * R_NSLOTS, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(land, h->acc, kLandBytes, cudaMemcpyDeviceToHost, st));
     if (rdf && (mask & KOMD_MEASURE_RDF) && e.rdf_bins > 0)
         CK(cudaMemcpyAsync(rdf, e.rdf, sizeof(double) * e.rdf_bins, cudaMemcpyDeviceToHost, st));
     if (lj_hist && (mask & KOMD_MEASURE_LJ_HIST))
@@ -534,14 +539,17 @@ int komd_gpu_create(const komd_config *cfg, int device, komd_gpu **out) {
         return fail(KOMD_ERR_CUDA, "stream creation failed");
     }
     if (dalloc(e.cell_count, g.ncell) || dalloc(e.cell_start, g.ncell + 1) || dalloc(e.cell_mcount, g.ncell) ||
-        dalloc(e.cell_mstart, g.ncell + 1) || dalloc(e.err, E_NFLAGS) || dalloc(h->acc, R_NSLOTS) || dalloc(h->thermo_acc, R_NSLOTS)) {
+        dalloc(e.cell_mstart, g.ncell + 1) || dalloc(h->acc, kLandBytes / sizeof(double)) || dalloc(h->thermo_acc, R_NSLOTS) ||
+        dalloc(e.kin_done, 1)) {
         komd_gpu_destroy(h);
         return fail(KOMD_ERR_NOMEM, "device allocation failed");
     }
-    cudaMemset(e.err, 0, sizeof(int) * E_NFLAGS);
-    if (cudaHostAlloc(reinterpret_cast<void **>(&h->flags_h), sizeof(int) * E_NFLAGS, cudaHostAllocDefault) != cudaSuccess) {
+    e.err = land_flags(h->acc);
+    cudaMemset(h->acc, 0, kLandBytes);
+    cudaMemset(e.kin_done, 0, sizeof(unsigned));
+    if (cudaHostAlloc(reinterpret_cast<void **>(&h->land), kLandBytes, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
-        h->flags_h = nullptr;   // read_flags then copies into the caller's array
+        h->land = nullptr;   // the copies then go to the caller's array
     }
     cudaMemset(e.cell_count, 0, sizeof(int) * g.ncell);    // the binning's counters start at zero
     cudaMemset(e.cell_mcount, 0, sizeof(int) * g.ncell);
@@ -611,13 +619,13 @@ int komd_gpu_destroy(komd_gpu *h) {
     if (e.stream) cudaStreamSynchronize(e.stream);
     if (e.graph) cudaGraphExecDestroy(e.graph);
     if (h->hgraph) cudaGraphExecDestroy(h->hgraph);
-    if (h->flags_h) cudaFreeHost(h->flags_h);
+    if (h->land) cudaFreeHost(h->land);
     dfree(e.r); dfree(e.v); dfree(e.f); dfree(e.m); dfree(e.eps); dfree(e.sig);
     dfree(e.key); dfree(e.site_mol); dfree(e.site_slot);
     dfree(e.mol_off); dfree(e.mol_cell); dfree(e.mol_rank); dfree(e.com);
     dfree(e.cell_count); dfree(e.cell_start); dfree(e.cell_mcount); dfree(e.cell_mstart); dfree(e.cell_mols);
     dfree(e.slot_site); dfree(e.skey); dfree(e.pos4); dfree(e.seps); dfree(e.posd); dfree(e.seps_d); dfree(e.sig_d);
-    dfree(e.nl); dfree(e.nl_count); dfree(e.bonds); dfree(e.angles); dfree(e.partials); dfree(e.err);
+    dfree(e.nl); dfree(e.nl_count); dfree(e.bonds); dfree(e.angles); dfree(e.partials); dfree(e.kin_done);
     dfree(e.tab_x); dfree(e.tab_y); dfree(e.tab_s); dfree(e.atm_acc); dfree(e.fown);
     dfree(e.rdf); dfree(e.lj_hist); dfree(e.counts); dfree(h->f_scratch); dfree(h->prof); dfree(h->acc); dfree(h->thermo_acc); dfree(e.offtab);
     dfree(e.nboff); dfree(e.vb_next); dfree(e.rebuild); dfree(e.bias); dfree(e.ref4); dfree(e.slot_cell); dfree(e.zkey); dfree(e.vl); dfree(e.vl_count);
@@ -832,6 +840,10 @@ int komd_gpu_update_container(komd_gpu *h) {
         CK(cudaMemsetAsync(e.f, 0, sizeof(double) * 3 * e.n, e.stream));   // FReset_Kernel
         int rc = check_launch("update_container");
         if (rc) return rc;
+        if (!e.verlet) {   // no list that could overflow
+            CK(cudaStreamSynchronize(e.stream));
+            break;
+        }
         int flags[E_NFLAGS];
         rc = read_flags(h, flags, false);
         if (rc) return rc;
@@ -892,16 +904,19 @@ int komd_gpu_integrate1(komd_gpu *h) {
     return KOMD_OK;
 }
 
-static int finish_steps(komd_gpu *h) {
-    int flags[E_NFLAGS];
-    int rc = read_flags(h, flags, true);
-    if (rc) return rc;
+static int check_step_flags(const int *flags) {
     if (flags[E_ATM_OVERFLOW])
         return fail(KOMD_ERR_OVERFLOW, "ATM neighbour list overflowed during the steps (raise atm_list_cap)");
     if (flags[E_VL_OVERFLOW])
         return fail(KOMD_ERR_OVERFLOW, "Verlet list overflowed during the steps (density rose; call update_container)");
     if (flags[E_NONFINITE]) return fail(KOMD_ERR_NONFINITE, "non-finite velocity after a step");
     return KOMD_OK;
+}
+
+static int finish_steps(komd_gpu *h) {
+    int flags[E_NFLAGS];
+    const int rc = read_flags(h, flags, true);
+    return rc ? rc : check_step_flags(flags);
 }
 
 // exact-ATM probe of the learned term at the current state (the ATM list of
@@ -1205,15 +1220,20 @@ int komd_gpu_measure(komd_gpu *h, uint32_t mask, komd_observables *obs, double *
     if (!h || !obs) return fail(KOMD_ERR_ARG, "null argument");
     if (!h->e.have_cells) return fail(KOMD_ERR_STATE, "update_container must run before measure");
     std::memset(obs, 0, sizeof(*obs));
-    double acc[R_NSLOTS];
-    int rc = measure_enqueue(h, mask, acc, rdf, lj_hist);
+    double local[kLandBytes / sizeof(double)];
+    double *land = h->land ? h->land : local;
+    int rc = measure_enqueue(h, mask, land, rdf, lj_hist);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->e.stream));
-    int flags[E_NFLAGS];
-    rc = read_flags(h, flags, true);
-    if (rc) return rc;
+    const int *flags = land_flags(land);
+    bool raised = false;
+    for (int k = 0; k < E_NFLAGS; k++) raised |= flags[k] != 0;
+    if (raised) {
+        CK(cudaMemsetAsync(h->e.err, 0, sizeof(int) * E_NFLAGS, h->e.stream));
+        CK(cudaStreamSynchronize(h->e.stream));
+    }
     if (flags[E_ATM_OVERFLOW]) return fail(KOMD_ERR_OVERFLOW, "ATM neighbour list overflow during measure");
-    measure_fill(acc, obs);
+    measure_fill(land, obs);
     return KOMD_OK;
 }
 
@@ -1989,6 +2009,26 @@ int batch_capture(komd_batch *b) {
 }
 }  // namespace
 
+namespace {
+// waits for the batch's graphs and checks every replica's error flags: the copies
+// queue behind the graphs and one synchronisation serves them all
+int batch_finish(komd_batch *b) {
+    bool landed = true;
+    for (komd_gpu *h : b->reps) landed = landed && h->land;
+    for (size_t r = 0; landed && r < b->reps.size(); r++)
+        CK(cudaMemcpyAsync(land_flags(b->reps[r]->land), b->reps[r]->e.err, sizeof(int) * E_NFLAGS,
+                           cudaMemcpyDeviceToHost, b->origin));
+    CK(cudaStreamSynchronize(b->origin));
+    for (size_t r = 0; r < b->reps.size(); r++) {
+        bool raised = !landed;
+        for (int k = 0; landed && k < E_NFLAGS; k++) raised |= land_flags(b->reps[r]->land)[k] != 0;
+        const int rc = raised ? finish_steps(b->reps[r]) : KOMD_OK;   // reads again, and clears
+        if (rc) return fail(rc, "replica " + std::to_string(r) + ": " + g_last_error);
+    }
+    return KOMD_OK;
+}
+}  // namespace
+
 extern "C" {
 
 int komd_batch_create(komd_gpu *const *replicas, int32_t n, int32_t n_streams, int32_t steps_per_graph,
@@ -2052,13 +2092,8 @@ int komd_batch_step(komd_batch *b, int64_t n_graphs) {
     if (!b) return fail(KOMD_ERR_ARG, "null batch");
     CK(cudaSetDevice(b->device));
     for (int64_t k = 0; k < n_graphs; k++) CK(cudaGraphLaunch(b->graph, b->origin));
-    CK(cudaStreamSynchronize(b->origin));
     b->steps += n_graphs * b->steps_per_graph;
-    for (size_t r = 0; r < b->reps.size(); r++) {
-        int rc = finish_steps(b->reps[r]);
-        if (rc) return fail(rc, "replica " + std::to_string(r) + ": " + g_last_error);
-    }
-    return KOMD_OK;
+    return batch_finish(b);
 }
 
 // enqueue only (no synchronisation, no flag check): for timing with events on the origin stream
@@ -2102,13 +2137,9 @@ int komd_batch_measure(komd_batch *b, uint32_t mask, komd_observables *obs, doub
         double *slot = b->stage + (size_t)r * per;
         const bool with_rdf = (mask & KOMD_MEASURE_RDF) && e.rdf_bins > 0;
         rc = measure_enqueue(b->reps[r], mask, slot, with_rdf ? b->stage + off : nullptr, nullptr);
-        if (!rc) {
-            // the flags as read_flags reads them (read, then cleared), into the landing area
-            int *fl = reinterpret_cast<int *>(slot + R_NSLOTS);
-            if (cudaMemcpyAsync(fl, e.err, sizeof(int) * E_NFLAGS, cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
-                cudaMemsetAsync(e.err, 0, sizeof(int) * E_NFLAGS, e.stream) != cudaSuccess)
-                rc = fail(KOMD_ERR_CUDA, "measure flags");
-        }
+        // the flags are cleared behind the copy, as komd_gpu_measure clears them
+        if (!rc && cudaMemsetAsync(e.err, 0, sizeof(int) * E_NFLAGS, e.stream) != cudaSuccess)
+            rc = fail(KOMD_ERR_CUDA, "measure flags");
         if (with_rdf) off += (size_t)e.rdf_bins;
         e.stream = keep;
     }
@@ -2121,7 +2152,7 @@ int komd_batch_measure(komd_batch *b, uint32_t mask, komd_observables *obs, doub
     for (int r = 0; r < nr; r++) {
         const Engine &e = b->reps[r]->e;
         const double *slot = b->stage + (size_t)r * per;
-        const int *fl = reinterpret_cast<const int *>(slot + R_NSLOTS);
+        const int *fl = land_flags(const_cast<double *>(slot));
         if (fl[E_ATM_OVERFLOW])
             return fail(KOMD_ERR_OVERFLOW, "replica " + std::to_string(r) + ": ATM neighbour list overflow during measure");
         measure_fill(slot, obs + r);
@@ -2141,12 +2172,7 @@ int komd_batch_form(komd_batch *b) {
 
 int komd_batch_check(komd_batch *b) {
     if (!b) return fail(KOMD_ERR_ARG, "null batch");
-    CK(cudaStreamSynchronize(b->origin));
-    for (size_t r = 0; r < b->reps.size(); r++) {
-        int rc = finish_steps(b->reps[r]);
-        if (rc) return fail(rc, "replica " + std::to_string(r) + ": " + g_last_error);
-    }
-    return KOMD_OK;
+    return batch_finish(b);
 }
 
 int komd_gpu_kernels_per_step(komd_gpu *h) {
@@ -2161,7 +2187,7 @@ int komd_gpu_kernels_per_step(komd_gpu *h) {
     if ((e.cfg.terms & KOMD_TERM_BONDED) && e.n_bonds > 0) k++;
     if ((e.cfg.terms & KOMD_TERM_BONDED) && e.n_angles > 0) k++;
     if (e.cfg.terms & KOMD_TERM_LIMIT) k++;
-    if (e.cfg.thermostat) k += 3;  /* kinetic sums, partial reduction, velocity scaling */
+    if (e.cfg.thermostat) k += 2;  /* kinetic sums, velocity scaling */
     if (surrogate_on(h)) k += 4;   /* descriptors, MLP, forces, apply */
     else if (e.cfg.terms & KOMD_TERM_ATM)   /* once-per-triplet kernel (inside the LJ pass on the Verlet path) + flush */
         k += (e.atm_acc != nullptr) ? (fused_lj_atm(h, false) ? 1 : 2) : 1;

@@ -416,12 +416,15 @@ __host__ __device__ inline double sci_pow10(int e) {
     for (int i = 22; i < k && i < 330; i++) p = p * 10.0;
     return e < 0 ? 1.0 / p : p;
 }
-__host__ __device__ inline double sci_temperature(double mv2, double n_in_box) {
-    if (!(n_in_box > 0.0)) return 0.0;
+// the units' factor (the same for every state: the device thermostat takes it as an argument)
+__host__ __device__ inline SciNum sci_factor() {
     const SciNum kB = sci_norm(1.380649, -23), da = sci_norm(1.66053906892, -27), aps = sci_norm(1.0, 2);
-    SciNum f = sci_norm(aps.m * aps.m, aps.e + aps.e);
+    const SciNum f = sci_norm(aps.m * aps.m, aps.e + aps.e);
     const SciNum q = sci_norm(da.m / kB.m, da.e - kB.e);
-    f = sci_norm(f.m * q.m, f.e + q.e);
+    return sci_norm(f.m * q.m, f.e + q.e);
+}
+__host__ __device__ inline double sci_temperature(SciNum f, double mv2, double n_in_box) {
+    if (!(n_in_box > 0.0)) return 0.0;
     const double x = mv2 / (n_in_box * 3);
     const SciNum v = x == 0.0 ? SciNum{0.0, 0} : sci_norm(x, 0);
     const SciNum t = sci_norm(f.m * v.m, f.e + v.e);
@@ -462,7 +465,8 @@ struct Engine {
     // reductions / flags
     double *partials = nullptr;
     int partial_blocks = 0;
-    int *err = nullptr;
+    int *err = nullptr;            // error flags, behind the measure's sums (komd_gpu::acc)
+    unsigned *kin_done = nullptr;  // blocks of the kinetic sums that have finished (zero between launches)
     double *rdf = nullptr;
     int64_t rdf_bins = 0;
     double *lj_hist = nullptr;

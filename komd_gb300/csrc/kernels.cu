@@ -962,17 +962,38 @@ __global__ void k_refresh(int n, const int *__restrict__ slot_site, const double
 // ===========================================================================
 // sensors
 // ===========================================================================
+// the warp sums of K values (2 or 8), the lanes splitting the values on the way:
+// lane l ends with value l / (32 / K); 9 additions a lane for eight values
+// instead of 40 (GB300's FP64 pipe bounds these reductions)
+template <int K>
+__device__ __forceinline__ double warp_sum_split(double (&v)[K], int lane) {
+    int o = 16;
+#pragma unroll
+    for (int k = K; k > 1; k >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int q = 0; q < k / 2; q++) {
+            const double send = up ? v[q] : v[q + k / 2], keep = up ? v[q + k / 2] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
 // TemperatureSensor::measure (sites inside [low, high]) + kinetic tensor
-// (PressureSensor::MomentumKernel) over the first n_terms sites.
+// (PressureSensor::MomentumKernel) over the first n_terms sites (TERMS).
 // Grid-stride over the sites (a resident grid, so each thread sums several
-// sites before the fixed-tree warp and block reductions; the order is fixed,
-// so the sums are deterministic).  TERMS adds the per-site kinetic tensor of
-// the first n_terms sites.
+// sites before the fixed-tree warp and block reductions).  The block that
+// finishes last sums the blocks' rows in their order into acc and zeroes
+// acc's other slots, so a measure needs neither a clearing nor a second
+// kernel: the sums are deterministic.  done: a counter, zero between launches.
 template <bool TERMS>
 __global__ void __launch_bounds__(kBlock) k_kinetic(Grid g, int n, int n_terms, const double *__restrict__ r,
                                                     const double *__restrict__ v, const double *__restrict__ m,
-                                                    double *__restrict__ partials) {
+                                                    double *partials, double *__restrict__ acc, unsigned *done) {
     __shared__ double s_part[kWarpsPerBlock][8];
+    __shared__ bool s_last;
     constexpr int kVals = TERMS ? 8 : 2;
     double vals[kVals];
     for (int k = 0; k < kVals; k++) vals[k] = 0.0;
@@ -990,24 +1011,36 @@ __global__ void __launch_bounds__(kBlock) k_kinetic(Grid g, int n, int n_terms, 
             }
         }
     }
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int k = 0; k < kVals; k++) {
-        double xk = vals[k];
-        for (int o = 16; o > 0; o >>= 1) xk += __shfl_xor_sync(0xffffffffu, xk, o);
-        if (lane == 0) s_part[wib][k] = xk;
+    const int t = threadIdx.x, lane = t & 31, wib = t >> 5;
+    const double mine = warp_sum_split<kVals>(vals, lane);
+    if (lane % (32 / kVals) == 0) s_part[wib][lane / (32 / kVals)] = mine;
+    __syncthreads();
+    if (t < kVals) {   // this block's row: R_NSLOTS doubles apart, the values in front
+        double sum = 0.0;
+        for (int w = 0; w < kWarpsPerBlock; w++) sum += s_part[w][t];
+        partials[(size_t)blockIdx.x * R_NSLOTS + t] = sum;
+        __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x < R_NSLOTS) {
-        const int t = threadIdx.x;
-        double acc = 0.0;
+    if (t == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (wib < kVals) {   // a value per warp, the rows over the lanes
+        double sum = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) sum += __ldcg(&partials[(size_t)b * R_NSLOTS + wib]);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) s_part[0][wib] = sum;
+    }
+    __syncthreads();
+    if (t < R_NSLOTS) {
         int src = -1;
         if (t == R_MV2) src = 0;
         else if (t == R_NBOX) src = 1;
         else if (TERMS && t >= R_K0 && t <= R_K5) src = 2 + t - R_K0;
-        if (src >= 0)
-            for (int w = 0; w < kWarpsPerBlock; w++) acc += s_part[w][src];
-        partials[(size_t)blockIdx.x * R_NSLOTS + t] = acc;
+        acc[t] = src >= 0 ? s_part[0][src] : 0.0;
     }
+    if (t == 0) *done = 0u;
 }
 
 // RDF over molecule COMs (RDFSensor::RDF_Kernel, RDFSensor.cpp:61-72):
@@ -1232,12 +1265,12 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_partials(int nblocks, const
 // overflowed force upstream) leaves v unscaled and raises E_NONFINITE, which
 // the host reads after the step.
 __global__ void k_velocity_scale(int n, double *__restrict__ v, const double *__restrict__ acc, double t_target,
-                                 double beta_in, int *__restrict__ err) {
+                                 SciNum factor, double beta_in, int *__restrict__ err) {
     __shared__ double s_beta;
     if (threadIdx.x == 0) {
         double beta = beta_in;
         if (acc) {
-            const double t = sci_temperature(acc[R_MV2], acc[R_NBOX]);
+            const double t = sci_temperature(factor, acc[R_MV2], acc[R_NBOX]);
             if (!isfinite(t)) {
                 beta = 1.0;
                 if (blockIdx.x == 0 && err) atomicOr(&err[E_NONFINITE], 1);
@@ -1621,12 +1654,15 @@ int kinetic_grid(const Engine &e) { return std::min(nblk(e.n, kBlock), e.num_sms
 
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta) {
     const int blocks = std::min(nblk(3 * e.n, 256), e.num_sms * 8);
-    k_velocity_scale<<<blocks, 256, 0, st>>>((int)e.n, e.v, acc, e.cfg.temperature_target, beta, e.err);
+    k_velocity_scale<<<blocks, 256, 0, st>>>((int)e.n, e.v, acc, e.cfg.temperature_target, sci_factor(), beta, e.err);
 }
 
-void launch_kinetic(Engine &e, cudaStream_t st, int n_terms) {
-    if (n_terms > 0) k_kinetic<true><<<kinetic_grid(e), kBlock, 0, st>>>(e.g, (int)e.n, n_terms, e.r, e.v, e.m, e.partials);
-    else k_kinetic<false><<<kinetic_grid(e), kBlock, 0, st>>>(e.g, (int)e.n, 0, e.r, e.v, e.m, e.partials);
+// the kinetic sums into acc (R_NSLOTS), whose other slots become zero
+void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc) {
+    const int grid = kinetic_grid(e);
+    if (n_terms > 0)
+        k_kinetic<true><<<grid, kBlock, 0, st>>>(e.g, (int)e.n, n_terms, e.r, e.v, e.m, e.partials, acc, e.kin_done);
+    else k_kinetic<false><<<grid, kBlock, 0, st>>>(e.g, (int)e.n, 0, e.r, e.v, e.m, e.partials, acc, e.kin_done);
 }
 
 void launch_sum_partials(cudaStream_t st, int nblocks, const double *partials, double *out) {

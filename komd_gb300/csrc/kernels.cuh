@@ -35,7 +35,7 @@ bool half_plain(const PairParams &p);
 // in_step (step graphs only): the fused drift path when the engine qualifies
 void launch_step0(Engine &e, cudaStream_t st, bool in_step = false);
 void launch_step1(Engine &e, cudaStream_t st);
-void launch_kinetic(Engine &e, cudaStream_t st, int n_terms);
+void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc);
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta);
 void launch_pair_table(Engine &e, cudaStream_t st);
 void launch_sum_partials(cudaStream_t st, int nblocks, const double *partials, double *out);
