@@ -158,6 +158,7 @@ int ensure_partials(komd_gpu *h) {
     Engine &e = h->e;
     int need = std::max(e.g.ncell, pair_cell_grid(e));   // one partial row per block of the pair kernels
     need = std::max(need, atm_grid(e));
+    if (e.verlet) need = std::max(need, vlist_blocks(e));
     need = std::max(need, kinetic_grid(e));
     if (need > h->partial_cap) {
         CK(dalloc(e.partials, (size_t)need * R_NSLOTS));

@@ -291,6 +291,8 @@ struct AtmParams {
     double nu;
     double rc2;
     double sign;               // +1 reference (+grad V), -1 physical
+    double share;              // 2 sign nu
+    float rc2f;                // rc2 in FP32
     int virial_compat;         // weights and missing ZZ of ATM_Pressure
     int atm_direct;            // COMPAT + direct: no virial contribution
     double *e_site;            // measure: per-site V/3 sums (site order), optional

@@ -459,11 +459,36 @@ __global__ void __launch_bounds__(kBlock) k_atm_d(AtmParams p) {
     }
 }
 
+// the warp sums of K values (2 or 8), the lanes splitting the values on the way:
+// lane l ends with value l / (32 / K); 9 additions a lane for eight values
+// instead of 40 (GB300's FP64 pipe bounds these reductions)
+template <typename T, int K>
+__device__ __forceinline__ T warp_sum_split(T (&v)[K], int lane) {
+    int o = 16;
+#pragma unroll
+    for (int k = K; k > 1; k >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int q = 0; q < k / 2; q++) {
+            const T send = up ? v[q] : v[q + k / 2], keep = up ? v[q + k / 2] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
 // FP32 ATM kernel with ballot compaction: lanes test candidate pairs (a, b)
 // of the vertex's neighbour list (round-robin pairing a, a+d mod n, so each
 // unordered pair is tested once) and queue the ones inside the cutoff; the
 // triplet arithmetic then always runs on 32 queued pairs at a time.  All
 // queued pairs share vertex i, so each lane keeps a private force sum.
+//
+// MEASURE runs a resident grid whose warps stride over the vertices: a vertex's
+// energy and virial leave the lanes' FP32 partials through a tree that leaves
+// value k in lane 4 k, so that one conversion and one FP64 addition per vertex
+// carry all seven into the warp's sums (a tree, conversions and a division per
+// vertex kept the FP64 pipe 76 % busy: 525 -> 380 us at 256,000 sites).
 template <bool MEASURE, bool COMPAT>
 __global__ void __launch_bounds__(kBlock) k_atm_q(AtmParams p) {
     extern __shared__ float4 s_dyn[];
@@ -474,14 +499,15 @@ __global__ void __launch_bounds__(kBlock) k_atm_q(AtmParams p) {
     const int cap = p.nl_cap;
     float4 *se = s_dyn + wib * cap;
     float4 *sq = s_dyn + kWarpsPerBlock * cap + wib * cap;   // (A, 1/A, 1/sqrt(A), -) per entry
-    const int i = blockIdx.x * kWarpsPerBlock + wib;
-    const float rc2 = (float)p.rc2;
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-    float m_e = 0.f, m_w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    int m_t = 0;   // triplet visits (each triplet is visited from its three vertices)
+    const float rc2 = p.rc2f;
+    double m_sum = 0.0;   // lane 4 k (k < 8): the warp's sum of value k
+    int m_t = 0;          // triplet visits (each triplet is visited from its three vertices)
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
 
+    for (int i = blockIdx.x * kWarpsPerBlock + wib; i < p.n; i += gridDim.x * kWarpsPerBlock) {
+    float gx = 0.f, gy = 0.f, gz = 0.f;
+    float m_e = 0.f, m_w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     auto triplet = [&](unsigned e, float C, bool valid) {
         if (!valid) return;
         const int a = (int)(e & 0xffffu), b = (int)(e >> 16);
@@ -535,7 +561,7 @@ __global__ void __launch_bounds__(kBlock) k_atm_q(AtmParams p) {
         }
     };
 
-    if (i < p.n) {
+    {
         const int ni = p.nl_count[i];
         for (int k = lane; k < ni; k += 32) {
             const float4 e = p.nl[(size_t)i * cap + k];
@@ -597,37 +623,24 @@ __global__ void __launch_bounds__(kBlock) k_atm_q(AtmParams p) {
             const float ce = v ? s_qc[wib][lane] : 1.f;
             triplet(e, ce, v);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            gx += __shfl_xor_sync(0xffffffffu, gx, o);
-            gy += __shfl_xor_sync(0xffffffffu, gy, o);
-            gz += __shfl_xor_sync(0xffffffffu, gz, o);
+        // lanes 0, 8 and 16 take a component each: one conversion and one fused
+        // operation on the FP64 pipe for the three
+        const float gs = warp_sum3(gx, gy, gz, lane);
+        const int site = p.slot_site[i];
+        if ((lane & 7) == 0 && lane < 24)   // reference: +2 nu (...); physical: -2 nu (...)
+            p.f[3 * (size_t)site + (lane >> 3)] += p.share * (double)gs;
+        if (MEASURE) {
+            float vals[8] = {m_e, 0.f, m_w[0], m_w[1], m_w[2], m_w[3], m_w[4], m_w[5]};
+            const double v = (double)warp_sum_split<float, 8>(vals, lane);
+            m_sum += v;
+            if (p.e_site && lane == 0) p.e_site[site] = p.nu * v;
         }
-        float ev = m_e;
-        if (MEASURE && p.e_site)
-            for (int o = 16; o > 0; o >>= 1) ev += __shfl_xor_sync(0xffffffffu, ev, o);
-        if (lane == 0) {
-            const int site = p.slot_site[i];
-            const double sc = 2.0 * p.sign * p.nu;   // reference: +2 nu (...); physical: -2 nu (...)
-            p.f[3 * site] += sc * (double)gx;
-            p.f[3 * site + 1] += sc * (double)gy;
-            p.f[3 * site + 2] += sc * (double)gz;
-            if (MEASURE && p.e_site) p.e_site[site] = p.nu * (double)ev;
-        }
+        __syncwarp();   // the staging is refilled by the next vertex
+    }
     }
     if (MEASURE) {
-        // FP32 warp tree over the lanes' FP32 partials, FP64 from the warp sums on
-        float vals[8] = {m_e, 0.f, m_w[0], m_w[1], m_w[2], m_w[3], m_w[4], m_w[5]};
-        for (int k = 0; k < 8; k++) {
-            float x = vals[k];
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            vals[k] = x;
-        }
-        int visits = m_t;   // an exact integer count, a third of a triplet per visit
-        for (int o = 16; o > 0; o >>= 1) visits += __shfl_xor_sync(0xffffffffu, visits, o);
-        if (lane == 0) {
-            for (int k = 0; k < 8; k++) s_part[wib][k] = (double)vals[k];
-            s_part[wib][1] = (double)visits / 3.0;
-        }
+        const int visits = __reduce_add_sync(0xffffffffu, m_t);   // a third of a triplet per visit
+        if ((lane & 3) == 0) s_part[wib][lane >> 2] = lane == 4 ? (double)visits / 3.0 : m_sum;
         __syncthreads();
         if (threadIdx.x < R_NSLOTS) {
             const int t = threadIdx.x;
@@ -962,25 +975,6 @@ __global__ void k_refresh(int n, const int *__restrict__ slot_site, const double
 // ===========================================================================
 // sensors
 // ===========================================================================
-// the warp sums of K values (2 or 8), the lanes splitting the values on the way:
-// lane l ends with value l / (32 / K); 9 additions a lane for eight values
-// instead of 40 (GB300's FP64 pipe bounds these reductions)
-template <int K>
-__device__ __forceinline__ double warp_sum_split(double (&v)[K], int lane) {
-    int o = 16;
-#pragma unroll
-    for (int k = K; k > 1; k >>= 1, o >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int q = 0; q < k / 2; q++) {
-            const double send = up ? v[q] : v[q + k / 2], keep = up ? v[q + k / 2] : v[q];
-            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    return v[0];
-}
-
 // TemperatureSensor::measure (sites inside [low, high]) + kinetic tensor
 // (PressureSensor::MomentumKernel) over the first n_terms sites (TERMS).
 // Grid-stride over the sites (a resident grid, so each thread sums several
@@ -1012,7 +1006,7 @@ __global__ void __launch_bounds__(kBlock) k_kinetic(Grid g, int n, int n_terms, 
         }
     }
     const int t = threadIdx.x, lane = t & 31, wib = t >> 5;
-    const double mine = warp_sum_split<kVals>(vals, lane);
+    const double mine = warp_sum_split<double, kVals>(vals, lane);
     if (lane % (32 / kVals) == 0) s_part[wib][lane / (32 / kVals)] = mine;
     __syncthreads();
     if (t < kVals) {   // this block's row: R_NSLOTS doubles apart, the values in front
@@ -1396,12 +1390,9 @@ PairParams pair_params(Engine &e) {
     return p;
 }
 
-// FP64: a resident grid whose warps stride over the vertices (at most one row
-// of partial sums per block, whatever the list capacity)
-int atm_grid(const Engine &e) {
-    const int g = nblk(e.n, kWarpsPerBlock);
-    return e.cfg.precision == KOMD_FP64 ? std::min(g, e.num_sms * 16) : g;
-}
+// measures and FP64: a resident grid whose warps stride over the vertices (one
+// row of partial sums per block, whatever the list capacity)
+int atm_grid(const Engine &e) { return std::min(nblk(e.n, kWarpsPerBlock), e.num_sms * 16); }
 // warps per block of the FP64 kernel: eight, fewer where their staging (64
 // bytes a neighbour) would pass 96 KB
 static int atm_warps(const Engine &e) {
@@ -1598,6 +1589,8 @@ AtmParams atm_params(const Engine &e) {
     p.nu = e.cfg.nu;
     p.rc2 = e.cfg.cutoff_3b * e.cfg.cutoff_3b;
     p.sign = e.cfg.atm_sign == KOMD_ATM_SIGN_REFERENCE ? 1.0 : -1.0;
+    p.share = 2.0 * p.sign * p.nu;
+    p.rc2f = (float)p.rc2;
     p.virial_compat = e.cfg.virial_mode == KOMD_VIRIAL_COMPAT;
     p.atm_direct = e.cfg.atm_direct;
     p.e_site = e.atm_esite;
@@ -1625,12 +1618,12 @@ bool launch_atm(Engine &e, cudaStream_t st, bool measure, bool with_step1) {
     const bool compat = e.cfg.atm_enum == KOMD_ATM_ENUM_COMPAT;
     if (!measure && !compat && e.cfg.precision == KOMD_FP32 && e.atm_acc) {
         // every triplet once (lowest slot), fixed-point scatter, then the flush into f
-        k_atm_s<<<atm_grid(e), kBlock, atm_smem(e), st>>>(p);
+        k_atm_s<<<nblk(e.n, kWarpsPerBlock), kBlock, atm_smem(e), st>>>(p);
         return launch_atm_flush(e, st, with_step1, false);
     }
     if (e.cfg.precision == KOMD_FP64)
         atm_dispatch_d(p, measure, compat, atm_grid(e), atm_warps(e), atm_smem(e), st);
-    else atm_dispatch_f(p, measure, compat, atm_grid(e), atm_smem(e), st);
+    else atm_dispatch_f(p, measure, compat, measure ? atm_grid(e) : nblk(e.n, kWarpsPerBlock), atm_smem(e), st);
     return false;
 }
 

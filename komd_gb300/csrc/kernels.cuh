@@ -13,6 +13,7 @@ int pair_cell_grid(const Engine &e);
 void launch_vlist_build(Engine &e, cudaStream_t st);
 int launch_lj_vlist(Engine &e, PairParams &p, bool measure, bool emit, cudaStream_t st);
 int vlist_grid(const Engine &e);
+int vlist_blocks(const Engine &e);
 void launch_counts(Engine &e, cudaStream_t st);
 void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc);
 void launch_limit(Engine &e, cudaStream_t st);

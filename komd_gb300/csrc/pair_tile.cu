@@ -584,20 +584,13 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, int lane, uns
             }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        fx += __shfl_xor_sync(0xffffffffu, fx, o);
-        fy += __shfl_xor_sync(0xffffffffu, fy, o);
-        fz += __shfl_xor_sync(0xffffffffu, fz, o);
-    }
-    if (lane == 0) {
-        const int site = p.slot_site[i];
-        p.f[3 * site] = (double)fx;
-        p.f[3 * site + 1] = (double)fy;
-        p.f[3 * site + 2] = (double)fz;
-        if (EMIT) {
-            if (!TO_SMEM) p.nl_count[i] = min(c_atm, p.nl_cap);
-            if (c_atm > p.nl_cap) atomicOr(&p.err[E_ATM_OVERFLOW], 1);
-        }
+    // lanes 0, 8 and 16 hold x, y and z: one FP32 -> FP64 conversion for the three (a
+    // conversion takes the FP64 pipe for a whole warp, whatever the active lanes)
+    const float fs = warp_sum3(fx, fy, fz, lane);
+    if ((lane & 7) == 0 && lane < 24) p.f[3 * (size_t)p.slot_site[i] + (lane >> 3)] = (double)fs;
+    if (EMIT && lane == 0) {
+        if (!TO_SMEM) p.nl_count[i] = min(c_atm, p.nl_cap);
+        if (c_atm > p.nl_cap) atomicOr(&p.err[E_ATM_OVERFLOW], 1);
     }
     return min(c_atm, p.nl_cap);
 }
@@ -920,6 +913,12 @@ int vlist_per(const Engine &e) {
     return groups <= target ? 1 : (groups + target - 1) / target;
 }
 
+// blocks of the single-system passes over the slots (rows of partial sums when measuring)
+int vlist_blocks(const Engine &e) {
+    const int per = vlist_per(e);
+    return (vlist_grid(e) + per - 1) / per;
+}
+
 // ---- packed replicas (kernels.cuh): the list build and the half-list pass of
 // every replica in one launch each
 __device__ __forceinline__ int packed_replica(const int *__restrict__ start, int nrep, int b) {
@@ -1032,7 +1031,7 @@ bool vlist_u3(const Engine &e) {
 int launch_lj_vlist(Engine &e, PairParams &p, bool measure, bool emit, cudaStream_t st) {
     // a block's partial sums cover all its groups (the lanes' sums run across them)
     const int per = vlist_per(e);
-    const int grid = (vlist_grid(e) + per - 1) / per;
+    const int grid = vlist_blocks(e);
     const bool u3 = vlist_u3(e);
     if (e.uniform) lj_vlist_dispatch<true>(p, (int)e.n, grid, per, measure, emit, u3, st);
     else lj_vlist_dispatch<false>(p, (int)e.n, grid, per, measure, emit, u3, st);
@@ -1043,7 +1042,7 @@ void launch_lj_atm(Engine &e, cudaStream_t st) {
     PairParams p = pair_params(e);
     const AtmParams a = atm_params(e);
     const int per = vlist_per(e);
-    const int grid = (vlist_grid(e) + per - 1) / per;
+    const int grid = vlist_blocks(e);
     if (lj_atm_half(e)) {
         const size_t sm = lj_atm_half_smem(e);
         const float sa = (float)(2.0 * a.sign * a.nu);   // share units (2 sign nu) to force units
