@@ -44,6 +44,14 @@ cudaError_t dalloc(T *&p, size_t count) {
     return cudaMalloc(reinterpret_cast<void **>(&p), sizeof(T) * count);
 }
 
+// the step graphs no longer match the engine's buffers, terms or capacities
+void drop_graphs(Engine &e) {
+    if (e.graph) cudaGraphExecDestroy(e.graph);
+    if (e.chain) cudaGraphExecDestroy(e.chain);
+    e.graph = e.chain = nullptr;
+    e.graph_valid = false;
+}
+
 // TemperatureSensor's conversion (TemperatureSensor.cpp:44-47), restated in engine.cuh
 double temperature_from(double mv2, double n_in_box) { return sci_temperature(sci_factor(), mv2, n_in_box); }
 
@@ -194,15 +202,16 @@ bool surrogate_on(komd_gpu *h) {
     return (h->e.cfg.terms & KOMD_TERM_ATM_SURROGATE) && h->sur.loaded && !h->sur.fallback;
 }
 
-// surrogate three-body forces: into f (fout == nullptr), with integrate1 of the
-// step (with_step1), or written to fout
-void enqueue_surrogate(komd_gpu *h, double *fout, bool with_step1 = false) {
+// surrogate three-body forces: into f (fout == nullptr), with the step's end, or
+// written to fout
+void enqueue_surrogate(komd_gpu *h, double *fout, StepEnd end = END_NONE) {
     Engine &e = h->e;
     SurParams p = sur_params(h);
     launch_sur_desc(p, e.stream);
     launch_sur_mlp(p, e.stream);
     launch_sur_force(p, e.stream);
-    if (with_step1) launch_sur_apply_step1(p, e, e.stream);
+    if (end == END_STEP1) launch_sur_apply_step1(p, e, e.stream);
+    else if (end == END_KICK_DRIFT) launch_learned_kick_drift(e, p.fsur, e.stream);
     else launch_sur_apply(p, e.slot_site, e.f, fout, e.stream);
 }
 
@@ -213,8 +222,8 @@ bool fused_lj_atm(komd_gpu *h, bool measure) {
 
 // the force sequence of Simulation::run: 2-body functors (LJ / FENE, bonded,
 // Limit), then the 3-body functor (ATM, exact or learned)
-// returns true when integrate1 was fused into the last force kernel (with_step1)
-bool enqueue_forces(komd_gpu *h, bool measure, double *lj_hist, bool with_step1 = false) {
+// returns true when the step's end was fused into the last force kernel
+bool enqueue_forces(komd_gpu *h, bool measure, double *lj_hist, StepEnd end = END_NONE) {
     Engine &e = h->e;
     cudaStream_t st = e.stream;
     bool fused = false;
@@ -251,14 +260,14 @@ bool enqueue_forces(komd_gpu *h, bool measure, double *lj_hist, bool with_step1 
     if (surrogate_on(h)) {
         {
             ProfScope ps(h, F_SURROGATE);
-            enqueue_surrogate(h, nullptr, with_step1);
-            fused = with_step1;
+            fused = end == END_STEP1 || (end == END_KICK_DRIFT && e.fused_drift);
+            enqueue_surrogate(h, nullptr, fused ? end : END_NONE);
         }
         if (measure) launch_sum_sites((int)e.n, h->sur.esite, h->acc + R_UATM, st);
     } else if (e.cfg.terms & KOMD_TERM_ATM) {
         {
             ProfScope ps(h, F_ATM);
-            fused = lj_atm ? launch_atm_flush(e, st, with_step1, lj_atm_half(e)) : launch_atm(e, st, measure, with_step1);
+            fused = lj_atm ? launch_atm_flush(e, st, end, lj_atm_half(e)) : launch_atm(e, st, measure, end);
         }
         if (measure) launch_sum_partials(st, atm_grid(e), e.partials, h->acc);
     }
@@ -291,7 +300,7 @@ void enqueue_step(komd_gpu *h) {
         launch_container(e, e.stream);
     }
     // the step's integrate1 rides on the ATM flush when the once-per-triplet path runs
-    if (!enqueue_forces(h, false, nullptr, true)) {
+    if (!enqueue_forces(h, false, nullptr, END_STEP1)) {
         ProfScope ps(h, F_INTEGRATE);
         launch_step1(e, e.stream);
     }
@@ -307,6 +316,24 @@ void enqueue_step(komd_gpu *h) {
             cudaMemcpyAsync(r_async, e.r, sizeof(double) * 3 * (size_t)e.n, cudaMemcpyDeviceToHost, e.stream);
         e.hout_r = r_async;
     }
+}
+
+// Several steps in one call share a pass at each boundary: integrate0 of the
+// first step, then per step the container and the forces with a pass that ends
+// the step and starts the next, and the last step's end.  Not with the device
+// thermostat (it scales between the two), the host-buffer I/O of a step, or a
+// Verlet step without a force pass over the list (that pass clears the flag).
+bool steps_chain(komd_gpu *h) {
+    const Engine &e = h->e;
+    return !e.cfg.thermostat && !e.profiling && !e.hin_r && !e.hin_v && !e.hout_r && !e.hout_v && !e.hout_f &&
+           (!e.verlet || (e.cfg.terms & (KOMD_TERM_LJ | KOMD_TERM_ATM)));
+}
+void enqueue_chained(komd_gpu *h, StepEnd end) {
+    Engine &e = h->e;
+    launch_container(e, e.stream);
+    if (enqueue_forces(h, false, nullptr, end)) return;
+    if (end == END_KICK_DRIFT) launch_kick_drift(e, e.stream);
+    else launch_step1(e, e.stream);
 }
 
 // the flags' place in a landing buffer of a measure's sums
@@ -341,8 +368,7 @@ int alloc_atm_list(komd_gpu *h, int cap) {
         CK(dalloc(e.nl_count, e.n));
         set_kernel_attributes(e);
     }
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -352,8 +378,7 @@ int ensure_posd(komd_gpu *h) {
     CK(dalloc(e.posd, 3 * (size_t)e.n));
     CK(dalloc(e.seps_d, e.n));
     CK(dalloc(e.sig_d, e.n));
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -366,8 +391,7 @@ int alloc_verlet(komd_gpu *h, int cap) {
     CK(dalloc(e.zkey, e.n));
     CK(dalloc(e.vl, (size_t)cap * (size_t)e.n));
     CK(dalloc(e.vl_count, e.n));
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -618,7 +642,7 @@ int komd_gpu_destroy(komd_gpu *h) {
     Engine &e = h->e;
     cudaSetDevice(e.device);
     if (e.stream) cudaStreamSynchronize(e.stream);
-    if (e.graph) cudaGraphExecDestroy(e.graph);
+    drop_graphs(e);
     if (h->hgraph) cudaGraphExecDestroy(h->hgraph);
     if (h->land) cudaFreeHost(h->land);
     dfree(e.r); dfree(e.v); dfree(e.f); dfree(e.m); dfree(e.eps); dfree(e.sig);
@@ -659,8 +683,7 @@ int komd_gpu_set_stream(komd_gpu *h, void *stream) {
         CK(cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking));
         e.own_stream = true;
     }
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -781,8 +804,7 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
     if (rc) return rc;
     e.have_sites = true;
     e.have_cells = e.have_forces = false;
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -815,8 +837,7 @@ int komd_gpu_set_topology(komd_gpu *h, int64_t n_bonds, const int64_t *bonds, in
     if (!a.empty()) CK(cudaMemcpy(e.angles, a.data(), sizeof(int) * a.size(), cudaMemcpyHostToDevice));
     e.n_bonds = std::max<int64_t>(n_bonds, 0);
     e.n_angles = std::max<int64_t>(n_angles, 0);
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -943,18 +964,19 @@ static int run_probe(komd_gpu *h) {
     if (!(u.last_rmse <= u.probe_threshold)) {
         u.fallback = true;
         u.fallback_step = u.steps;
-        if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-        e.graph_valid = false;
+        drop_graphs(e);
     }
     return KOMD_OK;
 }
 
-// one step captured into *out (replacing it)
-static int capture_step(komd_gpu *h, cudaGraphExec_t *out) {
+// one step, or (chained) one of several from its container to the next one's
+// drift, captured into *out (replacing it)
+static int capture_step(komd_gpu *h, cudaGraphExec_t *out, bool chained = false) {
     Engine &e = h->e;
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(h);
+    if (chained) enqueue_chained(h, END_KICK_DRIFT);
+    else enqueue_step(h);
     CK(cudaStreamEndCapture(e.stream, &graph));
     if (*out) cudaGraphExecDestroy(*out);
     *out = nullptr;
@@ -983,6 +1005,17 @@ static int run_steps(komd_gpu *h, int64_t n_steps) {
     Engine &e = h->e;
     if (e.profiling) {
         for (int64_t k = 0; k < n_steps; k++) enqueue_step(h);
+        return check_launch("step");
+    }
+    if (n_steps > 1 && steps_chain(h)) {
+        if (!e.chain) {
+            const int rc = capture_step(h, &e.chain, true);
+            if (rc) return rc;
+        }
+        launch_step0(e, e.stream, true);
+        for (int64_t k = 1; k < n_steps; k++) CK(cudaGraphLaunch(e.chain, e.stream));
+        enqueue_chained(h, END_STEP1);
+        h->graph_steps += n_steps;
         return check_launch("step");
     }
     const int rc = ensure_graph(h);
@@ -1125,8 +1158,7 @@ int komd_gpu_set_pair_table(komd_gpu *h, int32_t n, const double *x, const doubl
         CK(dalloc(e.tab_y, n));
         CK(dalloc(e.tab_s, n));
         e.tab_n = n;
-        if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-        e.graph_valid = false;
+        drop_graphs(e);
     }
     // same-size tables are replaced in place: graphs already captured read the new values
     CK(cudaMemcpy(e.tab_x, x, sizeof(double) * n, cudaMemcpyHostToDevice));
@@ -1138,8 +1170,7 @@ int komd_gpu_set_pair_table(komd_gpu *h, int32_t n, const double *x, const doubl
     if (e.tab_lo != below || e.tab_hi != above) {
         e.tab_lo = below;
         e.tab_hi = above;
-        if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-        e.graph_valid = false;
+        drop_graphs(e);
     }
     return KOMD_OK;
 }
@@ -1170,8 +1201,7 @@ int komd_gpu_set_terms(komd_gpu *h, uint32_t terms) {
         }
     }
     e.cfg.terms = terms;
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -1342,8 +1372,7 @@ int komd_gpu_surrogate_load(komd_gpu *h, const float *params, const float *fmean
     u.last_rmse = -1.0;
     u.max_rmse = 0.0;
     u.fallback_step = -1;
-    if (e.graph) { cudaGraphExecDestroy(e.graph); e.graph = nullptr; }
-    e.graph_valid = false;
+    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -1958,12 +1987,12 @@ int batch_capture(komd_batch *b) {
         const int G = (int)b->pk.size();
         cudaError_t ce = cudaSuccess;
         if (G == 1) {
-            for (int k = 0; k < b->steps_per_graph; k++) launch_packed_step(b->pk[0], b->origin);
+            launch_packed_steps(b->pk[0], b->steps_per_graph, b->origin);
         } else {
             ce = cudaEventRecord(b->ev[0], b->origin);
             for (int g = 0; g < G && ce == cudaSuccess; g++) ce = cudaStreamWaitEvent(b->branch[g], b->ev[0], 0);
             for (int g = 0; g < G && ce == cudaSuccess; g++)
-                for (int k = 0; k < b->steps_per_graph; k++) launch_packed_step(b->pk[g], b->branch[g]);
+                launch_packed_steps(b->pk[g], b->steps_per_graph, b->branch[g]);
             for (int g = 0; g < G && ce == cudaSuccess; g++) {
                 ce = cudaEventRecord(b->ev[1 + g], b->branch[g]);
                 if (ce == cudaSuccess) ce = cudaStreamWaitEvent(b->origin, b->ev[1 + g], 0);

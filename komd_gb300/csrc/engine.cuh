@@ -248,6 +248,7 @@ struct PairParams {
     const float *offtab;       // per dimension nd*3 FP32 offsets centre(k+d) + shift - centre(k)
     // Verlet path
     const int *rebuild;
+    int *rebuild_done;         // the force pass clears the step's rebuild flag here: its consumers have run
     unsigned *vl;
     int *vl_count;
     int vl_cap;
@@ -476,7 +477,8 @@ struct Engine {
     // state
     bool have_sites = false, have_cells = false, have_forces = false;
     // graph
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph = nullptr;   // one whole step
+    cudaGraphExec_t chain = nullptr;   // a step of several: its container, forces, end and the next one's drift
     bool graph_valid = false;
     // profiling
     bool profiling = false;

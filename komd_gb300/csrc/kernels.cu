@@ -848,6 +848,49 @@ __device__ __forceinline__ void rows_out(const double *src_s, double *dst, int b
     }
 }
 
+// the drift of site s past its new position x: periodic wrap with its bias
+// update (b: the site's bias), the FP32 cell-local position and the skin test.
+// The centres of mass are formed by the binning of a rebuild (k_com_wrap_bin),
+// before anything reads them.
+__device__ __forceinline__ void drift_finish(const Step0Args &a, int s, int slot, double (&x)[3], double (&b)[3]) {
+    const Grid &g = a.g;
+    // Periodic_Kernel on the COM (= the position): strict comparisons, made on
+    // order-preserving integer keys (the FP64 pipe is the bottleneck here);
+    // the cell-local position x - bias is unchanged by a wrap
+    double off[3];
+    bool moved = false;
+    for (int d = 0; d < 3; d++) {
+        off[d] = 0.0;
+        const long long kx = dkey(x[d]);
+        if (!dkey_nan(x[d])) {
+            if (kx < dkey(g.low[d])) {
+                off[d] = g.L[d];
+                moved = true;
+            }
+            if (kx > dkey(g.high[d])) {
+                off[d] = -g.L[d];
+                moved = true;
+            }
+        }
+    }
+    if (moved) {   // r += shift over all three components, as Periodic_Kernel
+        for (int d = 0; d < 3; d++) {
+            x[d] = dadd(x[d], off[d]);
+            b[d] = dadd(b[d], off[d]);
+            a.bias[3 * s + d] = b[d];
+        }
+    }
+    float4 p = a.pos4[slot];
+    const float4 q = a.ref4[s];
+    p.x = d2f_rn(dsub(x[0], b[0]));
+    p.y = d2f_rn(dsub(x[1], b[1]));
+    p.z = d2f_rn(dsub(x[2], b[2]));
+    a.pos4[slot] = p;
+    const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+    if (dx * dx + dy * dy + dz * dz > a.half_skin2) *a.rebuild = 1;
+    for (int d = 0; d < 3; d++) a.r[3 * s + d] = x[d];
+}
+
 // r_in / v_in: where this step's positions and velocities are read (the
 // engine's own arrays, or a caller's host buffers reached over the host link);
 // r_out: an extra host copy of the new positions (nullptr: none).  Launched
@@ -858,14 +901,8 @@ __device__ __forceinline__ void step0_fused_body(const Step0Args &a, int bid) {
     double *r = a.r, *v = a.v;
     const double *__restrict__ f = a.f, *__restrict__ hdtm = a.hdtm;
     const double dt = a.dt;
-    const Grid &g = a.g;
-    double *__restrict__ bias = a.bias;
-    const float4 *__restrict__ ref4 = a.ref4;
-    const float half_skin2 = a.half_skin2;
-    int *__restrict__ rebuild = a.rebuild;
-    double *__restrict__ com = a.com;
+    const double *__restrict__ bias = a.bias;
     const int *__restrict__ site_slot = a.site_slot;
-    float4 *__restrict__ pos4 = a.pos4;
     const double *r_in = a.r_in, *v_in = a.v_in;
     double *r_out = a.r_out;
     const int t = threadIdx.x;
@@ -890,46 +927,7 @@ __device__ __forceinline__ void step0_fused_body(const Step0Args &a, int bid) {
             x[d] = dadd(ri[d], dmul(vv, dt));
             b[d] = bias[3 * s + d];
         }
-        // Periodic_Kernel on the COM (= the position): strict comparisons, made on
-        // order-preserving integer keys (the FP64 pipe is the bottleneck here);
-        // the cell-local position x - bias is unchanged by a wrap
-        double off[3];
-        bool moved = false;
-        for (int d = 0; d < 3; d++) {
-            off[d] = 0.0;
-            const long long kx = dkey(x[d]);
-            if (!dkey_nan(x[d])) {
-                if (kx < dkey(g.low[d])) {
-                    off[d] = g.L[d];
-                    moved = true;
-                }
-                if (kx > dkey(g.high[d])) {
-                    off[d] = -g.L[d];
-                    moved = true;
-                }
-            }
-        }
-        if (moved) {   // r += shift over all three components, as Periodic_Kernel
-            for (int d = 0; d < 3; d++) {
-                x[d] = dadd(x[d], off[d]);
-                b[d] = dadd(b[d], off[d]);
-                bias[3 * s + d] = b[d];
-            }
-        }
-        float4 p = pos4[site_slot[s]];
-        p.x = d2f_rn(dsub(x[0], b[0]));
-        p.y = d2f_rn(dsub(x[1], b[1]));
-        p.z = d2f_rn(dsub(x[2], b[2]));
-        pos4[site_slot[s]] = p;
-        {
-            const float4 q = ref4[s];
-            const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-            if (dx * dx + dy * dy + dz * dz > half_skin2) *rebuild = 1;
-        }
-        for (int d = 0; d < 3; d++) {
-            r[3 * s + d] = x[d];
-            com[3 * s + d] = x[d];
-        }
+        drift_finish(a, s, site_slot[s], x, b);
         if (r_out)   // each thread overwrites only the entries it read
             for (int d = 0; d < 3; d++) s_r[3 * t + d] = x[d];
     }
@@ -1373,6 +1371,7 @@ PairParams pair_params(Engine &e) {
     p.virial_compat = e.cfg.virial_mode == KOMD_VIRIAL_COMPAT;
     p.offtab = e.offtab;
     p.rebuild = e.rebuild;
+    p.rebuild_done = e.verlet ? e.rebuild : nullptr;
     p.vl = e.vl;
     p.vl_count = e.vl_count;
     p.vl_cap = e.vl_cap;
@@ -1534,6 +1533,104 @@ __global__ void __launch_bounds__(kIoBlock) k_atm_flush_step1(FlushArgs a) {
     flush_step1_body(a, blockIdx.x);
 }
 
+// The end of one step and the start of the next in one pass over the sites
+// (several steps in one call): the last force term's sums into f (KICK_FLUSH:
+// the triplets' fixed-point sums; KICK_LEARNED: the learned term's, from fsur;
+// KICK_PLAIN: f is complete), integrate1 of the step and integrate0 of the next
+// -- the half-kick f dt/2m is formed once for both -- and the drift.  The
+// operations and their order are those of k_atm_flush_step1 / k_sur_apply_step1
+// / k_step1 and k_step0_fused.  The rebuild flag is set here for the next step;
+// the force pass has cleared it (PairParams::rebuild_done).  256,000 sites: 18 +
+// 13.7 us for the two kernels, 24.4 us for this one.
+enum { KICK_PLAIN = 0, KICK_FLUSH = 1, KICK_LEARNED = 2 };
+template <int MODE>
+__device__ __forceinline__ void kick_drift_body(const FlushArgs &a, const Step0Args &dr, float4 *fsur, int bid) {
+    const int s = bid * blockDim.x + threadIdx.x;
+    if (s >= a.n) return;
+    const int slot = a.site_slot[s];
+    long long q[3];
+    double fo[3], vo[3], ro[3], b[3];
+    float4 fs = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (MODE == KICK_FLUSH)
+        for (int d = 0; d < 3; d++) q[d] = (long long)a.acc[3 * slot + d];
+    if (MODE == KICK_LEARNED) fs = fsur[slot];
+    if (MODE == KICK_FLUSH && a.fown) {   // the half-list pass's FP32 force, widened exactly
+        const float4 o = a.fown[slot];
+        fo[0] = (double)o.x;
+        fo[1] = (double)o.y;
+        fo[2] = (double)o.z;
+    } else {
+        for (int d = 0; d < 3; d++) fo[d] = a.f[3 * s + d];
+    }
+    for (int d = 0; d < 3; d++) {
+        vo[d] = a.v[3 * s + d];
+        ro[d] = dr.r[3 * s + d];
+        b[d] = dr.bias[3 * s + d];
+    }
+    const double c = a.hdtm[s];
+    bool bad = false;
+    double x[3];
+    for (int d = 0; d < 3; d++) {
+        double fd = fo[d];
+        if (MODE == KICK_FLUSH) {
+            a.acc[3 * slot + d] = 0ull;
+            fd = fo[d] + a.scale_fix * (double)q[d];
+            a.f[3 * s + d] = fd;
+        }
+        if (MODE == KICK_LEARNED) {
+            fd = fo[d] + (double)(d == 0 ? fs.x : (d == 1 ? fs.y : fs.z));
+            a.f[3 * s + d] = fd;
+        }
+        const double kick = dmul(fd, c), v1 = dadd(vo[d], kick);
+        bad |= !isfinite(v1);
+        const double v2 = dadd(v1, kick);
+        a.v[3 * s + d] = v2;
+        x[d] = dadd(ro[d], dmul(v2, dr.dt));
+    }
+    if (MODE == KICK_LEARNED) fsur[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bad) atomicOr(&a.err[E_NONFINITE], 1);
+    drift_finish(dr, s, slot, x, b);
+}
+template <int MODE>
+__global__ void __launch_bounds__(kIoBlock) k_kick_drift(FlushArgs a, Step0Args dr, float4 *fsur) {
+    pdl_wait();
+    kick_drift_body<MODE>(a, dr, fsur, blockIdx.x);
+}
+
+// the same for systems outside the fused drift (per-step cells, molecules of
+// several sites): k_step1's and k_step0's operations
+__global__ void k_step10(int n, double *__restrict__ r, double *__restrict__ v, const double *__restrict__ f,
+                         const double *__restrict__ hdtm, double dt, const double *__restrict__ bias,
+                         const float4 *__restrict__ ref4, float half_skin2, int *__restrict__ rebuild,
+                         int *__restrict__ err) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const double c = hdtm[s];
+    double x[3], vo[3], fo[3];
+    for (int d = 0; d < 3; d++) {
+        vo[d] = v[3 * s + d];
+        fo[d] = f[3 * s + d];
+        x[d] = r[3 * s + d];
+    }
+    bool bad = false;
+    for (int d = 0; d < 3; d++) {
+        const double kick = dmul(fo[d], c), v1 = dadd(vo[d], kick);
+        bad |= !isfinite(v1);
+        const double v2 = dadd(v1, kick);
+        v[3 * s + d] = v2;
+        x[d] = dadd(x[d], dmul(v2, dt));
+        r[3 * s + d] = x[d];
+    }
+    if (bad) atomicOr(&err[E_NONFINITE], 1);
+    if (bias) {
+        const float4 q = ref4[s];
+        const float dx = __double2float_rn(dsub(x[0], bias[3 * s])) - q.x;
+        const float dy = __double2float_rn(dsub(x[1], bias[3 * s + 1])) - q.y;
+        const float dz = __double2float_rn(dsub(x[2], bias[3 * s + 2])) - q.z;
+        if (dx * dx + dy * dy + dz * dz > half_skin2) *rebuild = 1;
+    }
+}
+
 // f[site] += 2 sign nu g (fixed point -> FP64) and the accumulators back to 0
 __global__ void k_atm_flush(int n, const int *__restrict__ slot_site, unsigned long long *__restrict__ acc,
                             double *__restrict__ f, double scale_fix, const float4 *__restrict__ own) {
@@ -1599,27 +1696,32 @@ AtmParams atm_params(const Engine &e) {
     return p;
 }
 
-// the fixed-point sums of the once-per-triplet sweep into f (and, with_step1,
-// integrate1 of the step); returns with_step1
-bool launch_atm_flush(Engine &e, cudaStream_t st, bool with_step1, bool force_units) {
+// the fixed-point sums of the once-per-triplet sweep into f and, where a kernel
+// takes it along, the step's end; returns whether it did
+bool launch_atm_flush(Engine &e, cudaStream_t st, StepEnd end, bool force_units) {
     const double sign = e.cfg.atm_sign == KOMD_ATM_SIGN_REFERENCE ? 1.0 : -1.0;
     const double scale_fix = force_units ? 1.0 / kAtmFix : 2.0 * sign * e.cfg.nu / kAtmFix;
     const float4 *own = force_units ? half_own(e) : nullptr;   // force_units: the half-list pass ran
-    if (with_step1) {
+    if (end == END_STEP1) {
         launch_pdl(k_atm_flush_step1, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, scale_fix, own));
+        return true;
+    }
+    if (end == END_KICK_DRIFT && e.fused_drift) {
+        launch_pdl(k_kick_drift<KICK_FLUSH>, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, scale_fix, own),
+                   step0_args(e), (float4 *)nullptr);
         return true;
     }
     k_atm_flush<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.slot_site, e.atm_acc, e.f, scale_fix, own);
     return false;
 }
 
-bool launch_atm(Engine &e, cudaStream_t st, bool measure, bool with_step1) {
+bool launch_atm(Engine &e, cudaStream_t st, bool measure, StepEnd end) {
     AtmParams p = atm_params(e);
     const bool compat = e.cfg.atm_enum == KOMD_ATM_ENUM_COMPAT;
     if (!measure && !compat && e.cfg.precision == KOMD_FP32 && e.atm_acc) {
         // every triplet once (lowest slot), fixed-point scatter, then the flush into f
         k_atm_s<<<nblk(e.n, kWarpsPerBlock), kBlock, atm_smem(e), st>>>(p);
-        return launch_atm_flush(e, st, with_step1, false);
+        return launch_atm_flush(e, st, end, false);
     }
     if (e.cfg.precision == KOMD_FP64)
         atm_dispatch_d(p, measure, compat, atm_grid(e), atm_warps(e), atm_smem(e), st);
@@ -1636,6 +1738,25 @@ void launch_step0(Engine &e, cudaStream_t st, bool in_step) {
     k_step0<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
                                               e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, hs * hs,
                                               e.rebuild);
+}
+
+// integrate1 of a step and integrate0 of the next
+void launch_kick_drift(Engine &e, cudaStream_t st) {
+    if (e.fused_drift) {
+        launch_pdl(k_kick_drift<KICK_PLAIN>, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, 0.0, nullptr),
+                   step0_args(e), (float4 *)nullptr);
+        return;
+    }
+    const float hs = (float)(0.5 * e.cfg.skin);
+    k_step10<<<nblk(e.n, 128), 128, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
+                                             e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, hs * hs,
+                                             e.rebuild, e.err);
+}
+
+// the same with the learned term's forces (fsur, slot order) added first; needs the fused drift
+void launch_learned_kick_drift(Engine &e, float *fsur, cudaStream_t st) {
+    launch_pdl(k_kick_drift<KICK_LEARNED>, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, 0.0, nullptr),
+               step0_args(e), reinterpret_cast<float4 *>(fsur));
 }
 
 void launch_step1(Engine &e, cudaStream_t st) {
@@ -1746,23 +1867,35 @@ __global__ void __launch_bounds__(kIoBlock, 8) k_atm_flush_step1_p(const FlushAr
     flush_step1_body(a[r], blockIdx.x - start[r]);
 }
 
+__global__ void __launch_bounds__(kIoBlock, 5) k_kick_drift_p(const FlushArgs *a, const Step0Args *dr, const int *start,
+                                                              int nrep) {
+    const int r = packed_rep(start, nrep, blockIdx.x);
+    kick_drift_body<KICK_FLUSH>(a[r], dr[r], nullptr, blockIdx.x - start[r]);
+}
+
 // blocks per replica of the container stages: on a step without a rebuild
 // they exit at once; on a rebuild step a replica's blocks do its whole
 // binning, so too few of them make a long tail for the launch
 int packed_blocks_container(const Engine &e) { return std::max(1, std::min(nblk(e.n_mol, 256), 64)); }
 
-// one step of every replica: the stages of enqueue_step on the Verlet path
-// with the fused drift and the half-list pass, each stage one launch
-void launch_packed_step(const PackedStep &pk, cudaStream_t st) {
+// `steps` steps of every replica: the stages of enqueue_steps on the Verlet path
+// with the fused drift and the half-list pass, each stage one launch; a step's
+// flush takes the next one's drift along
+void launch_packed_steps(const PackedStep &pk, int steps, cudaStream_t st) {
     const int nr = pk.nrep;
-    k_step0_fused_p<<<pk.step0.blocks, kIoBlock, 0, st>>>((const Step0Args *)pk.step0.args, pk.step0.start, nr);
-    k_com_wrap_bin_p<<<pk.bin.blocks, 256, 0, st>>>((const BinArgs *)pk.bin.args, pk.bin.start, nr);
-    k_scan2_p<<<nr, 1024, 0, st>>>((const ScanArgs *)pk.scan.args);
-    k_scatter_mol_p<<<pk.scatter.blocks, 256, 0, st>>>((const ScatterArgs *)pk.scatter.args, pk.scatter.start, nr);
-    k_cell_sort_p<<<pk.sort.blocks, kBlock, 0, st>>>((const SortArgs *)pk.sort.args, pk.sort.start, nr);
-    launch_packed_pair_stages(pk, st, true);
-    launch_packed_pair_stages(pk, st, false);
-    k_atm_flush_step1_p<<<pk.flush.blocks, kIoBlock, 0, st>>>((const FlushArgs *)pk.flush.args, pk.flush.start, nr);
+    const Step0Args *dr = (const Step0Args *)pk.step0.args;
+    const FlushArgs *fl = (const FlushArgs *)pk.flush.args;
+    k_step0_fused_p<<<pk.step0.blocks, kIoBlock, 0, st>>>(dr, pk.step0.start, nr);
+    for (int k = 0; k < steps; k++) {
+        k_com_wrap_bin_p<<<pk.bin.blocks, 256, 0, st>>>((const BinArgs *)pk.bin.args, pk.bin.start, nr);
+        k_scan2_p<<<nr, 1024, 0, st>>>((const ScanArgs *)pk.scan.args);
+        k_scatter_mol_p<<<pk.scatter.blocks, 256, 0, st>>>((const ScatterArgs *)pk.scatter.args, pk.scatter.start, nr);
+        k_cell_sort_p<<<pk.sort.blocks, kBlock, 0, st>>>((const SortArgs *)pk.sort.args, pk.sort.start, nr);
+        launch_packed_pair_stages(pk, st, true);
+        launch_packed_pair_stages(pk, st, false);
+        if (k + 1 < steps) k_kick_drift_p<<<pk.flush.blocks, kIoBlock, 0, st>>>(fl, dr, pk.flush.start, nr);
+        else k_atm_flush_step1_p<<<pk.flush.blocks, kIoBlock, 0, st>>>(fl, pk.flush.start, nr);
+    }
 }
 
 

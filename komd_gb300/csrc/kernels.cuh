@@ -17,12 +17,15 @@ int vlist_blocks(const Engine &e);
 void launch_counts(Engine &e, cudaStream_t st);
 void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc);
 void launch_limit(Engine &e, cudaStream_t st);
-// ATM forces; with_step1 (step graphs only) lets the FULL FP32 path fuse
-// integrate1 into its flush: returns true when it did
-bool launch_atm(Engine &e, cudaStream_t st, bool measure, bool with_step1 = false);
+// what follows the last force term in a step: nothing here, integrate1, or
+// integrate1 and the next step's integrate0
+enum StepEnd { END_NONE, END_STEP1, END_KICK_DRIFT };
+// ATM forces; `end` (steps only) lets the FULL FP32 path take the step's end
+// along with its flush: returns true when it did
+bool launch_atm(Engine &e, cudaStream_t st, bool measure, StepEnd end = END_NONE);
 AtmParams atm_params(const Engine &e);
 // force_units: the sums are in force units (half-list pass), else in units of 2 sign nu
-bool launch_atm_flush(Engine &e, cudaStream_t st, bool with_step1, bool force_units);
+bool launch_atm_flush(Engine &e, cudaStream_t st, StepEnd end, bool force_units);
 // LJ forces and the once-per-triplet ATM sweep in one pass (FP32, FULL, Verlet)
 void launch_lj_atm(Engine &e, cudaStream_t st);
 // true when launch_lj_atm runs the half-list form, whose fixed-point sums are
@@ -36,6 +39,8 @@ bool half_plain(const PairParams &p);
 // in_step (step graphs only): the fused drift path when the engine qualifies
 void launch_step0(Engine &e, cudaStream_t st, bool in_step = false);
 void launch_step1(Engine &e, cudaStream_t st);
+void launch_kick_drift(Engine &e, cudaStream_t st);
+void launch_learned_kick_drift(Engine &e, float *fsur, cudaStream_t st);
 void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc);
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta);
 void launch_pair_table(Engine &e, cudaStream_t st);
@@ -80,7 +85,7 @@ int packed_blocks_container(const Engine &e);
 int packed_blocks_vbuild(const Engine &e);
 VbShape vb_shape(double sites, int64_t cells, int num_sms);
 size_t vb_smem(const VbShape &v);
-void launch_packed_step(const PackedStep &pk, cudaStream_t st);          // kernels.cu: all eight stages
+void launch_packed_steps(const PackedStep &pk, int steps, cudaStream_t st);   // kernels.cu: all stages
 void launch_packed_pair_stages(const PackedStep &pk, cudaStream_t st, bool vbuild);   // pair_tile.cu
 int kinetic_grid(const Engine &e);
 size_t atm_smem(const Engine &e);

@@ -602,6 +602,7 @@ __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, 
     const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq;
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
     float m_u = 0.f, m_pairs = 0.f, m_w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // each block walks `per` consecutive groups of 8 slots: neighbouring slots share
     // most of their neighbours, so the gathers of one group hit L1 lines of the last
@@ -647,6 +648,7 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm(PairParams p, AtmParams a, in
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float4 *se = s_dyn + w * 2 * p.nl_cap, *sq = se + p.nl_cap;
     const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq, rc3f = (float)a.rc2;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
     float m_u = 0.f, m_pairs = 0.f, m_w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -811,6 +813,7 @@ __device__ __forceinline__ void lj_atm_half_body(const PairParams &p, const AtmP
     float4 *se = s_dyn + (size_t)w * (2 * capa + capr), *sq = se + capa, *sr = sq + capa;
     const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq, rc3f = (float)a.rc2;
     const unsigned lt = lanemask_lt();
+    if (bid == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
     for (int it = 0; it < per; it++) {
         const int i = (bid * per + it) * 8 + w;
         if (i >= n) break;   // warp-uniform; later groups of this block are past n too
