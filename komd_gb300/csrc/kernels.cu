@@ -1283,6 +1283,11 @@ __global__ void k_velocity_scale(int n, double *__restrict__ v, const double *__
 // ===========================================================================
 static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
+// threads per block of the per-site kernels: 256 where that gives two blocks per
+// SM, else 64, so that a small system's FP64 work (the narrow pipe: 16 cycles a
+// warp instruction on its SM) spreads over more SMs
+static inline int site_block(const Engine &e, long long n) { return n >= 512ll * e.num_sms ? 256 : 64; }
+
 BinArgs bin_args(const Engine &e) {
     return BinArgs{e.g, (int)e.n_mol, e.mol_off, e.r, e.m, e.com, e.mol_cell, e.mol_rank, e.cell_count, e.cell_mcount,
                    e.verlet ? e.bias : nullptr, e.verlet ? e.rebuild : nullptr, e.exact_com, e.fused_drift ? 1 : 0,
@@ -1319,7 +1324,8 @@ void launch_container(Engine &e, cudaStream_t st) {
     // of every binning after reading them
     // grid-stride kernels on a resident grid: steps without a rebuild launch few blocks
     const int res = e.num_sms * 8;
-    launch_pdl(k_com_wrap_bin, std::min(nblk(e.n_mol, 256), res), 256, 0, st, bin_args(e));
+    const int mb = site_block(e, e.n_mol);
+    launch_pdl(k_com_wrap_bin, std::min(nblk(e.n_mol, mb), res * (256 / mb)), mb, 0, st, bin_args(e));
     launch_pdl(k_scan2, 1, 1024, 0, st, scan_args(e));
     launch_pdl(k_scatter_mol, std::min(nblk(e.n_mol, 256), res), 256, 0, st, scatter_args(e));
     // four warps a block: with few cells the chain of loads bounds the sort, not its throughput
@@ -1427,7 +1433,8 @@ void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc) {
 }
 
 void launch_limit(Engine &e, cudaStream_t st) {
-    k_limit<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.eps, e.sig, e.cfg.limit, e.f);
+    const int b = site_block(e, e.n);
+    k_limit<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.eps, e.sig, e.cfg.limit, e.f);
 }
 
 size_t atm_smem(const Engine &e) {
@@ -1703,12 +1710,14 @@ bool launch_atm_flush(Engine &e, cudaStream_t st, StepEnd end, bool force_units)
     const double scale_fix = force_units ? 1.0 / kAtmFix : 2.0 * sign * e.cfg.nu / kAtmFix;
     const float4 *own = force_units ? half_own(e) : nullptr;   // force_units: the half-list pass ran
     if (end == END_STEP1) {
-        launch_pdl(k_atm_flush_step1, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, scale_fix, own));
+        const int b = site_block(e, e.n);
+        launch_pdl(k_atm_flush_step1, nblk(e.n, b), b, 0, st, flush_args(e, scale_fix, own));
         return true;
     }
     if (end == END_KICK_DRIFT && e.fused_drift) {
-        launch_pdl(k_kick_drift<KICK_FLUSH>, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, scale_fix, own),
-                   step0_args(e), (float4 *)nullptr);
+        const int b = site_block(e, e.n);
+        launch_pdl(k_kick_drift<KICK_FLUSH>, nblk(e.n, b), b, 0, st, flush_args(e, scale_fix, own), step0_args(e),
+                   (float4 *)nullptr);
         return true;
     }
     k_atm_flush<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.slot_site, e.atm_acc, e.f, scale_fix, own);
@@ -1732,43 +1741,48 @@ bool launch_atm(Engine &e, cudaStream_t st, bool measure, StepEnd end) {
 void launch_step0(Engine &e, cudaStream_t st, bool in_step) {
     const float hs = (float)(0.5 * e.cfg.skin);
     if (in_step && e.fused_drift) {
-        k_step0_fused<<<nblk(e.n, kIoBlock), kIoBlock, 0, st>>>(step0_args(e));
+        const int b = site_block(e, e.n);
+        k_step0_fused<<<nblk(e.n, b), b, 0, st>>>(step0_args(e));
         return;
     }
-    k_step0<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
+    const int b = site_block(e, e.n);
+    k_step0<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
                                               e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, hs * hs,
                                               e.rebuild);
 }
 
 // integrate1 of a step and integrate0 of the next
 void launch_kick_drift(Engine &e, cudaStream_t st) {
+    const int b = site_block(e, e.n);
     if (e.fused_drift) {
-        launch_pdl(k_kick_drift<KICK_PLAIN>, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, 0.0, nullptr),
-                   step0_args(e), (float4 *)nullptr);
+        launch_pdl(k_kick_drift<KICK_PLAIN>, nblk(e.n, b), b, 0, st, flush_args(e, 0.0, nullptr), step0_args(e),
+                   (float4 *)nullptr);
         return;
     }
     const float hs = (float)(0.5 * e.cfg.skin);
-    k_step10<<<nblk(e.n, 128), 128, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
+    k_step10<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
                                              e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, hs * hs,
                                              e.rebuild, e.err);
 }
 
 // the same with the learned term's forces (fsur, slot order) added first; needs the fused drift
 void launch_learned_kick_drift(Engine &e, float *fsur, cudaStream_t st) {
-    launch_pdl(k_kick_drift<KICK_LEARNED>, nblk(e.n, kIoBlock), kIoBlock, 0, st, flush_args(e, 0.0, nullptr),
-               step0_args(e), reinterpret_cast<float4 *>(fsur));
+    const int b = site_block(e, e.n);
+    launch_pdl(k_kick_drift<KICK_LEARNED>, nblk(e.n, b), b, 0, st, flush_args(e, 0.0, nullptr), step0_args(e),
+               reinterpret_cast<float4 *>(fsur));
 }
 
 void launch_step1(Engine &e, cudaStream_t st) {
-    k_step1<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.v, e.f, e.hdtm, e.err,
+    const int b = site_block(e, e.n);
+    k_step1<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.v, e.f, e.hdtm, e.err,
                                               e.verlet ? e.rebuild : nullptr);
 }
 
 int kinetic_grid(const Engine &e) { return std::min(nblk(e.n, kBlock), e.num_sms * 2); }
 
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta) {
-    const int blocks = std::min(nblk(3 * e.n, 256), e.num_sms * 8);
-    k_velocity_scale<<<blocks, 256, 0, st>>>((int)e.n, e.v, acc, e.cfg.temperature_target, sci_factor(), beta, e.err);
+    const int b = site_block(e, 3 * e.n);
+    k_velocity_scale<<<std::min(nblk(3 * e.n, b), e.num_sms * 8), b, 0, st>>>((int)e.n, e.v, acc, e.cfg.temperature_target, sci_factor(), beta, e.err);
 }
 
 // the kinetic sums into acc (R_NSLOTS), whose other slots become zero
