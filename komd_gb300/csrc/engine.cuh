@@ -478,7 +478,7 @@ struct Engine {
     bool have_sites = false, have_cells = false, have_forces = false;
     // graph
     cudaGraphExec_t graph = nullptr;   // one whole step
-    cudaGraphExec_t chain = nullptr;   // a step of several: its container, forces, end and the next one's drift
+    cudaGraphExec_t several = nullptr; // several steps of one call
     bool graph_valid = false;
     // profiling
     bool profiling = false;
