@@ -650,7 +650,7 @@ int komd_gpu_destroy(komd_gpu *h) {
     dfree(e.mol_off); dfree(e.mol_cell); dfree(e.mol_rank); dfree(e.com);
     dfree(e.cell_count); dfree(e.cell_start); dfree(e.cell_mcount); dfree(e.cell_mstart); dfree(e.cell_mols);
     dfree(e.slot_site); dfree(e.skey); dfree(e.pos4); dfree(e.seps); dfree(e.posd); dfree(e.seps_d); dfree(e.sig_d);
-    dfree(e.nl); dfree(e.nl_count); dfree(e.bonds); dfree(e.angles); dfree(e.partials); dfree(e.kin_done);
+    dfree(e.nl); dfree(e.nl_count); dfree(e.bonds); dfree(e.angles); dfree(e.bond_block); dfree(e.comp_off); dfree(e.comp_terms); dfree(e.partials); dfree(e.kin_done);
     dfree(e.tab_x); dfree(e.tab_y); dfree(e.tab_s); dfree(e.atm_acc); dfree(e.fown);
     dfree(e.rdf); dfree(e.lj_hist); dfree(e.counts); dfree(h->f_scratch); dfree(h->prof); dfree(h->acc); dfree(h->thermo_acc); dfree(e.offtab);
     dfree(e.nboff); dfree(e.vb_next); dfree(e.rebuild); dfree(e.bias); dfree(e.ref4); dfree(e.slot_cell); dfree(e.zkey); dfree(e.vl); dfree(e.vl_count);
@@ -724,6 +724,7 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
     CK(dalloc(e.mol_off, e.n_mol + 1)); CK(dalloc(e.mol_cell, e.n_mol)); CK(dalloc(e.mol_rank, e.n_mol));
     CK(dalloc(e.com, 3 * e.n_mol)); CK(dalloc(e.cell_mols, e.n_mol));
     CK(dalloc(e.slot_site, n)); CK(dalloc(e.skey, n)); CK(dalloc(e.pos4, n)); CK(dalloc(e.seps, n));
+    CK(cudaMemset(e.site_slot, 0, sizeof(int) * n));   // a drift before the first container pass writes pos4 through it
     CK(dalloc(e.counts, n));
     dfree(e.posd); dfree(e.seps_d); dfree(e.sig_d);
     if (h->want_posd) {
@@ -818,6 +819,63 @@ int komd_gpu_set_state(komd_gpu *h, const double *r, const double *v) {
     return KOMD_OK;
 }
 
+// the terms by connected component for k_bonded_mol, where every component has at
+// most kBondTerms terms and a range of at most kBondSites sites to itself
+static int bond_layout(Engine &e, const std::vector<int> &b, const std::vector<int> &a) {
+    e.bond_blocks = 0;
+    e.bond_sites = e.n;
+    std::vector<int> root(e.n);
+    for (int64_t s = 0; s < e.n; s++) root[s] = (int)s;
+    auto find = [&](int x) {
+        while (root[x] != x) x = root[x] = root[root[x]];
+        return x;
+    };
+    auto join = [&](int x, int y) {   // the lowest site is the root
+        x = find(x);
+        y = find(y);
+        root[std::max(x, y)] = std::min(x, y);
+    };
+    const size_t nb = b.size() / 2, na = a.size() / 3;
+    for (size_t k = 0; k < nb; k++) join(b[2 * k], b[2 * k + 1]);
+    for (size_t k = 0; k < na; k++) {
+        join(a[3 * k], a[3 * k + 1]);
+        join(a[3 * k + 1], a[3 * k + 2]);
+    }
+    std::vector<int> count(e.n, 0), last(e.n, -1), comp(e.n, -1), off(1, 0);
+    for (size_t k = 0; k < nb; k++)
+        if (++count[find(b[2 * k])] > kBondTerms) return KOMD_OK;
+    for (size_t k = 0; k < na; k++)
+        if (++count[find(a[3 * k])] > kBondTerms) return KOMD_OK;
+    for (int64_t s = 0; s < e.n; s++) last[find((int)s)] = (int)s;
+    std::vector<int4> blocks;
+    int end = 0;   // of the components so far
+    for (int s = 0; s < (int)e.n; s++) {
+        if (root[s] != s || count[s] == 0) continue;
+        if (s < end || last[s] - s >= kBondSites) return KOMD_OK;
+        end = last[s] + 1;
+        comp[s] = (int)off.size() - 1;
+        if (blocks.empty() || comp[s] - blocks.back().x == kBondComps || end - blocks.back().z > kBondSites)
+            blocks.push_back(make_int4(comp[s], 0, s, 0));
+        blocks.back().y = comp[s] + 1;
+        blocks.back().w = end;
+        off.push_back(off.back() + count[s]);
+    }
+    if (blocks.empty()) return KOMD_OK;
+    std::vector<int> at(off.begin(), off.end() - 1);
+    std::vector<int4> terms(nb + na);
+    for (size_t k = 0; k < nb; k++) terms[at[comp[find(b[2 * k])]]++] = make_int4(b[2 * k], b[2 * k + 1], -1, 0);
+    for (size_t k = 0; k < na; k++)
+        terms[at[comp[find(a[3 * k])]]++] = make_int4(a[3 * k], a[3 * k + 1], a[3 * k + 2], 0);
+    CK(dalloc(e.bond_block, blocks.size()));
+    CK(dalloc(e.comp_off, off.size()));
+    CK(dalloc(e.comp_terms, terms.size()));
+    CK(cudaMemcpy(e.bond_block, blocks.data(), sizeof(int4) * blocks.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(e.comp_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(e.comp_terms, terms.data(), sizeof(int4) * terms.size(), cudaMemcpyHostToDevice));
+    e.bond_blocks = (int)blocks.size();
+    return KOMD_OK;
+}
+
 int komd_gpu_set_topology(komd_gpu *h, int64_t n_bonds, const int64_t *bonds, int64_t n_angles,
                           const int64_t *angles) {
     if (!h || !h->e.have_sites) return fail(KOMD_ERR_STATE, "no sites uploaded");
@@ -831,6 +889,7 @@ int komd_gpu_set_topology(komd_gpu *h, int64_t n_bonds, const int64_t *bonds, in
         if (angles[k] < 0 || angles[k] >= e.n) return fail(KOMD_ERR_ARG, "angle index out of range");
         a[k] = (int)angles[k];
     }
+    if (int rc = bond_layout(e, b, a)) return rc;
     CK(dalloc(e.bonds, b.size()));
     CK(dalloc(e.angles, a.size()));
     if (!b.empty()) CK(cudaMemcpy(e.bonds, b.data(), sizeof(int) * b.size(), cudaMemcpyHostToDevice));
@@ -2220,13 +2279,13 @@ int komd_gpu_kernels_per_step(komd_gpu *h) {
     if (!h) return -1;
     const Engine &e = h->e;
     // integrate0/1; the container pass (com/wrap/bin, scan, scatter, cell sort, and
-    // on the Verlet path the list build and the FP32 refresh unless the drift does it)
-    int k = 2 + 4 + (e.verlet ? (e.fused_drift ? 1 : 2) : 0);
+    // on the Verlet path the list build)
+    int k = 2 + 4 + (e.verlet ? 1 : 0);
     if (e.cfg.terms & (KOMD_TERM_LJ | KOMD_TERM_FENE | KOMD_TERM_ATM)) k++;   /* pair pass (else a memset) */
     if (e.cfg.terms & KOMD_TERM_TABULATED) k++;
     if (!surrogate_on(h) && (e.cfg.terms & KOMD_TERM_ATM) && e.atm_acc) k--;   /* integrate1 fused into the ATM flush */
-    if ((e.cfg.terms & KOMD_TERM_BONDED) && e.n_bonds > 0) k++;
-    if ((e.cfg.terms & KOMD_TERM_BONDED) && e.n_angles > 0) k++;
+    if (e.cfg.terms & KOMD_TERM_BONDED)   // one pass over small molecules, or one by bond and one by angle
+        k += e.bond_blocks > 0 && e.bond_sites == e.n ? 1 : (e.n_bonds > 0) + (e.n_angles > 0);
     if (e.cfg.terms & KOMD_TERM_LIMIT) k++;
     if (e.cfg.thermostat) k += 2;  /* kinetic sums, velocity scaling */
     if (surrogate_on(h)) k += 4;   /* descriptors, MLP, forces, apply */

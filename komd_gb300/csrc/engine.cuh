@@ -321,6 +321,9 @@ inline void sw_params(double rc, double width, int &on, float &rc2, float &iw) {
 // Arguments of the step kernels of the Verlet path, one struct per kernel, so
 // that one launch can serve one system (the struct by value) or all replicas
 // of a batch (an array of them, a block range per replica).
+// k_bonded_mol: components (and threads) and sites of a block, terms of a component.
+// Longer components would be a serial chain on one thread: they keep the atomics.
+constexpr int kBondComps = 64, kBondSites = 256, kBondTerms = 16;
 struct BinArgs {              // k_com_wrap_bin: COM, periodic wrap, binning
     Grid g;
     int n_mol;
@@ -334,6 +337,7 @@ struct BinArgs {              // k_com_wrap_bin: COM, periodic wrap, binning
     const unsigned char *exact_com;
     int wrapped;
     int single;               // every molecule has one site (the counts of both kinds are equal)
+    float in_lo[3], in_hi[3]; // the domain's bounds rounded inwards (com_inside)
 };
 struct ScanArgs {             // k_scan2: exclusive scans of the cell counts
     int nc;
@@ -464,6 +468,11 @@ struct Engine {
     int nl_cap = 64;
     // topology
     int *bonds = nullptr, *angles = nullptr;
+    // the same by connected component where all are small (k_bonded_mol)
+    int4 *bond_block = nullptr, *comp_terms = nullptr;
+    int *comp_off = nullptr;
+    int bond_blocks = 0;       // 0: not laid out
+    int64_t bond_sites = -1;   // the site count they were laid out for
     int64_t n_bonds = 0, n_angles = 0;
     // reductions / flags
     double *partials = nullptr;

@@ -20,6 +20,31 @@
 
 namespace komd {
 
+// double -> float rounded to nearest (ties to even) from the bits, in integer
+// instructions (GB300 converts FP64 -> FP32 on its narrow FP64 pipe): the 29
+// dropped mantissa bits decide the rounding, and a carry out of the mantissa
+// moves into the exponent as IEEE rounding does.  Results outside the FP32
+// normal range (zero, subnormal, overflow, NaN) take the conversion
+// instruction.  Bitwise equal to __double2float_rn.
+__device__ __forceinline__ float d2f_rn(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)((b >> 52) & 0x7ffu) - 1023 + 127;   // the FP32 biased exponent
+    if (e < 1 || e > 254) return __double2float_rn(x);
+    const unsigned long long mant = b & 0xfffffffffffffULL;
+    unsigned f = ((unsigned)e << 23) | (unsigned)(mant >> 29);
+    const unsigned rest = (unsigned)(mant & 0x1fffffffULL);
+    f += (rest > 0x10000000u || (rest == 0x10000000u && (f & 1u))) ? 1u : 0u;
+    return __uint_as_float(f | ((unsigned)(b >> 32) & 0x80000000u));
+}
+
+// float -> double (exact) from the bits, likewise
+__device__ __forceinline__ double f2d(float x) {
+    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+    if (m - 0x00800000u >= 0x7f000000u) return (double)x;   // zero, subnormal, infinity, NaN
+    return __longlong_as_double((long long)(((unsigned long long)(b & 0x80000000u) << 32) +
+                                            ((unsigned long long)m << 29) + (896ULL << 52)));
+}
+
 // ===========================================================================
 // container: COM, periodic wrap, binning (LinkedCells.cpp:65-121,390-400;
 // MoleculeContainer.cpp:55-75).  One thread per molecule.
@@ -40,6 +65,35 @@ __device__ __forceinline__ int cell_index(double x, double cs, double ics, int n
     return (int)q;
 }
 
+// On a step without a rebuild a molecule matters only if it wraps.  True when its
+// centre of mass is inside the domain by more than the error of this FP32 estimate:
+// with k sites of positive mass the rounded inputs, the products, the k - 1 additions
+// and those of the total mass are each within 2^-24 (the division 2^-22) of
+// sum |m r| / sum m.  The range of tm keeps underflow of the products far below that.
+// 18 FP64 operations and three divisions of a three-site molecule need not run:
+// 300,000 sites, 17.0 -> 7.0 us a step.
+__device__ __forceinline__ bool com_inside(const BinArgs &a, int s0, int s1) {
+    float c[3] = {0.f, 0.f, 0.f}, ca[3] = {0.f, 0.f, 0.f}, tm = 0.f;
+    bool in = true;
+    for (int s = s0; s < s1; s++) {
+        const float ms = d2f_rn(a.m[s]);
+        in = in && ms > 0.f;
+        for (int d = 0; d < 3; d++) {
+            const float x = d2f_rn(a.r[3 * s + d]) * ms;
+            c[d] += x;
+            ca[d] += fabsf(x);
+        }
+        tm += ms;
+    }
+    in = in && tm > 1e-20f && tm < 1e20f;
+    const float im = __fdividef(1.0f, tm), k = 6.0e-8f * (float)(2 * (s1 - s0) + 16);
+    for (int d = 0; d < 3; d++) {
+        const float x = c[d] * im, tol = fmaf(ca[d] * im, k, 1e-20f);
+        in = in && x - tol > a.in_lo[d] && x + tol < a.in_hi[d];
+    }
+    return in;   // false for NaN
+}
+
 __device__ __forceinline__ void com_wrap_bin_body(const BinArgs &a, int bid, int nblk) {
     const Grid &g = a.g;
     const int n_mol = a.n_mol;
@@ -56,6 +110,7 @@ __device__ __forceinline__ void com_wrap_bin_body(const BinArgs &a, int bid, int
     const bool bin = !(rebuild && !*rebuild);        // no rebuild in this step: cells stay as built
     for (int k = bid * blockDim.x + threadIdx.x; k < n_mol; k += nblk * blockDim.x) {
     const int s0 = a.single ? k : mol_off[k], s1 = a.single ? k + 1 : mol_off[k + 1];
+    if (!bin && com_inside(a, s0, s1)) continue;   // no wrap; the centre is formed again before anything reads it
     // com += r * m ; M += m ; com /= M   (updateCOM, no FMA).  For a single
     // site of power-of-two mass the scaling is exact and the result is r
     // itself (up to the sign of a zero), so the FP64 division is skipped.
@@ -738,6 +793,77 @@ __global__ void k_angles(int na, const int *__restrict__ angles, const double *_
     }
 }
 
+// The same forces without the sensors for small molecules: a thread evaluates every
+// term of a connected component (BondBlock: up to kBondComps components whose sites
+// lie in one range of kBondSites), so nothing is summed by atomics.  Positions and
+// forces pass through shared memory: coalesced, and the terms' reads and sums stay on
+// chip.  Bound by its FP64 instructions (33 for a three-site molecule; conversions are
+// in integers).  300,000 sites of three-site molecules: k_bonds + k_angles 20.1 ->
+// 16.8 us; a thread per site, which evaluates a term once from each of its sites,
+// took 25.7.
+__global__ void __launch_bounds__(kBondComps) k_bonded_mol(const int4 *__restrict__ blocks,
+                                                           const int *__restrict__ comp_off,
+                                                           const int4 *__restrict__ terms,
+                                                           const double *__restrict__ r, double *__restrict__ f,
+                                                           float kb, float r0, float ka, float th0) {
+    __shared__ double s_r[3 * kBondSites], s_f[3 * kBondSites];
+    const int4 b = blocks[blockIdx.x];   // components [x, y), sites [z, w)
+    const int n3 = 3 * (b.w - b.z), c = b.x + (int)threadIdx.x;
+    const size_t base = 3 * (size_t)b.z;
+    constexpr int kRows = 3 * kBondSites / kBondComps;
+    double x[kRows], y[kRows];   // all loads in flight at once
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const int t = threadIdx.x + k * kBondComps;
+        x[k] = t < n3 ? r[base + t] : 0.0;
+        y[k] = t < n3 ? f[base + t] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        s_r[threadIdx.x + k * kBondComps] = x[k];
+        s_f[threadIdx.x + k * kBondComps] = y[k];
+    }
+    const int t0 = c < b.y ? comp_off[c] : 0, t1 = c < b.y ? comp_off[c + 1] : 0;
+    __syncthreads();
+    for (int t = t0; t < t1; t++) {
+        const int4 q = terms[t];   // sites; z < 0: a bond
+        const int i = 3 * (q.x - b.z), j = 3 * (q.y - b.z);
+        float u[3];
+        for (int d = 0; d < 3; d++) u[d] = d2f_rn(dsub(s_r[i + d], s_r[j + d]));
+        const float uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+        if (q.z < 0) {
+            const float rr = sqrtf(uu);
+            const float fs = -kb * (rr - r0) / rr;
+            for (int d = 0; d < 3; d++) {
+                const double g = f2d(fs * u[d]);
+                s_f[i + d] = dadd(s_f[i + d], g);
+                s_f[j + d] = dsub(s_f[j + d], g);
+            }
+            continue;
+        }
+        const int k = 3 * (q.z - b.z);
+        float v[3];
+        for (int d = 0; d < 3; d++) v[d] = d2f_rn(dsub(s_r[k + d], s_r[j + d]));
+        const float vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+        const float uv = u[0] * v[0] + u[1] * v[1] + u[2] * v[2];
+        const float inu = rsqrtf(uu), inv_ = rsqrtf(vv);
+        float cs = uv * inu * inv_;
+        cs = fminf(1.0f, fmaxf(-1.0f, cs));
+        const float dth = acosf(cs) - th0;
+        const float sn = fmaxf(sqrtf(1.0f - cs * cs), 1e-6f);
+        const float pre = ka * dth / sn;
+        for (int d = 0; d < 3; d++) {
+            const float fi = pre * (v[d] * inu * inv_ - cs * u[d] * inu * inu);
+            const float fk = pre * (u[d] * inu * inv_ - cs * v[d] * inv_ * inv_);
+            s_f[i + d] = dadd(s_f[i + d], f2d(fi));
+            s_f[k + d] = dadd(s_f[k + d], f2d(fk));
+            s_f[j + d] = dsub(s_f[j + d], f2d(fi + fk));
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n3; t += kBondComps) f[base + t] = s_f[t];
+}
+
 // Limit_Force (Limit.cpp:19-25): clamp with Kokkos::min / max semantics
 __global__ void k_limit(int n, const double *__restrict__ eps, const double *__restrict__ sig, double limit,
                         double *__restrict__ f) {
@@ -755,13 +881,29 @@ __global__ void k_limit(int n, const double *__restrict__ eps, const double *__r
 // ===========================================================================
 // velocity Verlet (Integrator.cpp:28-37), FP64 without contraction
 // ===========================================================================
-// With a Verlet list (bias != nullptr) it also flags a rebuild when a site's
-// cell-local position r - bias has moved more than skin/2 since the build.
 // hdtm[s] = (dt * 0.5) / m[s], the reference's dtInv2m (Integrator.cpp:29), computed
-// once at upload with the same IEEE division
+// once at upload with the same IEEE division.  With a Verlet list (bias !=
+// nullptr) the drift also writes the site's FP32 position in its build cell's
+// frame, (float)(r - bias) -- a periodic wrap that follows moves both alike, and a
+// rebuild rewrites it -- and flags a rebuild when that has moved more than skin/2
+// since the build.
+__device__ __forceinline__ void local_position(int s, const double (&x)[3], const double *__restrict__ bias,
+                                               const float4 *__restrict__ ref4, const int *__restrict__ site_slot,
+                                               float4 *__restrict__ pos4, float half_skin2, int *__restrict__ rebuild) {
+    const int slot = site_slot[s];
+    const float4 q = ref4[s];
+    float4 p = pos4[slot];
+    p.x = d2f_rn(dsub(x[0], bias[3 * s]));
+    p.y = d2f_rn(dsub(x[1], bias[3 * s + 1]));
+    p.z = d2f_rn(dsub(x[2], bias[3 * s + 2]));
+    pos4[slot] = p;
+    const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+    if (dx * dx + dy * dy + dz * dz > half_skin2) *rebuild = 1;
+}
 __global__ void k_step0(int n, double *__restrict__ r, double *__restrict__ v, const double *__restrict__ f,
                         const double *__restrict__ hdtm, double dt, Grid g,
-                        const double *__restrict__ bias, const float4 *__restrict__ ref4, float half_skin2,
+                        const double *__restrict__ bias, const float4 *__restrict__ ref4,
+                        const int *__restrict__ site_slot, float4 *__restrict__ pos4, float half_skin2,
                         int *__restrict__ rebuild) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -773,43 +915,20 @@ __global__ void k_step0(int n, double *__restrict__ r, double *__restrict__ v, c
         x[d] = dadd(r[3 * s + d], dmul(vv, dt));
         r[3 * s + d] = x[d];
     }
-    if (bias) {
-        const float4 q = ref4[s];
-        const float dx = __double2float_rn(dsub(x[0], bias[3 * s])) - q.x;
-        const float dy = __double2float_rn(dsub(x[1], bias[3 * s + 1])) - q.y;
-        const float dz = __double2float_rn(dsub(x[2], bias[3 * s + 2])) - q.z;
-        if (dx * dx + dy * dy + dz * dz > half_skin2) *rebuild = 1;
-    }
+    if (bias) local_position(s, x, bias, ref4, site_slot, pos4, half_skin2, rebuild);
 }
 
 // Verlet path with single-site molecules whose COM is exactly the position
 // (power-of-two masses): integrate0, the skin test, the periodic wrap with
 // its bias update and COM (k_com_wrap_bin's operations) and the FP32
-// cell-local refresh (k_refresh's) in one pass over the sites.  The
-// results are those of the separate kernels; on a rebuild step the cell sort
-// rewrites pos4 afterwards.
+// cell-local position in one pass over the sites.  The results are those of
+// the separate kernels; on a rebuild step the cell sort rewrites pos4 afterwards.
 // integer key with key(x) < key(y) exactly when x < y for non-NaN doubles
 // (-0.0 and +0.0 share the key 0)
 __device__ __forceinline__ long long dkey(double x) {
     const long long b = __double_as_longlong(x);
     const long long m = b & 0x7fffffffffffffffLL;
     return b < 0 ? -m : m;
-}
-// double -> float rounded to nearest (ties to even) from the bits, in integer
-// instructions (GB300 converts FP64 -> FP32 on its narrow FP64 pipe): the 29
-// dropped mantissa bits decide the rounding, and a carry out of the mantissa
-// moves into the exponent as IEEE rounding does.  Results outside the FP32
-// normal range (zero, subnormal, overflow, NaN) take the conversion
-// instruction.  Bitwise equal to __double2float_rn.
-__device__ __forceinline__ float d2f_rn(double x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ffu) - 1023 + 127;   // the FP32 biased exponent
-    if (e < 1 || e > 254) return __double2float_rn(x);
-    const unsigned long long mant = b & 0xfffffffffffffULL;
-    unsigned f = ((unsigned)e << 23) | (unsigned)(mant >> 29);
-    const unsigned rest = (unsigned)(mant & 0x1fffffffULL);
-    f += (rest > 0x10000000u || (rest == 0x10000000u && (f & 1u))) ? 1u : 0u;
-    return __uint_as_float(f | ((unsigned)(b >> 32) & 0x80000000u));
 }
 __device__ __forceinline__ bool dkey_nan(double x) {
     return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
@@ -954,20 +1073,6 @@ __global__ void k_step1(int n, double *__restrict__ v, const double *__restrict_
         bad |= !isfinite(vv);
     }
     if (bad) atomicOr(&err[E_NONFINITE], 1);
-}
-
-// Verlet path, steps without rebuild: cell-local FP32 coordinates
-// (float)(r - bias) relative to each slot's build cell.
-__global__ void k_refresh(int n, const int *__restrict__ slot_site, const double *__restrict__ r,
-                          const double *__restrict__ bias, float4 *__restrict__ pos4, const int *__restrict__ rebuild) {
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= n || *rebuild) return;
-    const int s = slot_site[slot];
-    float4 p = pos4[slot];
-    p.x = __double2float_rn(dsub(r[3 * s], bias[3 * s]));
-    p.y = __double2float_rn(dsub(r[3 * s + 1], bias[3 * s + 1]));
-    p.z = __double2float_rn(dsub(r[3 * s + 2], bias[3 * s + 2]));
-    pos4[slot] = p;
 }
 
 // ===========================================================================
@@ -1289,9 +1394,14 @@ static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 static inline int site_block(const Engine &e, long long n) { return n >= 512ll * e.num_sms ? 256 : 64; }
 
 BinArgs bin_args(const Engine &e) {
-    return BinArgs{e.g, (int)e.n_mol, e.mol_off, e.r, e.m, e.com, e.mol_cell, e.mol_rank, e.cell_count, e.cell_mcount,
+    BinArgs a = BinArgs{e.g, (int)e.n_mol, e.mol_off, e.r, e.m, e.com, e.mol_cell, e.mol_rank, e.cell_count, e.cell_mcount,
                    e.verlet ? e.bias : nullptr, e.verlet ? e.rebuild : nullptr, e.exact_com, e.fused_drift ? 1 : 0,
-                   e.n_mol == e.n ? 1 : 0};
+                   e.n_mol == e.n ? 1 : 0, {}, {}};
+    for (int d = 0; d < 3; d++) {
+        a.in_lo[d] = nextafterf((float)e.g.low[d], INFINITY);
+        a.in_hi[d] = nextafterf((float)e.g.high[d], -INFINITY);
+    }
+    return a;
 }
 ScanArgs scan_args(const Engine &e) {
     return ScanArgs{e.g.ncell, e.n_mol == e.n ? nullptr : e.cell_count, e.cell_start, e.cell_mcount, e.cell_mstart,
@@ -1331,8 +1441,6 @@ void launch_container(Engine &e, cudaStream_t st) {
     // four warps a block: with few cells the chain of loads bounds the sort, not its throughput
     launch_pdl(k_cell_sort, std::min(nblk(g.ncell, 4), 2 * res), 128, 0, st, sort_args(e));
     if (e.verlet) {
-        if (!e.fused_drift)
-            k_refresh<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.slot_site, e.r, e.bias, e.pos4, e.rebuild);
         launch_vlist_build(e, st);
     }
 }
@@ -1424,6 +1532,12 @@ int launch_pair(Engine &e, cudaStream_t st, bool measure, double *lj_hist) {
 }
 
 void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc) {
+    if (!measure && e.bond_blocks > 0 && e.bond_sites == e.n) {
+        k_bonded_mol<<<e.bond_blocks, kBondComps, 0, st>>>(e.bond_block, e.comp_off, e.comp_terms, e.r, e.f,
+                                                           (float)e.cfg.bond_k, (float)e.cfg.bond_r0,
+                                                           (float)e.cfg.angle_k, (float)e.cfg.angle_theta0);
+        return;
+    }
     if (e.n_bonds > 0)
         k_bonds<<<nblk(e.n_bonds, 256), 256, 0, st>>>((int)e.n_bonds, e.bonds, e.r, e.f, (float)e.cfg.bond_k,
                                                         (float)e.cfg.bond_r0, acc, measure ? 1 : 0);
@@ -1608,7 +1722,8 @@ __global__ void __launch_bounds__(kIoBlock) k_kick_drift(FlushArgs a, Step0Args 
 // several sites): k_step1's and k_step0's operations
 __global__ void k_step10(int n, double *__restrict__ r, double *__restrict__ v, const double *__restrict__ f,
                          const double *__restrict__ hdtm, double dt, const double *__restrict__ bias,
-                         const float4 *__restrict__ ref4, float half_skin2, int *__restrict__ rebuild,
+                         const float4 *__restrict__ ref4, const int *__restrict__ site_slot,
+                         float4 *__restrict__ pos4, float half_skin2, int *__restrict__ rebuild,
                          int *__restrict__ err) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -1629,13 +1744,7 @@ __global__ void k_step10(int n, double *__restrict__ r, double *__restrict__ v, 
         r[3 * s + d] = x[d];
     }
     if (bad) atomicOr(&err[E_NONFINITE], 1);
-    if (bias) {
-        const float4 q = ref4[s];
-        const float dx = __double2float_rn(dsub(x[0], bias[3 * s])) - q.x;
-        const float dy = __double2float_rn(dsub(x[1], bias[3 * s + 1])) - q.y;
-        const float dz = __double2float_rn(dsub(x[2], bias[3 * s + 2])) - q.z;
-        if (dx * dx + dy * dy + dz * dz > half_skin2) *rebuild = 1;
-    }
+    if (bias) local_position(s, x, bias, ref4, site_slot, pos4, half_skin2, rebuild);
 }
 
 // f[site] += 2 sign nu g (fixed point -> FP64) and the accumulators back to 0
@@ -1747,8 +1856,8 @@ void launch_step0(Engine &e, cudaStream_t st, bool in_step) {
     }
     const int b = site_block(e, e.n);
     k_step0<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
-                                              e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, hs * hs,
-                                              e.rebuild);
+                                              e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4,
+                                          hs * hs, e.rebuild);
 }
 
 // integrate1 of a step and integrate0 of the next
@@ -1761,8 +1870,8 @@ void launch_kick_drift(Engine &e, cudaStream_t st) {
     }
     const float hs = (float)(0.5 * e.cfg.skin);
     k_step10<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
-                                             e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, hs * hs,
-                                             e.rebuild, e.err);
+                                             e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4,
+                                             hs * hs, e.rebuild, e.err);
 }
 
 // the same with the learned term's forces (fsur, slot order) added first; needs the fused drift
