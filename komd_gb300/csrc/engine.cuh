@@ -119,20 +119,20 @@ __device__ __forceinline__ double sqrt_d(double x, double y) {
     return __fma_rn(__fma_rn(-r, r, x), __dmul_rn(0.5, y), r);
 }
 
-// the warp sums of (x, y, z): a butterfly over offsets 16, 8, 4, 2, 1 whose
-// lanes split the components on the way (lanes 0-7 end with x, 8-15 with y,
-// 16-31 with z): 6 additions a lane instead of 15, the same pairing of partial
-// sums as a butterfly per component
-template <typename Real>
+// the sums of (x, y, z) over W = 32 or 16 lanes: a butterfly over offsets W/2 .. 1
+// whose lanes split the components on the way (of each W lanes the first quarter ends
+// with x, the second with y, the upper half with z): 6 additions a lane instead of 15,
+// the same pairing of partial sums as a butterfly per component
+template <typename Real, int W = 32>
 __device__ __forceinline__ Real warp_sum3(Real x, Real y, Real z, int lane) {
-    const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
-    const Real r1 = __shfl_xor_sync(0xffffffffu, up16 ? x : z, 16);
-    const Real r2 = __shfl_xor_sync(0xffffffffu, y, 16);
-    Real c0 = (up16 ? z : x) + r1;
+    const bool up = (lane & (W / 2)) != 0, upq = (lane & (W / 4)) != 0;
+    const Real r1 = __shfl_xor_sync(0xffffffffu, up ? x : z, W / 2);
+    const Real r2 = __shfl_xor_sync(0xffffffffu, y, W / 2);
+    Real c0 = (up ? z : x) + r1;
     const Real c1 = y + r2;
-    const Real r3 = __shfl_xor_sync(0xffffffffu, (up16 || up8) ? c0 : c1, 8);
-    c0 = ((up16 || !up8) ? c0 : c1) + r3;
-    for (int o = 4; o > 0; o >>= 1) c0 += __shfl_xor_sync(0xffffffffu, c0, o);
+    const Real r3 = __shfl_xor_sync(0xffffffffu, (up || upq) ? c0 : c1, W / 4);
+    c0 = ((up || !upq) ? c0 : c1) + r3;
+    for (int o = W / 8; o > 0; o >>= 1) c0 += __shfl_xor_sync(0xffffffffu, c0, o);
     return c0;
 }
 

@@ -488,28 +488,45 @@ __global__ void __launch_bounds__(32 * kVbMaxWarps) k_vlist_build(PairParams p, 
 // list in list order -- to the global list, or (TO_SMEM) staged in shared
 // memory (se, sq) for the sweep that follows in the same warp.  Returns the
 // number of ATM neighbours kept.
-// U = list entries per lane in flight (independent loads for latency hiding):
-// a warp covers 32 U entries of a row per pass
-template <bool MEASURE, bool EMIT, bool UNIFORM, int U, bool TO_SMEM>
-__device__ __forceinline__ int lj_site(const PairParams &p, int i, int lane, unsigned lt, float rc2, float rc3sq,
-                                       float4 *se, float4 *sq, float &m_u, float &m_pairs, float (&m_w)[6]) {
-    const int cw = p.vl_count[i];
+// U = list entries per lane in flight (independent loads for latency hiding)
+// W = lanes of the site: with 16 the warp holds two sites (live: this one is there), and
+// odd entries have sums of their own, (hx, hy, hz): those of lanes 16 to 31 with W = 32
+template <bool MEASURE, bool EMIT, bool UNIFORM, int U, bool TO_SMEM, int W = 32>
+__device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, int lane, unsigned lt, float rc2,
+                                       float rc3sq, float4 *se, float4 *sq, float &m_u, float &m_pairs,
+                                       float (&m_w)[6]) {
+    static_assert(W == 32 || (W == 16 && !MEASURE && !TO_SMEM && U % 2 == 0), "");
+    const int sub = lane & (W - 1);
+    const int cw = live ? p.vl_count[i] : 0;
     const int chi = cw & 0xffff, cnt = chi + (cw >> 16);   // both regions of the row
+    const int cmax = W == 32 ? cnt : max(cnt, __shfl_xor_sync(0xffffffffu, cnt, 16));
     const float4 pi = p.pos4[i];
     const float sei = UNIFORM ? 0.f : p.seps[i];
     const float4 *off = p.nboff + (size_t)p.slot_cell[i] * 27;
     const unsigned *row = p.vl + (size_t)i * p.vl_cap;
     const float sg2u = p.sig0 * p.sig0, eeu = p.eps0;
-    float fx = 0.f, fy = 0.f, fz = 0.f;
+    float fx = 0.f, fy = 0.f, fz = 0.f, hx = 0.f, hy = 0.f, hz = 0.f;
     int c_atm = 0;
-    for (int k0 = 0; k0 < cnt; k0 += 32 * U) {
+    const unsigned half = W == 32 ? 0xffffffffu : (lane < 16 ? 0xffffu : 0xffff0000u);
+    constexpr bool kAhead = W == 16;   // list entries read one pass ahead
+    unsigned en[U];
+    if (kAhead) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int k = u * W + sub;
+            en[u] = k < cnt ? __ldcs(row + vl_entry(k, chi, p.vl_cap)) : 0xffffffffu;
+        }
+    }
+    for (int k0 = 0; k0 < cmax; k0 += W * U) {
         unsigned e[U];
         float4 o[U], pj[U];
         float sej[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int k = k0 + u * 32 + lane;
-            e[u] = k < cnt ? __ldcs(row + vl_entry(k, chi, p.vl_cap)) : 0xffffffffu;   // read once per step: evict first
+            const int k = k0 + (kAhead ? W * U : 0) + u * W + sub;
+            if (kAhead) e[u] = en[u];
+            // read once per step: evict first
+            (kAhead ? en[u] : e[u]) = k < cnt ? __ldcs(row + vl_entry(k, chi, p.vl_cap)) : 0xffffffffu;
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -548,7 +565,11 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, int lane, uns
                         fac0 = fac0 * usw - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
                     }
                     const float fac = MEASURE ? fac0 : fac0 * p.lj_fscalef;   // ATM2B factor
-                    fx += dx * fac; fy += dy * fac; fz += dz * fac;
+                    if (W == 32 || (u & 1) == 0) {
+                        fx += dx * fac; fy += dy * fac; fz += dz * fac;
+                    } else {
+                        hx += dx * fac; hy += dy * fac; hz += dz * fac;
+                    }
                     if (MEASURE) {
                         const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
                         m_u += 2.0f * ee * (lj6 * lj6 - lj6) * usw;
@@ -565,7 +586,7 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, int lane, uns
             if (EMIT) {
                 // staged for the once-per-triplet sweep: neighbours above i only
                 const bool emit = valid && r2 <= rc3sq && (!TO_SMEM || (int)(e[u] & 0x3ffffffu) > i);
-                const unsigned m = __ballot_sync(0xffffffffu, emit);
+                const unsigned m = __ballot_sync(0xffffffffu, emit) & half;
                 if (emit) {
                     const int pos = c_atm + __popc(m & lt);
                     const int nb = (int)((e[u] >> 26) & 31u), j = (int)(e[u] & 0x3ffffffu);
@@ -584,11 +605,13 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, int lane, uns
             }
         }
     }
-    // lanes 0, 8 and 16 hold x, y and z: one FP32 -> FP64 conversion for the three (a
-    // conversion takes the FP64 pipe for a whole warp, whatever the active lanes)
-    const float fs = warp_sum3(fx, fy, fz, lane);
-    if ((lane & 7) == 0 && lane < 24) p.f[3 * (size_t)p.slot_site[i] + (lane >> 3)] = (double)fs;
-    if (EMIT && lane == 0) {
+    // lanes 0, W/4 and W/2 of a site hold x, y and z: one FP32 -> FP64 conversion for
+    // the three (a conversion takes the FP64 pipe for a whole warp, whatever the active lanes)
+    if (W == 16) { fx += hx; fy += hy; fz += hz; }
+    const float fs = warp_sum3<float, W>(fx, fy, fz, lane);
+    if ((sub & (W / 4 - 1)) == 0 && sub < 3 * W / 4 && live)
+        p.f[3 * (size_t)p.slot_site[i] + sub / (W / 4)] = (double)fs;
+    if (EMIT && sub == 0 && live) {
         if (!TO_SMEM) p.nl_count[i] = min(c_atm, p.nl_cap);
         if (c_atm > p.nl_cap) atomicOr(&p.err[E_ATM_OVERFLOW], 1);
     }
@@ -608,7 +631,9 @@ __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, 
     // most of their neighbours, so the gathers of one group hit L1 lines of the last
     for (int it = 0; it < per; it++) {
         const int i = (blockIdx.x * per + it) * 8 + w;
-        if (i < n) lj_site<MEASURE, EMIT, UNIFORM, U, false>(p, i, lane, lt, rc2, rc3sq, nullptr, nullptr, m_u, m_pairs, m_w);
+        if (i < n)
+            lj_site<MEASURE, EMIT, UNIFORM, U, false>(p, i, true, lane, lt, rc2, rc3sq, nullptr, nullptr, m_u, m_pairs,
+                                                      m_w);
     }
     if (MEASURE) {
         // the lanes' FP32 partials summed over the warp in FP32 (a fixed tree:
@@ -636,6 +661,32 @@ __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, 
     }
 }
 
+// The same with two sites a warp, sixteen lanes each.  The pass waits on its gathers
+// (with one site a warp and three entries a lane in flight: half of the issue slots, 40 %
+// of the L1 wavefronts), so what counts is how many sites are in flight and how little
+// each costs: a row of 74 entries takes five passes of 16 lanes where 32 lanes take 96
+// entries' worth, the reduction and the conversion to FP64 serve two sites, two entries
+// a lane in flight with the next two list entries read ahead fit in 48 registers (five
+// blocks an SM, not four).  A lane sums entries of equal place modulo 32 apart, so
+// every force is that of the kernel above bit for bit.  300,000 sites of three-site
+// molecules: 135 -> 90 us; 32,000 sites of liquid argon with the ATM list 25.4 -> 18.8.
+// Without the read-ahead 99, four entries in flight 119, six 132 us.
+template <bool EMIT, bool UNIFORM>
+__global__ void __launch_bounds__(256, 5) k_lj_vlist2(PairParams p, int n, int per) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq;
+    unsigned lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
+    float m_u, m_pairs, m_w[6];   // no sensors
+    for (int it = 0; it < per; it++) {
+        const int i0 = ((blockIdx.x * per + it) * 8 + w) * 2, i = i0 + (lane >> 4);
+        if (i0 >= n) return;
+        lj_site<false, EMIT, UNIFORM, 2, false, 16>(p, min(i, n - 1), i < n, lane, lt, rc2, rc3sq, nullptr, nullptr,
+                                                    m_u, m_pairs, m_w);
+    }
+}
+
 // LJ and ATM in one pass (FP32 forces, FULL triplets, Verlet path): each warp
 // runs the LJ pass of its site, stages the site's ATM neighbours above it in
 // shared memory instead of the global list, and sweeps its triplets at once.
@@ -655,7 +706,7 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm(PairParams p, AtmParams a, in
     for (int it = 0; it < per; it++) {
         const int i = (blockIdx.x * per + it) * 8 + w;
         if (i < n) {
-            const int m = lj_site<false, true, UNIFORM, U, true>(p, i, lane, lt, rc2, rc3sq, se, sq, m_u, m_pairs, m_w);
+            const int m = lj_site<false, true, UNIFORM, U, true>(p, i, true, lane, lt, rc2, rc3sq, se, sq, m_u, m_pairs, m_w);
             __syncwarp();
             atm_vertex(a, i, se, sq, m, lane, rc3f);
             __syncwarp();   // se / sq are refilled by the next site
@@ -1032,6 +1083,16 @@ bool vlist_u3(const Engine &e) {
 }
 
 int launch_lj_vlist(Engine &e, PairParams &p, bool measure, bool emit, cudaStream_t st) {
+    // two sites a warp once one site a warp (at most 32 warps an SM) takes more than one
+    // wave: 4000 sites 11.4 us a step either way, 2048 10.9 against 11.4, 5324 14.0 against
+    // 12.9, 16,384 19.5 against 16.9
+    if (!measure && e.n > 32 * (int64_t)e.num_sms) {
+        const int per2 = (vlist_per(e) + 1) / 2, grid2 = (int)((e.n + 16 * per2 - 1) / (16 * per2));
+        auto k = e.uniform ? (emit ? k_lj_vlist2<true, true> : k_lj_vlist2<false, true>)
+                           : (emit ? k_lj_vlist2<true, false> : k_lj_vlist2<false, false>);
+        k<<<grid2, 256, 0, st>>>(p, (int)e.n, per2);
+        return grid2;
+    }
     // a block's partial sums cover all its groups (the lanes' sums run across them)
     const int per = vlist_per(e);
     const int grid = vlist_blocks(e);
