@@ -23,19 +23,31 @@ namespace komd {
 // k_atm_flush adds them to f.
 constexpr double kAtmFix = 4294967296.0;   // 2^32 fixed-point units
 
+// 1/sqrt of a squared distance: rsqrtf's instruction without the scaling (three
+// more) that it wraps around it for subnormal arguments
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // staged (A, 1/A, 1/sqrt A) of a neighbour at squared distance A: the
 // hardware reciprocal (about 1 ulp) and reciprocal square root; A is a squared
 // distance of order one, never in the flush-to-zero range
 __device__ __forceinline__ float4 atm_stage_q(float A) {
     float ia;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ia) : "f"(A));
-    return make_float4(A, ia, rsqrtf(A), 0.f);
+    return make_float4(A, ia, rsqrt_ftz(A), 0.f);
 }
 
 // round(x * 2^32) to the nearest integer (ties to even) as int64, for finite
-// |x| < 2^31, built from two 32-bit conversions: GB300 runs FP32 -> int64
-// conversions on its narrow FP64 pipe, FP32 -> int32 on the wide ones.
-// With a = |x|: fl = floor(a) is an integer below 2^31 (the high word), and
+// |x| < 2^31, without an FP32 -> int64 conversion: GB300 runs those on its
+// narrow FP64 pipe, FP32 -> int32 on the wide ones.
+// Below 2^20, where forces are: t = x + 1.5 2^22 lies in a binade of ulp 1/2, so
+// its bits hold h = round(2 x), x - h / 2 is exact and within 1/4, and times 2^32 it
+// is exact and within the range of one 32-bit conversion; h 2^31 is even, so
+// rounding that part alone (to even) rounds the sum.
+// Otherwise, with a = |x|: fl = floor(a) is an integer below 2^31 (the high word), and
 // a - fl is exact (Sterbenz for a >= 1, a itself below 1), so (a - fl) * 2^32
 // is the exact low part in [0, 2^32 - 2^8]; it has a fraction only for
 // a < 2^-9, where rounding it is rounding x * 2^32.  The sign is applied last
@@ -43,6 +55,15 @@ __device__ __forceinline__ float4 atm_stage_q(float A) {
 // to int64 directly over all finite |x| < 2^31; a NaN contributes 0.
 __device__ __forceinline__ long long fix32_rn(float x) {
     const float a = fabsf(x);
+    if (a < 1048576.0f) {
+        const float big = 6291456.0f, t = __fadd_rn(x, big);
+        const float rem = __fsub_rn(x, __fsub_rn(t, big));
+        const long long lo = __float2int_rn(rem * 4294967296.0f);
+        long long q;   // -h * -2^31 + lo
+        asm("mad.wide.s32 %0, %1, %2, %3;"
+            : "=l"(q) : "r"(__float_as_int(big) - __float_as_int(t)), "r"((int)0x80000000), "l"(lo));
+        return q;
+    }
     const float fl = floorf(a);
     const unsigned hi = (unsigned)__float2int_rz(fl);
     const unsigned lo = __float2uint_rn((a - fl) * 4294967296.0f);
@@ -65,7 +86,7 @@ struct AtmV {
 // written around K = 3/8 (u + v + w), which the three share.
 __device__ __forceinline__ AtmV atm_derivs(float4 qa, float4 qb, float C) {
     const float A = qa.x, B = qb.x;
-    const float wc = rsqrtf(C);
+    const float wc = rsqrt_ftz(C);
     const float sv = qa.z * qb.z * wc;                  // 1/(abc)
     const float s2 = sv * sv;
     const float s5 = s2 * s2 * sv;
@@ -88,7 +109,7 @@ __device__ __forceinline__ AtmV atm_derivs(float4 qa, float4 qb, float C) {
 __device__ __forceinline__ AtmV atm_derivs_sw(float4 qa, float4 qb, float C, float sA, float dA, float rc2s,
                                               float iw) {
     const float A = qa.x, B = qb.x;
-    const float wc = rsqrtf(C);
+    const float wc = rsqrt_ftz(C);
     const float sv = qa.z * qb.z * wc;
     const float s2 = sv * sv;
     const float s5 = s2 * s2 * sv;
@@ -133,27 +154,27 @@ __device__ __forceinline__ void atm_sweep(const float4 *se, const float4 *sq, in
     int t_act = own ? d_last - d_first + 1 : 0;
     if (own && (m & 1) == 0 && d_last == (m >> 1) && li >= (m >> 1)) t_act--;
     // partner b = li + d and share source li - d (mod m), stepped per round;
-    // d <= m/2 keeps both within one wrap
-    int b = li + d_first, src = li - d_first;
+    // d <= m/2 keeps both within one wrap (lanes without a neighbour read entries
+    // from 0 on, 16 at most: nl_cap is 32 or more)
+    int b = own ? li + d_first : 0, src = li - d_first;
     if (b >= m) b -= m;
     if (src < 0) src += m;
     for (int t = 0; t < rounds; t++) {
-        float bx = 0.f, by = 0.f, bz = 0.f;
-        if (t < t_act) {
-            const float4 eb = se[b];
-            const float cx = eb.x - ea.x, cy = eb.y - ea.y, cz = eb.z - ea.z;
-            const float C = cx * cx + cy * cy + cz * cz;
-            if (C <= rc2) {
-                const AtmV v = SW ? atm_derivs_sw(qa, sq[b], C, sA, dA, rc2, sw_iw) : atm_derivs(qa, sq[b], C);
-                const float tx = v.vC * cx, ty = v.vC * cy, tz = v.vC * cz;
-                ax += tx - v.vA * ea.x;
-                ay += ty - v.vA * ea.y;
-                az += tz - v.vA * ea.z;
-                bx = -tx - v.vB * eb.x;
-                by = -ty - v.vB * eb.y;
-                bz = -tz - v.vB * eb.z;
-            }
-        }
+        // no branch: with one the partner's loads, the test and the arithmetic of a round
+        // wait for one another; the derivatives of a pair that does not count become 0
+        const float4 eb = se[b], qb = sq[b];
+        const float cx = eb.x - ea.x, cy = eb.y - ea.y, cz = eb.z - ea.z;
+        const float C = cx * cx + cy * cy + cz * cz;
+        const bool on = t < t_act && C <= rc2;
+        AtmV v = SW ? atm_derivs_sw(qa, qb, C, sA, dA, rc2, sw_iw) : atm_derivs(qa, qb, C);
+        v.vA = on ? v.vA : 0.f;
+        v.vB = on ? v.vB : 0.f;
+        v.vC = on ? v.vC : 0.f;
+        const float tx = v.vC * cx, ty = v.vC * cy, tz = v.vC * cz;
+        ax += tx - v.vA * ea.x;
+        ay += ty - v.vA * ea.y;
+        az += tz - v.vA * ea.z;
+        const float bx = -tx - v.vB * eb.x, by = -ty - v.vB * eb.y, bz = -tz - v.vB * eb.z;
         // lane li pulls the share computed, in this lane group, by the lane whose
         // partner it was.  In a round past d_last the source lane has no round
         // either and sends zero; lanes without a neighbour (li >= m) pull

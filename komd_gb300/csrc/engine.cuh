@@ -238,6 +238,7 @@ struct PairParams {
     int lj_bins;
     double max_sigma;
     double rc2, rc3sq, scan2;  // LJ cutoff^2, ATM cutoff^2, max of both
+    float rc2f, rc3sqf;        // the first two in FP32 (converted per site, they cost the FP64 pipe three instructions)
     float pre2;                // scan2 with the margin of the FP32 pre-test
     int uniform;               // one eps and one sigma for every site
     int multi_key;             // some sites share a molecule key

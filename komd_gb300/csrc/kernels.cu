@@ -1468,6 +1468,8 @@ PairParams pair_params(Engine &e) {
     p.max_sigma = e.cfg.max_sigma;
     p.rc2 = e.cfg.cutoff * e.cfg.cutoff;
     p.rc3sq = e.cfg.cutoff_3b * e.cfg.cutoff_3b;
+    p.rc2f = (float)p.rc2;
+    p.rc3sqf = (float)p.rc3sq;
     const bool atm = (e.cfg.terms & KOMD_TERM_ATM) != 0;
     const bool lj = (e.cfg.terms & KOMD_TERM_LJ) != 0;
     p.scan2 = 0.0;
@@ -1592,7 +1594,7 @@ __global__ void __launch_bounds__(kBlock) k_atm_s(AtmParams p) {
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
     const int m = atm_stage(p, i, se, sq, lane, lt);
     __syncwarp();
-    atm_vertex(p, i, se, sq, m, lane, (float)p.rc2);
+    atm_vertex(p, i, se, sq, m, lane, p.rc2f);
 }
 
 // the same flush fused with Integrator::integrate1 of the step (ATM is the

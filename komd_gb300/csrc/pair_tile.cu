@@ -622,7 +622,7 @@ template <bool MEASURE, bool EMIT, bool UNIFORM, int U>
 __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, int n, int per) {
     __shared__ double s_part[8][8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq;
+    const float rc2 = p.rc2f, rc3sq = p.rc3sqf;
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
@@ -674,7 +674,7 @@ __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, 
 template <bool EMIT, bool UNIFORM>
 __global__ void __launch_bounds__(256, 5) k_lj_vlist2(PairParams p, int n, int per) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq;
+    const float rc2 = p.rc2f, rc3sq = p.rc3sqf;
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm(PairParams p, AtmParams a, in
     extern __shared__ float4 s_dyn[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float4 *se = s_dyn + w * 2 * p.nl_cap, *sq = se + p.nl_cap;
-    const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq, rc3f = (float)a.rc2;
+    const float rc2 = p.rc2f, rc3sq = p.rc3sqf, rc3f = a.rc2f;
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
@@ -733,6 +733,12 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm(PairParams p, AtmParams a, in
 //      flush adds the fixed-point sums of the partners' contributions.
 // Against the full-row pass this reads half the list, evaluates each LJ
 // pair once instead of twice, and converts one FP32 partial per partner.
+// Bound by instruction issue (81 % of the slots, 740 a site, 44 % of them the
+// sweep): 256,000 sites of liquid argon at skin 0.6, 221 -> 195 us, from branches
+// around a dozen instructions replaced by selects, square roots without rsqrtf's
+// scaling, a shorter fixed-point conversion and the cutoffs' FP32 values in the
+// parameters (812 a site, 78 % before).  Five blocks an SM were slower (39 against
+// 35 us at 31,000 sites), two sites a warp gained nothing.
 // ---------------------------------------------------------------------------
 // what the half-list pass reads of a site before its arithmetic: the count
 // of its front region, the region's first 64 entries (rows hold vl_cap >= 64
@@ -785,65 +791,51 @@ __device__ __forceinline__ void lj_half(const PairParams &p, int i, const HalfRo
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            if (e[u] != 0xffffffffu) {
-                o[u] = off[(e[u] >> 26) & 31u];
-                pj[u] = p.pos4[e[u] & 0x3ffffffu];
-                if (!UNIFORM) sej[u] = p.seps[e[u] & 0x3ffffffu];
-            }
+            const unsigned x = e[u] != 0xffffffffu ? e[u] : 0u;   // slot 0 and its site's own cell: read, not used
+            o[u] = off[(x >> 26) & 31u];
+            pj[u] = p.pos4[x & 0x3ffffffu];
+            if (!UNIFORM) sej[u] = p.seps[x & 0x3ffffffu];
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const bool valid = e[u] != 0xffffffffu;
-            float dx = 0.f, dy = 0.f, dz = 0.f, r2 = 1e30f;
-            float gx = 0.f, gy = 0.f, gz = 0.f;
-            bool lj = false;
-            if (valid) {
-                dx = pi.x - (pj[u].x + o[u].x);
-                dy = pi.y - (pj[u].y + o[u].y);
-                dz = pi.z - (pj[u].z + o[u].z);
-                r2 = dx * dx + dy * dy + dz * dz;
-                lj = (PLAIN || p.use_lj) && r2 <= rc2 && !(e[u] >> 31);
-                if (lj) {
-                    const float inv = rcp_approx(r2);
-                    float x, ee;
-                    if (UNIFORM) {
-                        x = sg2u * inv;
-                        ee = eeu;
-                    } else {
-                        const float sg = pi.w + pj[u].w;
-                        x = sg * sg * inv;
-                        ee = sei * sej[u];
-                    }
-                    const float lj6 = x * x * x;
-                    float fac = 24.0f * ee * (2.0f * lj6 * lj6 - lj6) * inv;
-                    if (!PLAIN) fac *= p.lj_fscalef;   // ATM2B factor
-                    if (SW) {   // switched cutoff (no ATM2B with it): U S, force fac S - 2 U dS/dx
-                        float S, dS;
-                        sw_eval(r2, p.sw_rc2, p.sw_iw, S, dS);
-                        fac = fac * S - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
-                    }
-                    gx = dx * fac; gy = dy * fac; gz = dz * fac;
-                    fx += gx; fy += gy; fz += gz;
-                }
+            const float dx = pi.x - (pj[u].x + o[u].x), dy = pi.y - (pj[u].y + o[u].y), dz = pi.z - (pj[u].z + o[u].z);
+            const float r2 = valid ? dx * dx + dy * dy + dz * dz : 1e30f;
+            const bool lj = (PLAIN || p.use_lj) && r2 <= rc2 && !(e[u] >> 31);
+            const float inv = rcp_approx(r2);
+            float x, ee;
+            if (UNIFORM) {
+                x = sg2u * inv;
+                ee = eeu;
+            } else {
+                const float sg = pi.w + pj[u].w;
+                x = sg * sg * inv;
+                ee = sei * sej[u];
             }
+            const float lj6 = x * x * x;
+            float fac = 24.0f * ee * (2.0f * lj6 * lj6 - lj6) * inv;
+            if (!PLAIN) fac *= p.lj_fscalef;   // ATM2B factor
+            if (SW) {   // switched cutoff (no ATM2B with it): U S, force fac S - 2 U dS/dx
+                float S, dS;
+                sw_eval(r2, p.sw_rc2, p.sw_iw, S, dS);
+                fac = fac * S - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
+            }
+            fac = lj ? fac : 0.f;   // no branch around a dozen instructions
+            const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
+            fx += gx; fy += gy; fz += gz;
             const bool at = valid && r2 <= rc3sq;   // a triplet partner (LJ or not)
             const bool lo = lj && !at;              // an LJ-only partner
             const unsigned ma = __ballot_sync(0xffffffffu, at), ml = __ballot_sync(0xffffffffu, lo);
-            if (at || lo) {
+            const int pos = (at ? m : k) + __popc((at ? ma : ml) & lt);
+            if ((at && pos < capa) || lo) {
                 // the partner's slot j at bits 6-30 (j < 2^25 with ATM on): the list word
                 // shifted past its cell and molecule bits.  This pass reads only
                 // code >> 6 (the cell bits of atm_code are for the COMPAT filter)
                 const int code = (int)(e[u] << 6);
-                const float4 react = make_float4(-gx, -gy, -gz, __int_as_float(code));
+                sr[at ? pos : capr - 1 - pos] = make_float4(-gx, -gy, -gz, __int_as_float(code));
                 if (at) {
-                    const int pos = m + __popc(ma & lt);
-                    if (pos < capa) {
-                        se[pos] = make_float4(dx, dy, dz, __int_as_float(code));
-                        sq[pos] = atm_stage_q(r2);
-                        sr[pos] = react;
-                    }
-                } else {
-                    sr[capr - 1 - (k + __popc(ml & lt))] = react;
+                    se[pos] = make_float4(dx, dy, dz, __int_as_float(code));
+                    sq[pos] = atm_stage_q(r2);
                 }
             }
             m += __popc(ma);
@@ -862,7 +854,7 @@ __device__ __forceinline__ void lj_atm_half_body(const PairParams &p, const AtmP
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int capa = p.nl_cap, capr = p.vl_cap;
     float4 *se = s_dyn + (size_t)w * (2 * capa + capr), *sq = se + capa, *sr = sq + capa;
-    const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq, rc3f = (float)a.rc2;
+    const float rc2 = p.rc2f, rc3sq = p.rc3sqf, rc3f = a.rc2f;
     const unsigned lt = lanemask_lt();
     if (bid == 0 && threadIdx.x == 0 && p.rebuild_done) *p.rebuild_done = 0;
     for (int it = 0; it < per; it++) {
@@ -887,9 +879,10 @@ __device__ __forceinline__ void lj_atm_half_body(const PairParams &p, const AtmP
                 vz = fmaf(sa, az, vz);
             }
             unsigned long long *acc = a.acc + 3 * (size_t)(__float_as_int(rr.w) >> 6);
-            atm_fix_add(acc, vx);
-            atm_fix_add(acc + 1, vy);
-            atm_fix_add(acc + 2, vz);
+            // hardly a zero among them: added without a look
+            atomicAdd(acc, (unsigned long long)fix32_rn(vx));
+            atomicAdd(acc + 1, (unsigned long long)fix32_rn(vy));
+            atomicAdd(acc + 2, (unsigned long long)fix32_rn(vz));
         }
         // the site's own force: its LJ sum and its ATM share
         fx = fmaf(sa, gx, fx);
