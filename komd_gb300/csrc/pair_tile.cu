@@ -530,58 +530,52 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, in
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (e[u] != 0xffffffffu) {
-                o[u] = off[(e[u] >> 26) & 31u];
-                pj[u] = p.pos4[e[u] & 0x3ffffffu];
-                if (!UNIFORM) sej[u] = p.seps[e[u] & 0x3ffffffu];
-            }
+            const unsigned x = e[u] != 0xffffffffu ? e[u] : 0u;   // slot 0 and its site's own cell: read, not used
+            o[u] = off[(x >> 26) & 31u];
+            pj[u] = p.pos4[x & 0x3ffffffu];
+            if (!UNIFORM) sej[u] = p.seps[x & 0x3ffffffu];
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const bool valid = e[u] != 0xffffffffu;
-            float dx = 0.f, dy = 0.f, dz = 0.f, r2 = 1e30f;
-            if (valid) {
-                dx = pi.x - (pj[u].x + o[u].x);
-                dy = pi.y - (pj[u].y + o[u].y);
-                dz = pi.z - (pj[u].z + o[u].z);
-                r2 = dx * dx + dy * dy + dz * dz;
-                if (p.use_lj && r2 <= rc2 && !(e[u] >> 31)) {
-                    const float inv = rcp_approx(r2);
-                    float x, ee;
-                    if (UNIFORM) {
-                        x = sg2u * inv;
-                        ee = eeu;
-                    } else {
-                        const float sg = pi.w + pj[u].w;
-                        x = sg * sg * inv;
-                        ee = sei * sej[u];
-                    }
-                    const float lj6 = x * x * x;
-                    float fac0 = 24.0f * ee * (2.0f * lj6 * lj6 - lj6) * inv;
-                    float usw = 1.0f;
-                    if (p.sw) {   // switched cutoff: U S, force fac S - 2 U dS/dx
-                        float dS;
-                        sw_eval(r2, p.sw_rc2, p.sw_iw, usw, dS);
-                        fac0 = fac0 * usw - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
-                    }
-                    const float fac = MEASURE ? fac0 : fac0 * p.lj_fscalef;   // ATM2B factor
-                    if (W == 32 || (u & 1) == 0) {
-                        fx += dx * fac; fy += dy * fac; fz += dz * fac;
-                    } else {
-                        hx += dx * fac; hy += dy * fac; hz += dz * fac;
-                    }
-                    if (MEASURE) {
-                        const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
-                        m_u += 2.0f * ee * (lj6 * lj6 - lj6) * usw;
-                        m_pairs += 0.5f;
-                        m_w[0] += 0.5f * dx * gx;
-                        m_w[1] += 0.25f * (dx * gy + dy * gx);
-                        m_w[2] += 0.5f * dy * gy;
-                        m_w[3] += 0.25f * (dx * gz + dz * gx);
-                        m_w[4] += 0.25f * (dy * gz + dz * gy);
-                        m_w[5] += 0.5f * dz * gz;
-                    }
-                }
+            const float dx = pi.x - (pj[u].x + o[u].x), dy = pi.y - (pj[u].y + o[u].y), dz = pi.z - (pj[u].z + o[u].z);
+            const float r2 = valid ? dx * dx + dy * dy + dz * dz : 1e30f;
+            const bool lj = p.use_lj && r2 <= rc2 && !(e[u] >> 31);
+            const float inv = rcp_approx(r2);
+            float x, ee;
+            if (UNIFORM) {
+                x = sg2u * inv;
+                ee = eeu;
+            } else {
+                const float sg = pi.w + pj[u].w;
+                x = sg * sg * inv;
+                ee = sei * sej[u];
+            }
+            const float lj6 = x * x * x;
+            float fac0 = 24.0f * ee * (2.0f * lj6 * lj6 - lj6) * inv;
+            float usw = 1.0f;
+            if (p.sw) {   // switched cutoff: U S, force fac S - 2 U dS/dx
+                float dS;
+                sw_eval(r2, p.sw_rc2, p.sw_iw, usw, dS);
+                fac0 = fac0 * usw - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
+            }
+            if (!MEASURE) fac0 *= p.lj_fscalef;   // ATM2B factor
+            const float fac = lj ? fac0 : 0.f;    // no branch around a dozen instructions
+            if (W == 32 || (u & 1) == 0) {
+                fx += dx * fac; fy += dy * fac; fz += dz * fac;
+            } else {
+                hx += dx * fac; hy += dy * fac; hz += dz * fac;
+            }
+            if (MEASURE && lj) {
+                const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
+                m_u += 2.0f * ee * (lj6 * lj6 - lj6) * usw;
+                m_pairs += 0.5f;
+                m_w[0] += 0.5f * dx * gx;
+                m_w[1] += 0.25f * (dx * gy + dy * gx);
+                m_w[2] += 0.5f * dy * gy;
+                m_w[3] += 0.25f * (dx * gz + dz * gx);
+                m_w[4] += 0.25f * (dy * gz + dz * gy);
+                m_w[5] += 0.5f * dz * gz;
             }
             if (EMIT) {
                 // staged for the once-per-triplet sweep: neighbours above i only
@@ -669,7 +663,8 @@ __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, 
 // a lane in flight with the next two list entries read ahead fit in 48 registers (five
 // blocks an SM, not four).  A lane sums entries of equal place modulo 32 apart, so
 // every force is that of the kernel above bit for bit.  300,000 sites of three-site
-// molecules: 135 -> 90 us; 32,000 sites of liquid argon with the ATM list 25.4 -> 18.8.
+// molecules: 135 -> 90 us, and 86 with selects for the branches around a pair's
+// arithmetic; 32,000 sites of liquid argon with the ATM list 25.4 -> 18.8 -> 17.6.
 // Without the read-ahead 99, four entries in flight 119, six 132 us.
 template <bool EMIT, bool UNIFORM>
 __global__ void __launch_bounds__(256, 5) k_lj_vlist2(PairParams p, int n, int per) {
