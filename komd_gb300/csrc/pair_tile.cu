@@ -9,10 +9,15 @@
 //      coordinates (float4 position + slot, key, cell code, sqrt(eps));
 //   3. every warp owns a subset of home sites; for a home site the 32 lanes
 //      test 32 staged candidates at a time and ballot-compact the hits into a
-//      per-warp queue, so the force arithmetic always runs on full warps;
-//   4. each dequeued pair adds its LJ force to the home site's shared-memory
-//      accumulator and, inside cutoff_3b, appends (r_i - r_j, code) to the
-//      home site's ATM list in queue order (deterministic list order).
+//      per-warp queue, so the force arithmetic runs on full warps;
+//   4. each dequeued pair adds its LJ force to the lane's sum for the home site
+//      and, inside cutoff_3b, appends (r_i - r_j, code) to the home site's ATM
+//      list in queue order (deterministic list order).
+// With sensors the queue runs on over the home sites (their per-lane sums keep
+// their order); forces alone empty it at each site, which wastes some lanes of
+// the last evaluation but needs no grouping of the lanes by site, no segmented
+// sums (30 shuffles and adds an evaluation) and no read-modify-write of the
+// site's sum and count: 32,000 sites of liquid argon 44 -> 33 us.
 // Full shell: each site's force is summed by its own CTA, no global atomics.
 //
 // The Verlet path (skin > 0) has its own kernels here: the list build
@@ -98,6 +103,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
     const float rc2 = (float)p.rc2, rc3sq = (float)p.rc3sq, scan2 = (float)p.scan2;
     float4 *nl = p.nl;
     float m_u = 0.f, m_pairs = 0.f, m_w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // per-lane partials (MEASURE)
+    const unsigned lt = lanemask_lt();
 
     for (int hb = 0; hb < hn; hb += kHome) {
         const int hc = min(kHome, hn - hb);
@@ -127,7 +133,70 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                 s_pos[t] = q;
                 s_aux[t] = make_int4(j, p.skey[j], nb | s_nbc[nb], __float_as_int(p.seps[j]));
             }
+            if (ns + tid < ((ns + 31) & ~31)) s_pos[ns + tid] = make_float4(1e15f, 1e15f, 1e15f, 0.f);   // out of reach
             __syncthreads();
+
+            if (!MEASURE) {
+                // a home site at a time: its force stays in the lanes' registers, with one
+                // reduction at the end
+                for (int i = w; i < hc; i += kTileWarps) {
+                    const float4 pi = s_hpos[i];
+                    const int2 ha = s_haux[i];
+                    const float sei = __int_as_float(ha.y);
+                    const int self = self_base + i - sb;
+                    float4 *row = EMIT ? nl + (size_t)(hs + hb + i) * p.nl_cap : nullptr;
+                    float fx = 0.f, fy = 0.f, fz = 0.f;
+                    int cnt = EMIT ? s_cnt[i] : 0;
+                    auto pair = [&](int j, bool valid) {
+                        const float4 pj = s_pos[j];
+                        const int4 a = s_aux[j];
+                        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                        const float r2 = valid ? dx * dx + dy * dy + dz * dz : 1e30f;
+                        const float inv = rcp_approx(r2);
+                        const float sg = pi.w + pj.w;
+                        const float x = sg * sg * inv;
+                        const float lj6 = x * x * x;
+                        const float ee = sei * __int_as_float(a.w);
+                        const float ljd = 24.0f * ee * (2.0f * lj6 * lj6 - lj6);
+                        const float fac = p.use_lj && r2 <= rc2 && ha.x != a.y ? ljd * inv * p.lj_fscalef : 0.f;
+                        fx += dx * fac;
+                        fy += dy * fac;
+                        fz += dz * fac;
+                        if (EMIT) {
+                            const bool emit = r2 <= rc3sq;
+                            const unsigned em = __ballot_sync(0xffffffffu, emit);
+                            const int c = cnt + __popc(em & lt);
+                            if (emit && c < p.nl_cap) row[c] = make_float4(dx, dy, dz, __int_as_float(a.z | (a.x << 6)));
+                            cnt += __popc(em);
+                        }
+                    };
+                    int qn = 0;
+                    for (int j0 = 0; j0 < ns; j0 += 32) {
+                        const int j = j0 + lane;
+                        const float4 pj = s_pos[j];
+                        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                        const bool hit = dx * dx + dy * dy + dz * dz <= scan2 && j != self;
+                        const unsigned m = __ballot_sync(0xffffffffu, hit);
+                        if (hit) s_q[w][qn + __popc(m & lt)] = (unsigned)j;
+                        qn += __popc(m);
+                        if (qn >= 32) {
+                            __syncwarp();
+                            const unsigned e = s_q[w][lane], tail = s_q[w][lane + 32];
+                            __syncwarp();
+                            qn -= 32;
+                            if (lane < qn) s_q[w][lane] = tail;
+                            pair((int)e, true);
+                        }
+                    }
+                    __syncwarp();
+                    if (qn > 0) pair(lane < qn ? (int)s_q[w][lane] : 0, lane < qn);
+                    const float fs = warp_sum3(fx, fy, fz, lane);
+                    if ((lane & 7) == 0 && lane < 24) s_f[3 * i + (lane >> 3)] += fs;
+                    if (EMIT && lane == 0) s_cnt[i] = cnt;
+                    __syncwarp();   // the queue is refilled by the next site
+                }
+                continue;
+            }
 
             // Process one queued pair per lane (valid = lane holds an entry).
             // Entries of one home site occupy contiguous lanes (the queue is
@@ -152,7 +221,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                     const float lj6 = x * x * x;
                     const float ee = __int_as_float(s_haux[i].y) * __int_as_float(a.w);
                     const float ljd = 24.0f * ee * (2.0f * lj6 * lj6 - lj6);
-                    const float fac = MEASURE ? ljd * inv : ljd * inv * p.lj_fscalef;   // ATM2B factor
+                    const float fac = ljd * inv;
                     fx = dx * fac; fy = dy * fac; fz = dz * fac;
                     if (MEASURE) {
                         const float wt = (p.virial_compat && (a.z & 32)) ? 1.0f : 0.5f;
