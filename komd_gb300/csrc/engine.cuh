@@ -31,6 +31,13 @@ namespace komd {
 // access) holds it until the predecessor has completed and its writes are
 // visible, and pdl_trigger lets the successor be scheduled once every block
 // of this grid has started.  Both are no-ops without a programmatic launch.
+// Every kernel of a single system's step waits at its entry and is launched so: its
+// launch overlaps the end of its predecessor.  The passes of a few microseconds (the
+// container stages, the integrator) trigger as well; the force passes do not: their
+// successor's blocks, resident early, take their shared memory and slots.  Steps of 4096
+// sites 14.8 us with plain launches of the force and integrator passes, 15.3 with a
+// trigger in each, 14.3 with none there, 14.1 with the integrator's; without any, the container's
+// included, 15.6.  32,000 sites with the learned term 81.1, 86.7, 79.3, 78.6 (none: 80.0).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

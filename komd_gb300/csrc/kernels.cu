@@ -549,6 +549,7 @@ __device__ __forceinline__ T warp_sum_split(T (&v)[K], int lane) {
 // vertex kept the FP64 pipe 76 % busy: 525 -> 380 us at 256,000 sites).
 template <bool MEASURE, bool COMPAT>
 __global__ void __launch_bounds__(kBlock) k_atm_q(AtmParams p) {
+    pdl_wait();
     extern __shared__ float4 s_dyn[];
     __shared__ unsigned s_q[kWarpsPerBlock][64];
     __shared__ float s_qc[kWarpsPerBlock][64];
@@ -802,6 +803,7 @@ __global__ void __launch_bounds__(kBondComps) k_bonded_mol(const int4 *__restric
                                                            const int4 *__restrict__ terms,
                                                            const double *__restrict__ r, double *__restrict__ f,
                                                            float kb, float r0, float ka, float th0) {
+    pdl_wait();
     __shared__ double s_r[3 * kBondSites], s_f[3 * kBondSites];
     const int4 b = blocks[blockIdx.x];   // components [x, y), sites [z, w)
     const int n3 = 3 * (b.w - b.z), c = b.x + (int)threadIdx.x;
@@ -863,6 +865,8 @@ __global__ void __launch_bounds__(kBondComps) k_bonded_mol(const int4 *__restric
 // Limit_Force (Limit.cpp:19-25): clamp with Kokkos::min / max semantics
 __global__ void k_limit(int n, const double *__restrict__ eps, const double *__restrict__ sig, double limit,
                         double *__restrict__ f) {
+    pdl_trigger();
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const double fmax = limit * eps[s] / sig[s];
@@ -901,6 +905,8 @@ __global__ void k_step0(int n, double *__restrict__ r, double *__restrict__ v, c
                         const double *__restrict__ bias, const float4 *__restrict__ ref4,
                         const int *__restrict__ site_slot, float4 *__restrict__ pos4, float half_skin2,
                         int *__restrict__ rebuild) {
+    pdl_trigger();
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const double c = hdtm[s];
@@ -1053,11 +1059,14 @@ __device__ __forceinline__ void step0_fused_body(const Step0Args &a, int bid) {
 }
 __global__ void __launch_bounds__(kIoBlock) k_step0_fused(Step0Args a) {
     pdl_trigger();
+    pdl_wait();
     step0_fused_body(a, blockIdx.x);
 }
 
 __global__ void k_step1(int n, double *__restrict__ v, const double *__restrict__ f, const double *__restrict__ hdtm,
                         int *__restrict__ err, int *__restrict__ rebuild) {
+    pdl_trigger();
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (rebuild && s == 0) *rebuild = 0;   // every consumer of this step's flag has run
     if (s >= n) return;
@@ -1085,6 +1094,7 @@ template <bool TERMS>
 __global__ void __launch_bounds__(kBlock) k_kinetic(Grid g, int n, int n_terms, const double *__restrict__ r,
                                                     const double *__restrict__ v, const double *__restrict__ m,
                                                     double *partials, double *__restrict__ acc, unsigned *done) {
+    pdl_wait();
     __shared__ double s_part[kWarpsPerBlock][8];
     __shared__ bool s_last;
     constexpr int kVals = TERMS ? 8 : 2;
@@ -1338,6 +1348,7 @@ __global__ void k_rdf_all(Grid g, int n_mol, const double *__restrict__ com, dou
 constexpr int kSumThreads = 256;
 __global__ void __launch_bounds__(kSumThreads) k_sum_partials(int nblocks, const double *__restrict__ partials,
                                                               double *__restrict__ out) {
+    pdl_wait();
     __shared__ double s_w[kSumThreads / 32];
     const int slot = blockIdx.x, t = threadIdx.x, lane = t & 31;
     double s = 0.0;
@@ -1359,6 +1370,8 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_partials(int nblocks, const
 // the host reads after the step.
 __global__ void k_velocity_scale(int n, double *__restrict__ v, const double *__restrict__ acc, double t_target,
                                  SciNum factor, double beta_in, int *__restrict__ err) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ double s_beta;
     if (threadIdx.x == 0) {
         double beta = beta_in;
@@ -1531,9 +1544,8 @@ int launch_pair(Engine &e, cudaStream_t st, bool measure, double *lj_hist) {
 
 void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc) {
     if (!measure && e.bond_blocks > 0 && e.bond_sites == e.n) {
-        k_bonded_mol<<<e.bond_blocks, kBondComps, 0, st>>>(e.bond_block, e.comp_off, e.comp_terms, e.r, e.f,
-                                                           (float)e.cfg.bond_k, (float)e.cfg.bond_r0,
-                                                           (float)e.cfg.angle_k, (float)e.cfg.angle_theta0);
+        launch_pdl(k_bonded_mol, e.bond_blocks, kBondComps, 0, st, e.bond_block, e.comp_off, e.comp_terms, e.r, e.f,
+                   (float)e.cfg.bond_k, (float)e.cfg.bond_r0, (float)e.cfg.angle_k, (float)e.cfg.angle_theta0);
         return;
     }
     if (e.n_bonds > 0)
@@ -1546,7 +1558,7 @@ void launch_bonded(Engine &e, cudaStream_t st, bool measure, double *acc) {
 
 void launch_limit(Engine &e, cudaStream_t st) {
     const int b = site_block(e, e.n);
-    k_limit<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.eps, e.sig, e.cfg.limit, e.f);
+    launch_pdl(k_limit, nblk(e.n, b), b, 0, st, (int)e.n, e.eps, e.sig, e.cfg.limit, e.f);
 }
 
 size_t atm_smem(const Engine &e) {
@@ -1580,6 +1592,7 @@ __device__ __forceinline__ int atm_stage(const AtmParams &p, int i, float4 *se, 
 
 // one warp per vertex: stage its neighbours above it, then the sweep
 __global__ void __launch_bounds__(kBlock) k_atm_s(AtmParams p) {
+    pdl_wait();
     extern __shared__ float4 s_dyn[];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cap = p.nl_cap;
@@ -1712,6 +1725,7 @@ __device__ __forceinline__ void kick_drift_body(const FlushArgs &a, const Step0A
 }
 template <int MODE>
 __global__ void __launch_bounds__(kIoBlock) k_kick_drift(FlushArgs a, Step0Args dr, float4 *fsur) {
+    pdl_trigger();
     pdl_wait();
     kick_drift_body<MODE>(a, dr, fsur, blockIdx.x);
 }
@@ -1723,6 +1737,8 @@ __global__ void k_step10(int n, double *__restrict__ r, double *__restrict__ v, 
                          const float4 *__restrict__ ref4, const int *__restrict__ site_slot,
                          float4 *__restrict__ pos4, float half_skin2, int *__restrict__ rebuild,
                          int *__restrict__ err) {
+    pdl_trigger();
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const double c = hdtm[s];
@@ -1748,6 +1764,7 @@ __global__ void k_step10(int n, double *__restrict__ r, double *__restrict__ v, 
 // f[site] += 2 sign nu g (fixed point -> FP64) and the accumulators back to 0
 __global__ void k_atm_flush(int n, const int *__restrict__ slot_site, unsigned long long *__restrict__ acc,
                             double *__restrict__ f, double scale_fix, const float4 *__restrict__ own) {
+    pdl_wait();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= n) return;
     const int site = slot_site[slot];
@@ -1770,11 +1787,11 @@ __global__ void k_atm_flush(int n, const int *__restrict__ slot_site, unsigned l
 
 static void atm_dispatch_f(AtmParams &p, bool measure, bool compat, int grid, size_t sm, cudaStream_t st) {
     if (measure) {
-        if (compat) k_atm_q<true, true><<<grid, kBlock, sm, st>>>(p);
-        else k_atm_q<true, false><<<grid, kBlock, sm, st>>>(p);
+        if (compat) launch_pdl(k_atm_q<true, true>, grid, kBlock, sm, st, p);
+        else launch_pdl(k_atm_q<true, false>, grid, kBlock, sm, st, p);
     } else {
-        if (compat) k_atm_q<false, true><<<grid, kBlock, sm, st>>>(p);
-        else k_atm_q<false, false><<<grid, kBlock, sm, st>>>(p);
+        if (compat) launch_pdl(k_atm_q<false, true>, grid, kBlock, sm, st, p);
+        else launch_pdl(k_atm_q<false, false>, grid, kBlock, sm, st, p);
     }
 }
 
@@ -1827,7 +1844,7 @@ bool launch_atm_flush(Engine &e, cudaStream_t st, StepEnd end, bool force_units)
                    (float4 *)nullptr);
         return true;
     }
-    k_atm_flush<<<nblk(e.n, 256), 256, 0, st>>>((int)e.n, e.slot_site, e.atm_acc, e.f, scale_fix, own);
+    launch_pdl(k_atm_flush, nblk(e.n, 256), 256, 0, st, (int)e.n, e.slot_site, e.atm_acc, e.f, scale_fix, own);
     return false;
 }
 
@@ -1836,7 +1853,7 @@ bool launch_atm(Engine &e, cudaStream_t st, bool measure, StepEnd end) {
     const bool compat = e.cfg.atm_enum == KOMD_ATM_ENUM_COMPAT;
     if (!measure && !compat && e.cfg.precision == KOMD_FP32 && e.atm_acc) {
         // every triplet once (lowest slot), fixed-point scatter, then the flush into f
-        k_atm_s<<<nblk(e.n, kWarpsPerBlock), kBlock, atm_smem(e), st>>>(p);
+        launch_pdl(k_atm_s, nblk(e.n, kWarpsPerBlock), kBlock, atm_smem(e), st, p);
         return launch_atm_flush(e, st, end, false);
     }
     if (e.cfg.precision == KOMD_FP64)
@@ -1849,13 +1866,12 @@ void launch_step0(Engine &e, cudaStream_t st, bool in_step) {
     const float hs = (float)(0.5 * e.cfg.skin);
     if (in_step && e.fused_drift) {
         const int b = site_block(e, e.n);
-        k_step0_fused<<<nblk(e.n, b), b, 0, st>>>(step0_args(e));
+        launch_pdl(k_step0_fused, nblk(e.n, b), b, 0, st, step0_args(e));
         return;
     }
     const int b = site_block(e, e.n);
-    k_step0<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
-                                              e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4,
-                                          hs * hs, e.rebuild);
+    launch_pdl(k_step0, nblk(e.n, b), b, 0, st, (int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
+               e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4, hs * hs, e.rebuild);
 }
 
 // integrate1 of a step and integrate0 of the next
@@ -1867,9 +1883,9 @@ void launch_kick_drift(Engine &e, cudaStream_t st) {
         return;
     }
     const float hs = (float)(0.5 * e.cfg.skin);
-    k_step10<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
-                                             e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4,
-                                             hs * hs, e.rebuild, e.err);
+    launch_pdl(k_step10, nblk(e.n, b), b, 0, st, (int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
+               e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4, hs * hs, e.rebuild,
+               e.err);
 }
 
 // the same with the learned term's forces (fsur, slot order) added first; needs the fused drift
@@ -1881,27 +1897,29 @@ void launch_learned_kick_drift(Engine &e, float *fsur, cudaStream_t st) {
 
 void launch_step1(Engine &e, cudaStream_t st) {
     const int b = site_block(e, e.n);
-    k_step1<<<nblk(e.n, b), b, 0, st>>>((int)e.n, e.v, e.f, e.hdtm, e.err,
-                                              e.verlet ? e.rebuild : nullptr);
+    launch_pdl(k_step1, nblk(e.n, b), b, 0, st, (int)e.n, e.v, e.f, e.hdtm, e.err, e.verlet ? e.rebuild : nullptr);
 }
 
 int kinetic_grid(const Engine &e) { return std::min(nblk(e.n, kBlock), e.num_sms * 2); }
 
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta) {
     const int b = site_block(e, 3 * e.n);
-    k_velocity_scale<<<std::min(nblk(3 * e.n, b), e.num_sms * 8), b, 0, st>>>((int)e.n, e.v, acc, e.cfg.temperature_target, sci_factor(), beta, e.err);
+    launch_pdl(k_velocity_scale, std::min(nblk(3 * e.n, b), e.num_sms * 8), b, 0, st, (int)e.n, e.v, acc,
+               e.cfg.temperature_target, sci_factor(), beta, e.err);
 }
 
 // the kinetic sums into acc (R_NSLOTS), whose other slots become zero
 void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc) {
     const int grid = kinetic_grid(e);
     if (n_terms > 0)
-        k_kinetic<true><<<grid, kBlock, 0, st>>>(e.g, (int)e.n, n_terms, e.r, e.v, e.m, e.partials, acc, e.kin_done);
-    else k_kinetic<false><<<grid, kBlock, 0, st>>>(e.g, (int)e.n, 0, e.r, e.v, e.m, e.partials, acc, e.kin_done);
+        launch_pdl(k_kinetic<true>, grid, kBlock, 0, st, e.g, (int)e.n, n_terms, e.r, e.v, e.m, e.partials, acc,
+                   e.kin_done);
+    else launch_pdl(k_kinetic<false>, grid, kBlock, 0, st, e.g, (int)e.n, 0, e.r, e.v, e.m, e.partials, acc,
+                    e.kin_done);
 }
 
 void launch_sum_partials(cudaStream_t st, int nblocks, const double *partials, double *out) {
-    k_sum_partials<<<R_NSLOTS, kSumThreads, 0, st>>>(nblocks, partials, out);
+    launch_pdl(k_sum_partials, R_NSLOTS, kSumThreads, 0, st, nblocks, partials, out);
 }
 
 void launch_rdf(Engine &e, cudaStream_t st, double *bins, bool cells) {

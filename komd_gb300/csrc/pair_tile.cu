@@ -63,6 +63,7 @@ __device__ __forceinline__ int nb_cell(const Grid &g, int cx, int cy, int cz, in
 
 template <bool MEASURE, bool EMIT>
 __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
+    pdl_wait();
     __shared__ float4 s_pos[kStage];
     __shared__ int4 s_aux[kStage];        // slot, key, code (nb | crosses << 5), sqrt(eps) bits
     __shared__ float4 s_hpos[kHome];
@@ -683,6 +684,7 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, in
 
 template <bool MEASURE, bool EMIT, bool UNIFORM, int U>
 __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, int n, int per) {
+    pdl_wait();
     __shared__ double s_part[8][8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const float rc2 = p.rc2f, rc3sq = p.rc3sqf;
@@ -737,6 +739,7 @@ __global__ void __launch_bounds__(256, U == 3 ? 4 : 5) k_lj_vlist(PairParams p, 
 // Without the read-ahead 99, four entries in flight 119, six 132 us.
 template <bool EMIT, bool UNIFORM>
 __global__ void __launch_bounds__(256, 5) k_lj_vlist2(PairParams p, int n, int per) {
+    pdl_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const float rc2 = p.rc2f, rc3sq = p.rc3sqf;
     unsigned lt;
@@ -759,6 +762,7 @@ __global__ void __launch_bounds__(256, 5) k_lj_vlist2(PairParams p, int n, int p
 // the order of every sum are those of k_lj_vlist + k_atm_s.
 template <bool UNIFORM, int U>
 __global__ void __launch_bounds__(256, 4) k_lj_atm(PairParams p, AtmParams a, int n, int per) {
+    pdl_wait();
     extern __shared__ float4 s_dyn[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float4 *se = s_dyn + w * 2 * p.nl_cap, *sq = se + p.nl_cap;
@@ -1119,14 +1123,14 @@ template <bool UNIFORM>
 static void lj_vlist_dispatch(PairParams &p, int n, int grid, int per, bool measure, bool emit, bool u3,
                               cudaStream_t st) {
     if (measure) {
-        if (emit) k_lj_vlist<true, true, UNIFORM, 2><<<grid, 256, 0, st>>>(p, n, per);
-        else k_lj_vlist<true, false, UNIFORM, 2><<<grid, 256, 0, st>>>(p, n, per);
+        if (emit) launch_pdl(k_lj_vlist<true, true, UNIFORM, 2>, grid, 256, 0, st, p, n, per);
+        else launch_pdl(k_lj_vlist<true, false, UNIFORM, 2>, grid, 256, 0, st, p, n, per);
     } else if (u3) {
-        if (emit) k_lj_vlist<false, true, UNIFORM, 3><<<grid, 256, 0, st>>>(p, n, per);
-        else k_lj_vlist<false, false, UNIFORM, 3><<<grid, 256, 0, st>>>(p, n, per);
+        if (emit) launch_pdl(k_lj_vlist<false, true, UNIFORM, 3>, grid, 256, 0, st, p, n, per);
+        else launch_pdl(k_lj_vlist<false, false, UNIFORM, 3>, grid, 256, 0, st, p, n, per);
     } else {
-        if (emit) k_lj_vlist<false, true, UNIFORM, 2><<<grid, 256, 0, st>>>(p, n, per);
-        else k_lj_vlist<false, false, UNIFORM, 2><<<grid, 256, 0, st>>>(p, n, per);
+        if (emit) launch_pdl(k_lj_vlist<false, true, UNIFORM, 2>, grid, 256, 0, st, p, n, per);
+        else launch_pdl(k_lj_vlist<false, false, UNIFORM, 2>, grid, 256, 0, st, p, n, per);
     }
 }
 
@@ -1147,7 +1151,7 @@ int launch_lj_vlist(Engine &e, PairParams &p, bool measure, bool emit, cudaStrea
         const int per2 = (vlist_per(e) + 1) / 2, grid2 = (int)((e.n + 16 * per2 - 1) / (16 * per2));
         auto k = e.uniform ? (emit ? k_lj_vlist2<true, true> : k_lj_vlist2<false, true>)
                            : (emit ? k_lj_vlist2<true, false> : k_lj_vlist2<false, false>);
-        k<<<grid2, 256, 0, st>>>(p, (int)e.n, per2);
+        launch_pdl(k, grid2, 256, 0, st, p, (int)e.n, per2);
         return grid2;
     }
     // a block's partial sums cover all its groups (the lanes' sums run across them)
@@ -1183,29 +1187,29 @@ void launch_lj_atm(Engine &e, cudaStream_t st) {
     if (e.uniform) {
         if (u3) {
             if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_lj_atm<true, 3><<<grid, 256, sm, st>>>(p, a, (int)e.n, per);
+            launch_pdl(k_lj_atm<true, 3>, grid, 256, sm, st, p, a, (int)e.n, per);
         } else {
             if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_lj_atm<true, 2><<<grid, 256, sm, st>>>(p, a, (int)e.n, per);
+            launch_pdl(k_lj_atm<true, 2>, grid, 256, sm, st, p, a, (int)e.n, per);
         }
     } else {
         if (u3) {
             if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_lj_atm<false, 3><<<grid, 256, sm, st>>>(p, a, (int)e.n, per);
+            launch_pdl(k_lj_atm<false, 3>, grid, 256, sm, st, p, a, (int)e.n, per);
         } else {
             if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_lj_atm<false, 2><<<grid, 256, sm, st>>>(p, a, (int)e.n, per);
+            launch_pdl(k_lj_atm<false, 2>, grid, 256, sm, st, p, a, (int)e.n, per);
         }
     }
 }
 
 void launch_pair_tile(PairParams &p, int ncell, bool measure, bool emit, cudaStream_t st) {
     if (measure) {
-        if (emit) k_pair_tile<true, true><<<ncell, kTileThreads, 0, st>>>(p);
-        else k_pair_tile<true, false><<<ncell, kTileThreads, 0, st>>>(p);
+        if (emit) launch_pdl(k_pair_tile<true, true>, ncell, kTileThreads, 0, st, p);
+        else launch_pdl(k_pair_tile<true, false>, ncell, kTileThreads, 0, st, p);
     } else {
-        if (emit) k_pair_tile<false, true><<<ncell, kTileThreads, 0, st>>>(p);
-        else k_pair_tile<false, false><<<ncell, kTileThreads, 0, st>>>(p);
+        if (emit) launch_pdl(k_pair_tile<false, true>, ncell, kTileThreads, 0, st, p);
+        else launch_pdl(k_pair_tile<false, false>, ncell, kTileThreads, 0, st, p);
     }
 }
 

@@ -41,6 +41,7 @@ namespace komd {
 static_assert(kSurNC == 4 && kSurNR == 16, "a lane per channel, four radials each");
 
 __global__ void __launch_bounds__(128) k_sur_desc(SurParams p) {
+    pdl_wait();
     const int gi = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, c4 = threadIdx.x & 3;
     const bool in = gi < p.n;   // whole warps run on: the exchange needs every lane
     const int i = in ? gi : p.n - 1;
@@ -187,6 +188,7 @@ __device__ __forceinline__ void sur_stage_weights(const SurParams &p, __nv_bfloa
 }
 
 __global__ void __launch_bounds__(128) k_sur_mlp(SurParams p) {
+    pdl_wait();
     __shared__ __align__(16) __nv_bfloat16 sW1[kSurH * kSurNF], sW1T[kSurNF * kSurH], sW2[kSurH * kSurH],
         sW2T[kSurH * kSurH];
     __shared__ float sb1[kSurH], sb2[kSurH], sw3[kSurH];
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(128) k_sur_mlp(SurParams p) {
 // wave (a pass of 20 steps 1.72 ms; 1.75 at five, 1.78 at six, 1.76 at eight).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128, 7) k_sur_force(SurParams p) {
+    pdl_wait();
     const int gi = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 31, c4 = lane & 3;
     const bool in = gi < p.n;
     const int i = in ? gi : p.n - 1;
@@ -300,6 +303,7 @@ __global__ void k_sur_apply(int n, const int *__restrict__ slot_site, float *__r
 __global__ void k_sur_apply_step1(int n, const int *__restrict__ site_slot, float *__restrict__ fsur,
                                   double *__restrict__ f, double *__restrict__ v, const double *__restrict__ hdtm,
                                   int *__restrict__ err, int *__restrict__ rebuild) {
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (rebuild && s == 0) *rebuild = 0;   // every consumer of this step's flag has run
     if (s >= n) return;
@@ -443,7 +447,7 @@ __global__ void k_train_adam(TrainParams t, int step) {
 // ---------------------------------------------------------------------------
 // fstd == nullptr: raw features (training samples)
 void launch_sur_desc(SurParams &p, cudaStream_t st) {
-    if (p.fstd) k_sur_desc<<<(p.n + 31) / 32, 128, 0, st>>>(p);
+    if (p.fstd) launch_pdl(k_sur_desc, (p.n + 31) / 32, 128, 0, st, p);
     else k_sur_sample<<<(p.n + 127) / 128, 128, 0, st>>>(p);
 }
 void launch_sur_mlp(SurParams &p, cudaStream_t st) {
@@ -451,12 +455,12 @@ void launch_sur_mlp(SurParams &p, cudaStream_t st) {
     int blocks = (tiles + 3) / 4;
     const int cap = 4 * (p.num_sms > 0 ? p.num_sms : 152);
     if (blocks > cap) blocks = cap;   // persistent: weights staged once per block
-    k_sur_mlp<<<blocks, 128, 0, st>>>(p);
+    launch_pdl(k_sur_mlp, blocks, 128, 0, st, p);
 }
-void launch_sur_force(SurParams &p, cudaStream_t st) { k_sur_force<<<(p.n + 31) / 32, 128, 0, st>>>(p); }
+void launch_sur_force(SurParams &p, cudaStream_t st) { launch_pdl(k_sur_force, (p.n + 31) / 32, 128, 0, st, p); }
 void launch_sur_apply_step1(SurParams &p, const Engine &e, cudaStream_t st) {
-    k_sur_apply_step1<<<(p.n + 127) / 128, 128, 0, st>>>(p.n, e.site_slot, p.fsur, e.f, e.v, e.hdtm, e.err,
-                                                          e.verlet ? e.rebuild : nullptr);
+    launch_pdl(k_sur_apply_step1, (p.n + 127) / 128, 128, 0, st, p.n, e.site_slot, p.fsur, e.f, e.v, e.hdtm, e.err,
+               e.verlet ? e.rebuild : nullptr);
 }
 void launch_sur_apply(SurParams &p, const int *slot_site, double *f, double *fout, cudaStream_t st) {
     k_sur_apply<<<(p.n + 255) / 256, 256, 0, st>>>(p.n, slot_site, p.fsur, f, fout);

@@ -116,3 +116,26 @@ def test_wrap_at_the_faces_without_a_rebuild(sites):
     assert np.abs(a - free - k * L).max() < 1e-12
     assert (k != 0).any() and (np.abs(k) <= 1).all()
     g.close()
+
+
+@pytest.mark.parametrize("bonded", [False, True])
+def test_steps_without_a_pair_term(bonded):
+    """the forces start from a clearing, not from a pair kernel, in every step"""
+    from komd_gb300 import gpu, lattice
+    s = lattice.argon_fcc(3, rho=0.4, t_star=1.0, seed=2, jitter=0.1)
+    if bonded:
+        s.bonds = np.array([(k, k + 1) for k in range(0, s.n, 2)], np.int64)
+    cfg = gpu.make_config(s.low, s.high, float(s.high[0]) / 3, cutoff=1.0, terms=gpu.TERM_BONDED, dt=1e-3,
+                          bond_k=80.0, bond_r0=1.1, angle_k=30.0, angle_theta0=1.9)
+    a, b = gpu.GpuSystem(s, cfg), gpu.GpuSystem(s, cfg)
+    for g in (a, b):
+        g.update_container()
+        g.forces()
+    a.step(9)
+    for _ in range(9):
+        b.step(1)
+    for x, y in zip(a.download(), b.download()):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
+    assert np.any(a.download()[2]) == bonded
+    a.close()
+    b.close()
