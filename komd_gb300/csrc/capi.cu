@@ -76,6 +76,7 @@ struct Surrogate {
     float *x = nullptr, *mom = nullptr, *dedx = nullptr, *esite = nullptr, *fsur = nullptr;
     __nv_bfloat16 *w1 = nullptr, *w1t = nullptr, *w2 = nullptr, *w2t = nullptr;
     float *b1 = nullptr, *b2 = nullptr, *w3 = nullptr, *fmean = nullptr, *fstd = nullptr;
+    float *fgrad = nullptr;   // e_scale / fstd
     float b3 = 0.f, e_scale = 1.f, e_shift = 0.f;
     int probe_every = 0;
     double probe_threshold = 0.0, last_rmse = -1.0, max_rmse = 0.0;
@@ -186,6 +187,7 @@ SurParams sur_params(komd_gpu *h) {
     p.nl_cap = e.nl_cap;
     p.fmean = u.fmean;
     p.fstd = u.fstd;
+    p.fgrad = u.fgrad;
     p.x = u.x;
     p.mom = u.mom;
     p.dedx = u.dedx;
@@ -658,7 +660,7 @@ int komd_gpu_destroy(komd_gpu *h) {
     {
         Surrogate &u = h->sur;
         dfree(u.x); dfree(u.mom); dfree(u.dedx); dfree(u.esite); dfree(u.fsur); dfree(u.w1); dfree(u.w1t);
-        dfree(u.w2); dfree(u.w2t); dfree(u.b1); dfree(u.b2); dfree(u.w3); dfree(u.fmean); dfree(u.fstd);
+        dfree(u.w2); dfree(u.w2t); dfree(u.b1); dfree(u.b2); dfree(u.w3); dfree(u.fmean); dfree(u.fstd); dfree(u.fgrad);
         dfree(u.fprobe); dfree(u.fsur_d); dfree(u.probe_acc);
     }
     for (auto &p : h->pending) { h->pool.push_back(p.second.first); h->pool.push_back(p.second.second); }
@@ -1427,6 +1429,10 @@ int komd_gpu_surrogate_load(komd_gpu *h, const float *params, const float *fmean
     CK(cudaMemcpy(u.w3, w3, sizeof(float) * H, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(u.fmean, fmean, sizeof(float) * F, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(u.fstd, fstd, sizeof(float) * F, cudaMemcpyHostToDevice));
+    std::vector<float> fgrad(F);
+    for (int k = 0; k < F; k++) fgrad[k] = (float)e_scale / fstd[k];
+    CK(dalloc(u.fgrad, F));
+    CK(cudaMemcpy(u.fgrad, fgrad.data(), sizeof(float) * F, cudaMemcpyHostToDevice));
     u.b3 = b3[0];
     u.e_scale = (float)e_scale;
     u.e_shift = (float)e_shift;

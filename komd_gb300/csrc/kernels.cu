@@ -735,12 +735,11 @@ __global__ void k_bonds(int nb, const int *__restrict__ bonds, const double *__r
         }
     }
     if (measure) {
-        double vals[7] = {e, w[0], w[1], w[2], w[3], w[4], w[5]};
-        for (int k = 0; k < 7; k++) {
-            double x = vals[k];
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if ((threadIdx.x & 31) == 0) atomicAdd(&partials[k == 0 ? R_UBOND : R_W0 + k - 1], x);
-        }
+        const int lane = threadIdx.x & 31;
+        double vals[8] = {e, w[0], w[1], w[2], w[3], w[4], w[5], 0.0};
+        const double x = warp_sum_split<double, 8>(vals, lane);   // value k in lane 4 k
+        const int k = lane >> 2;
+        if ((lane & 3) == 0 && k < 7) atomicAdd(&partials[k == 0 ? R_UBOND : R_W0 + k - 1], x);
     }
 }
 
@@ -781,12 +780,11 @@ __global__ void k_angles(int na, const int *__restrict__ angles, const double *_
         }
     }
     if (measure) {
-        double vals[7] = {e, w[0], w[1], w[2], w[3], w[4], w[5]};
-        for (int q = 0; q < 7; q++) {
-            double x = vals[q];
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if ((threadIdx.x & 31) == 0) atomicAdd(&partials[q == 0 ? R_UBOND : R_W0 + q - 1], x);
-        }
+        const int lane = threadIdx.x & 31;
+        double vals[8] = {e, w[0], w[1], w[2], w[3], w[4], w[5], 0.0};
+        const double x = warp_sum_split<double, 8>(vals, lane);   // value k in lane 4 k
+        const int k = lane >> 2;
+        if ((lane & 3) == 0 && k < 7) atomicAdd(&partials[k == 0 ? R_UBOND : R_W0 + k - 1], x);
     }
 }
 

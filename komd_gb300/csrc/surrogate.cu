@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(128, 7) k_sur_force(SurParams p) {
         dr[4 * k] = t.x; dr[4 * k + 1] = t.y; dr[4 * k + 2] = t.z; dr[4 * k + 3] = t.w;
     }
 #pragma unroll
-    for (int k = 0; k < kSurNR; k++) dr[k] *= p.e_scale / p.fstd[k];
+    for (int k = 0; k < kSurNR; k++) dr[k] *= p.fgrad[k];
     float a[kSurNC][3], B[kSurNC][6];
     {
         const float *mo = p.mom + (size_t)i * kSurNC * 9 + 9 * c4;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(128, 7) k_sur_force(SurParams p) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int f = kSurNR + kSurNC * k + c4;
-            e[k] = dx[f] * (p.e_scale / p.fstd[f]);
+            e[k] = dx[f] * p.fgrad[f];
         }
         sur_channel_coeffs(mom, mom + 3, e[0], e[1], e[2], e[3], ca, cb);
 #pragma unroll

@@ -21,6 +21,7 @@ struct SurParams {
     const int *nl_count;
     int nl_cap;
     const float *fmean, *fstd;   // fstd == nullptr: raw features (training samples)
+    const float *fgrad;          // e_scale / fstd
     float *x;                    // n x 32 features
     float *mom;                  // n x 36 moments (M1 3 + M2 6 per channel)
     float *dedx;                 // n x 32 dE/dx
