@@ -609,7 +609,8 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, in
         for (int u = 0; u < U; u++) {
             const bool valid = e[u] != 0xffffffffu;
             const float dx = pi.x - (pj[u].x + o[u].x), dy = pi.y - (pj[u].y + o[u].y), dz = pi.z - (pj[u].z + o[u].z);
-            const float r2 = valid ? dx * dx + dy * dy + dz * dz : 1e30f;
+            // the roundings written out: left to the compiler they differ between the forms
+            const float r2 = valid ? fmaf(dz, dz, fmaf(dx, dx, dy * dy)) : 1e30f;
             const bool lj = p.use_lj && r2 <= rc2 && !(e[u] >> 31);
             const float inv = rcp_approx(r2);
             float x, ee;
@@ -622,7 +623,7 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, in
                 ee = sei * sej[u];
             }
             const float lj6 = x * x * x;
-            float fac0 = 24.0f * ee * (2.0f * lj6 * lj6 - lj6) * inv;
+            float fac0 = 24.0f * ee * fmaf(2.0f * lj6, lj6, -lj6) * inv;
             float usw = 1.0f;
             if (p.sw) {   // switched cutoff: U S, force fac S - 2 U dS/dx
                 float dS;
@@ -632,9 +633,9 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, in
             if (!MEASURE) fac0 *= p.lj_fscalef;   // ATM2B factor
             const float fac = lj ? fac0 : 0.f;    // no branch around a dozen instructions
             if (W == 32 || (u & 1) == 0) {
-                fx += dx * fac; fy += dy * fac; fz += dz * fac;
+                fx = fmaf(dx, fac, fx); fy = fmaf(dy, fac, fy); fz = fmaf(dz, fac, fz);
             } else {
-                hx += dx * fac; hy += dy * fac; hz += dz * fac;
+                hx = fmaf(dx, fac, hx); hy = fmaf(dy, fac, hy); hz = fmaf(dz, fac, hz);
             }
             if (MEASURE && lj) {
                 const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
