@@ -45,6 +45,9 @@ __device__ __forceinline__ double f2d(float x) {
                                             ((unsigned long long)m << 29) + (896ULL << 52)));
 }
 
+// an infinity or a NaN, from the exponent bits (a comparison would run on the FP64 pipe)
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+
 // ===========================================================================
 // container: COM, periodic wrap, binning (LinkedCells.cpp:65-121,390-400;
 // MoleculeContainer.cpp:55-75).  One thread per molecule.
@@ -1073,7 +1076,7 @@ __global__ void k_step1(int n, double *__restrict__ v, const double *__restrict_
     for (int d = 0; d < 3; d++) {
         const double vv = dadd(v[3 * s + d], dmul(f[3 * s + d], c));
         v[3 * s + d] = vv;
-        bad |= !isfinite(vv);
+        bad |= not_finite(vv);
     }
     if (bad) atomicOr(&err[E_NONFINITE], 1);
 }
@@ -1630,9 +1633,9 @@ __device__ __forceinline__ void flush_step1_body(const FlushArgs &a, int bid) {
         for (int d = 0; d < 3; d++) q[d] = (long long)acc[3 * slot + d];
         if (a.fown) {   // the half-list pass's FP32 force, widened exactly
             const float4 o = a.fown[slot];
-            fo[0] = (double)o.x;
-            fo[1] = (double)o.y;
-            fo[2] = (double)o.z;
+            fo[0] = f2d(o.x);
+            fo[1] = f2d(o.y);
+            fo[2] = f2d(o.z);
         } else {
             for (int d = 0; d < 3; d++) fo[d] = f[3 * site + d];
         }
@@ -1646,7 +1649,7 @@ __device__ __forceinline__ void flush_step1_body(const FlushArgs &a, int bid) {
             f[3 * site + d] = fd;
             const double vv = dadd(vo[d], dmul(fd, c));
             v[3 * site + d] = vv;
-            bad |= !isfinite(vv);
+            bad |= not_finite(vv);
             s_f[3 * t + d] = fd;
             s_v[3 * t + d] = vv;
         }
@@ -1671,7 +1674,8 @@ __global__ void __launch_bounds__(kIoBlock) k_atm_flush_step1(FlushArgs a) {
 // operations and their order are those of k_atm_flush_step1 / k_sur_apply_step1
 // / k_step1 and k_step0_fused.  The rebuild flag is set here for the next step;
 // the force pass has cleared it (PairParams::rebuild_done).  256,000 sites: 18 +
-// 13.7 us for the two kernels, 24.4 us for this one.
+// 13.7 us for the two kernels, 22.9 us for this one (24.4 with the FP32 forces
+// widened and finiteness tested on the FP64 pipe, which bounds it).
 enum { KICK_PLAIN = 0, KICK_FLUSH = 1, KICK_LEARNED = 2 };
 template <int MODE>
 __device__ __forceinline__ void kick_drift_body(const FlushArgs &a, const Step0Args &dr, float4 *fsur, int bid) {
@@ -1686,9 +1690,9 @@ __device__ __forceinline__ void kick_drift_body(const FlushArgs &a, const Step0A
     if (MODE == KICK_LEARNED) fs = fsur[slot];
     if (MODE == KICK_FLUSH && a.fown) {   // the half-list pass's FP32 force, widened exactly
         const float4 o = a.fown[slot];
-        fo[0] = (double)o.x;
-        fo[1] = (double)o.y;
-        fo[2] = (double)o.z;
+        fo[0] = f2d(o.x);
+        fo[1] = f2d(o.y);
+        fo[2] = f2d(o.z);
     } else {
         for (int d = 0; d < 3; d++) fo[d] = a.f[3 * s + d];
     }
@@ -1708,11 +1712,11 @@ __device__ __forceinline__ void kick_drift_body(const FlushArgs &a, const Step0A
             a.f[3 * s + d] = fd;
         }
         if (MODE == KICK_LEARNED) {
-            fd = fo[d] + (double)(d == 0 ? fs.x : (d == 1 ? fs.y : fs.z));
+            fd = fo[d] + f2d(d == 0 ? fs.x : (d == 1 ? fs.y : fs.z));
             a.f[3 * s + d] = fd;
         }
         const double kick = dmul(fd, c), v1 = dadd(vo[d], kick);
-        bad |= !isfinite(v1);
+        bad |= not_finite(v1);
         const double v2 = dadd(v1, kick);
         a.v[3 * s + d] = v2;
         x[d] = dadd(ro[d], dmul(v2, dr.dt));
@@ -1749,7 +1753,7 @@ __global__ void k_step10(int n, double *__restrict__ r, double *__restrict__ v, 
     bool bad = false;
     for (int d = 0; d < 3; d++) {
         const double kick = dmul(fo[d], c), v1 = dadd(vo[d], kick);
-        bad |= !isfinite(v1);
+        bad |= not_finite(v1);
         const double v2 = dadd(v1, kick);
         v[3 * s + d] = v2;
         x[d] = dadd(x[d], dmul(v2, dt));
@@ -1771,9 +1775,9 @@ __global__ void k_atm_flush(int n, const int *__restrict__ slot_site, unsigned l
     for (int d = 0; d < 3; d++) q[d] = (long long)acc[3 * slot + d];
     if (own) {   // the half-list pass's FP32 force, widened exactly
         const float4 o = own[slot];
-        fo[0] = (double)o.x;
-        fo[1] = (double)o.y;
-        fo[2] = (double)o.z;
+        fo[0] = f2d(o.x);
+        fo[1] = f2d(o.y);
+        fo[2] = f2d(o.z);
     } else {
         for (int d = 0; d < 3; d++) fo[d] = f[3 * site + d];
     }
