@@ -302,13 +302,14 @@ void enqueue_step(komd_gpu *h) {
         launch_container(e, e.stream);
     }
     // the step's integrate1 rides on the ATM flush when the once-per-triplet path runs
-    if (!enqueue_forces(h, false, nullptr, END_STEP1)) {
+    const bool ended = enqueue_forces(h, false, nullptr, END_STEP1);
+    if (!ended && !e.cfg.thermostat) {
         ProfScope ps(h, F_INTEGRATE);
         launch_step1(e, e.stream);
     }
     if (e.cfg.thermostat) {   // Simulation.cpp:72, after the step's sensors
         ProfScope ps(h, F_INTEGRATE);
-        launch_kinetic(e, e.stream, 0, h->thermo_acc);
+        launch_kinetic(e, e.stream, 0, h->thermo_acc, !ended);
         launch_velocity_scale(e, e.stream, h->thermo_acc, 1.0);
     }
     if (r_async) {
@@ -2293,7 +2294,8 @@ int komd_gpu_kernels_per_step(komd_gpu *h) {
     if (e.cfg.terms & KOMD_TERM_BONDED)   // one pass over small molecules, or one by bond and one by angle
         k += e.bond_blocks > 0 && e.bond_sites == e.n ? 1 : (e.n_bonds > 0) + (e.n_angles > 0);
     if (e.cfg.terms & KOMD_TERM_LIMIT) k++;
-    if (e.cfg.thermostat) k += 2;  /* kinetic sums, velocity scaling */
+    if (e.cfg.thermostat)   // velocity scaling and the kinetic sums, with integrate1 where the flush has it not
+        k += !surrogate_on(h) && (e.cfg.terms & KOMD_TERM_ATM) && e.atm_acc ? 2 : 1;
     if (surrogate_on(h)) k += 4;   /* descriptors, MLP, forces, apply */
     else if (e.cfg.terms & KOMD_TERM_ATM)   /* once-per-triplet kernel (inside the LJ pass on the Verlet path) + flush */
         k += (e.atm_acc != nullptr) ? (fused_lj_atm(h, false) ? 1 : 2) : 1;

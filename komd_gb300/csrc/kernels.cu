@@ -1091,11 +1091,15 @@ __global__ void k_step1(int n, double *__restrict__ v, const double *__restrict_
 // finishes last sums the blocks' rows in their order into acc and zeroes
 // acc's other slots, so a measure needs neither a clearing nor a second
 // kernel: the sums are deterministic.  done: a counter, zero between launches.
-template <bool TERMS>
+// STEP1: with integrate1 of the step before (k_step1's operations; a thermostatted step).
+template <bool TERMS, bool STEP1>
 __global__ void __launch_bounds__(kBlock) k_kinetic(Grid g, int n, int n_terms, const double *__restrict__ r,
-                                                    const double *__restrict__ v, const double *__restrict__ m,
-                                                    double *partials, double *__restrict__ acc, unsigned *done) {
+                                                    double *__restrict__ v, const double *__restrict__ m,
+                                                    double *partials, double *__restrict__ acc, unsigned *done,
+                                                    const double *__restrict__ f, const double *__restrict__ hdtm,
+                                                    int *__restrict__ err, int *__restrict__ rebuild) {
     pdl_wait();
+    if (STEP1 && rebuild && blockIdx.x == 0 && threadIdx.x == 0) *rebuild = 0;   // its consumers have run
     __shared__ double s_part[kWarpsPerBlock][8];
     __shared__ bool s_last;
     constexpr int kVals = TERMS ? 8 : 2;
@@ -1103,7 +1107,18 @@ __global__ void __launch_bounds__(kBlock) k_kinetic(Grid g, int n, int n_terms, 
     for (int k = 0; k < kVals; k++) vals[k] = 0.0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const double x = r[3 * s], y = r[3 * s + 1], z = r[3 * s + 2];
-        const double vx = v[3 * s], vy = v[3 * s + 1], vz = v[3 * s + 2], ms = m[s];
+        double vx = v[3 * s], vy = v[3 * s + 1], vz = v[3 * s + 2];
+        const double ms = m[s];
+        if (STEP1) {
+            const double c = hdtm[s];
+            vx = dadd(vx, dmul(f[3 * s], c));
+            vy = dadd(vy, dmul(f[3 * s + 1], c));
+            vz = dadd(vz, dmul(f[3 * s + 2], c));
+            v[3 * s] = vx;
+            v[3 * s + 1] = vy;
+            v[3 * s + 2] = vz;
+            if (not_finite(vx) || not_finite(vy) || not_finite(vz)) atomicOr(&err[E_NONFINITE], 1);
+        }
         if (x >= g.low[0] && y >= g.low[1] && z >= g.low[2] && x <= g.high[0] && y <= g.high[1] && z <= g.high[2]) {
             vals[0] = dadd(vals[0], dmul(ms, dadd(dadd(dmul(vx, vx), dmul(vy, vy)), dmul(vz, vz))));
             vals[1] = dadd(vals[1], 1.0);
@@ -1911,13 +1926,10 @@ void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double
 }
 
 // the kinetic sums into acc (R_NSLOTS), whose other slots become zero
-void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc) {
-    const int grid = kinetic_grid(e);
-    if (n_terms > 0)
-        launch_pdl(k_kinetic<true>, grid, kBlock, 0, st, e.g, (int)e.n, n_terms, e.r, e.v, e.m, e.partials, acc,
-                   e.kin_done);
-    else launch_pdl(k_kinetic<false>, grid, kBlock, 0, st, e.g, (int)e.n, 0, e.r, e.v, e.m, e.partials, acc,
-                    e.kin_done);
+void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc, bool step1) {
+    auto k = step1 ? k_kinetic<false, true> : n_terms > 0 ? k_kinetic<true, false> : k_kinetic<false, false>;
+    launch_pdl(k, kinetic_grid(e), kBlock, 0, st, e.g, (int)e.n, n_terms, e.r, e.v, e.m, e.partials, acc, e.kin_done,
+               e.f, e.hdtm, e.err, e.verlet ? e.rebuild : nullptr);
 }
 
 void launch_sum_partials(cudaStream_t st, int nblocks, const double *partials, double *out) {

@@ -41,7 +41,8 @@ void launch_step0(Engine &e, cudaStream_t st, bool in_step = false);
 void launch_step1(Engine &e, cudaStream_t st);
 void launch_kick_drift(Engine &e, cudaStream_t st);
 void launch_learned_kick_drift(Engine &e, float *fsur, cudaStream_t st);
-void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc);
+// step1: with integrate1 of the step, whose velocities are summed (n_terms 0)
+void launch_kinetic(Engine &e, cudaStream_t st, int n_terms, double *acc, bool step1 = false);
 void launch_velocity_scale(Engine &e, cudaStream_t st, const double *acc, double beta);
 void launch_pair_table(Engine &e, cudaStream_t st);
 void launch_sum_partials(cudaStream_t st, int nblocks, const double *partials, double *out);
