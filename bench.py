@@ -881,7 +881,7 @@ def run_ours(args, w, name):
         pairs = int(obs0["pairs_in_cutoff"])
         achieved = FLOP_PER_PAIR * pairs / t_launch / 1e12
         peak = fp32_simt_peak_tflops(torch)
-        roof = {"bound": "fp32", "kernel": "k_pair (LJ)", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+        roof = {"bound": "fp32", "kernel": "LJ pair kernel", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": committed_traffic("k_pair", name),
                 "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off", "launch_ms": t_launch * 1e3}
     cb = None
