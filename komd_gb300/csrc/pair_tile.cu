@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                         }
                     }
                     __syncwarp();
-                    if (qn > 0) pair(lane < qn ? (int)s_q[w][lane] : 0, lane < qn);
+                    if (qn > 0) pair((int)s_q[w][lane < qn ? lane : 0], lane < qn);   // the rest repeat a hit: its position is finite
                     const float fs = warp_sum3(fx, fy, fz, lane);
                     if ((lane & 7) == 0 && lane < 24) s_f[3 * i + (lane >> 3)] += fs;
                     if (EMIT && lane == 0) s_cnt[i] = cnt;
@@ -631,11 +631,14 @@ __device__ __forceinline__ int lj_site(const PairParams &p, int i, bool live, in
                 fac0 = fac0 * usw - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
             }
             if (!MEASURE) fac0 *= p.lj_fscalef;   // ATM2B factor
-            const float fac = lj ? fac0 : 0.f;    // no branch around a dozen instructions
+            // no branch around a dozen instructions; both factors are dropped, so that a
+            // position that is not finite reaches nobody else
+            const float fac = lj ? fac0 : 0.f;
+            const float ex = lj ? dx : 0.f, ey = lj ? dy : 0.f, ez = lj ? dz : 0.f;
             if (W == 32 || (u & 1) == 0) {
-                fx = fmaf(dx, fac, fx); fy = fmaf(dy, fac, fy); fz = fmaf(dz, fac, fz);
+                fx = fmaf(ex, fac, fx); fy = fmaf(ey, fac, fy); fz = fmaf(ez, fac, fz);
             } else {
-                hx = fmaf(dx, fac, hx); hy = fmaf(dy, fac, hy); hz = fmaf(dz, fac, hz);
+                hx = fmaf(ex, fac, hx); hy = fmaf(ey, fac, hy); hz = fmaf(ez, fac, hz);
             }
             if (MEASURE && lj) {
                 const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
@@ -889,8 +892,9 @@ __device__ __forceinline__ void lj_half(const PairParams &p, int i, const HalfRo
                 sw_eval(r2, p.sw_rc2, p.sw_iw, S, dS);
                 fac = fac * S - 8.0f * ee * (lj6 * lj6 - lj6) * dS;
             }
-            fac = lj ? fac : 0.f;   // no branch around a dozen instructions
-            const float gx = dx * fac, gy = dy * fac, gz = dz * fac;
+            // no branch around a dozen instructions; what does not count is dropped last, so
+            // that a position that is not finite reaches nobody else
+            const float gx = lj ? dx * fac : 0.f, gy = lj ? dy * fac : 0.f, gz = lj ? dz * fac : 0.f;
             fx += gx; fy += gy; fz += gz;
             const bool at = valid && r2 <= rc3sq;   // a triplet partner (LJ or not)
             const bool lo = lj && !at;              // an LJ-only partner
