@@ -9,15 +9,15 @@
 //      coordinates (float4 position + slot, key, cell code, sqrt(eps));
 //   3. every warp owns a subset of home sites; for a home site the 32 lanes
 //      test 32 staged candidates at a time and ballot-compact the hits into a
-//      per-warp queue, so the force arithmetic runs on full warps;
-//   4. each dequeued pair adds its LJ force to the lane's sum for the home site
-//      and, inside cutoff_3b, appends (r_i - r_j, code) to the home site's ATM
-//      list in queue order (deterministic list order).
-// With sensors the queue runs on over the home sites (their per-lane sums keep
-// their order); forces alone empty it at each site, which wastes some lanes of
-// the last evaluation but needs no grouping of the lanes by site, no segmented
-// sums (30 shuffles and adds an evaluation) and no read-modify-write of the
-// site's sum and count: 32,000 sites of liquid argon 44 -> 33 us.
+//      per-warp queue, so the force arithmetic always runs on full warps;
+//   4. each dequeued pair adds its LJ force to the home site's shared-memory
+//      accumulator and, inside cutoff_3b, appends (r_i - r_j, code) to the
+//      home site's ATM list in queue order (deterministic list order).
+// The lanes of a site are found by a ballot of the places where the site changes, and
+// the candidates of the last 32 that are not there are out of reach instead of
+// masked: 32,000 sites of liquid argon 44 -> 34.5 us.  Emptying the queue at each site, its
+// force in the lanes' registers, takes 33 us, but sums in another order: snapshots
+// for training then differ in their last bits, which BF16 roundings amplify.
 // Full shell: each site's force is summed by its own CTA, no global atomics.
 //
 // The Verlet path (skin > 0) has its own kernels here: the list build
@@ -137,68 +137,6 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
             if (ns + tid < ((ns + 31) & ~31)) s_pos[ns + tid] = make_float4(1e15f, 1e15f, 1e15f, 0.f);   // out of reach
             __syncthreads();
 
-            if (!MEASURE) {
-                // a home site at a time: its force stays in the lanes' registers, with one
-                // reduction at the end
-                for (int i = w; i < hc; i += kTileWarps) {
-                    const float4 pi = s_hpos[i];
-                    const int2 ha = s_haux[i];
-                    const float sei = __int_as_float(ha.y);
-                    const int self = self_base + i - sb;
-                    float4 *row = EMIT ? nl + (size_t)(hs + hb + i) * p.nl_cap : nullptr;
-                    float fx = 0.f, fy = 0.f, fz = 0.f;
-                    int cnt = EMIT ? s_cnt[i] : 0;
-                    auto pair = [&](int j, bool valid) {
-                        const float4 pj = s_pos[j];
-                        const int4 a = s_aux[j];
-                        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                        const float r2 = valid ? dx * dx + dy * dy + dz * dz : 1e30f;
-                        const float inv = rcp_approx(r2);
-                        const float sg = pi.w + pj.w;
-                        const float x = sg * sg * inv;
-                        const float lj6 = x * x * x;
-                        const float ee = sei * __int_as_float(a.w);
-                        const float ljd = 24.0f * ee * (2.0f * lj6 * lj6 - lj6);
-                        const float fac = p.use_lj && r2 <= rc2 && ha.x != a.y ? ljd * inv * p.lj_fscalef : 0.f;
-                        fx += dx * fac;
-                        fy += dy * fac;
-                        fz += dz * fac;
-                        if (EMIT) {
-                            const bool emit = r2 <= rc3sq;
-                            const unsigned em = __ballot_sync(0xffffffffu, emit);
-                            const int c = cnt + __popc(em & lt);
-                            if (emit && c < p.nl_cap) row[c] = make_float4(dx, dy, dz, __int_as_float(a.z | (a.x << 6)));
-                            cnt += __popc(em);
-                        }
-                    };
-                    int qn = 0;
-                    for (int j0 = 0; j0 < ns; j0 += 32) {
-                        const int j = j0 + lane;
-                        const float4 pj = s_pos[j];
-                        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                        const bool hit = dx * dx + dy * dy + dz * dz <= scan2 && j != self;
-                        const unsigned m = __ballot_sync(0xffffffffu, hit);
-                        if (hit) s_q[w][qn + __popc(m & lt)] = (unsigned)j;
-                        qn += __popc(m);
-                        if (qn >= 32) {
-                            __syncwarp();
-                            const unsigned e = s_q[w][lane], tail = s_q[w][lane + 32];
-                            __syncwarp();
-                            qn -= 32;
-                            if (lane < qn) s_q[w][lane] = tail;
-                            pair((int)e, true);
-                        }
-                    }
-                    __syncwarp();
-                    if (qn > 0) pair((int)s_q[w][lane < qn ? lane : 0], lane < qn);   // the rest repeat a hit: its position is finite
-                    const float fs = warp_sum3(fx, fy, fz, lane);
-                    if ((lane & 7) == 0 && lane < 24) s_f[3 * i + (lane >> 3)] += fs;
-                    if (EMIT && lane == 0) s_cnt[i] = cnt;
-                    __syncwarp();   // the queue is refilled by the next site
-                }
-                continue;
-            }
-
             // Process one queued pair per lane (valid = lane holds an entry).
             // Entries of one home site occupy contiguous lanes (the queue is
             // filled site by site), and a site belongs to exactly one warp:
@@ -212,8 +150,12 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                 const int4 a = s_aux[j];
                 const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 const float r2 = dx * dx + dy * dy + dz * dz;
-                const unsigned grp = __match_any_sync(0xffffffffu, valid ? i : (0x10000 | lane));
-                const int first = __ffs(grp) - 1, last = 31 - __clz(grp);
+                // the lane's group [first, last]: entries of a site are neighbours in the queue
+                const int site = valid ? i : (0x10000 | lane);
+                const int before = __shfl_up_sync(0xffffffffu, site, 1);
+                const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != site);
+                const unsigned upto = lt | (1u << lane), after = heads & ~upto;
+                const int first = 31 - __clz(heads & upto), last = after ? __ffs(after) - 2 : 31;
                 float fx = 0.f, fy = 0.f, fz = 0.f;
                 if (p.use_lj && valid && r2 <= rc2 && s_haux[i].x != a.y) {
                     const float inv = rcp_approx(r2);
@@ -222,7 +164,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                     const float lj6 = x * x * x;
                     const float ee = __int_as_float(s_haux[i].y) * __int_as_float(a.w);
                     const float ljd = 24.0f * ee * (2.0f * lj6 * lj6 - lj6);
-                    const float fac = ljd * inv;
+                    const float fac = MEASURE ? ljd * inv : ljd * inv * p.lj_fscalef;   // ATM2B factor
                     fx = dx * fac; fy = dy * fac; fz = dz * fac;
                     if (MEASURE) {
                         const float wt = (p.virial_compat && (a.z & 32)) ? 1.0f : 0.5f;
@@ -243,7 +185,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                     if (lane + o <= last) { fx += yx; fy += yy; fz += yz; }
                 }
                 const bool emit = EMIT && valid && r2 <= rc3sq;
-                const unsigned em = __ballot_sync(0xffffffffu, emit) & grp;
+                const unsigned em = __ballot_sync(0xffffffffu, emit) & (0xffffffffu << first) & (0xffffffffu >> (31 - last));
                 int base = 0;
                 if (EMIT && valid && lane == first) base = s_cnt[i];
                 base = __shfl_sync(0xffffffffu, base, first);
@@ -254,7 +196,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                     if (EMIT) s_cnt[i] = base + __popc(em);
                 }
                 if (emit) {
-                    const int c = base + __popc(em & lanemask_lt());
+                    const int c = base + __popc(em & lt);
                     const int slot_i = hs + hb + i;
                     if (c < p.nl_cap)
                         nl[(size_t)slot_i * p.nl_cap + c] = make_float4(dx, dy, dz, __int_as_float(a.z | (a.x << 6)));
@@ -268,14 +210,11 @@ __global__ void __launch_bounds__(kTileThreads) k_pair_tile(PairParams p) {
                 const int self = self_base + i - sb;
                 for (int j0 = 0; j0 < ns; j0 += 32) {
                     const int j = j0 + lane;
-                    bool hit = false;
-                    if (j < ns && j != self) {
-                        const float4 pj = s_pos[j];
-                        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                        hit = dx * dx + dy * dy + dz * dz <= scan2;
-                    }
+                    const float4 pj = s_pos[j];
+                    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                    const bool hit = dx * dx + dy * dy + dz * dz <= scan2 && j != self;
                     const unsigned m = __ballot_sync(0xffffffffu, hit);
-                    if (hit) s_q[w][qn + __popc(m & lanemask_lt())] = ((unsigned)i << 16) | (unsigned)j;
+                    if (hit) s_q[w][qn + __popc(m & lt)] = ((unsigned)i << 16) | (unsigned)j;
                     qn += __popc(m);
                     if (qn >= 32) {
                         __syncwarp();
