@@ -13,6 +13,7 @@
 #include <climits>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 
 #include "engine.cuh"
 #include "kernels.cuh"
@@ -1964,23 +1965,29 @@ void launch_rdf_bins(Engine &e, cudaStream_t st, double *bins, bool cells, doubl
         k_rdf_all<<<nblk(e.n_mol, 128), 128, 0, st>>>(e.g, (int)e.n_mol, e.com, max_r, dr, nbins, bins);
 }
 
-// the ATM kernels' staging; with their static arrays (up to 5 KB) it passes
-// the default 48 KB above 40
+// Shared memory above the default 48 KB (static and dynamic together) has to be
+// allowed kernel by kernel, and the limit is the process's, not the engine's: it is
+// only ever raised, so that an engine with small lists does not take from one with
+// larger ones what that one's launches need.
+void allow_smem(const void *kernel, size_t bytes) {
+    if (bytes <= 40 * 1024) return;   // the static arrays are below 8 KB
+    static std::mutex mutex;
+    std::lock_guard<std::mutex> lock(mutex);
+    const int want = std::max((int)bytes, 49 * 1024);   // above the default, so that it reads as allowed
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess && a.maxDynamicSharedSizeBytes >= want) return;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
+}
+
+// the ATM kernels' staging, whose size follows the list capacity
 void set_kernel_attributes(Engine &e) {
-    const int sm = (int)atm_smem(e);
-    if (sm <= 40 * 1024) return;
-    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const size_t sm = atm_smem(e);
     if (e.cfg.precision == KOMD_FP64) {
-        cudaFuncSetAttribute(k_atm_d<true, true>, attr, sm);
-        cudaFuncSetAttribute(k_atm_d<true, false>, attr, sm);
-        cudaFuncSetAttribute(k_atm_d<false, true>, attr, sm);
-        cudaFuncSetAttribute(k_atm_d<false, false>, attr, sm);
+        for (auto k : {k_atm_d<true, true>, k_atm_d<true, false>, k_atm_d<false, true>, k_atm_d<false, false>})
+            allow_smem((const void *)k, sm);
     } else {
-        cudaFuncSetAttribute(k_atm_s, attr, sm);
-        cudaFuncSetAttribute(k_atm_q<true, true>, attr, sm);
-        cudaFuncSetAttribute(k_atm_q<true, false>, attr, sm);
-        cudaFuncSetAttribute(k_atm_q<false, true>, attr, sm);
-        cudaFuncSetAttribute(k_atm_q<false, false>, attr, sm);
+        for (auto k : {k_atm_s, k_atm_q<true, true>, k_atm_q<true, false>, k_atm_q<false, true>, k_atm_q<false, false>})
+            allow_smem((const void *)k, sm);
     }
 }
 

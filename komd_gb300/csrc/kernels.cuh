@@ -49,6 +49,8 @@ void launch_sum_partials(cudaStream_t st, int nblocks, const double *partials, d
 void launch_rdf(Engine &e, cudaStream_t st, double *bins, bool cells);
 void launch_rdf_bins(Engine &e, cudaStream_t st, double *bins, bool cells, double max_r, double dr, int64_t nbins);
 void set_kernel_attributes(Engine &e);
+// allows a kernel this much dynamic shared memory (never less than before)
+void allow_smem(const void *kernel, size_t bytes);
 int atm_grid(const Engine &e);
 
 // ---- packed replicas: one launch per stage of the step for all replicas of a

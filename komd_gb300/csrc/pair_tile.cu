@@ -937,8 +937,7 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm_half(PairParams p, AtmParams 
 template <bool UNIFORM, bool SW, bool PLAIN = false>
 static void launch_half(const PairParams &p, const AtmParams &a, float sa, int n, int per, int grid, size_t sm,
                         cudaStream_t st) {
-    if (sm > 48 * 1024)
-        cudaFuncSetAttribute(k_lj_atm_half<UNIFORM, SW, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem((const void *)k_lj_atm_half<UNIFORM, SW, PLAIN>, sm);
     launch_pdl(k_lj_atm_half<UNIFORM, SW, PLAIN>, grid, 256, sm, st, p, a, sa, n, per);
 }
 
@@ -1008,9 +1007,7 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm_half_p(const PairParams *__re
 
 template <bool UNIFORM, bool SW, bool PLAIN = false>
 static void launch_half_p(const PackedStep &pk, cudaStream_t st) {
-    if (pk.force_smem > 48 * 1024)
-        cudaFuncSetAttribute(k_lj_atm_half_p<UNIFORM, SW, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)pk.force_smem);
+    allow_smem((const void *)k_lj_atm_half_p<UNIFORM, SW, PLAIN>, pk.force_smem);
     k_lj_atm_half_p<UNIFORM, SW, PLAIN><<<pk.force.blocks, 256, pk.force_smem, st>>>(pk.pp, pk.ap, pk.sa, pk.n,
                                                                                      pk.per, pk.force.start, pk.nrep);
 }
@@ -1130,18 +1127,18 @@ void launch_lj_atm(Engine &e, cudaStream_t st) {
     const bool u3 = vlist_u3(e);
     if (e.uniform) {
         if (u3) {
-            if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            allow_smem((const void *)k_lj_atm<true, 3>, sm);
             launch_pdl(k_lj_atm<true, 3>, grid, 256, sm, st, p, a, (int)e.n, per);
         } else {
-            if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            allow_smem((const void *)k_lj_atm<true, 2>, sm);
             launch_pdl(k_lj_atm<true, 2>, grid, 256, sm, st, p, a, (int)e.n, per);
         }
     } else {
         if (u3) {
-            if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            allow_smem((const void *)k_lj_atm<false, 3>, sm);
             launch_pdl(k_lj_atm<false, 3>, grid, 256, sm, st, p, a, (int)e.n, per);
         } else {
-            if (sm > 48 * 1024) cudaFuncSetAttribute(k_lj_atm<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            allow_smem((const void *)k_lj_atm<false, 2>, sm);
             launch_pdl(k_lj_atm<false, 2>, grid, 256, sm, st, p, a, (int)e.n, per);
         }
     }
