@@ -26,9 +26,11 @@ int fail(int code, const std::string &msg) {
 #define CK(call)                                                                                       \
     do {                                                                                               \
         cudaError_t _e = (call);                                                                       \
-        if (_e != cudaSuccess)                                                                         \
+        if (_e != cudaSuccess) {                                                                       \
+            cudaGetLastError();   /* reported here, not by the next launch check */                    \
             return fail(_e == cudaErrorMemoryAllocation ? KOMD_ERR_NOMEM : KOMD_ERR_CUDA,              \
                         std::string(#call) + ": " + cudaGetErrorString(_e));                          \
+        }                                                                                              \
     } while (0)
 
 template <typename T>
@@ -51,6 +53,38 @@ void drop_graphs(Engine &e) {
     e.graph = e.several = nullptr;
     e.graph_valid = false;
 }
+
+// While an engine's buffers are replaced it has no sites, cells, forces or step
+// graphs; they return with done().  Without it -- an allocation failed half-way --
+// the engine refuses everything until sites are uploaded again, so that neither a
+// kernel nor a captured graph meets a buffer that is gone.
+struct Replacing {
+    Engine &e;
+    const bool sites, cells, forces;
+    explicit Replacing(Engine &e_) : e(e_), sites(e_.have_sites), cells(e_.have_cells), forces(e_.have_forces) {
+        drop_graphs(e);
+        e.have_sites = e.have_cells = e.have_forces = false;
+    }
+    void done() {
+        e.have_sites = sites;
+        e.have_cells = cells;
+        e.have_forces = forces;
+    }
+};
+
+// a new device array that its owner gets by swap(), and that is freed otherwise
+template <typename T>
+struct Fresh {
+    T *p = nullptr;
+    ~Fresh() { dfree(p); }
+    cudaError_t copy(const std::vector<T> &v) {
+        const cudaError_t err = dalloc(p, v.size());
+        return err != cudaSuccess || v.empty()
+                   ? err
+                   : cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
+    }
+    void swap(T *&owner) { std::swap(p, owner); }
+};
 
 // TemperatureSensor's conversion (TemperatureSensor.cpp:44-47), restated in engine.cuh
 double temperature_from(double mv2, double n_in_box) { return sci_temperature(sci_factor(), mv2, n_in_box); }
@@ -170,6 +204,7 @@ int ensure_partials(komd_gpu *h) {
     if (e.verlet) need = std::max(need, vlist_blocks(e));
     need = std::max(need, kinetic_grid(e));
     if (need > h->partial_cap) {
+        h->partial_cap = 0;
         CK(dalloc(e.partials, (size_t)need * R_NSLOTS));
         h->partial_cap = need;
     }
@@ -361,6 +396,7 @@ int read_flags(komd_gpu *h, int flags[E_NFLAGS], bool clear) {
 
 int alloc_atm_list(komd_gpu *h, int cap) {
     Engine &e = h->e;
+    Replacing replacing(e);
     e.nl_cap = cap;
     if (e.cfg.terms & KOMD_TERM_ATM) {
         const size_t entry = e.cfg.precision == KOMD_FP64 ? 32 : 16;
@@ -371,22 +407,27 @@ int alloc_atm_list(komd_gpu *h, int cap) {
         CK(dalloc(e.nl_count, e.n));
         set_kernel_attributes(e);
     }
-    drop_graphs(e);
+    replacing.done();
     return KOMD_OK;
 }
 
 int ensure_posd(komd_gpu *h) {
     Engine &e = h->e;
     if (e.posd) return KOMD_OK;
-    CK(dalloc(e.posd, 3 * (size_t)e.n));
-    CK(dalloc(e.seps_d, e.n));
-    CK(dalloc(e.sig_d, e.n));
+    Fresh<double> posd, seps, sig;
+    CK(dalloc(posd.p, 3 * (size_t)e.n));
+    CK(dalloc(seps.p, e.n));
+    CK(dalloc(sig.p, e.n));
     drop_graphs(e);
+    posd.swap(e.posd);
+    seps.swap(e.seps_d);
+    sig.swap(e.sig_d);
     return KOMD_OK;
 }
 
 int alloc_verlet(komd_gpu *h, int cap) {
     Engine &e = h->e;
+    Replacing replacing(e);
     e.vl_cap = cap;
     CK(dalloc(e.bias, 3 * (size_t)e.n));
     CK(dalloc(e.ref4, e.n));
@@ -394,7 +435,7 @@ int alloc_verlet(komd_gpu *h, int cap) {
     CK(dalloc(e.zkey, e.n));
     CK(dalloc(e.vl, (size_t)cap * (size_t)e.n));
     CK(dalloc(e.vl_count, e.n));
-    drop_graphs(e);
+    replacing.done();
     return KOMD_OK;
 }
 
@@ -719,6 +760,7 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
         if (!(m[s] > 0)) return fail(KOMD_ERR_ARG, "site masses must be > 0");
     }
     off.push_back((int)n);
+    Replacing replacing(e);   // have_sites returns at the end
     e.n = n;
     e.n_mol = (int64_t)off.size() - 1;
     CK(dalloc(e.r, 3 * n)); CK(dalloc(e.v, 3 * n)); CK(dalloc(e.f, 3 * n)); CK(dalloc(h->f_scratch, 3 * n));
@@ -807,8 +849,6 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
     rc = ensure_partials(h);
     if (rc) return rc;
     e.have_sites = true;
-    e.have_cells = e.have_forces = false;
-    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -823,10 +863,9 @@ int komd_gpu_set_state(komd_gpu *h, const double *r, const double *v) {
 }
 
 // the terms by connected component for k_bonded_mol, where every component has at
-// most kBondTerms terms and a range of at most kBondSites sites to itself
-static int bond_layout(Engine &e, const std::vector<int> &b, const std::vector<int> &a) {
-    e.bond_blocks = 0;
-    e.bond_sites = e.n;
+// most kBondTerms terms and a range of at most kBondSites sites to itself (false otherwise)
+static bool bond_layout(const Engine &e, const std::vector<int> &b, const std::vector<int> &a,
+                        std::vector<int4> &blocks, std::vector<int> &off, std::vector<int4> &terms) {
     std::vector<int> root(e.n);
     for (int64_t s = 0; s < e.n; s++) root[s] = (int)s;
     auto find = [&](int x) {
@@ -844,17 +883,17 @@ static int bond_layout(Engine &e, const std::vector<int> &b, const std::vector<i
         join(a[3 * k], a[3 * k + 1]);
         join(a[3 * k + 1], a[3 * k + 2]);
     }
-    std::vector<int> count(e.n, 0), last(e.n, -1), comp(e.n, -1), off(1, 0);
+    std::vector<int> count(e.n, 0), last(e.n, -1), comp(e.n, -1);
+    off.assign(1, 0);
     for (size_t k = 0; k < nb; k++)
-        if (++count[find(b[2 * k])] > kBondTerms) return KOMD_OK;
+        if (++count[find(b[2 * k])] > kBondTerms) return false;
     for (size_t k = 0; k < na; k++)
-        if (++count[find(a[3 * k])] > kBondTerms) return KOMD_OK;
+        if (++count[find(a[3 * k])] > kBondTerms) return false;
     for (int64_t s = 0; s < e.n; s++) last[find((int)s)] = (int)s;
-    std::vector<int4> blocks;
     int end = 0;   // of the components so far
     for (int s = 0; s < (int)e.n; s++) {
         if (root[s] != s || count[s] == 0) continue;
-        if (s < end || last[s] - s >= kBondSites) return KOMD_OK;
+        if (s < end || last[s] - s >= kBondSites) return false;
         end = last[s] + 1;
         comp[s] = (int)off.size() - 1;
         if (blocks.empty() || comp[s] - blocks.back().x == kBondComps || end - blocks.back().z > kBondSites)
@@ -863,20 +902,12 @@ static int bond_layout(Engine &e, const std::vector<int> &b, const std::vector<i
         blocks.back().w = end;
         off.push_back(off.back() + count[s]);
     }
-    if (blocks.empty()) return KOMD_OK;
     std::vector<int> at(off.begin(), off.end() - 1);
-    std::vector<int4> terms(nb + na);
+    terms.resize(nb + na);
     for (size_t k = 0; k < nb; k++) terms[at[comp[find(b[2 * k])]]++] = make_int4(b[2 * k], b[2 * k + 1], -1, 0);
     for (size_t k = 0; k < na; k++)
         terms[at[comp[find(a[3 * k])]]++] = make_int4(a[3 * k], a[3 * k + 1], a[3 * k + 2], 0);
-    CK(dalloc(e.bond_block, blocks.size()));
-    CK(dalloc(e.comp_off, off.size()));
-    CK(dalloc(e.comp_terms, terms.size()));
-    CK(cudaMemcpy(e.bond_block, blocks.data(), sizeof(int4) * blocks.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(e.comp_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(e.comp_terms, terms.data(), sizeof(int4) * terms.size(), cudaMemcpyHostToDevice));
-    e.bond_blocks = (int)blocks.size();
-    return KOMD_OK;
+    return !blocks.empty();
 }
 
 int komd_gpu_set_topology(komd_gpu *h, int64_t n_bonds, const int64_t *bonds, int64_t n_angles,
@@ -892,14 +923,29 @@ int komd_gpu_set_topology(komd_gpu *h, int64_t n_bonds, const int64_t *bonds, in
         if (angles[k] < 0 || angles[k] >= e.n) return fail(KOMD_ERR_ARG, "angle index out of range");
         a[k] = (int)angles[k];
     }
-    if (int rc = bond_layout(e, b, a)) return rc;
-    CK(dalloc(e.bonds, b.size()));
-    CK(dalloc(e.angles, a.size()));
-    if (!b.empty()) CK(cudaMemcpy(e.bonds, b.data(), sizeof(int) * b.size(), cudaMemcpyHostToDevice));
-    if (!a.empty()) CK(cudaMemcpy(e.angles, a.data(), sizeof(int) * a.size(), cudaMemcpyHostToDevice));
+    std::vector<int4> blocks, terms;
+    std::vector<int> off;
+    const bool laid_out = bond_layout(e, b, a, blocks, off, terms);
+    Fresh<int> d_bonds, d_angles, d_off;
+    Fresh<int4> d_blocks, d_terms;
+    CK(d_bonds.copy(b));
+    CK(d_angles.copy(a));
+    if (laid_out) {
+        CK(d_blocks.copy(blocks));
+        CK(d_off.copy(off));
+        CK(d_terms.copy(terms));
+    }
+    // everything is there: the old topology, and the graphs that hold it, go
+    drop_graphs(e);
+    d_bonds.swap(e.bonds);
+    d_angles.swap(e.angles);
+    d_blocks.swap(e.bond_block);
+    d_off.swap(e.comp_off);
+    d_terms.swap(e.comp_terms);
+    e.bond_blocks = laid_out ? (int)blocks.size() : 0;
+    e.bond_sites = e.n;
     e.n_bonds = std::max<int64_t>(n_bonds, 0);
     e.n_angles = std::max<int64_t>(n_angles, 0);
-    drop_graphs(e);
     return KOMD_OK;
 }
 
@@ -1227,11 +1273,15 @@ int komd_gpu_set_pair_table(komd_gpu *h, int32_t n, const double *x, const doubl
         if (!(x[k] > x[k - 1])) return fail(KOMD_ERR_ARG, "table nodes must be strictly ascending");
     CK(cudaStreamSynchronize(e.stream));
     if (n != e.tab_n) {
-        CK(dalloc(e.tab_x, n));
-        CK(dalloc(e.tab_y, n));
-        CK(dalloc(e.tab_s, n));
-        e.tab_n = n;
+        Fresh<double> tx, ty, ts;
+        CK(dalloc(tx.p, n));
+        CK(dalloc(ty.p, n));
+        CK(dalloc(ts.p, n));
         drop_graphs(e);
+        tx.swap(e.tab_x);
+        ty.swap(e.tab_y);
+        ts.swap(e.tab_s);
+        e.tab_n = n;
     }
     // same-size tables are replaced in place: graphs already captured read the new values
     CK(cudaMemcpy(e.tab_x, x, sizeof(double) * n, cudaMemcpyHostToDevice));
@@ -1419,6 +1469,8 @@ int komd_gpu_surrogate_load(komd_gpu *h, const float *params, const float *fmean
     const std::vector<__nv_bfloat16> w1t = frag(F, H, [&](int n, int k) { return W1[k * F + n]; });
     const std::vector<__nv_bfloat16> w2 = frag(H, H, [&](int n, int k) { return W2[n * H + k]; });
     const std::vector<__nv_bfloat16> w2t = frag(H, H, [&](int n, int k) { return W2[k * H + n]; });
+    drop_graphs(e);
+    u.loaded = false;   // until everything below is there
     CK(dalloc(u.w1, w1.size())); CK(dalloc(u.w1t, w1t.size())); CK(dalloc(u.w2, w2.size())); CK(dalloc(u.w2t, w2t.size()));
     CK(dalloc(u.b1, H)); CK(dalloc(u.b2, H)); CK(dalloc(u.w3, H)); CK(dalloc(u.fmean, F)); CK(dalloc(u.fstd, F));
     CK(cudaMemcpy(u.w1, w1.data(), sizeof(__nv_bfloat16) * w1.size(), cudaMemcpyHostToDevice));
@@ -1449,7 +1501,6 @@ int komd_gpu_surrogate_load(komd_gpu *h, const float *params, const float *fmean
     u.last_rmse = -1.0;
     u.max_rmse = 0.0;
     u.fallback_step = -1;
-    drop_graphs(e);
     return KOMD_OK;
 }
 

@@ -32,6 +32,7 @@ def host(host_library, monkeypatch):
     lib = gpu.load()
     lib.fake_size.restype = ctypes.c_size_t
     lib.fake_size.argtypes = [ctypes.c_void_p]
+    lib.fake_count.argtypes = [ctypes.c_char_p]
     lib.fake_fail_malloc.argtypes = [ctypes.c_long]
     lib.fake_fail_malloc(-1)
     lib.fake_reset()
