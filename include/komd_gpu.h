@@ -163,7 +163,9 @@ int  komd_gpu_grid_dims(komd_gpu *h, int64_t nd[3]);
  * (container/MoleculeContainer.cpp:13-53) and CheckpointIO::loadCheckpoint.
  * Sites in molecule order; consecutive sites with equal mol_id form one
  * molecule.  r, v: n*3 doubles (x y z per site); m, eps (internal units),
- * sig: n doubles; mol_id: n uint64. */
+ * sig: n doubles; mol_id: n uint64.  A second upload replaces the sites (their
+ * number may change); a loaded learned term stays, and so does a topology
+ * unless it names sites that are gone, in which case it is dropped. */
 int  komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double *v, const double *m,
                            const double *eps, const double *sig, const uint64_t *mol_id);
 /* Overwrites positions and/or velocities only (NULL keeps a field). */

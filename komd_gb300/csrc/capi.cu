@@ -439,6 +439,18 @@ int alloc_verlet(komd_gpu *h, int cap) {
     return KOMD_OK;
 }
 
+// the learned term's arrays over the sites
+int alloc_learned_sites(komd_gpu *h) {
+    Surrogate &u = h->sur;
+    const size_t n = (size_t)h->e.n;
+    dfree(u.x);   // allocated last: its presence says that the others are there
+    CK(dalloc(u.mom, n * kSurNC * 9)); CK(dalloc(u.dedx, n * kSurNF)); CK(dalloc(u.esite, n)); CK(dalloc(u.fsur, 4 * n));
+    CK(dalloc(u.fprobe, 3 * n)); CK(dalloc(u.fsur_d, 3 * n)); CK(dalloc(u.probe_acc, 2));
+    CK(cudaMemset(u.fsur, 0, sizeof(float) * 4 * n));
+    CK(dalloc(u.x, n * kSurNF));
+    return KOMD_OK;
+}
+
 // forces a rebuild of cells (and, on the Verlet path, of the list) now
 void launch_rebuild(komd_gpu *h) {
     Engine &e = h->e;
@@ -761,6 +773,11 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
     }
     off.push_back((int)n);
     Replacing replacing(e);   // have_sites returns at the end
+    if (n != e.n) dfree(h->sur.x);   // the learned term's arrays follow the site count
+    if (e.topology_end > n) {        // a topology of sites that are gone
+        e.n_bonds = e.n_angles = e.topology_end = 0;
+        e.bond_blocks = 0;
+    }
     e.n = n;
     e.n_mol = (int64_t)off.size() - 1;
     CK(dalloc(e.r, 3 * n)); CK(dalloc(e.v, 3 * n)); CK(dalloc(e.f, 3 * n)); CK(dalloc(h->f_scratch, 3 * n));
@@ -848,6 +865,10 @@ int komd_gpu_upload_sites(komd_gpu *h, int64_t n, const double *r, const double 
     }
     rc = ensure_partials(h);
     if (rc) return rc;
+    if (h->sur.loaded && !h->sur.x) {
+        rc = alloc_learned_sites(h);
+        if (rc) return rc;
+    }
     e.have_sites = true;
     return KOMD_OK;
 }
@@ -946,6 +967,9 @@ int komd_gpu_set_topology(komd_gpu *h, int64_t n_bonds, const int64_t *bonds, in
     e.bond_sites = e.n;
     e.n_bonds = std::max<int64_t>(n_bonds, 0);
     e.n_angles = std::max<int64_t>(n_angles, 0);
+    e.topology_end = 0;
+    for (int s : b) e.topology_end = std::max<int64_t>(e.topology_end, s + 1);
+    for (int s : a) e.topology_end = std::max<int64_t>(e.topology_end, s + 1);
     return KOMD_OK;
 }
 
@@ -1489,10 +1513,7 @@ int komd_gpu_surrogate_load(komd_gpu *h, const float *params, const float *fmean
     u.b3 = b3[0];
     u.e_scale = (float)e_scale;
     u.e_shift = (float)e_shift;
-    CK(dalloc(u.x, (size_t)e.n * kSurNF)); CK(dalloc(u.mom, (size_t)e.n * kSurNC * 9));
-    CK(dalloc(u.dedx, (size_t)e.n * kSurNF)); CK(dalloc(u.esite, e.n)); CK(dalloc(u.fsur, 4 * (size_t)e.n));
-    CK(dalloc(u.fprobe, 3 * (size_t)e.n)); CK(dalloc(u.fsur_d, 3 * (size_t)e.n)); CK(dalloc(u.probe_acc, 2));
-    CK(cudaMemset(u.fsur, 0, sizeof(float) * 4 * e.n));
+    if (int rc = alloc_learned_sites(h)) return rc;
     u.probe_every = probe_every;
     u.probe_threshold = probe_threshold;
     u.loaded = true;
@@ -1511,10 +1532,8 @@ int komd_gpu_surrogate_sample(komd_gpu *h, float *features, double *e3, double *
     if (!(e.cfg.terms & KOMD_TERM_ATM) || e.cfg.precision != KOMD_FP32)
         return fail(KOMD_ERR_ARG, "samples need KOMD_TERM_ATM in FP32 mode");
     Surrogate &u = h->sur;
-    if (!u.x) {
-        CK(dalloc(u.x, (size_t)e.n * kSurNF)); CK(dalloc(u.mom, (size_t)e.n * kSurNC * 9));
-        CK(dalloc(u.fprobe, 3 * (size_t)e.n));
-    }
+    if (!u.x)
+        if (int rc = alloc_learned_sites(h)) return rc;
     double *e3d = nullptr;
     CK(dalloc(e3d, e.n));
     CK(cudaMemsetAsync(e3d, 0, sizeof(double) * e.n, e.stream));
@@ -1792,10 +1811,8 @@ int komd_gpu_surrogate_capture(komd_gpu *h, komd_sur_data *d) {
     int rc = data_reserve(d, d->n_snap + 1);
     if (rc) return rc;
     Surrogate &u = h->sur;
-    if (!u.x) {
-        CK(dalloc(u.x, (size_t)e.n * kSurNF)); CK(dalloc(u.mom, (size_t)e.n * kSurNC * 9));
-        CK(dalloc(u.fprobe, 3 * (size_t)e.n));
-    }
+    if (!u.x)
+        if (int rc = alloc_learned_sites(h)) return rc;
     double *e3d = nullptr;
     CK(dalloc(e3d, e.n));
     CK(cudaMemsetAsync(e3d, 0, sizeof(double) * e.n, e.stream));

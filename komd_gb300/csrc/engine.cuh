@@ -482,6 +482,7 @@ struct Engine {
     int bond_blocks = 0;       // 0: not laid out
     int64_t bond_sites = -1;   // the site count they were laid out for
     int64_t n_bonds = 0, n_angles = 0;
+    int64_t topology_end = 0;  // past the highest site they name
     // reductions / flags
     double *partials = nullptr;
     int partial_blocks = 0;

@@ -30,8 +30,7 @@ def host(host_library, monkeypatch):
     monkeypatch.setattr(gpu, "LIB_GPU", host_library)
     monkeypatch.setattr(gpu, "_lib", None)
     lib = gpu.load()
-    lib.fake_size.restype = ctypes.c_size_t
-    lib.fake_size.argtypes = [ctypes.c_void_p]
+    lib.fake_live.argtypes = [ctypes.c_size_t]
     lib.fake_count.argtypes = [ctypes.c_char_p]
     lib.fake_fail_malloc.argtypes = [ctypes.c_long]
     lib.fake_fail_malloc(-1)
