@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -50,6 +51,11 @@ cudaError_t dalloc(T *&p, size_t count) {
 void drop_graphs(Engine &e) {
     if (e.graph) cudaGraphExecDestroy(e.graph);
     if (e.several) cudaGraphExecDestroy(e.several);
+    for (cudaGraphExec_t &g : e.call) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    for (bool &seen : e.call_seen) seen = false;
     e.graph = e.several = nullptr;
     e.graph_valid = false;
 }
@@ -1101,16 +1107,12 @@ static int run_probe(komd_gpu *h) {
     return KOMD_OK;
 }
 
-// `steps` steps captured into *out (replacing it): whole ones, or (chained) each
-// from its container to the next one's drift
-static int capture_steps(komd_gpu *h, cudaGraphExec_t *out, int steps = 1, bool chained = false) {
+// what `enqueue` launches captured into *out (replacing it)
+static int capture(komd_gpu *h, cudaGraphExec_t *out, const std::function<void()> &enqueue) {
     Engine &e = h->e;
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < steps; k++) {
-        if (chained) enqueue_chained(h, END_KICK_DRIFT);
-        else enqueue_step(h);
-    }
+    enqueue();
     CK(cudaStreamEndCapture(e.stream, &graph));
     if (*out) cudaGraphExecDestroy(*out);
     *out = nullptr;
@@ -1128,30 +1130,53 @@ static int capture_steps(komd_gpu *h, cudaGraphExec_t *out, int steps = 1, bool 
 static int ensure_graph(komd_gpu *h) {
     Engine &e = h->e;
     if (e.graph_valid && e.graph) return KOMD_OK;
-    const int rc = capture_steps(h, &e.graph);
+    const int rc = capture(h, &e.graph, [h] { enqueue_step(h); });
     if (rc) return rc;
     e.graph_valid = true;
     h->graph_epoch++;
     return KOMD_OK;
 }
 
-// steps of one graph where a call has that many: the gap between two graphs is
-// paid once for them (100 LJ steps of 4,000 sites 1.675, 1.494 and 1.461 ms at 1,
-// 4 and 8; the first call captures that much more, 27 us at 4)
-constexpr int kGraphSteps = 4;
-
+// A call of up to kGraphSteps steps is one graph from its second time on (a small
+// system's step takes less than seven direct launches: 4,000 LJ sites, calls of 2, 3
+// and 4 steps 47, 58 and 70 us launched directly, 36, 48 and 53 as a graph, whose
+// capture takes some 80 us; one step 24).  A longer call replays a graph of that many
+// steps, and what is left over is launched directly, behind graphs that keep the device
+// busy meanwhile.  Graphs of 4 and 8 steps for 100 LJ steps of 4,000 sites: 1.494 and
+// 1.461 ms (1.675 with one step a graph); the first call captures that much more, 27 us at 4.
 static int run_steps(komd_gpu *h, int64_t n_steps) {
     Engine &e = h->e;
     if (e.profiling) {
         for (int64_t k = 0; k < n_steps; k++) enqueue_step(h);
         return check_launch("step");
     }
-    // chained: the first drift and the last end are launched by themselves
+    // chained: the first step's drift and the last one's end are passes of their own
     const bool chained = n_steps > 1 && steps_chain(h);
+    const bool again = chained && n_steps <= kGraphSteps && e.call_seen[n_steps - 2];
+    if (chained && n_steps <= kGraphSteps) e.call_seen[n_steps - 2] = true;
+    if (again) {
+        cudaGraphExec_t &g = e.call[n_steps - 2];
+        if (!g) {
+            const int rc = capture(h, &g, [&] {
+                launch_step0(e, e.stream, true);
+                for (int64_t k = 1; k < n_steps; k++) enqueue_chained(h, END_KICK_DRIFT);
+                enqueue_chained(h, END_STEP1);
+            });
+            if (rc) return rc;
+        }
+        CK(cudaGraphLaunch(g, e.stream));
+        h->graph_steps += n_steps;
+        return check_launch("step");
+    }
     const int64_t inner = chained ? n_steps - 1 : n_steps, many = inner / kGraphSteps;
     int64_t left = inner - many * kGraphSteps;
     if (many > 0 && !e.several) {
-        const int rc = capture_steps(h, &e.several, kGraphSteps, chained);
+        const int rc = capture(h, &e.several, [&] {
+            for (int k = 0; k < kGraphSteps; k++) {
+                if (chained) enqueue_chained(h, END_KICK_DRIFT);
+                else enqueue_step(h);
+            }
+        });
         if (rc) return rc;
     }
     if (chained) launch_step0(e, e.stream, true);
@@ -1239,7 +1264,7 @@ int step_host_direct(komd_gpu *h, int64_t n_steps, double *r, double *v, double 
             e.hin_r = rin;
             e.hin_v = vin;
             e.hout_r = rout; e.hout_v = vout; e.hout_f = fout;
-            rc = capture_steps(h, &h->hgraph);
+            rc = capture(h, &h->hgraph, [h] { enqueue_step(h); });
             e.hin_r = e.hin_v = nullptr;
             e.hout_r = e.hout_v = e.hout_f = nullptr;
             if (rc) return rc;

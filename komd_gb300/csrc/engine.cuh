@@ -446,6 +446,9 @@ __host__ __device__ inline double sci_temperature(SciNum f, double mv2, double n
     return t.m * sci_pow10(t.e);
 }
 
+// the steps of one graph (komd_gpu_step)
+constexpr int kGraphSteps = 4;
+
 struct Engine {
     komd_config cfg;
     Grid g;
@@ -496,7 +499,9 @@ struct Engine {
     bool have_sites = false, have_cells = false, have_forces = false;
     // graph
     cudaGraphExec_t graph = nullptr;   // one whole step
-    cudaGraphExec_t several = nullptr; // several steps of one call
+    cudaGraphExec_t several = nullptr; // kGraphSteps steps of a longer call
+    cudaGraphExec_t call[kGraphSteps - 1] = {};   // whole calls of 2 .. kGraphSteps chained steps
+    bool call_seen[kGraphSteps - 1] = {};
     bool graph_valid = false;
     // profiling
     bool profiling = false;
