@@ -805,7 +805,7 @@ def run_ours(args, w, name):
     value = world * s.n * args.steps / (ms / 1e3)
     rebuilds_timed = g.profile().get("list_rebuilds", (0, 0.0))[0]
     # engine launches in the timed region (counted before the other legs change the engine's terms)
-    kernels = g.kernels_per_step() * args.steps
+    kernels = g.step_kernels(args.steps)
 
     # per-kernel breakdown: K more steps launched kernel by kernel with CUDA
     # events around each kernel family (slower than the graph by the events)

@@ -362,8 +362,12 @@ int  komd_batch_form(komd_batch *b);
  * reset.  names is a '\n'-separated list of families (<= cap bytes). */
 int  komd_gpu_set_profiling(komd_gpu *h, int on);
 int  komd_gpu_profile(komd_gpu *h, int max_families, int64_t *launches, double *ms, char *names, int cap);
-/* Number of kernels one komd_gpu_step launches per step (for accounting). */
+/* Number of kernels that a komd_gpu_step call of one step launches (for accounting). */
 int  komd_gpu_kernels_per_step(komd_gpu *h);
+/* The same for the next call of n_steps steps, which share a pass at each step
+ * boundary where the configuration allows it (the kernels of the learned term's
+ * probes not included). */
+int64_t komd_gpu_step_kernels(komd_gpu *h, int64_t n_steps);
 
 /* ---- allocation-free variant ------------------------------------------- */
 /* No counterpart in the reference.  ATM forces (FULL triplet set) of one

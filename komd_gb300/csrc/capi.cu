@@ -2375,24 +2375,44 @@ int komd_batch_check(komd_batch *b) {
     return batch_finish(b);
 }
 
-int komd_gpu_kernels_per_step(komd_gpu *h) {
+// kernels of one step from its container on, with the pass that ends it (enqueue_step,
+// enqueue_chained)
+static int64_t pass_kernels(komd_gpu *h, StepEnd end) {
+    const Engine &e = h->e;
+    const uint32_t t = e.cfg.terms;
+    const bool learned = surrogate_on(h), atm = !learned && (t & KOMD_TERM_ATM);
+    // com/wrap/bin, scan, scatter, cell sort and, on the Verlet path, the list build
+    int64_t k = 4 + (e.verlet ? 1 : 0);
+    if (t & (KOMD_TERM_LJ | KOMD_TERM_FENE | KOMD_TERM_ATM)) k++;   // pair pass (else a memset)
+    if ((t & KOMD_TERM_TABULATED) && e.tab_x) k++;
+    if (t & KOMD_TERM_BONDED)   // one pass over small molecules, or one by bond and one by angle
+        k += e.bond_blocks > 0 && e.bond_sites == e.n ? 1 : (e.n_bonds > 0) + (e.n_angles > 0);
+    if (t & KOMD_TERM_LIMIT) k++;
+    if (learned) k += 4;   // descriptors, network, forces, apply
+    // the once-per-triplet kernel (inside the LJ pass on the Verlet path) and its flush, or one kernel
+    if (atm) k += !e.atm_acc ? 1 : (fused_lj_atm(h, false) ? 1 : 2);
+    const bool fused = (learned || (atm && e.atm_acc)) && (end == END_STEP1 || e.fused_drift);
+    return k + (fused ? 0 : 1);
+}
+
+int64_t komd_gpu_step_kernels(komd_gpu *h, int64_t n_steps) {
     if (!h) return -1;
     const Engine &e = h->e;
-    // integrate0/1; the container pass (com/wrap/bin, scan, scatter, cell sort, and
-    // on the Verlet path the list build)
-    int k = 2 + 4 + (e.verlet ? 1 : 0);
-    if (e.cfg.terms & (KOMD_TERM_LJ | KOMD_TERM_FENE | KOMD_TERM_ATM)) k++;   /* pair pass (else a memset) */
-    if (e.cfg.terms & KOMD_TERM_TABULATED) k++;
-    if (!surrogate_on(h) && (e.cfg.terms & KOMD_TERM_ATM) && e.atm_acc) k--;   /* integrate1 fused into the ATM flush */
-    if (e.cfg.terms & KOMD_TERM_BONDED)   // one pass over small molecules, or one by bond and one by angle
-        k += e.bond_blocks > 0 && e.bond_sites == e.n ? 1 : (e.n_bonds > 0) + (e.n_angles > 0);
-    if (e.cfg.terms & KOMD_TERM_LIMIT) k++;
-    if (e.cfg.thermostat)   // velocity scaling and the kinetic sums, with integrate1 where the flush has it not
-        k += !surrogate_on(h) && (e.cfg.terms & KOMD_TERM_ATM) && e.atm_acc ? 2 : 1;
-    if (surrogate_on(h)) k += 4;   /* descriptors, MLP, forces, apply */
-    else if (e.cfg.terms & KOMD_TERM_ATM)   /* once-per-triplet kernel (inside the LJ pass on the Verlet path) + flush */
-        k += (e.atm_acc != nullptr) ? (fused_lj_atm(h, false) ? 1 : 2) : 1;
+    const int64_t last = pass_kernels(h, END_STEP1);
+    // the thermostat's kinetic sums take integrate1 along where no force pass did
+    const bool ended = surrogate_on(h) || ((e.cfg.terms & KOMD_TERM_ATM) && e.atm_acc);
+    const int64_t single = 1 + last + (e.cfg.thermostat ? (ended ? 2 : 1) : 0);
+    const bool probing = surrogate_on(h) && h->sur.probe_every > 0;
+    int64_t k = 0, at = h->sur.steps;
+    while (n_steps > 0) {   // komd_gpu_step's pieces
+        const int64_t n = probing ? std::min<int64_t>(n_steps, h->sur.probe_every - at % h->sur.probe_every) : n_steps;
+        k += n > 1 && steps_chain(h) ? 1 + (n - 1) * pass_kernels(h, END_KICK_DRIFT) + last : n * single;
+        n_steps -= n;
+        at += n;
+    }
     return k;
 }
+
+int komd_gpu_kernels_per_step(komd_gpu *h) { return (int)komd_gpu_step_kernels(h, 1); }
 
 }  // extern "C"

@@ -64,6 +64,34 @@ def test_short_calls_are_graphs(host, form):  # noqa: F811
     g.close()
 
 
+@pytest.mark.parametrize("form", FORMS + ["bonds_by_atomics", "learned_probed", "no_table"])
+def test_reported_kernels_are_those_launched(host, form):  # noqa: F811
+    from komd_gb300 import gpu
+    g = engine({"bonds_by_atomics": "verlet_molecules", "learned_probed": "verlet_learned",
+                "no_table": "cells_lj"}.get(form, form))
+    if form == "bonds_by_atomics":   # one chain of all sites
+        b = np.array([[k, k + 1] for k in range(g.n - 1)], np.int64)
+        g._check(g.L.komd_gpu_set_topology(g.h, len(b), b.ctypes.data, 0, None))
+    if form == "learned_probed":
+        g.surrogate_load(dict(params=np.zeros(6337, np.float32), fmean=np.zeros(32, np.float32),
+                              fstd=np.ones(32, np.float32), e_scale=1.0, e_shift=0.0), probe_every=3,
+                         probe_threshold=1e9)
+        g.step(4)
+    if form == "no_table":
+        g.set_terms(gpu.TERM_LJ | gpu.TERM_TABULATED)
+    probes = lambda: g.surrogate_status()["probes"] if form == "learned_probed" else 0  # noqa: E731
+    for profiling in (False, True):
+        g.set_profiling(profiling)
+        for n in (1, 2, 3, 4, 5, 9, 22):
+            host.fake_reset()
+            before, said = probes(), g.step_kernels(n)
+            assert n != 1 or said == g.kernels_per_step()
+            g.step(n)
+            # a probe: the exact triplets and their flush, the learned term's four, the comparison
+            assert host.fake_direct() + host.fake_replayed() == said + 7 * (probes() - before)
+    g.close()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", [f for f in FORMS if not f.endswith("learned")])
 def test_calls_equal_single_steps(form):
