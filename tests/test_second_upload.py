@@ -89,3 +89,59 @@ def test_learned_forces_after_a_second_upload():
     a.step(9)
     a.close()
     b.close()
+
+
+def _verlet(s):
+    from komd_gb300 import gpu
+    g = gpu.GpuSystem(s, gpu.make_config(s.low, s.high, float(s.high[0]) / 3.0, cutoff=2.5, cutoff_3b=2.0, nu=0.073,
+                                         dt=0.005, terms=gpu.TERM_LJ | gpu.TERM_ATM, skin=0.3,
+                                         atm_sign=gpu.ATM_SIGN_PHYSICAL, atm_enum=gpu.ATM_ENUM_FULL,
+                                         virial_mode=gpu.VIRIAL_CORRECT))
+    g.update_container()
+    g.forces()
+    return g
+
+
+def _calls(g):
+    for n in (9, 9, 3, 3, 3, 1, 1):   # graphs of four steps, of three and of one
+        g.step(n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["same", "fewer"])
+def test_step_graphs_after_a_second_upload(form):
+    from komd_gb300 import lattice
+    s = lattice.argon_fcc(6, rho=0.8442, t_star=1.4, seed=9, jitter=0.05)
+    a = _verlet(s)
+    _calls(a)
+    keep = np.arange(0, s.n, 1 if form == "same" else 2)
+    t = lattice.System(r=s.r[keep], v=-s.v[keep], m=s.m[keep], eps=s.eps[keep], sig=s.sig[keep],
+                       mol_id=s.mol_id[keep], low=s.low, high=s.high)
+    _upload(a, t)
+    a.update_container()
+    a.forces()
+    b = _verlet(t)
+    for g in (a, b):
+        _calls(g)
+    assert all(np.isfinite(x).all() and np.array_equal(x, y) for x, y in zip(a.download(), b.download()))
+    a.close()
+    b.close()
+
+
+@pytest.mark.gpu
+def test_step_graphs_after_a_change_of_terms():
+    from komd_gb300 import gpu, lattice
+    s = lattice.argon_fcc(6, rho=0.8442, t_star=1.4, seed=9, jitter=0.05)
+    a, b = _verlet(s), _verlet(s)
+    for terms in (gpu.TERM_LJ, gpu.TERM_LJ | gpu.TERM_ATM):
+        _calls(a)
+        for _ in range(29):
+            b.step(1)
+        for g in (a, b):
+            g.set_terms(terms)
+    _calls(a)
+    for _ in range(29):
+        b.step(1)
+    assert all(np.isfinite(x).all() and np.array_equal(x, y) for x, y in zip(a.download(), b.download()))
+    a.close()
+    b.close()
