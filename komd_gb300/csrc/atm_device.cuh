@@ -23,8 +23,8 @@ namespace komd {
 // k_atm_flush adds them to f.
 constexpr double kAtmFix = 4294967296.0;   // 2^32 fixed-point units
 
-// 1/sqrt of a squared distance: rsqrtf's instruction without the scaling (three
-// more) that it wraps around it for subnormal arguments
+// 1/sqrt of a squared distance by PTX rsqrt.approx.ftz.f32, which takes a subnormal
+// argument for zero; squared distances are of order one
 __device__ __forceinline__ float rsqrt_ftz(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -154,8 +154,8 @@ __device__ __forceinline__ void atm_sweep(const float4 *se, const float4 *sq, in
     int t_act = own ? d_last - d_first + 1 : 0;
     if (own && (m & 1) == 0 && d_last == (m >> 1) && li >= (m >> 1)) t_act--;
     // partner b = li + d and share source li - d (mod m), stepped per round;
-    // d <= m/2 keeps both within one wrap (lanes without a neighbour read entries
-    // from 0 on, 16 at most: nl_cap is 32 or more)
+    // d <= m/2 keeps both within one wrap, and lanes without a neighbour start at
+    // entry 0: b stays below m, so every lane reads staged entries, whatever nl_cap is
     int b = own ? li + d_first : 0, src = li - d_first;
     if (b >= m) b -= m;
     if (src < 0) src += m;

@@ -31,13 +31,18 @@ namespace komd {
 // access) holds it until the predecessor has completed and its writes are
 // visible, and pdl_trigger lets the successor be scheduled once every block
 // of this grid has started.  Both are no-ops without a programmatic launch.
-// Every kernel of a single system's step waits at its entry and is launched so: its
-// launch overlaps the end of its predecessor.  The passes of a few microseconds (the
-// container stages, the integrator) trigger as well; the force passes do not: their
-// successor's blocks, resident early, take their shared memory and slots.  Steps of 4096
-// sites 14.8 us with plain launches of the force and integrator passes, 15.3 with a
-// trigger in each, 14.3 with none there, 14.1 with the integrator's; without any, the container's
-// included, 15.6.  32,000 sites with the learned term 81.1, 86.7, 79.3, 78.6 (none: 80.0).
+// The kernels of a single system's FP32 step are launched so and wait at their entry:
+// their launch overlaps the end of their predecessor.  Plain launches, without a wait
+// in the kernel -- a kernel has to get one before it may be launched so -- are
+// k_pair_cell and k_atm_d (launched beside their predecessor, ten FP64 LJ steps of 4,000
+// sites went from 565 to 607 us), k_bonds, k_angles, k_sur_apply, the kernels of samples,
+// probes, RDF and training, and the packed replicas' stages.  The passes of a few
+// microseconds (the container stages, the integrator) trigger as well.  Of the force passes only
+// k_lj_atm_half does; of the others the successor's blocks, resident early, take shared
+// memory and slots.  Steps of 4096 sites 14.8 us with plain launches of the force and
+// integrator passes, 15.3 with a trigger in each, 14.3 with none there, 14.1 with the
+// integrator's; without any, the container's included, 15.6.  32,000 sites with the
+// learned term 81.1, 86.7, 79.3, 78.6 (none: 80.0).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -326,12 +331,13 @@ inline void sw_params(double rc, double width, int &on, float &rc2, float &iw) {
     iw = on ? (float)(1.0 / (rc * rc - rs * rs)) : 0.f;
 }
 
-// Arguments of the step kernels of the Verlet path, one struct per kernel, so
-// that one launch can serve one system (the struct by value) or all replicas
-// of a batch (an array of them, a block range per replica).
 // k_bonded_mol: components (and threads) and sites of a block, terms of a component.
 // Longer components would be a serial chain on one thread: they keep the atomics.
 constexpr int kBondComps = 64, kBondSites = 256, kBondTerms = 16;
+
+// Arguments of the step kernels of the Verlet path, one struct per kernel, so
+// that one launch can serve one system (the struct by value) or all replicas
+// of a batch (an array of them, a block range per replica).
 struct BinArgs {              // k_com_wrap_bin: COM, periodic wrap, binning
     Grid g;
     int n_mol;

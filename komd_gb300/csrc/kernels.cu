@@ -55,8 +55,8 @@ __device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x)
 // ===========================================================================
 // (int64)(x / cs) clamped to [0, nd - 1] (writeIndices).  The truncated quotient
 // is read off x * (1 / cs) where that is not within 1e-9 of an integer (its
-// error is below 4e-10 for quotients up to 1e6); the IEEE division, a dozen
-// instructions on the narrow FP64 pipe, runs for the rest.
+// error is below 4e-10 for quotients up to 1e6); the IEEE division, which costs the
+// narrow FP64 pipe several times as much, runs for the rest.
 __device__ __forceinline__ int cell_index(double x, double cs, double ics, int nd) {
     const double t = dmul(x, ics);
     const int q0 = __double2int_rz(t);

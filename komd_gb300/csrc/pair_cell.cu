@@ -22,11 +22,10 @@
 // their components over the lanes (6 additions instead of 15).
 // Real = float: the staged coordinates are the operands; issue-bound.
 //
-// Against one warp per home cell with every candidate in the result type (10
-// steps with the sensors and the state read back): FP64 LJ on 4,000 sites
-// 11.1 -> 0.65 ms (944 -> 30 us a launch), FP64 LJ + ATM on 32,000 35.4 -> 22.4 ms, LJ + FENE on 1,536
-// sites of molecules 2.19 -> 1.64 ms (a call per hook), the tabulated force on
-// 32,000 sites (a warp per cell staged for itself before) 4.30 -> 2.88 ms.
+// Against one warp per home cell with every candidate in the result type, a launch:
+// FP64 LJ on 4,000 sites 944 -> 30 us (with the sensors 1326 -> 50), on 32,000 with the
+// ATM list 1344 -> 149, FP32 LJ + FENE on 1,536 sites of molecules 68 -> 11, and the
+// tabulated force on 32,000 sites (a warp per cell that staged for itself) 347 -> 145.
 #include <climits>
 #include <cstdint>
 

@@ -746,9 +746,9 @@ __global__ void __launch_bounds__(256, 4) k_lj_atm(PairParams p, AtmParams a, in
 // pair once instead of twice, and converts one FP32 partial per partner.
 // Bound by instruction issue (81 % of the slots, 740 a site, 44 % of them the
 // sweep): 256,000 sites of liquid argon at skin 0.6, 221 -> 195 us, from branches
-// around a dozen instructions replaced by selects, square roots without rsqrtf's
-// scaling, a shorter fixed-point conversion and the cutoffs' FP32 values in the
-// parameters (812 a site, 78 % before).  Five blocks an SM were slower (39 against
+// around a dozen instructions replaced by selects, reciprocal roots by PTX
+// rsqrt.approx.ftz, a shorter fixed-point conversion and the cutoffs' FP32 values in
+// the parameters (812 a site, 78 % before).  Five blocks an SM were slower (39 against
 // 35 us at 31,000 sites), two sites a warp gained nothing.
 // ---------------------------------------------------------------------------
 // what the half-list pass reads of a site before its arithmetic: the count
