@@ -99,6 +99,14 @@ __device__ __forceinline__ bool dabove(double a, double b) {
     return ka > __double_as_longlong(b) && ka <= 0x7ff0000000000000LL;
 }
 
+// integer key with key(x) < key(y) exactly when x < y for non-NaN doubles
+// (-0.0 and +0.0 share the key 0)
+__device__ __forceinline__ long long dkey(double x) {
+    const long long b = __double_as_longlong(x);
+    const long long m = b & 0x7fffffffffffffffLL;
+    return b < 0 ? -m : m;
+}
+
 // Reciprocal square root and square root in FP64 for kernels that GB300's FP64
 // pipe bounds: an FP32 seed y0 (24 bits, from the hardware's approximation; both
 // conversions are integer shifts of the bits) and one Householder step of third
@@ -391,7 +399,6 @@ struct Step0Args {            // k_step0_fused: half-kick, drift, wrap, skin tes
     const float4 *ref4;
     float half_skin2;
     int *rebuild;
-    double *com;
     const int *site_slot;
     float4 *pos4;
     const double *r_in, *v_in;

@@ -903,7 +903,7 @@ __device__ __forceinline__ void local_position(int s, const double (&x)[3], cons
     if (dx * dx + dy * dy + dz * dz > half_skin2) *rebuild = 1;
 }
 __global__ void k_step0(int n, double *__restrict__ r, double *__restrict__ v, const double *__restrict__ f,
-                        const double *__restrict__ hdtm, double dt, Grid g,
+                        const double *__restrict__ hdtm, double dt,
                         const double *__restrict__ bias, const float4 *__restrict__ ref4,
                         const int *__restrict__ site_slot, float4 *__restrict__ pos4, float half_skin2,
                         int *__restrict__ rebuild) {
@@ -924,16 +924,9 @@ __global__ void k_step0(int n, double *__restrict__ r, double *__restrict__ v, c
 
 // Verlet path with single-site molecules whose COM is exactly the position
 // (power-of-two masses): integrate0, the skin test, the periodic wrap with
-// its bias update and COM (k_com_wrap_bin's operations) and the FP32
-// cell-local position in one pass over the sites.  The results are those of
-// the separate kernels; on a rebuild step the cell sort rewrites pos4 afterwards.
-// integer key with key(x) < key(y) exactly when x < y for non-NaN doubles
-// (-0.0 and +0.0 share the key 0)
-__device__ __forceinline__ long long dkey(double x) {
-    const long long b = __double_as_longlong(x);
-    const long long m = b & 0x7fffffffffffffffLL;
-    return b < 0 ? -m : m;
-}
+// its bias update (k_com_wrap_bin's operations) and the FP32 cell-local
+// position in one pass over the sites.  The results are those of the separate
+// kernels; on a rebuild step the cell sort rewrites pos4 afterwards.
 __device__ __forceinline__ bool dkey_nan(double x) {
     return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
 }
@@ -1445,7 +1438,7 @@ SortArgs sort_args(const Engine &e) {
 }
 Step0Args step0_args(const Engine &e) {
     const float hs = (float)(0.5 * e.cfg.skin);
-    return Step0Args{(int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g, e.bias, e.ref4, hs * hs, e.rebuild, e.com,
+    return Step0Args{(int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g, e.bias, e.ref4, hs * hs, e.rebuild,
                      e.site_slot, e.pos4, e.hin_r ? e.hin_r : e.r, e.hin_v ? e.hin_v : e.v, e.hout_r};
 }
 FlushArgs flush_args(const Engine &e, double scale_fix, const float4 *own) {
@@ -1888,7 +1881,7 @@ void launch_step0(Engine &e, cudaStream_t st, bool in_step) {
         return;
     }
     const int b = site_block(e, e.n);
-    launch_pdl(k_step0, nblk(e.n, b), b, 0, st, (int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t, e.g,
+    launch_pdl(k_step0, nblk(e.n, b), b, 0, st, (int)e.n, e.r, e.v, e.f, e.hdtm, e.cfg.delta_t,
                e.verlet ? e.bias : nullptr, e.verlet ? e.ref4 : nullptr, e.site_slot, e.pos4, hs * hs, e.rebuild);
 }
 

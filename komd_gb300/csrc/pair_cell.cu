@@ -42,26 +42,19 @@ enum PairKind { PC_LJ = 0, PC_TABLE = 1, PC_COUNT = 2 };
 __device__ __forceinline__ bool above(double a, double b) { return dabove(a, b); }
 __device__ __forceinline__ bool above(float a, float b) { return a > b; }
 
-// integer key with key(x) < key(y) exactly when x < y for non-NaN doubles
-__device__ __forceinline__ long long order_key(double x) {
-    const long long b = __double_as_longlong(x);
-    const long long m = b & 0x7fffffffffffffffLL;
-    return b < 0 ? -m : m;
-}
-
 // FunctionPL::evaluateAt (plugins/IBI/IBI_Math.h:30-44): the upper node is the
 // first node >= r (by binary search on integer keys, the node the reference's
 // linear scan finds), slope[k] = (y[k+1] - y[k]) / (x[k+1] - x[k]) is the
 // reference's quotient, computed once with the same IEEE operations.  At
 // r == x[0] the reference reads x[-1]; here the first segment is used.
 __device__ __forceinline__ double table_eval(double r, const PairTable &t) {
-    const long long kr = order_key(r);
-    if (kr > order_key(t.xs[t.n - 1])) return t.hi;
-    if (kr < order_key(t.xs[0])) return t.lo;
+    const long long kr = dkey(r);
+    if (kr > dkey(t.xs[t.n - 1])) return t.hi;
+    if (kr < dkey(t.xs[0])) return t.lo;
     int a = 0, b = t.n - 1;           // lower_bound: first index with xs[i] >= r
     while (a < b) {
         const int m = (a + b) >> 1;
-        if (kr > order_key(t.xs[m])) a = m + 1;
+        if (kr > dkey(t.xs[m])) a = m + 1;
         else b = m;
     }
     const int lb = (a < 1 ? 1 : a) - 1;

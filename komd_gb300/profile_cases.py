@@ -5,6 +5,7 @@
     python -m komd_gb300.profile_cases replicas   [--count 64] [--steps 2] [--equil 0] [--groups 4]
     python -m komd_gb300.profile_cases tabulated  [--ncell 40] [--steps 3]
     python -m komd_gb300.profile_cases train      [--snaps 40] [--epochs 2] [--batch 4]
+    python -m komd_gb300.profile_cases case --name NAME
 
 `exact`: LJ + FULL ATM argon (rho* 0.8442, T* 0.722, rc 2.5 / 2.0, nu* 0.073,
 cell 2.8, skin 0.3 by default; the benchmark's timed configuration is
@@ -17,9 +18,10 @@ benchmark's uneven replicas (2000-20000 atoms) advanced by one batched graph
 tabulated pair force (FP64, per-step cells of edge >= 2.5, a 200-node table
 of the LJ force) on the jittered lattice, then one RDF_Profiler sample (100
 bins to 2.5).  `train`: force-matched training of the learned term on a small
-dataset from the exact kernel.  Each prints its mean step
-time; the launches before the measured steps are few, so that a profiler can
-skip to them.
+dataset from the exact kernel.  `case`: one pass of a listed case of
+perf/cases.py, after two passes that are not profiled (for ncu's
+--profile-from-start off).  The others print their mean step time; the
+launches before the measured steps are few, so that a profiler can skip to them.
 """
 from __future__ import annotations
 
@@ -108,9 +110,25 @@ def tabulated(ncell, steps):
     g.close()
 
 
+def case(name):
+    import torch
+    from perf import cases
+    c = next(c for c in cases.listed() if c["name"] == name)
+    state = cases.prepare(c, 3)
+    for _ in range(2):
+        cases.run(state)
+    torch.cuda.synchronize()
+    torch.cuda.cudart().cudaProfilerStart()
+    cases.run(state)
+    torch.cuda.synchronize()
+    torch.cuda.cudart().cudaProfilerStop()
+    print("one pass of", name)
+
+
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["exact", "surrogate", "replicas", "tabulated", "train"])
+    ap.add_argument("case", choices=["exact", "surrogate", "replicas", "tabulated", "train", "case"])
+    ap.add_argument("--name", default="verlet_lj_atm_256k")
     ap.add_argument("--ncell", type=int, default=40)
     ap.add_argument("--steps", type=int, default=3)
     ap.add_argument("--equil", type=int, default=0)
@@ -122,7 +140,9 @@ def main():
     ap.add_argument("--skin", type=float, default=0.3)
     ap.add_argument("--cell", type=float, default=2.8)
     a = ap.parse_args()
-    if a.case == "train":
+    if a.case == "case":
+        case(a.name)
+    elif a.case == "train":
         train(a.snaps, a.epochs, a.batch)
     elif a.case == "replicas":
         replicas(a.count, a.steps, a.equil, a.groups)
