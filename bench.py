@@ -900,7 +900,7 @@ def run_ours(args, w, name):
                        "triplets_per_step": triplets, "parallelism": f"replicas x{world}",
                        "l2": "no flush: inputs larger than L2 -- the Verlet list (about 88 MB at 256k, of which "
                              "the half-list force pass reads the 44 MB front regions) is read every step, and the "
-                             "dominant kernel moves about 77 MB of DRAM traffic per launch"},
+                             "dominant kernel moves 83-84 MB of DRAM traffic per launch"},
             "gpu_launches": kernels, "list_rebuilds_timed": rebuilds_timed,
             "events_ms_per_step": events_ms / args.steps,
             "kernel_ms": {k: {"launches": v[0], "ms": v[1]} for k, v in prof.items()},
