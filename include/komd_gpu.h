@@ -189,9 +189,10 @@ int  komd_gpu_forces(komd_gpu *h);
 int  komd_gpu_integrate0(komd_gpu *h);
 int  komd_gpu_integrate1(komd_gpu *h);
 /* n full steps of Simulation::run's loop body without thermostat or plugins
- * (integrate0, updateContainer, forces, integrate1), replayed from one CUDA
- * graph.  Requires forces of the current positions (call update_container +
- * forces once before the first step_n). */
+ * (integrate0, updateContainer, forces, integrate1), replayed from CUDA graphs
+ * (a call of two to four steps from its second time on, and the steps left
+ * over of a longer one never).  Requires forces of the current positions (call
+ * update_container + forces once before the first step_n). */
 int  komd_gpu_step(komd_gpu *h, int64_t n_steps);
 /* Same as komd_gpu_step, end to end from host buffers: takes r, v (n*3) from
  * the host, runs n_steps, returns r, v and f.  When the GPU can address the
